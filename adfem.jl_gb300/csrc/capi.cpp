@@ -140,8 +140,20 @@ int system_set_bd(adfem_system* s, const long long* bd, long long nbd, const dou
   ADFEM_TRY(to_dev(s->isbd, tag.data(), tag.size()));
   ADFEM_TRY(to_dev(s->isbd_ref, tref.data(), tref.size()));
   ADFEM_TRY(to_dev(s->bdval, val.data(), val.size()));
+  s->solver.mg_isbd = s->isbd.as<uint8_t>();
+  s->solver.mg_fixed = nbd > 0;
   s->assembled = false;
   return ADFEM_OK;
+}
+
+// Solves of resident systems use the multigrid-preconditioned CG unless ADFEM_MG=0 or one of
+// the variables that pick a variant of the Jacobi iterations is set at creation.
+bool mg_wanted() {
+  const char* e = std::getenv("ADFEM_MG");
+  if (e && e[0] == '0') return false;
+  for (const char* v : {"ADFEM_ZCG", "ADFEM_ZCG64", "ADFEM_ZCG_SMAX", "ADFEM_ZCG_RING", "ADFEM_ZCG_RING_REFILL"})
+    if (std::getenv(v)) return false;
+  return true;
 }
 
 // vectors between the reference DOF order and the solver's
@@ -167,9 +179,9 @@ size_t system_device_bytes(const adfem_system* s) {
   const Solver& v = s->solver;
   for (const DevBuf* d : {&v.s32, &v.state, &v.partials, &v.b, &v.y64, &v.r64, &v.p64, &v.q64, &v.z64, &v.r32, &v.pa32,
                           &v.pb32, &v.q32, &v.yh32, &v.yl32, &v.z1, &v.zq1, &v.dz32, &v.valz64, &v.valz32,
-                          &v.colz16, &v.zpid32, &v.zpool32, &v.bz32})
+                          &v.colz16, &v.zpid32, &v.zpool32, &v.bz32, &v.vals64})
     b += d->bytes;
-  return b;
+  return b + mg_device_bytes(v);
 }
 
 const Mesh* mesh_of(const adfem_mesh* h) { return h ? h->m : nullptr; }
@@ -1155,6 +1167,21 @@ int adfem_system_create(adfem_mesh* mesh, int kind, adfem_system** out) {
   ADFEM_TRY(s->t1.alloc(sizeof(double) * s->ndof));
   ADFEM_TRY(s->t2.alloc(sizeof(double) * s->ndof));
   ADFEM_TRY(s->solver.init(&s->A, s->ndof));
+  if (mg_wanted()) {
+    Solver& sv = s->solver;
+    sv.mg_allowed = true;
+    sv.mg_nb = kind == ADFEM_SYS_ELASTICITY ? 2 : 1;
+    sv.mg_rp = std::move(rpS);
+    sv.mg_ci = std::move(ciS);
+    if (kind == ADFEM_SYS_ELASTICITY) {
+      sv.mg_x.resize(nn);
+      sv.mg_y.resize(nn);
+      for (int64_t i = 0; i < nn; i++) {
+        sv.mg_x[pi[i]] = m.xy[2 * i];
+        sv.mg_y[pi[i]] = m.xy[2 * i + 1];
+      }
+    }
+  }
   ADFEM_TRY(system_set_bd(s.get(), nullptr, 0, nullptr));
   *out = s.release();
   return ADFEM_OK;

@@ -111,6 +111,12 @@ size_t estimate_system_bytes(const adfem::Mesh* m, int kind) {
   return (size_t)b;
 }
 
+// Multigrid hierarchy of a system, which its first solve outside a pack builds (per unknown:
+// operators, interpolation and work vectors of all levels, as mg_plan lays them out).
+size_t estimate_hierarchy_bytes(const adfem::Mesh* m, int kind) {
+  return (size_t)((kind == ADFEM_SYS_ELASTICITY ? 380.0 : 230.0) * (double)ndof_of(m, kind)) + 64 * 1024;
+}
+
 // Worker buffers a request needs (inputs at Gauss points, u, g, lambda, gradient).
 size_t estimate_worker_bytes(const adfem::Mesh* m, int kind) {
   const size_t ng = 3 * (size_t)m->ne, nd = (size_t)ndof_of(m, kind);
@@ -172,6 +178,12 @@ struct adfem_server {
     }
     job->done = true;
     cv_done.notify_all();
+  }
+  // whether a request's solves run in packed launches
+  bool goes_packed(const adfem_request& q) const {
+    const int prec = q.precision >= 0 ? q.precision : cfg.opts.precision;
+    return pack_max_dof > 0 && prec == ADFEM_PREC_MIXED &&
+           (long long)ndof_of(adfem::mesh_of(q.mesh), q.kind) <= pack_max_dof;
   }
   Resident* find_free(const adfem_mesh* mesh, int kind) {
     for (auto& r : residents)
@@ -329,7 +341,7 @@ int adfem_server::run_job(Worker& W, Resident& R, Job& job) {
     ADFEM_CUDA(cudaMemcpyAsync(W.u.p, R.uprev.p, sizeof(double) * nd, cudaMemcpyDeviceToDevice, st));
     o.warm_start = 1;
   }
-  const bool packed = pack_max_dof > 0 && o.precision == ADFEM_PREC_MIXED && (long long)nd <= pack_max_dof;
+  const bool packed = goes_packed(q);
   adfem_solver_stats fs{};
   if (packed) {
     ADFEM_CUDA(cudaStreamSynchronize(st));  // assembly and the warm-start copy are done
@@ -420,7 +432,8 @@ void adfem_server::run_worker(int wid) {
         hits++;
       } else {
         const adfem::Mesh* m = adfem::mesh_of(job->req.mesh);
-        const size_t est = estimate_system_bytes(m, job->req.kind);
+        const size_t est = estimate_system_bytes(m, job->req.kind) +
+                           (goes_packed(job->req) ? 0 : estimate_hierarchy_bytes(m, job->req.kind));
         while (used + est > budget && evict_one_idle()) {
         }
         if (used + est > budget) {
@@ -453,7 +466,9 @@ void adfem_server::run_worker(int wid) {
       status = adfem_system_create(const_cast<adfem_mesh*>(R->mesh), R->kind, &R->sys);
       std::lock_guard<std::mutex> lk(mu);
       if (status == ADFEM_OK) {
-        const size_t actual = adfem::system_device_bytes(R->sys);
+        // (the hierarchy is built by the first solve: its estimate stays booked until then)
+        const size_t actual = adfem::system_device_bytes(R->sys) +
+                              (goes_packed(job->req) ? 0 : estimate_hierarchy_bytes(adfem::mesh_of(R->mesh), R->kind));
         used = used - R->bytes + actual;
         R->bytes = actual;
       }
@@ -462,6 +477,11 @@ void adfem_server::run_worker(int wid) {
     if (status != ADFEM_OK) std::snprintf(job->resp.message, sizeof(job->resp.message), "%s", adfem_last_error());
     {
       std::lock_guard<std::mutex> lk(mu);
+      if (R->sys) {
+        const size_t actual = adfem::system_device_bytes(R->sys) + R->uprev.bytes;
+        used = used - R->bytes + actual;
+        R->bytes = actual;
+      }
       running--;
       R->busy = false;
       R->last_use = ++tick;
@@ -577,7 +597,8 @@ int adfem_server_submit(adfem_server* srv, const adfem_request* req, long long* 
     return adfem::fail(ADFEM_ERR_INVALID, "server: unknown precision");
   std::lock_guard<std::mutex> lk(srv->mu);
   if (srv->stopping) return adfem::fail(ADFEM_ERR_INVALID, "server: shutting down");
-  const size_t need = estimate_system_bytes(m, req->kind) + estimate_worker_bytes(m, req->kind);
+  const size_t need = estimate_system_bytes(m, req->kind) + estimate_worker_bytes(m, req->kind) +
+                      (srv->goes_packed(*req) ? 0 : estimate_hierarchy_bytes(m, req->kind));
   if (need > srv->budget) {
     srv->rejected++;
     return adfem::fail(ADFEM_ERR_BUSY, "server: request needs ~" + std::to_string(need >> 20) +

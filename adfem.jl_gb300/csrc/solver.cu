@@ -65,7 +65,7 @@ __global__ void k_scale_diag(int64_t n, const int32_t* __restrict__ sptr, const 
   s[r] = rsqrtf(df);
 }
 
-// val64 <- s_i K_ij s_j (FP64, in place, standard form).  The difference-form copies
+// vals <- s_i K_ij s_j (FP64, standard form).  The difference-form copies
 // (FP64 valD for residuals, FP32 val32 for the inner iteration) hold w_ij = s_i K_ij
 // in off-diagonal slots and d_i = s_i^2 sum_j K_ij (the row sum, zero for rows of a
 // pure Laplacian) in the diagonal slot, so that
@@ -75,7 +75,8 @@ __global__ void k_scale_diag(int64_t n, const int32_t* __restrict__ sptr, const 
 // their accuracy; a plain FP32 copy of K~ loses them once cond(K~) * 2^-24 ~ 1.
 template <bool D16>
 __global__ void k_scale_values(int64_t n, const int32_t* __restrict__ sptr, const void* __restrict__ col,
-                               double* __restrict__ val, double* __restrict__ valD, float* __restrict__ val32,
+                               const double* __restrict__ val, double* __restrict__ vals,
+                               double* __restrict__ valD, float* __restrict__ val32,
                                const float* __restrict__ s, const int32_t* __restrict__ diagpos) {
   const int64_t r = gtid();
   if (r >= n) return;
@@ -91,7 +92,7 @@ __global__ void k_scale_values(int64_t n, const int32_t* __restrict__ sptr, cons
     const double t = si * v;
     int j = colof<D16>(col, idx, r);
     if (!ADFEM_DCHECK(j >= 0 && j < n)) j = (int)r;
-    val[idx] = t * (double)s[j];
+    if (vals) vals[idx] = t * (double)s[j];
     valD[idx] = t;
     val32[idx] = (float)t;
   }
@@ -538,11 +539,10 @@ __global__ void k_unscale(int64_t n, const double* __restrict__ y, const float* 
   else u[i] = (double)s[i] * y[i];
 }
 
-// y = K x = S^-1 K~ S^-1 x
+// y = K x
 template <bool D16>
 __global__ void k_apply(int64_t n, const int32_t* __restrict__ sptr, const void* __restrict__ col,
-                        const double* __restrict__ val, const float* __restrict__ s, const double* __restrict__ x,
-                        double* __restrict__ y) {
+                        const double* __restrict__ val, const double* __restrict__ x, double* __restrict__ y) {
   const int64_t r = gtid();
   if (r >= n) return;
   int64_t base;
@@ -553,9 +553,9 @@ __global__ void k_apply(int64_t n, const int32_t* __restrict__ sptr, const void*
     const int64_t idx = base + 32 * (int64_t)k;
     int j = colof<D16>(col, idx, r);
     if (!ADFEM_DCHECK(j >= 0 && j < n)) j = (int)r;
-    acc = fma(val[idx], x[j] / (double)s[j], acc);
+    acc = fma(val[idx], x[j], acc);
   }
-  y[r] = acc / (double)s[r];
+  y[r] = acc;
 }
 
 // ---------------------------------------------------------------------------
@@ -644,6 +644,7 @@ int Solver::init(const Sell* A_, int64_t n_) {
   grid_spmv = std::min(g2, g3);
   ADFEM_TRY(zcg_plan(*this, sms));
   ADFEM_TRY(state.alloc(sizeof(CgState)));
+  ADFEM_TRY(bad.alloc(sizeof(int)));
   ADFEM_CUDA(cudaMemset(state.p, 0, sizeof(CgState)));
   ADFEM_TRY(partials.alloc(sizeof(double) * 4 * (size_t)std::max(std::max(grid, grid_spmv), zgrid)));
   const size_t n8 = sizeof(double) * (size_t)n, n4 = sizeof(float) * (size_t)n;
@@ -680,59 +681,81 @@ int Solver::init(const Sell* A_, int64_t n_) {
   return ADFEM_OK;
 }
 
-// After an assembly: the copies the system's default solve needs are made at once (the
-// banded mixed copies when the band fits, else the Jacobi-scaled copies), which also
-// checks the diagonal; the Jacobi-scaled copies of a banded system (FP64 solves, the
-// scaled mixed path, packed solves, apply) are made on first use (solver_ensure_scaled),
-// so an assembly followed by mixed solves does not pay for them.
+// Reads back the diagonal check of the kernels before it.
+static int check_diagonal(Solver& S, cudaStream_t user) {
+  int hbad = 0;
+  ADFEM_CUDA(cudaMemcpyAsync(&hbad, S.bad.p, sizeof(int), cudaMemcpyDeviceToHost, user));
+  ADFEM_CUDA(cudaStreamSynchronize(user));
+  if (hbad) return fail(ADFEM_ERR_BREAKDOWN, "operator has a non-positive or non-finite diagonal entry");
+  return ADFEM_OK;
+}
+
+static void enqueue_scale_diag(Solver& S, cudaStream_t user) {
+  const Sell& A = *S.A;
+  k_scale_diag<<<(unsigned)((S.n + kT - 1) / kT), kT, 0, user>>>(S.n, A.sptr.as<int32_t>(), A.val64.as<double>(),
+                                                                 S.diagpos, S.s32.as<float>(), S.bad.as<int>());
+}
+
+// The copies of the banded mixed iteration, once per assembly.
+static int ensure_banded(Solver& S, cudaStream_t user) {
+  if (S.prep_z) return ADFEM_OK;
+  ADFEM_CUDA(cudaMemsetAsync(S.bad.p, 0, sizeof(int), user));
+  ADFEM_TRY(zcg_prepare(S, S.diagpos, S.bad.as<int>(), user));
+  ADFEM_TRY(check_diagonal(S, user));
+  S.prep_z = true;
+  return ADFEM_OK;
+}
+
+// After an assembly: what the system's default solve needs first is made at once and checks the
+// diagonal (multigrid: the scales; else the banded mixed copies when the band fits, or the
+// Jacobi-scaled copies); the other copies of the operator (multigrid values, banded, Jacobi-scaled
+// ones) are made on first use, so an assembly does not pay for solvers it is not followed by.
 int solver_prepare(Solver& S, const int32_t* diagpos_dev, cudaStream_t user) {
   S.prepared = false;
   S.prep_scaled = false;
+  S.prep_vals64 = false;
+  S.prep_z = false;
+  if (S.mg) S.mg->current = false;
   if (!diagpos_dev) return fail(ADFEM_ERR_INVALID, "solver_prepare: diagonal positions required");
   S.diagpos = diagpos_dev;
-  if (!S.zcg) {
-    ADFEM_TRY(solver_ensure_scaled(S, user));
-    S.prepared = true;
-    return ADFEM_OK;
+  if (S.mg_allowed) {
+    ADFEM_CUDA(cudaMemsetAsync(S.bad.p, 0, sizeof(int), user));
+    enqueue_scale_diag(S, user);
+    ADFEM_CUDA(cudaGetLastError());
+    ADFEM_TRY(check_diagonal(S, user));
+  } else if (S.zcg) {
+    ADFEM_TRY(ensure_banded(S, user));
+  } else {
+    ADFEM_TRY(solver_ensure_scaled(S, true, user));
   }
-  DevBuf bad;
-  ADFEM_TRY(bad.alloc(sizeof(int)));
-  ADFEM_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), user));
-  ADFEM_TRY(zcg_prepare(S, diagpos_dev, bad.as<int>(), user));  // reads the unscaled values
-  int hbad = 0;
-  ADFEM_CUDA(cudaMemcpyAsync(&hbad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, user));
-  ADFEM_CUDA(cudaStreamSynchronize(user));
-  if (hbad) return fail(ADFEM_ERR_BREAKDOWN, "operator has a non-positive or non-finite diagonal entry");
   S.prepared = true;
   return ADFEM_OK;
 }
 
-// Jacobi-scaled copies: s_i = rsqrt(K_ii), val64 <- s_i K_ij s_j in place (standard form),
-// valD64 / val32 the FP64 / FP32 difference forms (k_scale_values).  Once per assembly.
-int solver_ensure_scaled(Solver& S, cudaStream_t user) {
-  if (S.prep_scaled) return ADFEM_OK;
+// Jacobi-scaled copies: s_i = rsqrt(K_ii), vals64 = s_i K_ij s_j (standard form), valD64 / val32
+// the FP64 / FP32 difference forms (k_scale_values).  Once per assembly.  standard64: vals64 is
+// needed (the FP64 iterations).
+int solver_ensure_scaled(Solver& S, bool standard64, cudaStream_t user) {
+  if (S.prep_scaled && (S.prep_vals64 || !standard64)) return ADFEM_OK;
   if (!S.diagpos) return fail(ADFEM_ERR_INVALID, "solver: operator not prepared");
   const Sell& A = *S.A;
-  DevBuf bad;
-  ADFEM_TRY(bad.alloc(sizeof(int)));
-  ADFEM_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), user));
+  if (standard64) ADFEM_TRY(S.vals64.alloc(sizeof(double) * (size_t)std::max<int64_t>(A.nent, 1)));
+  double* vals = standard64 ? S.vals64.as<double>() : nullptr;
+  ADFEM_CUDA(cudaMemsetAsync(S.bad.p, 0, sizeof(int), user));
   const unsigned nb = (unsigned)((S.n + kT - 1) / kT);
-  k_scale_diag<<<nb, kT, 0, user>>>(S.n, A.sptr.as<int32_t>(), A.val64.as<double>(), S.diagpos, S.s32.as<float>(),
-                                    bad.as<int>());
+  enqueue_scale_diag(S, user);
   if (A.delta16)
     k_scale_values<true><<<nb, kT, 0, user>>>(S.n, A.sptr.as<int32_t>(), A.col.p, A.val64.as<double>(),
-                                              A.valD64.as<double>(), A.val32.as<float>(), S.s32.as<float>(),
-                                              S.diagpos);
+                                              vals, A.valD64.as<double>(), A.val32.as<float>(),
+                                              S.s32.as<float>(), S.diagpos);
   else
     k_scale_values<false><<<nb, kT, 0, user>>>(S.n, A.sptr.as<int32_t>(), A.col.p, A.val64.as<double>(),
-                                               A.valD64.as<double>(), A.val32.as<float>(), S.s32.as<float>(),
-                                               S.diagpos);
+                                               vals, A.valD64.as<double>(), A.val32.as<float>(),
+                                               S.s32.as<float>(), S.diagpos);
   ADFEM_CUDA(cudaGetLastError());
-  int hbad = 0;
-  ADFEM_CUDA(cudaMemcpyAsync(&hbad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, user));
-  ADFEM_CUDA(cudaStreamSynchronize(user));
-  if (hbad) return fail(ADFEM_ERR_BREAKDOWN, "operator has a non-positive or non-finite diagonal entry");
+  ADFEM_TRY(check_diagonal(S, user));
   S.prep_scaled = true;
+  S.prep_vals64 = standard64;
   return ADFEM_OK;
 }
 
@@ -799,18 +822,23 @@ struct Timer {
   }
 };
 
+void solver_enqueue_spmv64(Solver& S, const double* vals, cudaStream_t st) {
+  const Sell& A = *S.A;
+  ADFEM_SELL_DISPATCH(S, k_cg64_spmv, S.grid_spmv, st, S.n, A.sptr.as<int32_t>(), A.col.p, sell_pat(A), vals,
+                      S.p64.as<double>(), S.q64.as<double>(), S.state.as<CgState>(), S.partials.as<double>());
+}
+
+void solver_enqueue_fold64(Solver& S, int force, cudaStream_t st) {
+  k_fold64<<<S.grid, kT, 0, st>>>(S.n, S.y64.as<double>(), S.z64.as<double>(), S.state.as<CgState>(), force);
+}
+
 // enqueue one FP64 CG iteration
 static void enqueue_cg64(Solver& S, cudaStream_t st, Timer* tm = nullptr) {
   Timer none;
   if (!tm) tm = &none;
-  const Sell& A = *S.A;
-  auto* sp = A.sptr.as<int32_t>();
   auto* cs = S.state.as<CgState>();
   auto* part = S.partials.as<double>();
-  tm->run(0, st, [&] {
-    ADFEM_SELL_DISPATCH(S, k_cg64_spmv, S.grid_spmv, st, S.n, sp, A.col.p, sell_pat(A), A.val64.as<double>(),
-                        S.p64.as<double>(), S.q64.as<double>(), cs, part);
-  });
+  tm->run(0, st, [&] { solver_enqueue_spmv64(S, S.vals64.as<double>(), st); });
   tm->run(1, st, [&] {
     k_cg64_update<<<S.grid, kT, 0, st>>>(S.n, S.z64.as<double>(), S.r64.as<double>(), S.p64.as<double>(),
                                          S.q64.as<double>(), cs, part);
@@ -872,9 +900,7 @@ static void enqueue_reliable_update(Solver& S, cudaStream_t st, int force, Timer
 static void enqueue_fp64_replacement(Solver& S, cudaStream_t st, int force, Timer* tm = nullptr) {
   Timer none;
   if (!tm) tm = &none;
-  tm->run(2, st, [&] {
-    k_fold64<<<S.grid, kT, 0, st>>>(S.n, S.y64.as<double>(), S.z64.as<double>(), S.state.as<CgState>(), force);
-  });
+  tm->run(2, st, [&] { solver_enqueue_fold64(S, force, st); });
   enqueue_residual(S, st, 3, force, tm);
 }
 
@@ -987,9 +1013,18 @@ int solver_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_ro
   const bool mixed = o.precision == ADFEM_PREC_MIXED;
   if (o.precision != ADFEM_PREC_FP64 && !mixed) return fail(ADFEM_ERR_INVALID, "solver: unknown precision");
   if (!(o.rtol > 0.0) || o.max_iter < 1) return fail(ADFEM_ERR_INVALID, "solver: rtol must be > 0, max_iter >= 1");
+  if (S.mg_allowed && S.mg_fixed && !prof) {
+    ADFEM_TRY(mg_plan(S));
+    if (S.mg) {
+      bool gave_up = false;
+      const int r = mg_solve(S, rhs, u, zero_rows, fix_rows, fix_vals, o, stats, user, &gave_up);
+      if (!gave_up) return r;
+    }
+  }
   const int chunk = std::max(1, std::min(o.chunk > 0 ? o.chunk : 32, 512));
   const Path path = !mixed ? (S.dcg ? Path::DBANDED : Path::FP64) : (S.zcg ? Path::BANDED : Path::MIXED);
-  if (path != Path::BANDED) ADFEM_TRY(solver_ensure_scaled(S, user));
+  if (path != Path::BANDED) ADFEM_TRY(solver_ensure_scaled(S, path != Path::MIXED, user));
+  else ADFEM_TRY(ensure_banded(S, user));
   cudaStream_t st = S.stream;
   cudaGraphExec_t* gx = path == Path::FP64 ? &S.g64
                         : (path == Path::MIXED ? &S.g32 : (path == Path::BANDED ? &S.gz : &S.gd));
@@ -1120,7 +1155,7 @@ int solver_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_ro
                                   S.state.as<CgState>(), 1);
     launches += 1;
   } else {
-    k_fold64<<<S.grid, kT, 0, st>>>(S.n, S.y64.as<double>(), S.z64.as<double>(), S.state.as<CgState>(), 1);
+    solver_enqueue_fold64(S, 1, st);
     launches += 1;
   }
   if (path == Path::BANDED) {
@@ -1161,19 +1196,21 @@ int solver_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_ro
 }
 
 int solver_apply(Solver& S, const double* x, double* y, cudaStream_t user) {
-  ADFEM_TRY(solver_ensure_scaled(S, user));
   const Sell& A = *S.A;
   const unsigned nb = (unsigned)((S.n + kT - 1) / kT);
   if (A.delta16)
-    k_apply<true><<<nb, kT, 0, user>>>(S.n, A.sptr.as<int32_t>(), A.col.p, A.val64.as<double>(), S.s32.as<float>(), x,
-                                       y);
+    k_apply<true><<<nb, kT, 0, user>>>(S.n, A.sptr.as<int32_t>(), A.col.p, A.val64.as<double>(), x, y);
   else
-    k_apply<false><<<nb, kT, 0, user>>>(S.n, A.sptr.as<int32_t>(), A.col.p, A.val64.as<double>(), S.s32.as<float>(),
-                                        x, y);
+    k_apply<false><<<nb, kT, 0, user>>>(S.n, A.sptr.as<int32_t>(), A.col.p, A.val64.as<double>(), x, y);
   ADFEM_CUDA(cudaGetLastError());
   return ADFEM_OK;
 }
 
-ADFEM_CHECK_READER(check_line_solver)
+ADFEM_CHECK_READER(check_line_solver_own)
+int check_line_mg();  // mg.cu
+int check_line_solver() {
+  const int a = check_line_solver_own(), b = check_line_mg();
+  return a != 0 ? a : (b > 0 ? 50000 + b : b);
+}
 
 }  // namespace adfem

@@ -1,6 +1,7 @@
 // Solver internals shared by solver.cu and capi.cpp.
 #pragma once
 #include "adfem_internal.h"
+#include "mg.cuh"
 
 namespace adfem {
 
@@ -35,7 +36,7 @@ struct Solver {
   int grid = 0;            // blocks of the grid-stride kernels (resident blocks per SM x SMs)
   int grid_spmv = 0;       // same for the unrolled SpMV kernels (higher register use)
   bool prefetch = false;   // SpMV software pipelining (ADFEM_SPMV_PREFETCH=1)
-  const Sell* A = nullptr; // sliced-ELL operator (val64 scaled in place, val32 scaled copy)
+  const Sell* A = nullptr; // sliced-ELL operator (val64 as assembled, val32 scaled copy)
   DevBuf s32;              // Jacobi scaling s_i = 1/sqrt(K_ii) (float, exact in double)
   DevBuf state;            // CgState
   DevBuf partials;         // 4 * grid doubles
@@ -52,6 +53,7 @@ struct Solver {
   int g64_chunk = 0, g32_chunk = 0;
   bool prepared = false;
   bool prep_scaled = false;        // the Jacobi-scaled copies are current (see solver_ensure_scaled)
+  bool prep_vals64 = false;        // vals64 too
   const int32_t* diagpos = nullptr; // device: entry index of the diagonal in each row
   // banded mixed path (zcg.cu): used by mixed solves when the band fits the ring
   bool zcg = false;
@@ -85,6 +87,19 @@ struct Solver {
   DevBuf dr1, dp1, dq1;    // second buffers of the r, p, q pairs (first: r64, p64, q64)
   cudaGraphExec_t gd = nullptr;
   int gd_chunk = 0;
+  // multigrid preconditioner (mg.cu) of resident systems: the matrix graph in solver order (node
+  // graph, mg_nb unknowns per node; node positions for two) is kept until the first solve
+  // builds the hierarchy from it
+  bool mg_allowed = false;
+  int mg_nb = 1;
+  std::vector<int32_t> mg_rp, mg_ci;
+  std::vector<double> mg_x, mg_y;
+  const uint8_t* mg_isbd = nullptr;  // device: Dirichlet tags in solver order
+  bool mg_fixed = false;             // there are Dirichlet rows (the operator is not singular)
+  std::unique_ptr<Mg> mg;
+  DevBuf vals64;           // Jacobi-scaled FP64 copy (A->val64 keeps the assembled values)
+  DevBuf bad;              // int: a diagonal entry is not positive and finite
+  bool prep_z = false;     // the banded mixed copies are current
   ~Solver();
   int init(const Sell* A, int64_t n);
 };
@@ -92,9 +107,10 @@ struct Solver {
 // After an assembly (diagpos: entry index k of the diagonal in row i): makes the copies
 // the default solve needs now and marks the others for first use.
 int solver_prepare(Solver& S, const int32_t* diagpos_dev, cudaStream_t user);
-// The Jacobi-scaled copies: s_i = rsqrt(K_ii) (FP32), val64 <- s_i K_ij s_j, valD64 / val32
-// the FP64 / FP32 difference-form copies (see k_scale_values); no-op when current.
-int solver_ensure_scaled(Solver& S, cudaStream_t user);
+// The Jacobi-scaled copies: s_i = rsqrt(K_ii) (FP32), vals64 = s_i K_ij s_j, valD64 / val32
+// the FP64 / FP32 difference-form copies (see k_scale_values); standard64: vals64 too; no-op when
+// current.
+int solver_ensure_scaled(Solver& S, bool standard64, cudaStream_t user);
 // Per-kernel timing of a profiled solve: 0 SpMV+dot, 1 update+dot, 2 p update / fold,
 // 3 FP64 residual.
 struct SolveProfile {
@@ -108,8 +124,21 @@ struct SolveProfile {
 int solver_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_rows, const uint8_t* fix_rows,
                  const double* fix_vals, const adfem_solver_opts& o, adfem_solver_stats* stats, cudaStream_t user,
                  SolveProfile* prof = nullptr);
-// y = K x with the unscaled operator (via the scaled copy)
+// y = K x with the unscaled operator
 int solver_apply(Solver& S, const double* x, double* y, cudaStream_t user);
+
+// Multigrid-preconditioned FP64 CG (mg.cu): hierarchy on first use (clears mg_allowed when the
+// graph does not coarsen), its values once per assembly, the solve.  gave_up: no outcome (a
+// breakdown, or more iterations than the multigrid cap); u untouched, the caller falls back.
+int mg_plan(Solver& S);
+int mg_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_rows, const uint8_t* fix_rows,
+             const double* fix_vals, const adfem_solver_opts& o, adfem_solver_stats* stats, cudaStream_t user,
+             bool* gave_up);
+size_t mg_device_bytes(const Solver& S);
+// kernels of the FP64 CG that mg.cu shares: q64 = K p64 with alpha = rho / p.q for the given
+// values, and y64 += z64, z64 = 0 (when a residual is due, or forced)
+void solver_enqueue_spmv64(Solver& S, const double* vals, cudaStream_t st);
+void solver_enqueue_fold64(Solver& S, int force, cudaStream_t st);
 
 // Banded mixed path (zcg.cu).  zcg_plan decides whether the operator's band fits
 // the shared-memory ring and allocates the path's buffers; zcg_prepare derives its

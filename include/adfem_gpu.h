@@ -59,8 +59,8 @@ ADFEM_API int adfem_debug_fail_alloc(long long k);
 /* Testing hook, no counterpart in the reference: in the debug build (-DADFEM_CHECKS, a
  * second library built by build.py --checks) kernels check the indices they compute before
  * using them and record the first failure instead of faulting; this returns it as
- * 100000 * unit + source line (unit 1: solver.cu, 2: zcg.cu, 3: assemble.cu, 4: generic.cu), 0 when no check
- * failed (always 0 in release builds), -1 if the flags cannot be read, and clears it. */
+ * 100000 * unit + source line (unit 1: solver.cu, and mg.cu from line 50000 on, 2: zcg.cu,
+ * 3: assemble.cu, 4: generic.cu), 0 when no check failed (always 0 in release builds), -1 if the flags cannot be read, and clears it. */
 ADFEM_API int adfem_debug_check_code(void);
 
 /* ====================================================================
@@ -297,11 +297,14 @@ enum { ADFEM_PREC_FP64 = 0, ADFEM_PREC_MIXED = 1 };
 typedef struct {
   double rtol;     /* stop when ||b~ - K~ y|| <= rtol ||b~|| in the Jacobi-scaled system (default 1e-12) */
   int max_iter;    /* cap on CG iterations (default 200000) */
-  int precision;   /* ADFEM_PREC_FP64: FP64 Jacobi-CG; ADFEM_PREC_MIXED: FP32 inner CG with FP64
-                      reliable updates (FP64 residual r = F - K u, FP64 solution, FP64 stop test) */
-  double ru_delta; /* mixed: replace the FP32 residual by the FP64 one when it dropped by this factor
-                      since the last replacement (default 0.1) */
-  int chunk;       /* iterations per device-resident chunk between host checks (default 32) */
+  int precision;   /* Jacobi-CG (adfem_csc_solve, packed solves, resident systems that do not use
+                      multigrid): ADFEM_PREC_FP64: FP64; ADFEM_PREC_MIXED: FP32 inner CG with FP64
+                      reliable updates (FP64 residual r = F - K u, FP64 solution, FP64 stop test).
+                      Resident systems: FP64 CG preconditioned by an FP32 multigrid cycle in either
+                      precision, same stop test; see adfem_system_create */
+  double ru_delta; /* mixed Jacobi-CG: replace the FP32 residual by the FP64 one when it dropped by
+                      this factor since the last replacement (default 0.1) */
+  int chunk;       /* Jacobi-CG: iterations per device-resident chunk between host checks (default 32) */
   int warm_start;  /* 1: start from the u passed in; 0: from zero */
 } adfem_solver_opts;
 
@@ -328,7 +331,15 @@ ADFEM_API int adfem_csc_solve(long long n, const long long *colptr1, const long 
  * sliced-ELL form (FP64 and FP32 Jacobi-scaled copies) with its right-hand side and
  * CG work vectors, so repeated solves and adjoint solves reuse them. */
 enum { ADFEM_SYS_POISSON = 0, ADFEM_SYS_ELASTICITY = 1 };
-/* Poisson systems on P1 or P2 meshes (P2: the vertex-then-edge DOFs of the mesh's space,
+/* Solves of a system with Dirichlet DOFs run FP64 CG preconditioned by one V-cycle of smoothed
+ * aggregation multigrid (hierarchy of the matrix graph built by the first solve, its values
+ * once per assembly): tens of iterations at every size where Jacobi-CG needs thousands.  The
+ * Jacobi iterations serve systems without Dirichlet DOFs (singular), graphs that do not
+ * coarsen, solves in which the preconditioned iteration breaks down (indefinite operators) or
+ * needs more than 300 iterations, profiled solves, and systems created while ADFEM_MG=0 or one
+ * of ADFEM_ZCG, ADFEM_ZCG64, ADFEM_ZCG_SMAX, ADFEM_ZCG_RING, ADFEM_ZCG_RING_REFILL (which pick
+ * a variant of them) is set in the environment.
+ * Poisson systems on P1 or P2 meshes (P2: the vertex-then-edge DOFs of the mesh's space,
  * kappa and f at the 6 points per element of the order-4 rule; DOFs renumbered for the
  * solver by reverse Cuthill-McKee, inputs and outputs in the reference order); elasticity
  * systems on P1 meshes (a P2 mesh gives ADFEM_ERR_UNSUPPORTED: assemble its stiffness
@@ -371,7 +382,7 @@ ADFEM_API int adfem_system_grad_E_d(adfem_system *sys, const double *u_d, const 
 ADFEM_API int adfem_system_apply_d(adfem_system *sys, const double *x_d, double *y_d, void *stream);
 /* copy out the assembled right-hand side (reference DOF ordering) */
 ADFEM_API int adfem_system_rhs_d(adfem_system *sys, double *rhs_d, void *stream);
-/* Same solve as adfem_system_solve_d with CUDA event pairs on the solver's stream, for
+/* The system's Jacobi-CG solve with CUDA event pairs on the solver's stream, for
  * measurement: launched kernel by kernel with an event pair around every launch, except
  * that on the banded mixed path each run of iterations between two replacement checks
  * (16) is one captured graph (as in the solve) with an event pair around the run, whose
