@@ -38,7 +38,7 @@ namespace {
 constexpr float kSmoothP = 1.6f;
 constexpr float kFrac0 = 0.125f, kFrac = 0.06f;  // lower end of the Chebyshev interval over lam
 constexpr int kCoef = 2 * kMgDeg;
-constexpr int kTailT = 1024;
+constexpr size_t kTailSmem = 224 * 1024;  // shared memory of a tail block, at most
 constexpr int kMgIterations = 300;  // a solve that needs more is left to the Jacobi iteration
 
 template <int NB>
@@ -65,19 +65,36 @@ __device__ __forceinline__ void store_vec(float* __restrict__ p, int64_t i, cons
 #pragma unroll
     for (int c = 0; c < NB; c++) p[NB * i + c] = r.v[c];
 }
-// acc += M x, M an R x C block
+// R x C blocks of an array of n entries: 2 x 2 blocks as one 16-byte word each, other blocks as
+// R C planes of n floats (a warp's loads of one component are then consecutive; 36-byte blocks
+// side by side cost nine times the L1 wavefronts).
 template <int R, int C>
-__device__ __forceinline__ void block_fma(const float* __restrict__ m, const Vec<C>& x, Vec<R>& acc) {
+__device__ __forceinline__ void load_block(const float* __restrict__ m, int64_t idx, int64_t n, float (&v)[R * C]) {
   if constexpr (R == 2 && C == 2) {
-    const float4 t = *reinterpret_cast<const float4*>(m);
-    acc.v[0] = fmaf(t.x, x.v[0], fmaf(t.y, x.v[1], acc.v[0]));
-    acc.v[1] = fmaf(t.z, x.v[0], fmaf(t.w, x.v[1], acc.v[1]));
+    const float4 t = reinterpret_cast<const float4*>(m)[idx];
+    v[0] = t.x;
+    v[1] = t.y;
+    v[2] = t.z;
+    v[3] = t.w;
   } else {
 #pragma unroll
-    for (int r = 0; r < R; r++)
-#pragma unroll
-      for (int c = 0; c < C; c++) acc.v[r] = fmaf(m[r * C + c], x.v[c], acc.v[r]);
+    for (int e = 0; e < R * C; e++) v[e] = m[e * n + idx];
   }
+}
+template <int R, int C>
+__device__ __forceinline__ int64_t block_at(int e, int64_t idx, int64_t n) {
+  return R == 2 && C == 2 ? 4 * idx + e : e * n + idx;
+}
+// acc += M x
+template <int R, int C>
+__device__ __forceinline__ void block_fma(const float* __restrict__ m, int64_t idx, int64_t n, const Vec<C>& x,
+                                          Vec<R>& acc) {
+  float v[R * C];
+  load_block<R, C>(m, idx, n, v);
+#pragma unroll
+  for (int r = 0; r < R; r++)
+#pragma unroll
+    for (int c = 0; c < C; c++) acc.v[r] = fmaf(v[r * C + c], x.v[c], acc.v[r]);
 }
 template <int NB, int LPR>
 __device__ __forceinline__ void lane_sum(Vec<NB>& a) {
@@ -131,7 +148,7 @@ __device__ __forceinline__ Vec<NB> row_product(const MgLev& L, int r, int lane, 
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const int k = k0 + u * LPR;
-      if (k < w) block_fma<NB, NB>(L.val + (base + 32 * (int64_t)k) * (NB * NB), load_vec<NB>(x, j[u]), acc);
+      if (k < w) block_fma<NB, NB>(L.val, base + 32 * (int64_t)k, L.nv, load_vec<NB>(x, j[u]), acc);
     }
   }
   if (LPR > 1) lane_sum<NB, LPR>(acc);
@@ -222,7 +239,7 @@ __global__ void __launch_bounds__(kT) k_mg_restrict(MgLev L, const float* __rest
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const int k = k0 + u * LPR;
-      if (k < w) block_fma<NC, NB>(L.pt_val + (base + 32 * (int64_t)k) * (NB * NC), load_vec<NB>(r, i[u]), acc);
+      if (k < w) block_fma<NC, NB>(L.pt_val, base + 32 * (int64_t)k, L.npt, load_vec<NB>(r, i[u]), acc);
     }
   }
   if (LPR > 1) lane_sum<NC, LPR>(acc);
@@ -247,187 +264,448 @@ __global__ void __launch_bounds__(kT) k_mg_prolong(MgLev L, const float* __restr
 #pragma unroll
     for (int u = 0; u < U; u++)
       if (k0 + u < w)
-        block_fma<NB, NC>(L.p_val + (base + 32 * (int64_t)(k0 + u)) * (NB * NC), load_vec<NC>(xc, J[u]), acc);
+        block_fma<NB, NC>(L.p_val, base + 32 * (int64_t)(k0 + u), L.np, load_vec<NC>(xc, J[u]), acc);
   }
   store_vec<NB>(x, i, acc);
 }
 
 // ---------------------------------------------------------------------------
-// The levels from Mg::tail on in one block: all vectors in shared memory, the operators read
-// through L1/L2; `reps` cycles (two cycles below a larger level: its coarse problem is then
-// solved nearly exactly).  The coarsest operator is applied as its dense inverse.
+// The levels from Mg::tail on in one launch, `reps` cycles (two below a larger level: its coarse
+// problem is then solved nearly exactly).  Two forms:
+//  * one block (first level of at most kTailLocal unknowns): every level's vectors in shared
+//    memory, a barrier of the block per sweep;
+//  * a cluster of kTailC blocks (EX): each block owns a contiguous range of the first level's
+//    rows and keeps both iterates of that level whole in its shared memory (gathers are local);
+//    a row's new value goes to the blocks whose rows refer to it (MgLev::to; one or two of
+//    eight, as the numbering is banded) by asynchronous stores that count on the receiver's
+//    mbarrier, and a block goes on when what it needs has arrived.  (A cluster barrier instead
+//    would also drop the operator's rows from L1, where they stay from sweep to sweep.)  Every
+//    block sends every other one word per exchange, after it has read its operands, so that a
+//    block is at most one exchange ahead of another: two mbarriers in turn suffice, and nothing
+//    is overwritten before it has been read.  The smaller levels are computed by every block
+//    for itself, which costs no exchange.
+// What bounds it is latency and instruction issue: a thread owns one unknown's row and keeps its
+// entries in registers over the steps of a smoother, and the operators of the levels that a
+// block runs alone are copied to shared memory in bulk while it is busy with the first level.
+// The coarsest operator is applied as its dense inverse.
 struct TailArgs {
   MgLev L[kMgMaxTail];
   int nl;
   const float* dense;
   int N;         // unknowns of the coarsest level
+  // patterns and values of the levels a block runs alone, each one range of device memory
+  // (bytes 0: they do not fit and are read through L1)
+  const char *pat, *vals;
+  int pat_bytes, val_bytes;
   const float* b;
   float* x;
   int reps;
-  CgState* st;   // level 0 in the tail: r.z from here
+  int dot;       // level 0 in the tail: r.z from here
+  CgState* st;
 };
 struct TailVecs {
-  float *b, *x, *y, *d;
+  float *x, *y;  // whole: current iterate, other iterate (or right-hand side, residual)
+  float *b, *d;  // own rows
+  int r0, r1;    // own rows of the level
+  int floats;    // EX: values an exchange of the level brings here
 };
 
-template <int NB, class Body>
-__device__ __forceinline__ void tail_rows(const MgLev& L, const float* x, Body body) {
-  const int lpr = L.lpr, lane = threadIdx.x & (lpr - 1);
-  const int rows = (L.n + (kTailT / lpr) - 1) / (kTailT / lpr) * (kTailT / lpr);
-  for (int r0 = threadIdx.x / lpr; r0 < rows; r0 += kTailT / lpr) {
-    const int r = r0 < L.n ? r0 : L.n - 1;
-    Vec<NB> acc;
-#pragma unroll
-    for (int c = 0; c < NB; c++) acc.v[c] = 0.0f;
-    int64_t base;
-    int w;
-    slice_row(L.sptr, r, base, w);
-    const int32_t* col = reinterpret_cast<const int32_t*>(L.col);
-    constexpr int U = 4;
-    for (int k0 = lane; k0 < w; k0 += U * lpr) {
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int k = k0 + u * lpr;
-        if (k < w) {
-          int j = __ldg(col + base + 32 * (int64_t)k);
-          if (!ADFEM_DCHECK(j >= 0 && j < L.n)) j = r;
-          block_fma<NB, NB>(L.val + (base + 32 * (int64_t)k) * (NB * NB), load_vec<NB>(x, j), acc);
-        }
-      }
-    }
-    for (int o = lpr >> 1; o > 0; o >>= 1)
-#pragma unroll
-      for (int c = 0; c < NB; c++) acc.v[c] += __shfl_xor_sync(0xffffffffu, acc.v[c], o);
-    if (lane == 0 && r0 < L.n) body(r, acc);
-  }
-  __syncthreads();
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// shared-memory address p of this block, in the block of the given rank
+__device__ __forceinline__ unsigned rank_addr(const void* p, int rank) {
+  unsigned m;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(m) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+  return m;
+}
+__device__ __forceinline__ void store_rank(const float* p, int rank, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(rank_addr(p, rank)), "f"(v) : "memory");
 }
 
-// Chebyshev of the level's degree on (b, x) -> x; zero: x = 0 on entry.  v.y: the other iterate.
+// The exchanges of a block, numbered: exchange k counts on bar[k & 1] in its (k >> 1)-th phase.
+struct TailSync {
+  unsigned long long* bar;
+  float* tok;    // kTailC words
+  int rank;
+  CgState* st;
+  int k = 0;
+  // this exchange brings `floats` values here
+  __device__ __forceinline__ void expect(int floats) {
+    if (threadIdx.x == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(bar + (k & 1))),
+                   "r"(4 * (floats + kTailC))
+                   : "memory");
+  }
+  __device__ __forceinline__ void send(const float* p, int rk, float v) const {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(rank_addr(p, rk)),
+                 "f"(v), "r"(rank_addr(bar + (k & 1), rk))
+                 : "memory");
+  }
+  // the block has sent its rows: tell every block, and wait for what it needs itself
+  __device__ __forceinline__ void exchange() {
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      if (threadIdx.x < kTailC) send(tok + rank, threadIdx.x, 0.0f);
+      const unsigned a = (unsigned)__cvta_generic_to_shared(bar + (k & 1)), parity = (k >> 1) & 1;
+      unsigned ok = 0;
+      // (bounded: a wait that gives up ends the solve, which falls back to the Jacobi iteration)
+      for (int i = 0; i < (1 << 16) && !ok; i++)
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(ok)
+                     : "r"(a), "r"(parity)
+                     : "memory");
+      if (!ok) st->done = 5;
+    }
+    __syncthreads();
+    k++;
+  }
+};
+
+// The level as the tail's threads see it (pointers into shared memory where it was copied).
+struct TailLev {
+  const int32_t *sptr, *col, *p_sptr, *p_col, *pt_sptr, *pt_col;
+  const float *val, *p_val, *pt_val, *coef;
+  const uint8_t* to;
+  int n, nv, np, npt;
+};
+
+// Row of one unknown (component c of node r): the first E entries in registers.
 template <int NB>
-__device__ void tail_smooth(const MgLev& L, TailVecs& v, int deg, bool zero) {
+struct RowCache {
+  static constexpr int E = NB == 1 ? 14 : (NB == 2 ? 8 : 6);
+  float v[E][NB];
+  int j[E];
+  int base, w, c;
+  __device__ __forceinline__ void load(const TailLev& L, int r, int comp) {
+    const int s0 = L.sptr[r >> 5];
+    w = (L.sptr[(r >> 5) + 1] - s0) >> 5;
+    base = s0 + (r & 31);
+    c = comp;
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      if (e >= w) continue;
+      j[e] = NB * L.col[base + 32 * e];
+      if (!ADFEM_DCHECK(j[e] >= 0 && j[e] < NB * L.n)) j[e] = NB * r;
+#pragma unroll
+      for (int q = 0; q < NB; q++) v[e][q] = L.val[block_at<NB, NB>(c * NB + q, base + 32 * e, L.nv)];
+    }
+  }
+  __device__ __forceinline__ float product(const TailLev& L, const float* x) const {
+    float acc = 0.0f;
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      if (e >= w) continue;
+#pragma unroll
+      for (int q = 0; q < NB; q++) acc = fmaf(v[e][q], x[j[e] + q], acc);
+    }
+    for (int e = E; e < w; e++) {
+      const int k = base + 32 * e, jj = NB * L.col[k];
+#pragma unroll
+      for (int q = 0; q < NB; q++) acc = fmaf(L.val[block_at<NB, NB>(c * NB + q, k, L.nv)], x[jj + q], acc);
+    }
+    return acc;
+  }
+};
+
+constexpr int kTailT = kMgTailDofs / kTailC;  // threads of a tail block: one per own unknown
+
+// publish unknown u (of a row that the ranks in the bit mask need): out[u] here or there
+template <bool EX>
+__device__ __forceinline__ void tail_put(const TailSync& sync, unsigned ranks, float* out, int u, float v) {
+  if (EX) {
+    for (; ranks; ranks &= ranks - 1) sync.send(out + u, __ffs(ranks) - 1, v);
+  } else {
+    out[u] = v;
+  }
+}
+template <bool EX>
+__device__ __forceinline__ void tail_end(TailSync& sync) {
+  if (EX) sync.exchange();
+  else __syncthreads();
+}
+
+// Chebyshev steps on (b, x) -> x, then (res) the residual into y.  fresh: x = 0 and the right-hand
+// side stands whole in y; the first two steps are one sweep (as kPre).
+template <bool EX, int NB, int T>
+__device__ __forceinline__ void tail_smooth(TailSync& sync, const TailLev& L, TailVecs& v, int deg, bool fresh,
+                                            bool res) {
+  TailVecs f = v;
+  const int m = (f.r1 - f.r0) * NB, u0 = f.r0 * NB;
+  const bool one = m <= T;  // at most one row per thread: its entries stay in registers
+  RowCache<NB> rc;
+  unsigned ranks = 0;
+  if (one && (int)threadIdx.x < m) {
+    const int r = f.r0 + threadIdx.x / NB;
+    rc.load(L, r, threadIdx.x % NB);
+    if (EX) ranks = L.to[r];
+  }
   const float th = L.coef[0];
-  if (zero) {
-    for (int t = threadIdx.x; t < L.n * NB; t += kTailT) {
-      const float x1 = th * v.b[t];
-      v.d[t] = x1;
-      v.x[t] = x1;
+  const int k1 = res ? deg + 1 : deg;
+  for (int k = fresh ? 1 : 0; k < k1; k++) {
+    const bool pre = fresh && k == 1, last = k == deg;
+    const float a1 = k > 0 && !last ? L.coef[2 * k] : 0.0f;
+    const float a2 = k > 0 && !last ? L.coef[2 * k + 1] : th;
+    const float* x = pre ? f.y : f.x;
+    float* out = pre ? f.x : f.y;
+    if (EX) sync.expect(f.floats);
+    for (int q = threadIdx.x; q < m; q += T) {
+      if (!one) {
+        const int r = f.r0 + q / NB;
+        rc.load(L, r, q % NB);
+        if (EX) ranks = L.to[r];
+      }
+      const float ax = rc.product(L, x), bi = f.b[q];
+      float o;
+      if (last) {
+        o = bi - ax;
+      } else {
+        const float x1 = pre ? th * bi : f.x[u0 + q];
+        const float d0 = pre ? x1 : (a1 != 0.0f ? f.d[q] : 0.0f);
+        const float d = fmaf(a1, d0, a2 * (bi - (pre ? th : 1.0f) * ax));
+        f.d[q] = d;
+        o = x1 + d;
+      }
+      tail_put<EX>(sync, ranks, out, u0 + q, o);
+    }
+    tail_end<EX>(sync);
+    if (!pre && !last) {
+      float* s = f.x;
+      f.x = f.y;
+      f.y = s;
+    }
+  }
+  v.x = f.x;
+  v.y = f.y;
+}
+
+// out = M x (+ add) for the rows [r0, r1) of a rectangular M with R unknowns per row, X per column.
+// `to`: EX, the ranks that need a row (null: all); own: a second copy.
+template <bool EX, int R, int X, int T>
+__device__ __forceinline__ void tail_transfer(TailSync& sync, const int32_t* sp, const int32_t* col, const float* val,
+                                              int nent, const uint8_t* to, int r0, int r1, int lg, const float* x,
+                                              const float* add, float* out, float* own) {
+  const int lane = threadIdx.x & ((1 << lg) - 1), rows = (r1 - r0) * R;
+  for (int q0 = 0; q0 < rows; q0 += T >> lg) {
+    if (q0 + ((int)(threadIdx.x & ~31u) >> lg) >= rows) break;  // (whole warps without a row)
+    const int q = q0 + ((int)threadIdx.x >> lg);
+    const bool live = q < rows;
+    const int u = r0 * R + (live ? q : rows - 1), r = u / R, c = u % R;
+    const int s0 = sp[r >> 5], w = (sp[(r >> 5) + 1] - s0) >> 5, base = s0 + (r & 31);
+    float acc = 0.0f;
+    for (int k = lane; k < w; k += 1 << lg) {
+      const int j = X * col[base + 32 * k];
+#pragma unroll
+      for (int e = 0; e < X; e++) acc = fmaf(val[block_at<R, X>(c * X + e, base + 32 * k, nent)], x[j + e], acc);
+    }
+    for (int o = (1 << lg) >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (!live || lane) continue;
+    if (add) acc += add[u];
+    if (own) own[u] = acc;
+    tail_put<EX>(sync, EX ? (to ? to[r] : (1u << kTailC) - 1u) : 0u, out, u, acc);
+  }
+  tail_end<EX>(sync);
+}
+
+// log2 of the lanes per row of a transfer with that many rows
+__device__ __forceinline__ int tail_lanes(int rows, int T) {
+  int lg = 0;
+  while (lg < 4 && (rows << (lg + 1)) <= T) lg++;
+  return lg;
+}
+
+// the levels from l on, each whole in this block: (b in y and b) -> x
+template <int NB, int T>
+__device__ __noinline__ void tail_local(TailSync& sync, const TailLev* L, TailVecs* v, int l0, int last, int dot,
+                                        bool fresh0, const float* dense, int N) {
+  for (int l = l0; l < last; l++) {
+    tail_smooth<false, NB, T>(sync, L[l], v[l], dot && l == 0 ? kMgDeg0 : kMgDeg, l > l0 || fresh0, true);
+    TailVecs& c = v[l + 1];
+    tail_transfer<false, NB, NB, T>(sync, L[l].pt_sptr, L[l].pt_col, L[l].pt_val, L[l].npt, nullptr, 0, c.r1,
+                                    tail_lanes(c.r1 * NB, T), v[l].y, nullptr, c.y, c.b);
+  }
+  {
+    // coarsest: some lanes per row of the dense inverse
+    const int lg = tail_lanes(N, T), lane = threadIdx.x & ((1 << lg) - 1);
+    const float* bb = v[last].y;
+    for (int q0 = 0; q0 < N; q0 += T >> lg) {
+      if (q0 + ((int)(threadIdx.x & ~31u) >> lg) >= N) break;
+      const int q = q0 + ((int)threadIdx.x >> lg), r = min(q, N - 1);
+      float s = 0.0f;
+      for (int k = lane; k < N; k += 1 << lg) s = fmaf(dense[r + k * N], bb[k], s);  // (symmetric)
+      for (int o = (1 << lg) >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0 && q < N) v[last].x[q] = s;
     }
     __syncthreads();
   }
-  for (int k = zero ? 1 : 0; k < deg; k++) {
-    const float a1 = k > 0 ? L.coef[2 * k] : 0.0f, a2 = k > 0 ? L.coef[2 * k + 1] : th;
-    tail_rows<NB>(L, v.x, [&](int r, const Vec<NB>& ax) {
-#pragma unroll
-      for (int c = 0; c < NB; c++) {
-        const int t = NB * r + c;
-        const float res = v.b[t] - ax.v[c];
-        const float d = k > 0 ? fmaf(a1, v.d[t], a2 * res) : a2 * res;
-        v.d[t] = d;
-        v.y[t] = v.x[t] + d;
-      }
-    });
-    float* s = v.x;
-    v.x = v.y;
-    v.y = s;
+  for (int l = last - 1; l >= l0; l--) {
+    tail_transfer<false, NB, NB, T>(sync, L[l].p_sptr, L[l].p_col, L[l].p_val, L[l].np, nullptr, 0, v[l].r1, 0,
+                                    v[l + 1].x, v[l].x, v[l].x, nullptr);
+    tail_smooth<false, NB, T>(sync, L[l], v[l], dot && l == 0 ? kMgDeg0 : kMgDeg, false, false);
   }
 }
 
-template <int NB, int NC>
-__device__ void tail_down(const MgLev& L, TailVecs& f, TailVecs& c, int deg, bool zero) {
-  tail_smooth<NB>(L, f, deg, zero);
-  tail_rows<NB>(L, f.x, [&](int r, const Vec<NB>& ax) {
-#pragma unroll
-    for (int q = 0; q < NB; q++) f.d[NB * r + q] = f.b[NB * r + q] - ax.v[q];
-  });
-  const int J8 = threadIdx.x >> 3, lane = threadIdx.x & 7;
-  for (int J0 = J8; J0 < (L.nc + 127) / 128 * 128; J0 += kTailT / 8) {
-    const int J = J0 < L.nc ? J0 : L.nc - 1;
-    Vec<NC> acc;
-#pragma unroll
-    for (int q = 0; q < NC; q++) acc.v[q] = 0.0f;
-    int64_t base;
-    int w;
-    slice_row(L.pt_sptr, J, base, w);
-    for (int k = lane; k < w; k += 8)
-      block_fma<NC, NB>(L.pt_val + (base + 32 * (int64_t)k) * (NB * NC),
-                        load_vec<NB>(f.d, __ldg(L.pt_col + base + 32 * (int64_t)k)), acc);
-    lane_sum<NC, 8>(acc);
-    if (lane == 0 && J0 < L.nc) store_vec<NC>(c.b, J, acc);
-  }
-  __syncthreads();
-}
-template <int NB, int NC>
-__device__ void tail_up(const MgLev& L, TailVecs& f, const TailVecs& c, int deg) {
-  for (int i = threadIdx.x; i < L.n; i += kTailT) {
-    Vec<NB> acc = load_vec<NB>(f.x, i);
-    int64_t base;
-    int w;
-    slice_row(L.p_sptr, i, base, w);
-    for (int k = 0; k < w; k++)
-      block_fma<NB, NC>(L.p_val + (base + 32 * (int64_t)k) * (NB * NC),
-                        load_vec<NC>(c.x, __ldg(L.p_col + base + 32 * (int64_t)k)), acc);
-    store_vec<NB>(f.x, i, acc);
-  }
-  __syncthreads();
-  tail_smooth<NB>(L, f, deg, false);
+__host__ __device__ inline int pad4(int n) { return (n + 3) & ~3; }
+__host__ __device__ inline int tail_chunk(int n) { return (n + kTailC - 1) / kTailC; }
+// floats of one level: two whole vectors and two of the block's own rows
+__host__ __device__ inline int tail_floats(int n, int nb, bool ex) {
+  return 2 * pad4(n * nb) + 2 * pad4((ex ? tail_chunk(n) : n) * nb);
 }
 
 // NT: unknowns per node of the tail's first level, NC: of the others
-template <int NT, int NC>
-__global__ void __launch_bounds__(kTailT) k_mg_tail(TailArgs a) {
+template <int NT, int NC, bool EX>
+__global__ void __launch_bounds__(kTailT, 1) k_mg_tail(const __grid_constant__ TailArgs a) {
+  constexpr int T = kTailT;
   extern __shared__ float4 tail_sm4[];
+  __shared__ float dots[kTailC], tokens[kTailC];
+  __shared__ unsigned long long bars[3];
+  __shared__ TailLev lev[kMgMaxTail];
   float* sm = reinterpret_cast<float*>(tail_sm4);
-  TailVecs v[kMgMaxTail];
-  {
-    float* p = sm;
-    for (int l = 0; l < a.nl; l++) {
-      const int m = (a.L[l].n * (l == 0 ? NT : NC) + 3) & ~3;
-      v[l].b = p;
-      v[l].x = p + m;
-      v[l].y = p + 2 * m;
-      v[l].d = p + 3 * m;
-      p += 4 * m;
+  const int rank = EX ? (int)cluster_rank() : 0;
+  char* pat = reinterpret_cast<char*>(sm);
+  char* vals = pat + a.pat_bytes;
+  const bool copy = a.pat_bytes > 0;
+  const unsigned fill = (unsigned)__cvta_generic_to_shared(bars + 2);
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < 3; k++)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(bars + k)));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (copy) {
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fill),
+                   "r"(a.pat_bytes + a.val_bytes)
+                   : "memory");
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(pat)),
+                   "l"(a.pat), "r"(a.pat_bytes), "r"(fill)
+                   : "memory");
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(vals)),
+                   "l"(a.vals), "r"(a.val_bytes), "r"(fill)
+                   : "memory");
     }
   }
-  const int n0 = a.L[0].n * NT;
-  for (int t = threadIdx.x; t < n0; t += kTailT) v[0].b[t] = a.b[t];
-  __syncthreads();
+  sm += (a.pat_bytes + a.val_bytes) / sizeof(float);
+  // where the copies of a level's arrays stand (level 0 of a cluster is read through L1)
+  if (threadIdx.x < a.nl) {
+    const int l = threadIdx.x;
+    const MgLev& G = a.L[l];
+    const bool in = copy && !(EX && l == 0);
+    auto ip = [&](const void* p) {
+      return reinterpret_cast<const int32_t*>(in && p ? pat + (reinterpret_cast<const char*>(p) - a.pat) : p);
+    };
+    auto fp = [&](const float* p) {
+      return in && p ? reinterpret_cast<const float*>(vals + (reinterpret_cast<const char*>(p) - a.vals)) : p;
+    };
+    TailLev& S = lev[l];
+    S.sptr = ip(G.sptr);
+    S.col = ip(G.col);
+    S.p_sptr = ip(G.p_sptr);
+    S.p_col = ip(G.p_col);
+    S.pt_sptr = ip(G.pt_sptr);
+    S.pt_col = ip(G.pt_col);
+    S.val = fp(G.val);
+    S.p_val = fp(G.p_val);
+    S.pt_val = fp(G.pt_val);
+    S.coef = fp(G.coef);
+    S.to = G.to;
+    S.n = G.n;
+    S.nv = G.nv;
+    S.np = G.np;
+    S.npt = G.npt;
+  }
+  const float* dense =
+      copy ? reinterpret_cast<const float*>(vals + (reinterpret_cast<const char*>(a.dense) - a.vals)) : a.dense;
+  TailVecs v[kMgMaxTail];
+  for (int l = 0; l < a.nl; l++) {
+    const bool ex = EX && l == 0;
+    const int nb = l == 0 ? NT : NC, n = a.L[l].n, own = ex ? tail_chunk(n) : n;
+    v[l].x = sm;
+    v[l].y = sm + pad4(n * nb);
+    v[l].b = sm + 2 * pad4(n * nb);
+    v[l].d = v[l].b + pad4(own * nb);
+    v[l].r0 = ex ? min(n, rank * own) : 0;
+    v[l].r1 = ex ? min(n, rank * own + own) : n;
+    v[l].floats = ex ? nb * __ldg(a.L[l].cnt + rank) : 0;
+    sm += tail_floats(n, nb, ex);
+  }
+  TailSync sync{bars, tokens, rank, a.st};
+  const int n0 = a.L[0].n * NT, own0 = (v[0].r1 - v[0].r0) * NT, off0 = v[0].r0 * NT;
+  for (int t = threadIdx.x; t < n0; t += T) v[0].y[t] = a.b[t];
+  for (int t = threadIdx.x; t < own0; t += T) v[0].b[t] = a.b[off0 + t];
+  // (EX also: no block stores to another's shared memory before that block runs and has its barriers)
+  if (EX) cluster_barrier();
+  else __syncthreads();
+  auto filled = [&] {
+    if (!copy) return;
+    unsigned ok = 0;
+    for (int i = 0; i < (1 << 16) && !ok; i++)
+      asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\nselp.u32 %0, 1, 0, p;\n}"
+                   : "=r"(ok)
+                   : "r"(fill)
+                   : "memory");
+    if (!ok) a.st->done = 5;
+  };
   const int last = a.nl - 1;
   for (int rep = 0; rep < a.reps; rep++) {
-    for (int l = 0; l < last; l++) {
-      const int deg = a.st && l == 0 ? kMgDeg0 : kMgDeg;
-      if (l == 0) tail_down<NT, NC>(a.L[0], v[0], v[1], deg, rep == 0);
-      else tail_down<NC, NC>(a.L[l], v[l], v[l + 1], deg, true);
-    }
-    {
-      // coarsest: one warp per row of the dense inverse
-      const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-      const float* bb = v[last].b;
-      for (int r = wid; r < a.N; r += kTailT / 32) {
-        float s = 0.0f;
-        for (int k = lane; k < a.N; k += 32) s = fmaf(__ldg(a.dense + (int64_t)r * a.N + k), bb[k], s);
-        s = warp_sum(s);
-        if (lane == 0) v[last].x[r] = s;
+    if constexpr (!EX && NT == NC) {
+      if (rep == 0) filled();
+      tail_local<NC, T>(sync, lev, v, 0, last, a.dot, rep == 0, dense, a.N);
+    } else {
+      const TailLev& L = lev[0];
+      const int deg = a.dot ? kMgDeg0 : kMgDeg;
+      if (!EX && rep == 0) filled();
+      tail_smooth<EX, NT, T>(sync, L, v[0], deg, rep == 0, true);
+      TailVecs& c = v[1];
+      const int nc = lev[1].n;
+      if (EX) {
+        // coarse right-hand side: rows dealt in ranges, whole to every block
+        const int ch = tail_chunk(nc), c0 = min(nc, rank * ch), c1 = min(nc, c0 + ch);
+        sync.expect(nc * NC);
+        tail_transfer<true, NC, NT, T>(sync, L.pt_sptr, L.pt_col, L.pt_val, L.npt, nullptr, c0, c1,
+                                       tail_lanes(ch * NC, T), v[0].y, nullptr, c.y, nullptr);
+        for (int t = threadIdx.x; t < nc * NC; t += T) c.b[t] = c.y[t];
+        if (rep == 0) filled();
+        __syncthreads();
+      } else {
+        tail_transfer<false, NC, NT, T>(sync, L.pt_sptr, L.pt_col, L.pt_val, L.npt, nullptr, 0, c.r1,
+                                        tail_lanes(c.r1 * NC, T), v[0].y, nullptr, c.y, c.b);
       }
-      __syncthreads();
-    }
-    for (int l = last - 1; l >= 0; l--) {
-      const int deg = a.st && l == 0 ? kMgDeg0 : kMgDeg;
-      if (l == 0) tail_up<NT, NC>(a.L[0], v[0], v[1], deg);
-      else tail_up<NC, NC>(a.L[l], v[l], v[l + 1], deg);
+      tail_local<NC, T>(sync, lev, v, 1, last, 0, true, dense, a.N);
+      if (EX) sync.expect(v[0].floats);
+      tail_transfer<EX, NT, NC, T>(sync, L.p_sptr, L.p_col, L.p_val, L.np, L.to, v[0].r0, v[0].r1, 0, v[1].x, v[0].x,
+                                   v[0].y, nullptr);
+      float* s = v[0].x;
+      v[0].x = v[0].y;
+      v[0].y = s;
+      tail_smooth<EX, NT, T>(sync, L, v[0], deg, false, false);
     }
   }
   float dot = 0.0f;
-  for (int t = threadIdx.x; t < n0; t += kTailT) {
-    a.x[t] = v[0].x[t];
-    dot = fmaf(v[0].x[t], v[0].b[t], dot);
+  for (int t = threadIdx.x; t < own0; t += T) {
+    const float xi = v[0].x[off0 + t];
+    a.x[off0 + t] = xi;
+    dot = fmaf(xi, v[0].b[t], dot);
   }
-  if (a.st) {
+  if (a.dot) {
     float w[1] = {dot};
-    block_sum<float, 1, kTailT>(w);
-    if (threadIdx.x == 0 && !a.st->done) {
-      const double rz = (double)w[0] / a.st->ar;
+    block_sum<float, 1, T>(w);
+    if (EX) {
+      if (threadIdx.x == 0) store_rank(dots + rank, 0, w[0]);
+      cluster_barrier();
+    }
+    if (rank == 0 && threadIdx.x == 0 && !a.st->done) {
+      float tot = w[0];
+      if (EX) {
+        tot = 0.0f;
+        for (int k = 0; k < kTailC; k++) tot += dots[k];
+      }
+      const double rz = (double)tot / a.st->ar;  // (b carries the factor st->ar, and so does z)
       if (!(rz > 0.0) || !isfinite(rz)) {
         a.st->done = 2;
       } else {
@@ -478,7 +756,7 @@ __global__ void __launch_bounds__(kT) k_mg_vals0(int64_t n, const int32_t* __res
 #pragma unroll
       for (int q = 0; q < NB; q++)
         if (k % NB == q) rs[q] += v;
-      L.val[(nbase + 32 * (int64_t)(k / NB)) * (NB * NB) + c * NB + k % NB] = f;
+      L.val[block_at<NB, NB>(c * NB + k % NB, nbase + 32 * (int64_t)(k / NB), L.nv)] = f;
     }
   }
 #pragma unroll
@@ -507,10 +785,12 @@ __device__ __forceinline__ void tentative(const MgLev& L, int j, float (&T)[NB *
 
 // P = P0 - (1.6 / q) A P0 and the level's eigenvalue bound max q.  q: absolute row sums,
 // weighted by P0 for scalar operators (then exactly 2 where the row sums to zero with
-// non-positive off-diagonals, whatever the coefficients' jumps).
+// non-positive off-diagonals, whatever the coefficients' jumps).  One thread per node; the
+// loads of U neighbours are issued together (the kernel is a chain of dependent loads).
 template <int NB, int NC, bool D16, int BT>
 __global__ void __launch_bounds__(BT) k_mg_p(MgLev L) {
   __shared__ float acc[kMgMaxP * NB * NC][BT];
+  __shared__ int pc[kMgMaxP][BT];
   const int t = threadIdx.x;
   const int64_t i64 = gtid();
   float qmax = 0.0f;
@@ -521,34 +801,48 @@ __global__ void __launch_bounds__(BT) k_mg_p(MgLev L) {
     slice_row(L.p_sptr, i, pb, pw);
     slice_row(L.sptr, i, base, w);
     if (pw > kMgMaxP) pw = kMgMaxP;
+    for (int s = 0; s < pw; s++) pc[s][t] = __ldg(L.p_col + pb + 32 * (int64_t)s);
     for (int e = 0; e < pw * NB * NC; e++) acc[e][t] = 0.0f;
     float ti[NB], Ti[NB * NC], q[NB];
     tentative<NB, NC>(L, i, Ti, ti);
 #pragma unroll
     for (int c = 0; c < NB; c++) q[c] = 0.0f;
     const Cols<D16> cols(L, i);
-    for (int k = 0; k < w; k++) {
-      const int64_t idx = base + 32 * (int64_t)k;
-      int j = cols.at(k, idx);
-      if (!ADFEM_DCHECK(j >= 0 && j < L.n)) j = i;
-      const float* a = L.val + idx * (NB * NB);
-      float T[NB * NC], tj[NB];
-      tentative<NB, NC>(L, j, T, tj);
-      const int J = __ldg(L.agg + j);
-      int s = 0;
-      while (s < pw && __ldg(L.p_col + pb + 32 * (int64_t)s) != J) s++;
+    constexpr int U = NB == 1 ? 8 : 2;
+    for (int k0 = 0; k0 < w; k0 += U) {
+      int j[U], J[U];
+      float a[U][NB * NB], T[U][NB * NC], tj[U][NB];
 #pragma unroll
-      for (int c = 0; c < NB; c++) {
+      for (int u = 0; u < U; u++) {
+        j[u] = k0 + u < w ? cols.at(k0 + u, base + 32 * (int64_t)(k0 + u)) : i;
+        if (!ADFEM_DCHECK(j[u] >= 0 && j[u] < L.n)) j[u] = i;
+      }
 #pragma unroll
-        for (int e = 0; e < NB; e++) q[c] += NB == 1 ? fabsf(a[0]) * tj[0] : fabsf(a[c * NB + e]);
-        if (s < pw)
+      for (int u = 0; u < U; u++) {
+        J[u] = __ldg(L.agg + j[u]);
+        tentative<NB, NC>(L, j[u], T[u], tj[u]);
+        if (k0 + u < w) load_block<NB, NB>(L.val, base + 32 * (int64_t)(k0 + u), L.nv, a[u]);
+        else
 #pragma unroll
-          for (int m = 0; m < NC; m++) {
-            float v = 0.0f;
+          for (int e = 0; e < NB * NB; e++) a[u][e] = 0.0f;
+      }
 #pragma unroll
-            for (int e = 0; e < NB; e++) v = fmaf(a[c * NB + e], T[e * NC + m], v);
-            acc[s * NB * NC + c * NC + m][t] -= v;
-          }
+      for (int u = 0; u < U; u++) {
+        int s = 0;
+        while (s < pw && pc[s][t] != J[u]) s++;
+#pragma unroll
+        for (int c = 0; c < NB; c++) {
+#pragma unroll
+          for (int e = 0; e < NB; e++) q[c] += NB == 1 ? fabsf(a[u][0]) * tj[u][0] : fabsf(a[u][c * NB + e]);
+          if (s < pw)
+#pragma unroll
+            for (int m = 0; m < NC; m++) {
+              float v = 0.0f;
+#pragma unroll
+              for (int e = 0; e < NB; e++) v = fmaf(a[u][c * NB + e], T[u][e * NC + m], v);
+              acc[s * NB * NC + c * NC + m][t] -= v;
+            }
+        }
       }
     }
 #pragma unroll
@@ -557,17 +851,17 @@ __global__ void __launch_bounds__(BT) k_mg_p(MgLev L) {
       q[c] = fmaxf(q[c], 1.0f);
       qmax = fmaxf(qmax, q[c]);
     }
-    // (padding repeats column 0 behind the row's entries: the first match is the own aggregate)
+    // (padding repeats the first column behind the row's entries: the first match is the own aggregate)
     const int Ji = __ldg(L.agg + i);
     int own = 0;
-    while (own < pw && __ldg(L.p_col + pb + 32 * (int64_t)own) != Ji) own++;
+    while (own < pw && pc[own][t] != Ji) own++;
     for (int s = 0; s < pw; s++)
 #pragma unroll
       for (int c = 0; c < NB; c++) {
         const float f = ti[c] > 0.0f ? kSmoothP / q[c] : 0.0f;
 #pragma unroll
         for (int m = 0; m < NC; m++)
-          L.p_val[(pb + 32 * (int64_t)s) * (NB * NC) + c * NC + m] =
+          L.p_val[block_at<NB, NC>(c * NC + m, pb + 32 * (int64_t)s, L.np)] =
               f * acc[s * NB * NC + c * NC + m][t] + (s == own ? Ti[c * NC + m] : 0.0f);
       }
   }
@@ -577,10 +871,11 @@ __global__ void __launch_bounds__(BT) k_mg_p(MgLev L) {
   if ((t & 31) == 0) atomicMax(L.lam, __float_as_int(qmax));
 }
 
-// rows of A P
+// rows of A P, one thread per node: the P rows of U neighbours are walked side by side
 template <int NB, int NC, bool D16, int BT>
 __global__ void __launch_bounds__(BT) k_mg_ap(MgLev L) {
   __shared__ float acc[kMgMaxAP * NB * NC][BT];
+  __shared__ int ac[kMgMaxAP][BT];
   const int t = threadIdx.x;
   const int64_t i64 = gtid();
   if (i64 >= L.n) return;
@@ -590,54 +885,75 @@ __global__ void __launch_bounds__(BT) k_mg_ap(MgLev L) {
   slice_row(L.ap_sptr, i, ab, aw);
   slice_row(L.sptr, i, base, w);
   if (aw > kMgMaxAP) aw = kMgMaxAP;
+  for (int s = 0; s < aw; s++) ac[s][t] = __ldg(L.ap_col + ab + 32 * (int64_t)s);
   for (int e = 0; e < aw * NB * NC; e++) acc[e][t] = 0.0f;
   const Cols<D16> cols(L, i);
-  for (int k = 0; k < w; k++) {
-    const int64_t idx = base + 32 * (int64_t)k;
-    int j = cols.at(k, idx);
-    if (!ADFEM_DCHECK(j >= 0 && j < L.n)) j = i;
-    float a[NB * NB];
-    bool any = false;
+  constexpr int U = NB == 1 ? 8 : 2;
+  for (int k0 = 0; k0 < w; k0 += U) {
+    int j[U], pw[U], pm = 0;
+    int64_t pb[U];
+    float a[U][NB * NB];
 #pragma unroll
-    for (int e = 0; e < NB * NB; e++) {
-      a[e] = L.val[idx * (NB * NB) + e];
-      any |= a[e] != 0.0f;
+    for (int u = 0; u < U; u++) {
+      j[u] = k0 + u < w ? cols.at(k0 + u, base + 32 * (int64_t)(k0 + u)) : i;
+      if (!ADFEM_DCHECK(j[u] >= 0 && j[u] < L.n)) j[u] = i;
     }
-    if (!any) continue;
-    int64_t pb;
-    int pw;
-    slice_row(L.p_sptr, j, pb, pw);
-    for (int p = 0; p < pw; p++) {
-      const int64_t pe = pb + 32 * (int64_t)p;
-      const int K = __ldg(L.p_col + pe);
-      int s = 0;
-      while (s < aw && __ldg(L.ap_col + ab + 32 * (int64_t)s) != K) s++;
-      if (s == aw) continue;
-      float v[NB * NC];
 #pragma unroll
-      for (int e = 0; e < NB * NC; e++) v[e] = L.p_val[pe * (NB * NC) + e];
+    for (int u = 0; u < U; u++) {
+      slice_row(L.p_sptr, j[u], pb[u], pw[u]);
+      if (k0 + u < w) load_block<NB, NB>(L.val, base + 32 * (int64_t)(k0 + u), L.nv, a[u]);
+      else
 #pragma unroll
-      for (int c = 0; c < NB; c++)
+        for (int e = 0; e < NB * NB; e++) a[u][e] = 0.0f;
+      bool any = false;
 #pragma unroll
-        for (int m = 0; m < NC; m++) {
-          float x = acc[s * NB * NC + c * NC + m][t];
+      for (int e = 0; e < NB * NB; e++) any |= a[u][e] != 0.0f;
+      if (!any) pw[u] = 0;
+      pm = max(pm, pw[u]);
+    }
+    for (int p = 0; p < pm; p++) {
+      int K[U];
+      float v[U][NB * NC];
 #pragma unroll
-          for (int e = 0; e < NB; e++) x = fmaf(a[c * NB + e], v[e * NC + m], x);
-          acc[s * NB * NC + c * NC + m][t] = x;
+      for (int u = 0; u < U; u++) {
+        K[u] = -1;
+        if (p < pw[u]) {
+          const int64_t pe = pb[u] + 32 * (int64_t)p;
+          K[u] = __ldg(L.p_col + pe);
+          load_block<NB, NC>(L.p_val, pe, L.np, v[u]);
         }
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (K[u] < 0) continue;
+        int s = 0;
+        while (s < aw && ac[s][t] != K[u]) s++;
+        if (s == aw) continue;
+#pragma unroll
+        for (int c = 0; c < NB; c++)
+#pragma unroll
+          for (int m = 0; m < NC; m++) {
+            float x = acc[s * NB * NC + c * NC + m][t];
+#pragma unroll
+            for (int e = 0; e < NB; e++) x = fmaf(a[u][c * NB + e], v[u][e * NC + m], x);
+            acc[s * NB * NC + c * NC + m][t] = x;
+          }
+      }
     }
   }
   for (int s = 0; s < aw; s++)
 #pragma unroll
     for (int e = 0; e < NB * NC; e++)
-      L.ap_val[(ab + 32 * (int64_t)s) * (NB * NC) + e] = acc[s * NB * NC + e][t];
+      L.ap_val[block_at<NB, NC>(e, ab + 32 * (int64_t)s, L.nap)] = acc[s * NB * NC + e][t];
 }
 
-// Coarse rows P^T (A P), one warp per row: lane k owns entries k and k + 32 of the row and
-// picks its terms from the walk over the row's nodes (in ascending order).
+// Coarse rows P^T (A P), one warp per row, one lane per node of the row's column of P: the
+// lanes load their nodes' rows of A P together, then each entry of the coarse row is the sum
+// over the lanes of the one term (if any) that each contributes, by a fixed shuffle tree.
 template <int NB, int NC>
 __global__ void __launch_bounds__(128) k_mg_ac(MgLev L, MgLev C) {
-  const int lane = threadIdx.x & 31;
+  __shared__ int kk[4][kMgMaxAP][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t J64 = gtid() >> 5;
   if (J64 >= L.nc) return;
   const int J = (int)J64;
@@ -652,37 +968,52 @@ __global__ void __launch_bounds__(128) k_mg_ac(MgLev L, MgLev C) {
   for (int h = 0; h < 2; h++) {
     const int k = lane + 32 * h;
     K[h] = k < cw ? __ldg(ccol + cb + 32 * (int64_t)k) : -1;
-    // (padding repeats column 0 behind the row's entries: the first match owns the sum)
-    if (k > 0 && K[h] == 0) K[h] = -1;
+    // (padding repeats the first column behind the row's entries: the first match owns the sum)
+    if (k > 0 && K[h] == __ldg(ccol + cb)) K[h] = -1;
 #pragma unroll
     for (int e = 0; e < NC * NC; e++) acc[h][e] = 0.0f;
   }
-  for (int q = 0; q < tw; q++) {
-    const int src = __ldg(L.pt_src + tb + 32 * (int64_t)q);
-    if (src < 0) continue;
-    const int i = __ldg(L.pt_col + tb + 32 * (int64_t)q);
+  for (int q0 = 0; q0 < tw; q0 += 32) {
+    const int q = q0 + lane;
+    const int src = q < tw ? __ldg(L.pt_src + tb + 32 * (int64_t)q) : -1;
+    int64_t ab = 0;
+    int aw = 0;
     float p[NB * NC];
-#pragma unroll
-    for (int e = 0; e < NB * NC; e++) p[e] = L.p_val[(int64_t)src * (NB * NC) + e];
-    int64_t ab;
-    int aw;
-    slice_row(L.ap_sptr, i, ab, aw);
-    for (int s = 0; s < aw; s++) {
-      const int64_t ae = ab + 32 * (int64_t)s;
-      const int k = __ldg(L.ap_col + ae);
-#pragma unroll
-      for (int h = 0; h < 2; h++)
-        if (k == K[h]) {
-#pragma unroll
-          for (int e = 0; e < NB; e++)
-#pragma unroll
-            for (int m = 0; m < NC; m++) {
-              const float v = L.ap_val[ae * (NB * NC) + e * NC + m];
-#pragma unroll
-              for (int c = 0; c < NC; c++) acc[h][c * NC + m] = fmaf(p[e * NC + c], v, acc[h][c * NC + m]);
-            }
-        }
+    if (src >= 0) {
+      slice_row(L.ap_sptr, __ldg(L.pt_col + tb + 32 * (int64_t)q), ab, aw);
+      if (aw > kMgMaxAP) aw = kMgMaxAP;
+      load_block<NB, NC>(L.p_val, src, L.np, p);
+#pragma unroll 4
+      for (int s = 0; s < aw; s++) kk[wid][s][lane] = __ldg(L.ap_col + ab + 32 * (int64_t)s);
     }
+    __syncwarp();
+    for (int k = 0; k < cw; k++) {
+      const int col = __shfl_sync(0xffffffffu, k < 32 ? K[0] : K[1], k & 31);
+      if (col < 0) continue;
+      float v[NB * NC], T[NC * NC];
+      int s = 0;
+      while (s < aw && kk[wid][s][lane] != col) s++;
+      if (s < aw) load_block<NB, NC>(L.ap_val, ab + 32 * (int64_t)s, L.nap, v);
+#pragma unroll
+      for (int c = 0; c < NC; c++)
+#pragma unroll
+        for (int m = 0; m < NC; m++) {
+          float x = 0.0f;
+          if (s < aw)
+#pragma unroll
+            for (int e = 0; e < NB; e++) x = fmaf(p[e * NC + c], v[e * NC + m], x);
+          T[c * NC + m] = x;
+        }
+#pragma unroll
+      for (int e = 0; e < NC * NC; e++) {
+        const float x = warp_sum(T[e]);
+        if (lane == (k & 31)) {
+          if (k < 32) acc[0][e] += x;
+          else acc[1][e] += x;
+        }
+      }
+    }
+    __syncwarp();
   }
 #pragma unroll
   for (int h = 0; h < 2; h++) {
@@ -690,7 +1021,7 @@ __global__ void __launch_bounds__(128) k_mg_ac(MgLev L, MgLev C) {
     if (k >= cw) continue;
 #pragma unroll
     for (int e = 0; e < NC * NC; e++)
-      C.val[(cb + 32 * (int64_t)k) * (NC * NC) + e] = K[h] >= 0 ? acc[h][e] : 0.0f;
+      C.val[block_at<NC, NC>(e, cb + 32 * (int64_t)k, C.nv)] = K[h] >= 0 ? acc[h][e] : 0.0f;
     if (K[h] == J)
 #pragma unroll
       for (int c = 0; c < NC; c++) {
@@ -700,37 +1031,49 @@ __global__ void __launch_bounds__(128) k_mg_ac(MgLev L, MgLev C) {
   }
 }
 
-// unit diagonal: A_JK <- s_J A_JK s_K (1 on the diagonal of unknowns without a scale), and
-// the interpolation in those unknowns, P <- P S, with its transpose
+// Unit diagonal: A_JK <- s_J A_JK s_K (1 on the diagonal of unknowns without a scale), and
+// the interpolation in those unknowns, P <- P S, with its transpose.  One warp per coarse row.
+// The first thread also turns the level's eigenvalue bound into the Chebyshev coefficients:
+// 1 / theta, then (c1, c2) of step k at 2k, 2k + 1.
 template <int NB, int NC>
-__global__ void __launch_bounds__(128) k_mg_scale(MgLev L, MgLev C) {
-  const int64_t J64 = gtid();
+__global__ void __launch_bounds__(128) k_mg_scale(MgLev L, MgLev C, int deg, float frac) {
+  const int lane = threadIdx.x & 31;
+  const int64_t J64 = gtid() >> 5;
+  if (gtid() == 0) {
+    const float hi = __int_as_float(*L.lam), lo = frac * hi;
+    const float th = 0.5f * (hi + lo), de = 0.5f * (hi - lo), s1 = th / de;
+    float rho = 1.0f / s1;
+    L.coef[0] = 1.0f / th;
+    for (int k = 1; k < deg; k++) {
+      const float rn = 1.0f / (2.0f * s1 - rho);
+      L.coef[2 * k] = rn * rho;
+      L.coef[2 * k + 1] = 2.0f * rn / de;
+      rho = rn;
+    }
+  }
   if (J64 >= L.nc) return;
   const int J = (int)J64;
   float sJ[NC];
 #pragma unroll
-  for (int c = 0; c < NC; c++) sJ[c] = C.s[(int64_t)NC * J + c];
+  for (int c = 0; c < NC; c++) sJ[c] = __ldg(C.s + (int64_t)NC * J + c);
   int64_t base;
   int w;
   slice_row(C.sptr, J, base, w);
   const int32_t* ccol = reinterpret_cast<const int32_t*>(C.col);
-  bool diag = false;
-  for (int k = 0; k < w; k++) {
+  for (int k = lane; k < w; k += 32) {
     const int64_t e = base + 32 * (int64_t)k;
     const int K = __ldg(ccol + e);
-    const bool own = K == J && !diag;
-    diag |= own;
+    const bool own = K == J && (k == 0 || K != __ldg(ccol + base));  // (padding repeats the first column)
 #pragma unroll
     for (int c = 0; c < NC; c++)
 #pragma unroll
       for (int m = 0; m < NC; m++) {
-        float* v = C.val + e * (NC * NC) + c * NC + m;
-        const float sk = C.s[(int64_t)NC * K + m];
-        *v = own && c == m ? 1.0f : *v * (sJ[c] * sk);
+        float* v = C.val + block_at<NC, NC>(c * NC + m, e, C.nv);
+        *v = own && c == m ? 1.0f : *v * (sJ[c] * __ldg(C.s + (int64_t)NC * K + m));
       }
   }
   slice_row(L.pt_sptr, J, base, w);
-  for (int q = 0; q < w; q++) {
+  for (int q = lane; q < w; q += 32) {
     const int64_t e = base + 32 * (int64_t)q;
     const int64_t src = __ldg(L.pt_src + e);
     if (src < 0) continue;
@@ -738,71 +1081,90 @@ __global__ void __launch_bounds__(128) k_mg_scale(MgLev L, MgLev C) {
     for (int r = 0; r < NB; r++)
 #pragma unroll
       for (int c = 0; c < NC; c++) {
-        const float v = L.p_val[src * (NB * NC) + r * NC + c] * sJ[c];
-        L.p_val[src * (NB * NC) + r * NC + c] = v;
-        L.pt_val[e * (NB * NC) + c * NB + r] = v;
+        float* pv = L.p_val + block_at<NB, NC>(r * NC + c, src, L.np);
+        const float v = *pv * sJ[c];
+        *pv = v;
+        L.pt_val[block_at<NC, NB>(c * NB + r, e, L.npt)] = v;
       }
   }
 }
 
-// Chebyshev coefficients of one level: 1 / theta, then (c1, c2) of step k at 2k, 2k + 1
-__global__ void k_mg_coef(MgLev L, int deg, float frac) {
-  if (threadIdx.x || blockIdx.x) return;
-  const float hi = __int_as_float(*L.lam), lo = frac * hi;
-  const float th = 0.5f * (hi + lo), de = 0.5f * (hi - lo), s1 = th / de;
-  float rho = 1.0f / s1;
-  L.coef[0] = 1.0f / th;
-  for (int k = 1; k < deg; k++) {
-    const float rn = 1.0f / (2.0f * s1 - rho);
-    L.coef[2 * k] = rn * rho;
-    L.coef[2 * k + 1] = 2.0f * rn / de;
-    rho = rn;
-  }
-}
-
-// Inverse of the coarsest operator (N <= kMgDense, unit diagonal) by Gauss-Jordan in shared
-// memory; a pivot at rounding level (a near-null space the Dirichlet data leave in) drops its
-// unknown from the inverse, which stays symmetric positive semi-definite.
+// Inverse of the coarsest operator (N <= kMgDense, unit diagonal) by Gauss-Jordan in one block
+// of 32 x 32 threads, each holding the entries (ty + 32 a, tx + 32 b) in registers; a step
+// exchanges the pivot row and column through shared memory (one barrier).  A pivot at rounding
+// level (a near-null space the Dirichlet data leave in) drops its unknown from the inverse,
+// which stays symmetric positive semi-definite.
 template <int NC>
-__global__ void __launch_bounds__(kTailT) k_mg_dense(MgLev C, float* __restrict__ inv) {
+__global__ void __launch_bounds__(1024) k_mg_dense(MgLev C, float* __restrict__ inv) {
+  constexpr int S = kMgDense / 32;
+  static_assert(kMgDense % 32 == 0, "whole tiles");
   extern __shared__ float4 dense_sm4[];
-  float* A = reinterpret_cast<float*>(dense_sm4);
+  float* A = reinterpret_cast<float*>(dense_sm4);  // N x N, then two pivot rows and columns
   const int N = C.n * NC;
-  float* f = A + N * N;  // the pivot column
+  float* piv = A + N * N;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   for (int t = threadIdx.x; t < N * N; t += blockDim.x) A[t] = 0.0f;
   __syncthreads();
   const int32_t* col = reinterpret_cast<const int32_t*>(C.col);
-  for (int t = threadIdx.x; t < C.n; t += blockDim.x) {
+  for (int r = ty; r < C.n; r += 32) {
     int64_t base;
     int w;
-    slice_row(C.sptr, t, base, w);
-    for (int k = 0; k < w; k++) {
+    slice_row(C.sptr, r, base, w);
+    for (int k = tx; k < w; k += 32) {
       const int64_t e = base + 32 * (int64_t)k;
       const int K = col[e];
+      if (k > 0 && K == col[base]) continue;  // (padding)
       for (int c = 0; c < NC; c++)
-        for (int m = 0; m < NC; m++) A[(t * NC + c) * N + K * NC + m] += C.val[e * (NC * NC) + c * NC + m];
+        for (int m = 0; m < NC; m++)
+          A[(r * NC + c) * N + K * NC + m] = C.val[block_at<NC, NC>(c * NC + m, e, C.nv)];
     }
   }
   __syncthreads();
-  for (int k = 0; k < N; k++) {
-    const float p = A[k * N + k];
-    const float ip = p > 1e-5f ? 1.0f / p : 0.0f;
-    for (int t = threadIdx.x; t < N; t += blockDim.x) f[t] = A[t * N + k];
-    __syncthreads();
-    for (int t = threadIdx.x; t < N; t += blockDim.x) A[k * N + t] = t == k ? ip : A[k * N + t] * ip;
-    __syncthreads();
-    for (int t = threadIdx.x; t < N * N; t += blockDim.x) {
-      const int r = t / N, c = t - r * N;
-      if (r == k) continue;
-      A[t] = c == k ? -f[r] * ip : fmaf(-f[r], A[k * N + c], A[t]);
+  float x[S][S];
+#pragma unroll
+  for (int a = 0; a < S; a++)
+#pragma unroll
+    for (int b = 0; b < S; b++) {
+      const int r = ty + 32 * a, c = tx + 32 * b;
+      x[a][b] = r < N && c < N ? A[r * N + c] : 0.0f;
     }
+  for (int k = 0; k < N; k++) {
+    float* row = piv + (k & 1) * 2 * kMgDense;
+    float* cl = row + kMgDense;
+#pragma unroll
+    for (int a = 0; a < S; a++)
+#pragma unroll
+      for (int b = 0; b < S; b++) {
+        if (ty + 32 * a == k) row[tx + 32 * b] = x[a][b];
+        if (tx + 32 * b == k) cl[ty + 32 * a] = x[a][b];
+      }
     __syncthreads();
+    const float p = row[k];
+    const float ip = p > 1e-5f ? 1.0f / p : 0.0f;
+#pragma unroll
+    for (int a = 0; a < S; a++) {
+      const int r = ty + 32 * a;
+      const float f = cl[r];
+#pragma unroll
+      for (int b = 0; b < S; b++) {
+        const int c = tx + 32 * b;
+        const float s = c == k ? ip : row[c] * ip;  // the scaled pivot row
+        x[a][b] = r == k ? s : (c == k ? -f * ip : fmaf(-f, s, x[a][b]));
+      }
+    }
   }
+  __syncthreads();
+#pragma unroll
+  for (int a = 0; a < S; a++)
+#pragma unroll
+    for (int b = 0; b < S; b++) {
+      const int r = ty + 32 * a, c = tx + 32 * b;
+      if (r < N && c < N) A[r * N + c] = x[a][b];
+    }
+  __syncthreads();
   // (symmetrised: the cycle has to be symmetric)
-  for (int t = threadIdx.x; t < N * N; t += blockDim.x) {
-    const int r = t / N, c = t - r * N;
-    inv[t] = 0.5f * (A[t] + A[c * N + r]);
-  }
+  for (int r = ty; r < N; r += 32)
+    for (int c = tx; c < N; c += 32) inv[r * N + c] = 0.5f * (A[r * N + c] + A[c * N + r]);
 }
 
 // ---------------------------------------------------------------------------
@@ -995,6 +1357,10 @@ struct Slab {
     std::memcpy(host.data() + off, v.data(), sizeof(T) * v.size());
     fix.emplace_back((void**)p, off);
   }
+  size_t mark() {
+    host.resize((host.size() + 255) / 256 * 256);
+    return host.size();
+  }
   void seal() { total = (host.size() + 255) / 256 * 256; }
   template <class T>
   void room(T** p, size_t count) {
@@ -1006,7 +1372,7 @@ struct Slab {
   }
 };
 
-// slices of 32 rows with absolute columns (padding: column 0)
+// slices of 32 rows with absolute columns (padding: the row's first column)
 void slices(int64_t n, const MgPattern& P, std::vector<int32_t>& sptr, std::vector<int32_t>& col) {
   const int64_t ns = (n + 31) / 32;
   sptr.assign(ns + 1, 0);
@@ -1016,19 +1382,33 @@ void slices(int64_t n, const MgPattern& P, std::vector<int32_t>& sptr, std::vect
     sptr[s + 1] = sptr[s] + 32 * w;
   }
   col.assign(std::max<int32_t>(sptr[ns], 1), 0);
-  for (int64_t r = 0; r < n; r++)
-    for (int32_t k = P.rp[r]; k < P.rp[r + 1]; k++) col[sptr[r >> 5] + 32 * (k - P.rp[r]) + (r & 31)] = P.ci[k];
+  for (int64_t r = 0; r < n; r++) {
+    const int32_t len = P.rp[r + 1] - P.rp[r], w = (sptr[(r >> 5) + 1] - sptr[r >> 5]) / 32;
+    for (int32_t k = 0; k < w; k++)
+      col[sptr[r >> 5] + 32 * k + (r & 31)] = len ? P.ci[P.rp[r] + (k < len ? k : 0)] : 0;
+  }
+}
+
+// Tail blocks that need each row's value of the tail's first level: those that own a row that
+// refers to it in A (sweeps) or a coarse row whose restriction reads it; cnt: how many rows each
+// block needs.
+void tail_targets(const MgHostLevel& H, int64_t nc, std::vector<uint8_t>& to, std::vector<int32_t>& cnt) {
+  to.assign(H.n, 0);
+  auto owner = [](int64_t r, int64_t n) { return (int)(r / tail_chunk((int)n)); };
+  for (int64_t r = 0; r < H.n; r++)
+    for (int32_t k = H.A.rp[r]; k < H.A.rp[r + 1]; k++) to[H.A.ci[k]] |= (uint8_t)(1 << owner(r, H.n));
+  for (int64_t i = 0; i < H.n; i++)
+    for (int32_t k = H.P.rp[i]; k < H.P.rp[i + 1]; k++) to[i] |= (uint8_t)(1 << owner(H.P.ci[k], nc));
+  cnt.assign(kTailC, 0);
+  for (uint8_t m : to)
+    for (int k = 0; k < kTailC; k++) cnt[k] += (m >> k) & 1;
 }
 
 int lanes_per_row(int64_t n) {
   // one lane while the rows alone fill the chip (152 SMs x 2048 threads), more below
   return n >= 150000 ? 1 : (n >= 40000 ? 4 : 8);
 }
-int tail_lanes(int64_t n) {
-  int l = 1;
-  while (l < 8 && 2 * l * n <= kTailT) l *= 2;
-  return l;
-}
+
 
 }  // namespace
 
@@ -1057,14 +1437,17 @@ int mg_plan(Solver& S) {
   Mg& M = *mg;
   M.nlev = (int)lv.size();
   while (M.tail < M.nlev - 1 && lv[M.tail].n * (M.tail ? nbc : nb0) > kMgTailDofs) M.tail++;
-  if (M.nlev < 2 || M.nlev - M.tail > kMgMaxTail) {
+  M.cluster = lv[M.tail].n * (M.tail ? nbc : nb0) > kTailLocal;
+  if (M.nlev < 2 || M.nlev - M.tail > kMgMaxTail || M.tail + 1 >= M.nlev) {
     S.mg_allowed = false;
     return ADFEM_OK;
   }
   const Sell& A = *S.A;
   Slab sl;
-  std::vector<int32_t> sptr, col;
-  std::vector<int64_t> vals(M.nlev), pv(M.nlev), apv(M.nlev), ptv(M.nlev);
+  std::vector<int32_t> sptr, col, cnt;
+  std::vector<uint8_t> to;
+  std::vector<int64_t> vals(M.nlev);
+  const int local = M.tail + (M.cluster ? 1 : 0);  // first level that a tail block runs alone
   for (int l = 0; l < M.nlev; l++) {
     MgLev& L = M.lev[l];
     MgHostLevel& H = lv[l];
@@ -1072,8 +1455,37 @@ int mg_plan(Solver& S) {
     L.nb = l ? nbc : nb0;
     L.nbc = nbc;
     const bool tail = l >= M.tail;
-    L.lpr = tail ? tail_lanes(H.n) : lanes_per_row(H.n);
-    if (l == 0) L.lpr = tail ? L.lpr : (nb0 == 1 ? 1 : (H.n >= 150000 ? 1 : 4));
+    L.lpr = l == 0 ? (nb0 == 1 || H.n >= 150000 ? 1 : 4) : lanes_per_row(H.n);
+    if (l == M.tail && M.cluster) {
+      tail_targets(lv[l], lv[l + 1].n, to, cnt);
+      sl.put(&L.to, to);
+      sl.put(&L.cnt, cnt);
+    }
+    if (l + 1 < M.nlev) {
+      L.nc = (int)lv[l + 1].n;
+      // (what only the value kernels read comes before the range that the tail copies)
+      slices(H.n, H.AP, sptr, col);
+      sl.put(&L.ap_sptr, sptr);
+      sl.put(&L.ap_col, col);
+      L.nap = sptr.back();
+      slices(H.n, H.P, sptr, col);
+      const std::vector<int32_t> psptr = sptr;
+      slices(L.nc, H.PT, sptr, col);
+      std::vector<int32_t> src(col.size(), -1);
+      for (int64_t J = 0; J < L.nc; J++)
+        for (int32_t k = H.PT.rp[J]; k < H.PT.rp[J + 1]; k++) {
+          const int32_t i = H.PT.ci[k];
+          src[sptr[J >> 5] + 32 * (k - H.PT.rp[J]) + (J & 31)] = psptr[i >> 5] + 32 * H.PTslot[k] + (i & 31);
+        }
+      sl.put(&L.pt_src, src);
+      sl.put(&L.agg, H.agg);
+      if (nbc == 3) {
+        std::vector<float2> dp(H.n);
+        for (int64_t i = 0; i < H.n; i++)
+          dp[i] = make_float2((float)(H.x[i] - lv[l + 1].x[H.agg[i]]), (float)(H.y[i] - lv[l + 1].y[H.agg[i]]));
+        sl.put(&L.dpos, dp);
+      }
+    }
     if (l == 0 && nb0 == 1 && !tail) {
       // the system's own pattern
       L.sptr = A.sptr.as<int32_t>();
@@ -1082,87 +1494,89 @@ int mg_plan(Solver& S) {
       L.pat = A.pat.as<int16_t>();
       L.d16 = A.delta16 ? 1 : 0;
       vals[l] = A.nent;
-    } else {
+    }
+  }
+  size_t pat0 = 0, val0 = 0;
+  for (int l = 0; l < M.nlev; l++) {
+    MgLev& L = M.lev[l];
+    MgHostLevel& H = lv[l];
+    if (l == local) pat0 = sl.mark();
+    if (!(l == 0 && nb0 == 1 && M.tail > 0)) {
       slices(H.n, H.A, sptr, col);
       sl.put(&L.sptr, sptr);
       sl.put((const int32_t**)&L.col, col);
       vals[l] = sptr.back();
     }
+    L.nv = (int)vals[l];
     if (l + 1 == M.nlev) continue;
-    L.nc = (int)lv[l + 1].n;
     slices(H.n, H.P, sptr, col);
     sl.put(&L.p_sptr, sptr);
     sl.put(&L.p_col, col);
-    pv[l] = sptr.back();
-    const std::vector<int32_t> psptr = sptr;
-    slices(H.n, H.AP, sptr, col);
-    sl.put(&L.ap_sptr, sptr);
-    sl.put(&L.ap_col, col);
-    apv[l] = sptr.back();
+    L.np = sptr.back();
     slices(L.nc, H.PT, sptr, col);
     sl.put(&L.pt_sptr, sptr);
     sl.put(&L.pt_col, col);
-    ptv[l] = sptr.back();
-    std::vector<int32_t> src(col.size(), -1);
-    for (int64_t J = 0; J < L.nc; J++)
-      for (int32_t k = H.PT.rp[J]; k < H.PT.rp[J + 1]; k++) {
-        const int32_t i = H.PT.ci[k];
-        src[sptr[J >> 5] + 32 * (k - H.PT.rp[J]) + (J & 31)] = psptr[i >> 5] + 32 * H.PTslot[k] + (i & 31);
-      }
-    sl.put(&L.pt_src, src);
-    sl.put(&L.agg, H.agg);
-    if (nbc == 3) {
-      std::vector<float2> dp(H.n);
-      for (int64_t i = 0; i < H.n; i++)
-        dp[i] = make_float2((float)(H.x[i] - lv[l + 1].x[H.agg[i]]), (float)(H.y[i] - lv[l + 1].y[H.agg[i]]));
-      sl.put(&L.dpos, dp);
-    }
+    L.npt = sptr.back();
   }
   sl.seal();
+  M.pat_bytes = (int)(sl.total - pat0);
   for (int l = 0; l < M.nlev; l++) {
     MgLev& L = M.lev[l];
     const size_t nb = L.nb, n = (size_t)L.n * nb;
-    sl.room(&L.val, (size_t)vals[l] * nb * nb);
     sl.room(&L.s, n);
     sl.room(&L.b, n);
     sl.room(&L.x, n);
     sl.room(&L.x2, n);
     sl.room(&L.d, n);
+    if (l + 1 < M.nlev) sl.room(&L.ap_val, (size_t)L.nap * nb * nbc);
+  }
+  sl.room(&M.rowsum, (size_t)S.n * nb0);
+  sl.room(&M.lam, kMgMaxLevels);
+  for (int l = 0; l < M.nlev; l++) {
+    MgLev& L = M.lev[l];
+    const size_t nb = L.nb;
+    if (l == local) val0 = sl.total;
+    sl.room(&L.val, (size_t)vals[l] * nb * nb);
     sl.room(&L.coef, kCoef + 2);
-    sl.room(&L.lam, 1);
     if (l + 1 == M.nlev) continue;
-    sl.room(&L.p_val, (size_t)pv[l] * nb * nbc);
-    sl.room(&L.ap_val, (size_t)apv[l] * nb * nbc);
-    sl.room(&L.pt_val, (size_t)ptv[l] * nb * nbc);
+    sl.room(&L.p_val, (size_t)L.np * nb * nbc);
+    sl.room(&L.pt_val, (size_t)L.npt * nb * nbc);
   }
   M.ndense = M.lev[M.nlev - 1].n * M.lev[M.nlev - 1].nb;
   sl.room(&M.dense, (size_t)M.ndense * M.ndense);
-  sl.room(&M.rowsum, (size_t)S.n * nb0);
+  M.val_bytes = (int)(sl.total - val0);
   ADFEM_TRY(M.slab.alloc(sl.total));
   sl.resolve(M.slab.as<char>());
+  for (int l = 0; l < M.nlev; l++) M.lev[l].lam = M.lam + l;
   ADFEM_CUDA(cudaMemcpy(M.slab.p, sl.host.data(), sl.host.size(), cudaMemcpyHostToDevice));
   ADFEM_CUDA(cudaMemset(M.slab.as<char>() + sl.host.size(), 0, sl.total - sl.host.size()));
   // (legacy-stream sync, not a device-wide one: other threads may be capturing graphs)
   ADFEM_CUDA(cudaStreamSynchronize(0));
   size_t fl = 0;
-  for (int l = M.tail; l < M.nlev; l++) fl += 4 * (((size_t)M.lev[l].n * M.lev[l].nb + 3) / 4 * 4);
+  for (int l = M.tail; l < M.nlev; l++) fl += (size_t)tail_floats(M.lev[l].n, M.lev[l].nb, M.cluster && l == M.tail);
   M.tail_smem = sizeof(float) * fl;
+  M.pat = M.slab.as<char>() + pat0;
+  M.vals = M.slab.as<char>() + val0;
+  if (M.tail_smem + M.pat_bytes + M.val_bytes > kTailSmem) M.pat_bytes = M.val_bytes = 0;  // read through L1
+  M.tail_smem += M.pat_bytes + M.val_bytes;
   {
     // (once per process: changing a kernel attribute while another thread captures that
     // kernel would invalidate the capture)
     static std::once_flag once;
     static cudaError_t err = cudaSuccess;
     std::call_once(once, [] {
-      const int tmax = (int)(sizeof(float) * 4 * (2 * kMgTailDofs + 64));
-      const int dmax = (int)(sizeof(float) * (kMgDense * kMgDense + kMgDense));
+      const int tmax = (int)kTailSmem;
+      const int dmax = (int)(sizeof(float) * (kMgDense * kMgDense + 4 * kMgDense));
       const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-      for (cudaError_t e : {cudaFuncSetAttribute(k_mg_tail<1, 1>, a, tmax), cudaFuncSetAttribute(k_mg_tail<2, 3>, a, tmax),
-                            cudaFuncSetAttribute(k_mg_tail<3, 3>, a, tmax), cudaFuncSetAttribute(k_mg_dense<1>, a, dmax),
-                            cudaFuncSetAttribute(k_mg_dense<3>, a, dmax)})
+      for (cudaError_t e :
+           {cudaFuncSetAttribute(k_mg_tail<1, 1, false>, a, tmax), cudaFuncSetAttribute(k_mg_tail<2, 3, false>, a, tmax),
+            cudaFuncSetAttribute(k_mg_tail<3, 3, false>, a, tmax), cudaFuncSetAttribute(k_mg_tail<1, 1, true>, a, tmax),
+            cudaFuncSetAttribute(k_mg_tail<2, 3, true>, a, tmax), cudaFuncSetAttribute(k_mg_tail<3, 3, true>, a, tmax),
+            cudaFuncSetAttribute(k_mg_dense<1>, a, dmax), cudaFuncSetAttribute(k_mg_dense<3>, a, dmax)})
         if (e != cudaSuccess) err = e;
     });
     if (err != cudaSuccess) return cuda_fail(err, "cudaFuncSetAttribute (multigrid)");
-    if (M.tail_smem > sizeof(float) * 4 * (2 * kMgTailDofs + 64)) {
+    if (M.tail_smem > kTailSmem) {
       S.mg_allowed = false;
       return ADFEM_OK;
     }
@@ -1177,12 +1591,12 @@ namespace {
 unsigned blocks(int64_t n, int b) { return (unsigned)std::max<int64_t>(1, (n + b - 1) / b); }
 
 template <int NB, int NC, bool D16>
-void level_values(const MgLev& L, const MgLev& C, cudaStream_t st) {
+void level_values(const MgLev& L, const MgLev& C, int deg, float frac, cudaStream_t st) {
   constexpr int BP = 64, BA = NB * NC == 1 ? 128 : 32;
   k_mg_p<NB, NC, D16, BP><<<blocks(L.n, BP), BP, 0, st>>>(L);
   k_mg_ap<NB, NC, D16, BA><<<blocks(L.n, BA), BA, 0, st>>>(L);
   k_mg_ac<NB, NC><<<blocks(32 * (int64_t)L.nc, 128), 128, 0, st>>>(L, C);
-  k_mg_scale<NB, NC><<<blocks(L.nc, 128), 128, 0, st>>>(L, C);
+  k_mg_scale<NB, NC><<<blocks(32 * (int64_t)L.nc, 128), 128, 0, st>>>(L, C, deg, frac);
 }
 
 }  // namespace
@@ -1194,7 +1608,7 @@ int mg_values(Solver& S, cudaStream_t st) {
   const Sell& A = *S.A;
   const MgLev& L0 = M.lev[0];
   const unsigned nb = blocks(S.n, kT);
-  for (int l = 0; l < M.nlev; l++) ADFEM_CUDA(cudaMemsetAsync(M.lev[l].lam, 0, sizeof(int), st));
+  ADFEM_CUDA(cudaMemsetAsync(M.lam, 0, sizeof(int) * kMgMaxLevels, st));
   auto vals0 = [&](auto nbt, auto d16) {
     k_mg_vals0<decltype(nbt)::value, decltype(d16)::value><<<nb, kT, 0, st>>>(
         S.n, A.sptr.as<int32_t>(), A.col.p, A.val64.as<double>(), S.s32.as<float>(), S.mg_isbd, L0, M.rowsum);
@@ -1209,20 +1623,21 @@ int mg_values(Solver& S, cudaStream_t st) {
   }
   for (int l = 0; l + 1 < M.nlev; l++) {
     const MgLev &L = M.lev[l], &C = M.lev[l + 1];
+    const int deg = l == 0 ? kMgDeg0 : kMgDeg;
+    const float frac = l == 0 ? kFrac0 : kFrac;
     if (L.nb == 1) {
-      if (L.d16) level_values<1, 1, true>(L, C, st);
-      else level_values<1, 1, false>(L, C, st);
+      if (L.d16) level_values<1, 1, true>(L, C, deg, frac, st);
+      else level_values<1, 1, false>(L, C, deg, frac, st);
     } else if (L.nb == 2) {
-      level_values<2, 3, false>(L, C, st);
+      level_values<2, 3, false>(L, C, deg, frac, st);
     } else {
-      level_values<3, 3, false>(L, C, st);
+      level_values<3, 3, false>(L, C, deg, frac, st);
     }
-    k_mg_coef<<<1, 32, 0, st>>>(L, l == 0 ? kMgDeg0 : kMgDeg, l == 0 ? kFrac0 : kFrac);
   }
   const MgLev& C = M.lev[M.nlev - 1];
-  const size_t dsm = sizeof(float) * ((size_t)M.ndense * M.ndense + M.ndense);
-  if (C.nb == 1) k_mg_dense<1><<<1, kTailT, dsm, st>>>(C, M.dense);
-  else k_mg_dense<3><<<1, kTailT, dsm, st>>>(C, M.dense);
+  const size_t dsm = sizeof(float) * ((size_t)M.ndense * M.ndense + 4 * kMgDense);
+  if (C.nb == 1) k_mg_dense<1><<<1, 1024, dsm, st>>>(C, M.dense);
+  else k_mg_dense<3><<<1, 1024, dsm, st>>>(C, M.dense);
   ADFEM_CUDA(cudaGetLastError());
   M.current = true;
   return ADFEM_OK;
@@ -1273,6 +1688,23 @@ void prolong_from(const MgLev& L, const float* xc, float* x, cudaStream_t st) {
   else k_mg_prolong<3, 3><<<g, kT, 0, st>>>(L, xc, x);
 }
 
+template <int NT, int NC>
+void launch_tail(const Mg& M, const TailArgs& a, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(M.cluster ? kTailC : 1);
+  cfg.blockDim = dim3(kTailT);
+  cfg.dynamicSmemBytes = M.tail_smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = kTailC;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = M.cluster ? 1 : 0;
+  if (M.cluster) cudaLaunchKernelEx(&cfg, k_mg_tail<NT, NC, true>, a);
+  else cudaLaunchKernelEx(&cfg, k_mg_tail<NT, NC, false>, a);
+}
+
 // One cycle: lev[0].b -> the vector returned; returns the launches through *count.
 const float* enqueue_cycle(Solver& S, cudaStream_t st, int* count) {
   Mg& M = *S.mg;
@@ -1302,14 +1734,19 @@ const float* enqueue_cycle(Solver& S, cudaStream_t st, int* count) {
     for (int l = 0; l < a.nl; l++) a.L[l] = M.lev[M.tail + l];
     a.dense = M.dense;
     a.N = M.ndense;
+    a.pat = M.pat;
+    a.vals = M.vals;
+    a.pat_bytes = M.pat_bytes;
+    a.val_bytes = M.val_bytes;
     a.b = M.lev[M.tail].b;
     a.x = M.lev[M.tail].x;
     a.reps = M.tail == 0 ? 1 : 2;
-    a.st = M.tail == 0 ? cs : nullptr;
-    const int nt = a.L[0].nb, nc = a.L[0].nbc;
-    if (nt == 1) k_mg_tail<1, 1><<<1, kTailT, M.tail_smem, st>>>(a);
-    else if (nt == 2 && nc == 3) k_mg_tail<2, 3><<<1, kTailT, M.tail_smem, st>>>(a);
-    else k_mg_tail<3, 3><<<1, kTailT, M.tail_smem, st>>>(a);
+    a.dot = M.tail == 0;
+    a.st = cs;
+    const int nt = a.L[0].nb;
+    if (nt == 1) launch_tail<1, 1>(M, a, st);
+    else if (nt == 2) launch_tail<2, 3>(M, a, st);
+    else launch_tail<3, 3>(M, a, st);
     xs[M.tail] = M.lev[M.tail].x;
     nl++;
   }
@@ -1442,6 +1879,7 @@ int mg_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_rows, 
   ADFEM_CUDA(cudaGetLastError());
   ADFEM_CUDA(cudaEventSynchronize(S.ev[2]));
   const CgState fin = S.h_state[0];
+  if (std::getenv("MGDBG")) { std::fprintf(stderr, "mg: done %d iters %d rr %.3e b %.3e rho %.3e alpha %.3e lev", fin.done, fin.iters, fin.rr64, fin.bnorm2, fin.rho, fin.alpha); for (int l = 0; l < M.nlev; l++) std::fprintf(stderr, " %d", M.lev[l].n); std::fprintf(stderr, " tail %d\n", M.tail); }
   if (fin.done != 1 && !(fin.done == 4 && fin.iters >= o.max_iter)) {
     *gave_up = true;
     ADFEM_CUDA(cudaStreamWaitEvent(user, S.ev[2], 0));

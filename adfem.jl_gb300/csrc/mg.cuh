@@ -5,7 +5,7 @@
 // after every assembly the device forms the interpolation values P = P0 - c D^-1 A P0 and the
 // coarse operators P^T A P on those fixed patterns (mg.cu).  Every level is scaled to unit
 // diagonal, so its smoother (Chebyshev) needs no diagonal; levels of at most kTailDofs
-// unknowns run in one thread block (k_mg_tail).
+// unknowns run in one launch (k_mg_tail).
 #pragma once
 #include <stdint.h>
 
@@ -22,7 +22,9 @@ constexpr int kMgMaxP = 16;       // entries per interpolation row
 constexpr int kMgMaxAP = 32;      // entries per row of A P
 constexpr int kMgMaxA = 64;       // entries per coarse row
 constexpr int kMgDense = 160;     // unknowns of the directly solved coarsest level
-constexpr int kMgTailDofs = 4096; // unknowns of the largest level of the one-block tail
+constexpr int kMgTailDofs = 5120; // unknowns of the largest level of the one-launch tail
+constexpr int kTailC = 8;         // blocks of the tail's cluster
+constexpr int kTailLocal = kMgTailDofs / kTailC;  // unknowns of a tail that one block runs alone
 constexpr int kMgDeg0 = 2, kMgDeg = 4;  // Chebyshev degree: level 0, coarser levels
 
 // Patterns of one level (host), rows in solver order at level 0.  Rows are in compressed
@@ -47,6 +49,7 @@ bool mg_build_host(int64_t n, std::vector<int32_t>&& rp, std::vector<int32_t>&& 
 // Device view of one level
 struct MgLev {
   int n = 0, nc = 0, nb = 1, nbc = 1, lpr = 1;
+  int nv = 0, np = 0, nap = 0, npt = 0;  // entries of val, p_val, ap_val, pt_val
   int d16 = 0;                 // level 0 only: the system's own pattern (int16 deltas, slice patterns)
   const int32_t *sptr = nullptr, *spat = nullptr;
   const void* col = nullptr;
@@ -62,18 +65,23 @@ struct MgLev {
   const float2* dpos = nullptr;  // position relative to the aggregate's centre (rotation mode)
   float* s = nullptr;          // scale of each unknown (0: unknown without a degree of freedom)
   float *b = nullptr, *x = nullptr, *x2 = nullptr, *d = nullptr;
+  const uint8_t* to = nullptr;  // tail: the blocks that need each row's value (one bit each)
+  const int32_t* cnt = nullptr; // tail: rows each block needs
   float* coef = nullptr;       // Chebyshev coefficients
   int* lam = nullptr;          // bound of the largest eigenvalue (float bits)
 };
 
 struct Mg {
-  int nlev = 0, tail = 0;      // levels, first level of the one-block tail
+  int nlev = 0, tail = 0;      // levels, first level of the one-launch tail
   MgLev lev[kMgMaxLevels];
   float* dense = nullptr;      // inverse of the coarsest operator
   int ndense = 0;
   double* rowsum = nullptr;    // FP64 row sums of K per component of the column (nb per row)
-  float* inv_scale = nullptr;
+  int* lam = nullptr;          // MgLev::lam of every level
   DevBuf slab;                 // all of the above
+  bool cluster = false;        // the tail's first level is shared by a cluster
+  const char *pat = nullptr, *vals = nullptr;  // of the levels that a tail block runs alone
+  int pat_bytes = 0, val_bytes = 0;            // (0: too large for its shared memory)
   size_t tail_smem = 0;
   bool current = false;        // values belong to the current assembly
   cudaGraphExec_t solve = nullptr;  // while (not finished) one iteration
