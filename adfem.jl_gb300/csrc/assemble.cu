@@ -23,14 +23,6 @@ static constexpr int kBlock = 256;
 __device__ __forceinline__ int64_t gtid() { return (int64_t)blockIdx.x * blockDim.x + threadIdx.x; }
 static inline unsigned nblocks(int64_t n, int b = kBlock) { return (unsigned)((n + b - 1) / b); }
 
-// barycentric coordinate of vertex r at quadrature point k: points 0,1,2 are
-// (xi,eta) = (1/6,1/6), (1/6,2/3), (2/3,1/6) so phi = (1-xi-eta, xi, eta)
-__device__ __forceinline__ double lam(int k, int r) {
-  const double qx = (k == 2) ? 2.0 / 3.0 : 1.0 / 6.0;
-  const double qy = (k == 1) ? 2.0 / 3.0 : 1.0 / 6.0;
-  return r == 0 ? 1.0 - qx - qy : (r == 1 ? qx : qy);
-}
-
 // g of the vertex pair (a, b), a != b, from {g01, g02, g12}
 __device__ __forceinline__ double gpair(const double4& g, int a, int b) {
   int s = a + b;  // 1 -> (0,1), 2 -> (0,2), 3 -> (1,2)
@@ -40,7 +32,7 @@ __device__ __forceinline__ double gpair(const double4& g, int a, int b) {
 // ---------------------------------------------------------------------------
 // src_e[r] = w sum_k f_k phi_r(x_k).  With the degree-2 rule above, phi_r is 2/3 at one
 // point k*(r) and 1/6 at the other two (k* = 0, 2, 1 for r = 0, 1, 2), so the sum is
-// w (S/6 + f_{k*}/2) with S = f0 + f1 + f2: 11 FP64 operations per element instead of 14
+// (w/6) S + (w/2) f_{k*} with S = f0 + f1 + f2: 7 FP64 operations per element instead of 14
 // (the element pass is FP64-instruction bound on GB300).
 // WEIGHTED = false leaves out the factor w (8 FP64 operations per element, and no read of
 // the 32-byte geometry record, whose other three doubles came along with w in the same
@@ -55,13 +47,13 @@ __global__ void k_element_prepass(int64_t ne, const double* __restrict__ kappa, 
   if (kappa) sigma[e] = kappa[3 * e] + kappa[3 * e + 1] + kappa[3 * e + 2];
   if (f) {
     const double f0 = f[3 * e], f1 = f[3 * e + 1], f2 = f[3 * e + 2];
-    const double s6 = (f0 + f1 + f2) * (1.0 / 6.0);
     if (WEIGHTED) {
-      const double w = geo[e].w;
-      src3[3 * e] = w * fma(f0, 0.5, s6);
-      src3[3 * e + 1] = w * fma(f2, 0.5, s6);
-      src3[3 * e + 2] = w * fma(f1, 0.5, s6);
+      const double w = geo[e].w, wh = 0.5 * w, t = (f0 + f1 + f2) * (w * (1.0 / 6.0));
+      src3[3 * e] = fma(f0, wh, t);
+      src3[3 * e + 1] = fma(f2, wh, t);
+      src3[3 * e + 2] = fma(f1, wh, t);
     } else {
+      const double s6 = (f0 + f1 + f2) * (1.0 / 6.0);
       src3[3 * e] = fma(f0, 0.5, s6);
       src3[3 * e + 1] = fma(f2, 0.5, s6);
       src3[3 * e + 2] = fma(f1, 0.5, s6);
@@ -503,72 +495,121 @@ cudaError_t launch_poisson_system(const Mesh& m, const double* sigma, const doub
 // ---------------------------------------------------------------------------
 // Unsummed COO of FemLaplaceScalar_forward (FemLaplaceScalar.h:3-26): entry
 // z = 27 e + 9 k + 3 p + q is (dof_p, dof_q, (w grad_p.grad_q) kappa_{3e+k}).
-// One thread per entry keeps the 16-byte index and 8-byte value stores coalesced.
-__global__ void k_laplace_coo(int64_t ne, const int4* __restrict__ conn, const double4* __restrict__ geo,
-                              const double* __restrict__ kappa, longlong2* __restrict__ idx,
-                              double* __restrict__ vv) {
-  const int64_t z = gtid();
-  if (z >= 27 * ne) return;
-  const int64_t e = z / 27;
-  const int rem = (int)(z - 27 * e);
-  const int k = rem / 9, p = (rem / 3) % 3, q = rem % 3;
-  const int4 c = conn[e];
-  const double4 g = geo[e];
-  double gpq;
-  if (p != q) {
-    gpq = gpair(g, p, q);
-  } else {
-    const int b = (p == 0) ? 1 : 0, cc = (p == 2) ? 1 : 2;
-    gpq = -(gpair(g, p, b) + gpair(g, p, cc));
+// A block takes kCooPts Gauss points: one thread per point forms its 6 distinct values (6 FP64
+// operations; an operation per entry issued 9 and the divisions of a 64-bit entry index held the
+// kernel at 3.7 TB/s), then all threads write values and indices in order.
+constexpr int kCooPts = 120;  // whole elements
+__global__ void __launch_bounds__(kBlock) k_laplace_coo(int64_t ne, const int4* __restrict__ conn,
+                                                        const double4* __restrict__ geo,
+                                                        const double* __restrict__ kappa, longlong2* __restrict__ idx,
+                                                        double* __restrict__ vv) {
+  __shared__ double sv[kCooPts][6];       // (0,1) (0,2) (1,2) (0,0) (1,1) (2,2)
+  __shared__ int32_t sd[kCooPts / 3][3];
+  const int64_t e0 = (int64_t)blockIdx.x * (kCooPts / 3);
+  const int np = (int)min((int64_t)kCooPts, 3 * (ne - e0));
+  const int t = threadIdx.x;
+  if (t < np) {
+    const int64_t e = e0 + t / 3;
+    const double4 g = geo[e];
+    const double c = kappa[3 * e0 + t];
+    const double x = g.x * c, y = g.y * c, z = g.z * c;
+    sv[t][0] = x;
+    sv[t][1] = y;
+    sv[t][2] = z;
+    sv[t][3] = -(x + y);
+    sv[t][4] = -(x + z);
+    sv[t][5] = -(y + z);
+    if (t % 3 == 0) {
+      const int4 cn = conn[e];
+      sd[t / 3][0] = cn.x;
+      sd[t / 3][1] = cn.y;
+      sd[t / 3][2] = cn.z;
+    }
   }
-  const int vp = p == 0 ? c.x : (p == 1 ? c.y : c.z);
-  const int vq = q == 0 ? c.x : (q == 1 ? c.y : c.z);
-  idx[z] = make_longlong2(vp, vq);
-  vv[z] = gpq * kappa[3 * e + k];
+  __syncthreads();
+  for (int q = t; q < 9 * np; q += kBlock) {
+    const int p = q / 9, m = q - 9 * p, r = m / 3, c = m - 3 * r;
+    __stcs(vv + 27 * e0 + q, sv[p][r == c ? 3 + r : r + c - 1]);
+    const int32_t* d = sd[p / 3];
+    __stcs(reinterpret_cast<int4*>(idx) + 27 * e0 + q, make_int4(d[r], 0, d[c], 0));  // (two 64-bit indices)
+  }
 }
 
 cudaError_t launch_laplace_coo(const Mesh& m, const double* kappa, long long* indices, double* vv, cudaStream_t st) {
-  k_laplace_coo<<<nblocks(27 * m.ne), kBlock, 0, st>>>(m.ne, m.d_conn.as<int4>(), m.d_geo.as<double4>(), kappa,
-                                                       reinterpret_cast<longlong2*>(indices), vv);
+  k_laplace_coo<<<nblocks(m.ne, kCooPts / 3), kBlock, 0, st>>>(m.ne, m.d_conn.as<int4>(), m.d_geo.as<double4>(), kappa,
+                                                               reinterpret_cast<longlong2*>(indices), vv);
   return cudaGetLastError();
 }
 
-// FemLaplaceScalar_backward (FemLaplaceScalar.h:28-54): grad_kappa[3e+k] = sum_pq grad_vv * (w grad_p.grad_q)
-__global__ void k_laplace_coo_backward(int64_t ne, const double4* __restrict__ geo, const double* __restrict__ gvv,
-                                       double* __restrict__ gk) {
-  const int64_t s = gtid();
-  if (s >= 3 * ne) return;
-  const int64_t e = s / 3;
-  const double4 g = geo[e];
-  const double g00 = -(g.x + g.y), g11 = -(g.x + g.z), g22 = -(g.y + g.z);
-  const double G[9] = {g00, g.x, g.y, g.x, g11, g.z, g.y, g.z, g22};
-  const double* src = gvv + 9 * s;
-  double v = 0.0;
+// FemLaplaceScalar_backward (FemLaplaceScalar.h:28-54): grad_kappa[3e+k] = sum_pq grad_vv * (w grad_p.grad_q).
+// FP64 issue bounds it: one thread per element shares the diagonal products of its three points,
+// 30 operations per element instead of 36.  The block reads its elements' entries in order into
+// shared memory (a thread's own are 216 bytes apart from its neighbour's).
+constexpr int kBwdEl = 128;
+__global__ void __launch_bounds__(kBwdEl) k_laplace_coo_backward(int64_t ne, const double4* __restrict__ geo,
+                                                                 const double* __restrict__ gvv,
+                                                                 double* __restrict__ gk) {
+  __shared__ double sv[27 * kBwdEl];
+  const int64_t e0 = (int64_t)blockIdx.x * kBwdEl;
+  const int nel = (int)min((int64_t)kBwdEl, ne - e0), cnt = 27 * nel, t = threadIdx.x;
+  const double* src = gvv + 27 * e0;
+  if ((reinterpret_cast<uintptr_t>(gvv) & 15) == 0) {  // (27 e0 is even)
+    for (int q = t; q < cnt / 2; q += kBwdEl) {
+      const double2 v = __ldcs(reinterpret_cast<const double2*>(src) + q);
+      sv[2 * q] = v.x;
+      sv[2 * q + 1] = v.y;
+    }
+    if ((cnt & 1) && t == 0) sv[cnt - 1] = src[cnt - 1];
+  } else {
+    for (int q = t; q < cnt; q += kBwdEl) sv[q] = __ldcs(src + q);
+  }
+  __syncthreads();
+  double o[3];
+  if (t < nel) {
+    const double4 g = geo[e0 + t];
+    const double g00 = -(g.x + g.y), g11 = -(g.x + g.z), g22 = -(g.y + g.z);
 #pragma unroll
-  for (int j = 0; j < 9; j++) v = fma(src[j], G[j], v);
-  gk[s] = v;
+    for (int k = 0; k < 3; k++) {
+      const double* G = sv + 27 * t + 9 * k;
+      double v = g00 * G[0];
+      v = fma(g11, G[4], v);
+      v = fma(g22, G[8], v);
+      v = fma(g.x, G[1] + G[3], v);
+      v = fma(g.y, G[2] + G[6], v);
+      o[k] = fma(g.z, G[5] + G[7], v);
+    }
+  }
+  __syncthreads();
+  if (t < nel)
+#pragma unroll
+    for (int k = 0; k < 3; k++) sv[3 * t + k] = o[k];
+  __syncthreads();
+  for (int q = t; q < 3 * nel; q += kBwdEl) gk[3 * e0 + q] = sv[q];
 }
 
 cudaError_t launch_laplace_coo_backward(const Mesh& m, const double* grad_vv, double* grad_kappa, cudaStream_t st) {
-  k_laplace_coo_backward<<<nblocks(3 * m.ne), kBlock, 0, st>>>(m.ne, m.d_geo.as<double4>(), grad_vv, grad_kappa);
+  k_laplace_coo_backward<<<nblocks(m.ne, kBwdEl), kBwdEl, 0, st>>>(m.ne, m.d_geo.as<double4>(), grad_vv, grad_kappa);
   return cudaGetLastError();
 }
 
-// FemSourceScalar_backward (FemSourceScalar.h:17-32)
+// FemSourceScalar_backward (FemSourceScalar.h:17-32), one thread per element: with the rule's
+// algebra of k_element_prepass, gf_k = (w/6) (g0 + g1 + g2) + (w/2) g_{r*(k)} -- 8 FP64 operations
+// per element instead of 18.
 __global__ void k_source_backward(int64_t ne, const int4* __restrict__ conn, const double4* __restrict__ geo,
                                   const double* __restrict__ grhs, double* __restrict__ gf) {
-  const int64_t s = gtid();
-  if (s >= 3 * ne) return;
-  const int64_t e = s / 3;
-  const int k = (int)(s - 3 * e);
+  const int64_t e = gtid();
+  if (e >= ne) return;
   const int4 c = conn[e];
-  const double w = geo[e].w;
-  gf[s] = w * (lam(k, 0) * grhs[c.x] + lam(k, 1) * grhs[c.y] + lam(k, 2) * grhs[c.z]);
+  const double w = geo[e].w, g0 = grhs[c.x], g1 = grhs[c.y], g2 = grhs[c.z];
+  const double wh = 0.5 * w, t = (g0 + g1 + g2) * (w * (1.0 / 6.0));
+  gf[3 * e] = fma(wh, g0, t);
+  gf[3 * e + 1] = fma(wh, g2, t);
+  gf[3 * e + 2] = fma(wh, g1, t);
 }
 
 cudaError_t launch_source_backward(const Mesh& m, const double* grad_rhs, double* grad_f, cudaStream_t st) {
-  k_source_backward<<<nblocks(3 * m.ne), kBlock, 0, st>>>(m.ne, m.d_conn.as<int4>(), m.d_geo.as<double4>(),
-                                                          grad_rhs, grad_f);
+  k_source_backward<<<nblocks(m.ne), kBlock, 0, st>>>(m.ne, m.d_conn.as<int4>(), m.d_geo.as<double4>(), grad_rhs,
+                                                      grad_f);
   return cudaGetLastError();
 }
 

@@ -17,44 +17,53 @@ __device__ __forceinline__ int64_t gtid() { return (int64_t)blockIdx.x * blockDi
 static inline unsigned nblk(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
 
 // ---------------------------------------------------------------------------
-// PlaneStrainAndStress.h:5-78
-__global__ void k_plane_strain(int mode, int64_t n, const double* __restrict__ E, const double* __restrict__ nu,
-                               double* __restrict__ D) {
-  const int64_t i = gtid();
-  if (i >= n) return;
-  const double e = E[i], v = nu[i];
-  double* o = D + 9 * i;
-  if (mode == 0) {
-    const double s = e * (1 - v) / (1 + v) / (1 - 2 * v);
-    const double a = s * v / (1 - v);
-    o[0] = s; o[1] = a; o[2] = a;
-    o[3] = a; o[4] = s; o[5] = a;
-    o[6] = a; o[7] = a; o[8] = s;
-  } else {
-    const double s = e / (1 + v) / (1 - 2 * v);
-    o[0] = s * (1 - v); o[1] = s * v; o[2] = 0.0;
-    o[3] = s * v; o[4] = s * (1 - v); o[5] = 0.0;
-    o[6] = 0.0; o[7] = 0.0; o[8] = s * (1 - 2 * v) / 2.0;
+// PlaneStrainAndStress.h:5-78.  FP64 divisions (about ten operations each) bound these kernels:
+// one reciprocal per point instead of two to four quotients; the nine entries of a point are
+// written (read) in order by the whole block.
+__global__ void __launch_bounds__(256) k_plane_strain(int mode, int64_t n, const double* __restrict__ E,
+                                                      const double* __restrict__ nu, double* __restrict__ D) {
+  __shared__ double sv[256][3];  // diagonal, off-diagonal, last entry
+  const int64_t i0 = (int64_t)blockIdx.x * 256;
+  const int np = (int)min((int64_t)256, n - i0);
+  if ((int)threadIdx.x < np) {
+    const double e = E[i0 + threadIdx.x], v = nu[i0 + threadIdx.x];
+    const double d = 1 - 2 * v, s = e / ((1 + v) * d);
+    sv[threadIdx.x][0] = s * (1 - v);
+    sv[threadIdx.x][1] = s * v;
+    sv[threadIdx.x][2] = mode == 0 ? s * (1 - v) : s * d / 2.0;
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < 9 * np; q += 256) {
+    const int p = q / 9, m = q - 9 * p;
+    double v = sv[p][m == 8 ? 2 : (m % 4 == 0 ? 0 : 1)];
+    if (mode != 0 && (m == 2 || (m >= 5 && m <= 7))) v = 0.0;
+    D[9 * i0 + q] = v;
   }
 }
 
 // derivative of the entries above (the reference obtains it with an AD tape)
-__global__ void k_plane_strain_backward(int mode, int64_t n, const double* __restrict__ g,
-                                        const double* __restrict__ E, const double* __restrict__ nu,
-                                        double* __restrict__ gE, double* __restrict__ gnu) {
-  const int64_t i = gtid();
-  if (i >= n) return;
-  const double* q = g + 9 * i;
-  const double v = nu[i], D = (1 + v) * (1 - 2 * v);
+__global__ void __launch_bounds__(256) k_plane_strain_backward(int mode, int64_t n, const double* __restrict__ g,
+                                                               const double* __restrict__ E,
+                                                               const double* __restrict__ nu, double* __restrict__ gE,
+                                                               double* __restrict__ gnu) {
+  __shared__ double sv[9 * 256];
+  const int64_t i0 = (int64_t)blockIdx.x * 256;
+  const int np = (int)min((int64_t)256, n - i0);
+  for (int q = threadIdx.x; q < 9 * np; q += 256) sv[q] = __ldcs(g + 9 * i0 + q);
+  __syncthreads();
+  if ((int)threadIdx.x >= np) return;
+  const int64_t i = i0 + threadIdx.x;
+  const double* q = sv + 9 * threadIdx.x;
+  const double v = nu[i], r = 1.0 / ((1 + v) * (1 - 2 * v)), er2 = E[i] * r * r;
   if (mode == 0) {
     const double gd = q[0] + q[4] + q[8];
     const double go = q[1] + q[2] + q[3] + q[5] + q[6] + q[7];
-    gE[i] = gd * (1 - v) / D + go * v / D;
-    gnu[i] = E[i] * (gd * 2 * v * (2 - v) + go * (1 + 2 * v * v)) / (D * D);
+    gE[i] = (gd * (1 - v) + go * v) * r;
+    gnu[i] = er2 * (gd * 2 * v * (2 - v) + go * (1 + 2 * v * v));
   } else {
-    const double a = q[0] + q[4], b = q[1] + q[3], c = q[8];
-    gE[i] = (a * (1 - v) + b * v + c * (1 - 2 * v) / 2.0) / D;
-    gnu[i] = E[i] * (a * 2 * v * (2 - v) / (D * D) + b * (1 + 2 * v * v) / (D * D) + c * -0.5 / ((1 + v) * (1 + v)));
+    const double a = q[0] + q[4], b = q[1] + q[3], c = q[8], d = 1 - 2 * v;
+    gE[i] = (a * (1 - v) + b * v + c * d / 2.0) * r;
+    gnu[i] = er2 * (a * 2 * v * (2 - v) + b * (1 + 2 * v * v) - c * 0.5 * d * d);
   }
 }
 
@@ -312,94 +321,140 @@ cudaError_t launch_elastic_system(const Mesh& m, const double* Dbar, const doubl
 }
 
 // ---------------------------------------------------------------------------
-// Unsummed COO of ComputeFemStiffnessMatrixMfem_forward: thread per (e, k, l) writes
-// the 6 entries of row l of NN_k = B^T D_k B w.  Entry index 108 e + 36 k + 6 l + s.
-__global__ void k_stiffness_coo(int64_t ne, int64_t ndof, const int4* __restrict__ conn,
-                                const double2* __restrict__ grad, const double4* __restrict__ geo,
-                                const double* __restrict__ D, longlong2* __restrict__ idx, double* __restrict__ vv) {
-  const int64_t t = gtid();
-  if (t >= 18 * ne) return;
-  const int64_t e = t / 18;
-  const int rem = (int)(t - 18 * e);
-  const int k = rem / 6, l = rem % 6;
-  const int4 cn = conn[e];
-  const int vtx[3] = {cn.x, cn.y, cn.z};
-  const double2* gr = grad + 3 * e;
-  const double* d = D + 27 * e + 9 * k;
-  const double w = geo[e].w;
-  const int a = l % 3;
-  const double2 ga = gr[a];
-  double v0, v1, v2;
-  if (l < 3) {
-    v0 = fma(ga.x, d[0], ga.y * d[6]);
-    v1 = fma(ga.x, d[1], ga.y * d[7]);
-    v2 = fma(ga.x, d[2], ga.y * d[8]);
-  } else {
-    v0 = fma(ga.y, d[3], ga.x * d[6]);
-    v1 = fma(ga.y, d[4], ga.x * d[7]);
-    v2 = fma(ga.y, d[5], ga.x * d[8]);
-  }
-  const long long row = vtx[a] + (l < 3 ? 0 : ndof);
-  const int64_t z0 = 108 * e + 36 * k + 6 * l;
+// Unsummed COO of ComputeFemStiffnessMatrixMfem_forward: entry 108 e + 36 k + 6 l + s of
+// NN_k = w B^T D_k B.  The gradients of the three vertices sum to zero, so the rows and columns
+// of vertex 2 are the negated sums of the other two: one thread per Gauss point forms the 4 x 4
+// block of vertices 0 and 1 and extends it, 80 FP64 operations instead of 144 (FP64 issue bounds
+// the kernel); the block then writes values and indices in order through shared memory.
+constexpr int kStiffPts = 126, kStiffT = 128;  // whole elements; every warp of the block has points
+__global__ void __launch_bounds__(kStiffT) k_stiffness_coo(int64_t ne, int64_t ndof, const int4* __restrict__ conn,
+                                                       const double2* __restrict__ grad,
+                                                       const double4* __restrict__ geo, const double* __restrict__ D,
+                                                       longlong2* __restrict__ idx, double* __restrict__ vv) {
+  __shared__ double sv[kStiffPts][37];
+  __shared__ int32_t sd[kStiffPts / 3][3];
+  const int64_t e0 = (int64_t)blockIdx.x * (kStiffPts / 3);
+  const int np = (int)min((int64_t)kStiffPts, 3 * (ne - e0));
+  if ((int)threadIdx.x < np) {
+    const int64_t e = e0 + threadIdx.x / 3;
+    const double2 h0 = grad[3 * e], h1 = grad[3 * e + 1];
+    const double w = geo[e].w;
+    double d[9];
 #pragma unroll
-  for (int s = 0; s < 6; s++) {
-    const int b = s % 3;
-    const double2 gb = gr[b];
-    const double val = s < 3 ? fma(v0, gb.x, v2 * gb.y) : fma(v1, gb.y, v2 * gb.x);
-    idx[z0 + s] = make_longlong2(row, (long long)vtx[b] + (s < 3 ? 0 : ndof));
-    vv[z0 + s] = val * w;
+    for (int q = 0; q < 9; q++) d[q] = __ldg(D + 27 * e0 + 9 * threadIdx.x + q);
+    double* N = sv[threadIdx.x];
+    // row l of the 4 x 4 block: x of vertex i (B column (hx, 0, hy)), y of vertex i ((0, hy, hx))
+    auto row = [&](int l, const double2& h, bool y) {
+      const double a = w * h.x, b = w * h.y;
+      double v[3];
+#pragma unroll
+      for (int q = 0; q < 3; q++) v[q] = y ? fma(b, d[3 + q], a * d[6 + q]) : fma(a, d[q], b * d[6 + q]);
+      const double x0 = fma(v[0], h0.x, v[2] * h0.y), x1 = fma(v[0], h1.x, v[2] * h1.y);
+      const double y0 = fma(v[1], h0.y, v[2] * h0.x), y1 = fma(v[1], h1.y, v[2] * h1.x);
+      N[6 * l] = x0;
+      N[6 * l + 1] = x1;
+      N[6 * l + 2] = -(x0 + x1);
+      N[6 * l + 3] = y0;
+      N[6 * l + 4] = y1;
+      N[6 * l + 5] = -(y0 + y1);
+    };
+    row(0, h0, false);
+    row(1, h1, false);
+    row(3, h0, true);
+    row(4, h1, true);
+#pragma unroll
+    for (int q = 0; q < 6; q++) {
+      N[12 + q] = -(N[q] + N[6 + q]);
+      N[30 + q] = -(N[18 + q] + N[24 + q]);
+    }
+    if (threadIdx.x % 3 == 0) {
+      const int4 cn = conn[e];
+      sd[threadIdx.x / 3][0] = cn.x;
+      sd[threadIdx.x / 3][1] = cn.y;
+      sd[threadIdx.x / 3][2] = cn.z;
+    }
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < 36 * np; q += kStiffT) {
+    const int p = q / 36, m = q - 36 * p, r = m / 6, c = m - 6 * r;
+    __stcs(vv + 108 * e0 + q, sv[p][m]);
+    const int32_t* v = sd[p / 3];
+    idx[108 * e0 + q] = make_longlong2(v[r % 3] + (r < 3 ? 0 : ndof), v[c % 3] + (c < 3 ? 0 : ndof));
   }
 }
 
 cudaError_t launch_stiffness_coo(const Mesh& m, const double* D, long long* indices, double* vv, cudaStream_t st) {
-  k_stiffness_coo<<<nblk(18 * m.ne, 256), 256, 0, st>>>(m.ne, m.nv, m.d_conn.as<int4>(), m.d_grad.as<double2>(),
-                                                        m.d_geo.as<double4>(), D,
-                                                        reinterpret_cast<longlong2*>(indices), vv);
+  k_stiffness_coo<<<nblk(m.ne, kStiffPts / 3), kStiffT, 0, st>>>(m.ne, m.nv, m.d_conn.as<int4>(), m.d_grad.as<double2>(),
+                                                             m.d_geo.as<double4>(), D,
+                                                             reinterpret_cast<longlong2*>(indices), vv);
   return cudaGetLastError();
 }
 
-// ComputeFemStiffnessMatrixMfem_backward: grad_D_k = w B G B^T, G = grad_vv block (6x6)
-__global__ void k_stiffness_coo_backward(int64_t ne, const double2* __restrict__ grad,
-                                         const double4* __restrict__ geo, const double* __restrict__ gvv,
-                                         double* __restrict__ gD) {
-  const int64_t t = gtid();
-  if (t >= 3 * ne) return;
-  const int64_t e = t / 3;
-  const double2* gr = grad + 3 * e;
-  const double* G = gvv + 36 * t;
-  double B[3][6];
-#pragma unroll
-  for (int b = 0; b < 3; b++) {
-    B[0][b] = gr[b].x; B[0][b + 3] = 0.0;
-    B[1][b] = 0.0;     B[1][b + 3] = gr[b].y;
-    B[2][b] = gr[b].y; B[2][b + 3] = gr[b].x;
+// ComputeFemStiffnessMatrixMfem_backward: grad_D_k = w B G B^T, G = grad_vv block (6x6).  By the
+// same zero sum G enters through the differences of its rows and columns to those of vertex 2: a
+// 4 x 4 block (40 additions), then 60 operations, against 126 on the full block.  The block reads
+// and writes its points' entries in order through shared memory.
+__global__ void __launch_bounds__(kStiffT) k_stiffness_coo_backward(int64_t ne, const double2* __restrict__ grad,
+                                                                const double4* __restrict__ geo,
+                                                                const double* __restrict__ gvv,
+                                                                double* __restrict__ gD) {
+  __shared__ double sv[kStiffPts][37];
+  const int64_t e0 = (int64_t)blockIdx.x * (kStiffPts / 3);
+  const int np = (int)min((int64_t)kStiffPts, 3 * (ne - e0));
+  const double* src = gvv + 108 * e0;
+  if ((reinterpret_cast<uintptr_t>(gvv) & 15) == 0) {
+    for (int q = threadIdx.x; q < 18 * np; q += kStiffT) {
+      const double2 v = __ldcs(reinterpret_cast<const double2*>(src) + q);
+      const int p = q / 18, m = 2 * (q - 18 * p);
+      sv[p][m] = v.x;
+      sv[p][m + 1] = v.y;
+    }
+  } else {
+    for (int q = threadIdx.x; q < 36 * np; q += kStiffT) sv[q / 36][q % 36] = __ldcs(src + q);
   }
-  double T[3][6];
+  __syncthreads();
+  if ((int)threadIdx.x < np) {
+    const int64_t e = e0 + threadIdx.x / 3;
+    const double2 h0 = grad[3 * e], h1 = grad[3 * e + 1];
+    const double w = geo[e].w;
+    double* G = sv[threadIdx.x];
+    // H: rows and columns x0, x1, y0, y1
+    double H[4][4];
 #pragma unroll
-  for (int p = 0; p < 3; p++)
+    for (int r = 0; r < 4; r++) {
+      const int gr = r < 2 ? r : r + 1, g2 = r < 2 ? 2 : 5;
+      double R[6];
 #pragma unroll
-    for (int s = 0; s < 6; s++) {
-      double acc = 0.0;
-#pragma unroll
-      for (int l = 0; l < 6; l++)
-        if (B[p][l] != 0.0) acc = fma(B[p][l], G[6 * l + s], acc);
-      T[p][s] = acc;
+      for (int c = 0; c < 6; c++) R[c] = G[6 * gr + c] - G[6 * g2 + c];
+      H[r][0] = R[0] - R[2];
+      H[r][1] = R[1] - R[2];
+      H[r][2] = R[3] - R[5];
+      H[r][3] = R[4] - R[5];
     }
-  const double w = geo[e].w;
+    double T[3][4];
+    {
+      const double a0 = w * h0.x, a1 = w * h1.x, b0 = w * h0.y, b1 = w * h1.y;
 #pragma unroll
-  for (int p = 0; p < 3; p++)
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-      double acc = 0.0;
-#pragma unroll
-      for (int s = 0; s < 6; s++) acc = fma(T[p][s], B[q][s], acc);
-      gD[9 * t + 3 * p + q] = acc * w;
+      for (int c = 0; c < 4; c++) {
+        T[0][c] = fma(a0, H[0][c], a1 * H[1][c]);
+        T[1][c] = fma(b0, H[2][c], b1 * H[3][c]);
+        T[2][c] = fma(b0, H[0][c], fma(b1, H[1][c], fma(a0, H[2][c], a1 * H[3][c])));
+      }
     }
+#pragma unroll
+    for (int p = 0; p < 3; p++) {
+      G[3 * p] = fma(T[p][0], h0.x, T[p][1] * h1.x);
+      G[3 * p + 1] = fma(T[p][2], h0.y, T[p][3] * h1.y);
+      G[3 * p + 2] = fma(T[p][0], h0.y, fma(T[p][1], h1.y, fma(T[p][2], h0.x, T[p][3] * h1.x)));
+    }
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < 9 * np; q += kStiffT) gD[27 * e0 + q] = sv[q / 9][q % 9];
 }
 
 cudaError_t launch_stiffness_coo_backward(const Mesh& m, const double* grad_vv, double* grad_D, cudaStream_t st) {
-  k_stiffness_coo_backward<<<nblk(3 * m.ne, 256), 256, 0, st>>>(m.ne, m.d_grad.as<double2>(), m.d_geo.as<double4>(),
-                                                                grad_vv, grad_D);
+  k_stiffness_coo_backward<<<nblk(m.ne, kStiffPts / 3), kStiffT, 0, st>>>(m.ne, m.d_grad.as<double2>(),
+                                                                      m.d_geo.as<double4>(), grad_vv, grad_D);
   return cudaGetLastError();
 }
 

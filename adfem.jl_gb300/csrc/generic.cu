@@ -55,6 +55,7 @@ struct Tab {
   double t[NG][ND][3];  // d phi_r / d l_c at point k
   double l[NG][3];      // barycentric coordinates of point k
   double w[NG];         // rule weight of point k
+  double hw[NG][ND];    // phi_r w / 0.5 at point k
 };
 
 // Lagrange basis in barycentric coordinates.  P1: phi_r = l_r.  P2 (nodes at the
@@ -86,6 +87,7 @@ __device__ void tab_init(Tab<DEG>& T) {
         T.t[k][3 + j][b] = 4.0 * l[a];
       }
     }
+    for (int r = 0; r < ND; r++) T.hw[k][r] = T.h[k][r] * T.w[k] / 0.5;
   }
   __syncthreads();
 }
@@ -111,9 +113,346 @@ __device__ __forceinline__ double weight_at(const Tab<DEG>& T, int k, double are
   return T.w[k] * area / 0.5;
 }
 
+// Callers' arrays are 8-byte aligned at least; 16-byte accesses only where they are 16-byte
+// aligned (an element's six values keep the array's alignment).
+__device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+__device__ __forceinline__ void load6(const double* __restrict__ p, double (&v)[6]) {
+  if (aligned16(p)) {
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const double2 x = __ldg(reinterpret_cast<const double2*>(p) + k);
+      v[2 * k] = x.x;
+      v[2 * k + 1] = x.y;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 6; k++) v[k] = __ldg(p + k);
+  }
+}
+
+// sum_k f_k t(k) over an element's points
+template <int NG, class F>
+__device__ __forceinline__ double point_sum(const double* __restrict__ f, F t) {
+  double v[NG];
+  if constexpr (NG == 6) {
+    load6(f, v);
+  } else {
+#pragma unroll
+    for (int k = 0; k < NG; k++) v[k] = __ldg(f + k);
+  }
+  double s = v[0] * t(0);
+#pragma unroll
+  for (int k = 1; k < NG; k++) s = fma(v[k], t(k), s);
+  return s;
+}
+
 int grid_for(int64_t n, int bt = kGT) {
   int64_t b = (n + bt - 1) / bt;
   return (int)std::max<int64_t>(1, std::min<int64_t>(b, 152 * 32));
+}
+
+// ---------------------------------------------------------------- P2 by orbits
+// The order-4 rule has two orbits of three points; at the point with special vertex i the
+// barycentric coordinates are b at i and a at the other two.  A sum over an orbit of a
+// coefficient times a product of basis values (or of their derivatives' factors) is therefore
+// base * (c_0 + c_1 + c_2) + alpha * c_i (+ beta * c_j), so the sums that an element matrix, a
+// load or an interpolation needs cost one or two FP64 operations each instead of six, which is
+// what bounds these kernels (FP64 issues at 1/64 of FP32 here).  Laplace: the basis gradients
+// are combinations of the barycentric ones, so the matrix is a contraction of the moments
+//   VV_ab = sum c w t_a t_b, Q_ab = sum c w t_a 4 l_b, R_ab = sum c w 16 l_a l_b  (t = 4 l - 1)
+// with the three products g_ab of the P1 geometry record.  ~125 FP64 operations per element
+// against ~500 with gradients formed at every point.
+namespace p2 {
+__device__ constexpr double A[2] = {0.091576213509770743460, 0.44594849091596488632};
+__device__ constexpr double B[2] = {0.81684757298045851308, 0.10810301816807022736};
+__device__ constexpr double W[2] = {0.054975871827660933819, 0.11169079483900573285};
+// point k of an orbit -> its special vertex: (a, a), (a, b), (b, a) in (xi, eta)
+__host__ __device__ constexpr int special(int k) { return k == 0 ? 0 : 3 - k; }
+// local edge opposite to vertex m: edges (0,1), (1,2), (2,0) are DOFs 3, 4, 5
+__host__ __device__ constexpr int edge_opp(int m) { return m == 0 ? 4 : (m == 1 ? 5 : 3); }
+__host__ __device__ constexpr int third(int i, int j) { return 3 - i - j; }
+
+// the six values of an element by orbit and special vertex
+__device__ __forceinline__ void by_special(const double* __restrict__ c6, double (&c)[2][3]) {
+  double v[6];
+  load6(c6, v);
+#pragma unroll
+  for (int k = 0; k < 6; k++) c[k / 3][special(k % 3)] = v[k];
+}
+
+// symmetric family: D[i] (both factors at i) and O[k] (factors at i, j with third vertex k) of
+// sum c x_i x_j, x = xs at the special vertex, xo elsewhere
+__device__ __forceinline__ void sym_sums(const double (&c)[2][3], const double (&cs)[2], const double (&xs)[2],
+                                         const double (&xo)[2], const double (&w)[2], double (&D)[3], double (&O)[3]) {
+  const double d = fma(w[1] * xo[1] * xo[1], cs[1], w[0] * xo[0] * xo[0] * cs[0]);
+  const double o = fma(w[1] * xs[1] * xo[1], cs[1], w[0] * xs[0] * xo[0] * cs[0]);
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    D[i] = fma(w[1] * (xs[1] * xs[1] - xo[1] * xo[1]), c[1][i], fma(w[0] * (xs[0] * xs[0] - xo[0] * xo[0]), c[0][i], d));
+    O[i] = fma(w[1] * (xo[1] * xo[1] - xs[1] * xo[1]), c[1][i], fma(w[0] * (xo[0] * xo[0] - xs[0] * xo[0]), c[0][i], o));
+  }
+}
+// mixed family: M[i][j] of sum c x_i y_j
+__device__ __forceinline__ void mixed_sums(const double (&c)[2][3], const double (&cs)[2], const double (&xs)[2],
+                                           const double (&xo)[2], const double (&ys)[2], const double (&yo)[2],
+                                           const double (&w)[2], double (&M)[3][3]) {
+  const double m = fma(w[1] * xo[1] * yo[1], cs[1], w[0] * xo[0] * yo[0] * cs[0]);
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    M[i][i] = fma(w[1] * (xs[1] * ys[1] - xo[1] * yo[1]), c[1][i],
+                  fma(w[0] * (xs[0] * ys[0] - xo[0] * yo[0]), c[0][i], m));
+    const double mi = fma(w[1] * (xs[1] * yo[1] - xo[1] * yo[1]), c[1][i],
+                          fma(w[0] * (xs[0] * yo[0] - xo[0] * yo[0]), c[0][i], m));
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+      if (j != i)
+        M[i][j] = fma(w[1] * (xo[1] * ys[1] - xo[1] * yo[1]), c[1][j],
+                      fma(w[0] * (xo[0] * ys[0] - xo[0] * yo[0]), c[0][j], mi));
+  }
+}
+// values of a P2 function at the six points: sums over vertices and edges, then two operations
+// per point (f: the point weights, 1 for plain values)
+template <class F>
+__device__ __forceinline__ void at_points(const double (&u)[6], F put, const double (&f)[2]) {
+  const double U = u[0] + u[1] + u[2], E = u[3] + u[4] + u[5];
+#pragma unroll
+  for (int o = 0; o < 2; o++) {
+    const double hs = B[o] * (2 * B[o] - 1), ho = A[o] * (2 * A[o] - 1), es = 4 * A[o] * A[o], eo = 4 * A[o] * B[o];
+    const double base = fma(f[o] * eo, E, f[o] * ho * U);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const int i = special(k);
+      put(3 * o + k, fma(f[o] * (es - eo), u[edge_opp(i)], fma(f[o] * (hs - ho), u[i], base)));
+    }
+  }
+}
+}  // namespace p2
+
+// P2 element matrices, one thread per element, stored as the full 6 x 6 matrix (a row gather
+// reads one contiguous row)
+template <int OP>
+__global__ void __launch_bounds__(kGT) k_p2_ke(int64_t ne, const double4* __restrict__ geo,
+                                               const double* __restrict__ area, const double* __restrict__ coef,
+                                               double* __restrict__ ke) {
+  for (int64_t e = gtid(); e < ne; e += gstride()) {
+    double c[2][3];
+    p2::by_special(coef + 6 * e, c);
+    const double cs[2] = {c[0][0] + c[0][1] + c[0][2], c[1][0] + c[1][1] + c[1][2]};
+    double K[6][6];
+    if (OP == (int)GenOp::LAPLACE) {
+      // 2 area grad_a.grad_b = 6 g_ab of the record (whose weight is area / 3)
+      constexpr double w6[2] = {6 * p2::W[0], 6 * p2::W[1]}, w16[2] = {96 * p2::W[0], 96 * p2::W[1]},
+                       w4[2] = {24 * p2::W[0], 24 * p2::W[1]};
+      constexpr double ts[2] = {4 * p2::B[0] - 1, 4 * p2::B[1] - 1}, to[2] = {4 * p2::A[0] - 1, 4 * p2::A[1] - 1};
+      const double4 gr = geo[e];
+      const double g[3][3] = {{-(gr.x + gr.y), gr.x, gr.y}, {gr.x, -(gr.x + gr.z), gr.z}, {gr.y, gr.z, -(gr.y + gr.z)}};
+      double D[3], O[3], Q[3][3], RD[3], RO[3];
+      p2::sym_sums(c, cs, ts, to, w6, D, O);
+      p2::mixed_sums(c, cs, ts, to, p2::B, p2::A, w4, Q);
+      p2::sym_sums(c, cs, p2::B, p2::A, w16, RD, RO);
+      auto R = [&](int i, int j) { return i == j ? RD[i] : RO[p2::third(i, j)]; };
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        K[i][i] = D[i] * g[i][i];
+#pragma unroll
+        for (int j = 0; j < i; j++) K[i][j] = K[j][i] = O[p2::third(i, j)] * g[i][j];
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+          const int q = (j + 1) % 3;  // edge j joins j and q
+          K[i][3 + j] = K[3 + j][i] = fma(Q[i][q], g[i][j], Q[i][j] * g[i][q]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        const int q = (i + 1) % 3;
+        K[3 + i][3 + i] = fma(R(q, q), g[i][i], fma(2 * R(i, q), g[i][q], R(i, i) * g[q][q]));
+#pragma unroll
+        for (int j = 0; j < i; j++) {
+          const int s = (j + 1) % 3;
+          K[3 + i][3 + j] = K[3 + j][3 + i] =
+              fma(R(q, s), g[i][j], fma(R(q, j), g[i][s], fma(R(i, s), g[q][j], R(i, j) * g[q][s])));
+        }
+      }
+    } else {
+      constexpr double w2[2] = {2 * p2::W[0], 2 * p2::W[1]};
+      constexpr double hs[2] = {p2::B[0] * (2 * p2::B[0] - 1), p2::B[1] * (2 * p2::B[1] - 1)};
+      constexpr double ho[2] = {p2::A[0] * (2 * p2::A[0] - 1), p2::A[1] * (2 * p2::A[1] - 1)};
+      constexpr double es[2] = {4 * p2::A[0] * p2::A[0], 4 * p2::A[1] * p2::A[1]};
+      constexpr double eo[2] = {4 * p2::A[0] * p2::B[0], 4 * p2::A[1] * p2::B[1]};
+      const double ar = area[e];
+      double D[3], O[3], M[3][3], ED[3], EO[3];
+      p2::sym_sums(c, cs, hs, ho, w2, D, O);
+      p2::mixed_sums(c, cs, hs, ho, es, eo, w2, M);
+      p2::sym_sums(c, cs, es, eo, w2, ED, EO);
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        K[i][i] = ar * D[i];
+        K[p2::edge_opp(i)][p2::edge_opp(i)] = ar * ED[i];
+#pragma unroll
+        for (int j = 0; j < i; j++) {
+          K[i][j] = K[j][i] = ar * O[p2::third(i, j)];
+          K[p2::edge_opp(i)][p2::edge_opp(j)] = K[p2::edge_opp(j)][p2::edge_opp(i)] = ar * EO[p2::third(i, j)];
+        }
+#pragma unroll
+        for (int j = 0; j < 3; j++) K[i][p2::edge_opp(j)] = K[p2::edge_opp(j)][i] = ar * M[i][j];
+      }
+    }
+    double2* out = reinterpret_cast<double2*>(ke + 36 * e);
+#pragma unroll
+    for (int a = 0; a < 6; a++)
+#pragma unroll
+      for (int b = 0; b < 3; b++) out[3 * a + b] = make_double2(K[a][2 * b], K[a][2 * b + 1]);
+  }
+}
+
+// Gradient factors of the P2 basis at point k of the rule: t[a] = 4 l_a - 1 (vertex a), l4[a] = 4 l_a
+// (edge (p, q) has 4 l_q grad_p + 4 l_p grad_q)
+__device__ __forceinline__ void p2_factors(int k, double (&t)[3], double (&l4)[3]) {
+  const int o = k >= 3 ? 1 : 0, i = p2::special(k - 3 * o);
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    const double l = a == i ? (o ? p2::B[1] : p2::B[0]) : (o ? p2::A[1] : p2::A[0]);
+    l4[a] = 4 * l;
+    t[a] = 4 * l - 1;
+  }
+}
+
+// Unsummed P2 Laplace COO: a block takes kCooPts Gauss points; one thread per point forms the 21
+// distinct entries from the element's g_ab (51 FP64 operations; recomputing the gradients per row
+// took ~400), all threads write values and indices in order through shared memory.
+// (The points fill every warp of the block: two warps of eight left half of the SM's FP64 pipes
+// idle, 54 instead of 40 us at 39k elements.)
+constexpr int kCooPts = 126, kCooT = 128;  // whole elements
+__global__ void __launch_bounds__(kCooT) k_p2_coo(int64_t ne, const int32_t* __restrict__ dof,
+                                                const double4* __restrict__ geo, const double* __restrict__ coef,
+                                                longlong2* __restrict__ idx, double* __restrict__ vv) {
+  __shared__ double sv[kCooPts][37];
+  __shared__ int32_t sd[kCooPts / 6][6];
+  const int64_t ngp = 6 * ne;
+  for (int64_t g0 = (int64_t)blockIdx.x * kCooPts; g0 < ngp; g0 += (int64_t)gridDim.x * kCooPts) {
+    const int np = (int)std::min<int64_t>(kCooPts, ngp - g0);
+    const int64_t e0 = g0 / 6;
+    const int nel = np / 6;
+    __syncthreads();  // the previous tile has been written
+    for (int t = threadIdx.x; t < 6 * nel; t += kCooT) sd[t / 6][t % 6] = dof[6 * e0 + t];
+    if ((int)threadIdx.x < np) {
+      const int64_t gp = g0 + threadIdx.x, e = gp / 6;
+      const int k = (int)(gp - 6 * e);
+      const double4 gr = geo[e];
+      const double cw = coef[gp] * (6 * p2::W[k >= 3 ? 1 : 0]);
+      const double x = gr.x * cw, y = gr.y * cw, z = gr.z * cw;
+      const double g[3][3] = {{-(x + y), x, y}, {x, -(x + z), z}, {y, z, -(y + z)}};
+      double t[3], l4[3], h[3][3];  // h[i][c] = (edge i's gradient) . grad_c
+      p2_factors(k, t, l4);
+      double* K = sv[threadIdx.x];
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        const int q = (i + 1) % 3;
+#pragma unroll
+        for (int c = 0; c < 3; c++) h[i][c] = fma(l4[q], g[i][c], l4[i] * g[q][c]);
+      }
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        K[6 * i + i] = t[i] * t[i] * g[i][i];
+#pragma unroll
+        for (int j = 0; j < i; j++) K[6 * i + j] = K[6 * j + i] = t[i] * t[j] * g[i][j];
+#pragma unroll
+        for (int j = 0; j < 3; j++) K[6 * (3 + j) + i] = K[6 * i + 3 + j] = t[i] * h[j][i];
+#pragma unroll
+        for (int j = 0; j <= i; j++) {
+          const int s = (j + 1) % 3;
+          K[6 * (3 + i) + 3 + j] = K[6 * (3 + j) + 3 + i] = fma(l4[s], h[i][j], l4[j] * h[i][s]);
+        }
+      }
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < 36 * np; q += kCooT) {
+      const int p = q / 36, m = q - 36 * p, r = m / 6, c = m - 6 * r;
+      const int le = p / 6;
+      __stcs(vv + 36 * g0 + q, sv[p][m]);
+      idx[36 * g0 + q] = make_longlong2(sd[le][r], sd[le][c]);
+    }
+  }
+}
+
+// Its transpose: grad_coef[gp] = sum_pq grad_vv[gp, p, q] (d N_pq / d coef).  The block reads its
+// points' entries in order into shared memory, one thread per point contracts them with the
+// basis' gradient factors to the 3 x 3 matrix of the barycentric gradients, then with the g_ab.
+__global__ void __launch_bounds__(kCooT) k_p2_coo_backward(int64_t ne, const double4* __restrict__ geo,
+                                                         const double* __restrict__ gv, double* __restrict__ out) {
+  __shared__ double sv[kCooPts][37];
+  const int64_t ngp = 6 * ne;
+  for (int64_t g0 = (int64_t)blockIdx.x * kCooPts; g0 < ngp; g0 += (int64_t)gridDim.x * kCooPts) {
+    const int np = (int)std::min<int64_t>(kCooPts, ngp - g0);
+    __syncthreads();
+    if (aligned16(gv)) {
+      for (int q = threadIdx.x; q < 18 * np; q += kCooT) {
+        const double2 v = __ldcs(reinterpret_cast<const double2*>(gv + 36 * g0) + q);
+        const int p = q / 18, m = 2 * (q - 18 * p);
+        sv[p][m] = v.x;
+        sv[p][m + 1] = v.y;
+      }
+    } else {
+      for (int q = threadIdx.x; q < 36 * np; q += kCooT) sv[q / 36][q % 36] = __ldcs(gv + 36 * g0 + q);
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < np) {
+      const int64_t gp = g0 + threadIdx.x, e = gp / 6;
+      const int k = (int)(gp - 6 * e);
+      double t[3], l4[3], S[3][3];
+      p2_factors(k, t, l4);
+      const double* G = sv[threadIdx.x];
+      double y[6][3];
+#pragma unroll
+      for (int p = 0; p < 6; p++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          const int q = (c + 1) % 3, r = (c + 2) % 3;  // edges c = (c, q) and r = (r, c) touch vertex c
+          y[p][c] = fma(t[c], G[6 * p + c], fma(l4[q], G[6 * p + 3 + c], l4[r] * G[6 * p + 3 + r]));
+        }
+#pragma unroll
+      for (int b = 0; b < 3; b++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          const int q = (b + 1) % 3, r = (b + 2) % 3;
+          S[b][c] = fma(t[b], y[b][c], fma(l4[q], y[3 + b][c], l4[r] * y[3 + r][c]));
+        }
+      const double4 gr = geo[e];
+      double v = gr.x * ((S[0][1] + S[1][0]) - (S[0][0] + S[1][1]));
+      v = fma(gr.y, (S[0][2] + S[2][0]) - (S[0][0] + S[2][2]), v);
+      v = fma(gr.z, (S[1][2] + S[2][1]) - (S[1][1] + S[2][2]), v);
+      out[gp] = v * (6 * p2::W[k >= 3 ? 1 : 0]);
+    }
+  }
+}
+
+// P2 values at the Gauss points, one thread per element (SRC: the load's transpose, times w_k)
+template <bool SRC>
+__global__ void __launch_bounds__(kGT) k_p2_to_gauss(int64_t ne, const int32_t* __restrict__ dof,
+                                                     const double* __restrict__ area, const double* __restrict__ u,
+                                                     double* __restrict__ out) {
+  for (int64_t e = gtid(); e < ne; e += gstride()) {
+    const int2* d = reinterpret_cast<const int2*>(dof + 6 * e);
+    const int2 a = __ldg(d), b = __ldg(d + 1), c = __ldg(d + 2);
+    const double v[6] = {__ldg(u + a.x), __ldg(u + a.y), __ldg(u + b.x), __ldg(u + b.y), __ldg(u + c.x), __ldg(u + c.y)};
+    double o[6];
+    if (SRC) {
+      constexpr double w[2] = {2 * p2::W[0], 2 * p2::W[1]};
+      const double ar = area[e];
+      p2::at_points(v, [&](int k, double x) { o[k] = ar * x; }, w);
+    } else {
+      constexpr double one[2] = {1.0, 1.0};
+      p2::at_points(v, [&](int k, double x) { o[k] = x; }, one);
+    }
+    if (aligned16(out)) {
+      double2* q = reinterpret_cast<double2*>(out + 6 * e);
+#pragma unroll
+      for (int k = 0; k < 3; k++) q[k] = make_double2(o[2 * k], o[2 * k + 1]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 6; k++) out[6 * e + k] = o[k];
+    }
+  }
 }
 
 // ---------------------------------------------------------------- unsummed COO
@@ -510,6 +849,78 @@ __global__ void __launch_bounds__(BT) k_gen_rows(int64_t ndof, int64_t nnz, cons
   }
 }
 
+// Summed rows of a scalar operator, one thread per DOF row as above.  The rows of the element
+// matrices of four incident elements are loaded before they are added (the walk is a chain of
+// dependent loads), and the write-out finds the row of an entry in a table of bytes that the
+// rows' threads fill, instead of a search per entry.
+template <int DEG, int BT, int CAP>
+__global__ void __launch_bounds__(BT) k_gen_scalar_rows(int64_t ndof, const int32_t* __restrict__ rowptr,
+                                                        const int32_t* __restrict__ inc_ptr,
+                                                        const uint4* __restrict__ inc, const double* __restrict__ ke,
+                                                        double* __restrict__ vals) {
+  constexpr int ND = Tab<DEG>::ND;
+  static_assert(BT <= 256, "a row of the tile is a byte");
+  __shared__ double buf[CAP][BT];
+  __shared__ uint8_t owner[CAP * BT];
+  const int tid = threadIdx.x;
+  const int64_t i0 = (int64_t)blockIdx.x * BT, i = i0 + tid;
+  const int nrow = (int)std::min<int64_t>(BT, ndof - i0);
+  const int32_t b0 = rowptr[i0], total = rowptr[i0 + nrow] - b0;
+  if (tid < nrow) {
+    const int32_t p0 = rowptr[i], len = rowptr[i + 1] - p0;
+    const bool fits = len <= CAP;
+    const int32_t s0 = inc_ptr[i], s1 = inc_ptr[i + 1];
+    double* row = vals + p0;
+    for (int j = 0; j < len; j++) {
+      if (fits) buf[j][tid] = 0.0;
+      else row[j] = 0.0;
+      if (p0 - b0 + j < CAP * BT) owner[p0 - b0 + j] = (uint8_t)tid;
+    }
+    auto load = [&](const uint4& r, double (&v)[ND]) {
+      const double* K = ke + ((int64_t)r.x * ND + r.y) * ND;
+      if constexpr (ND == 6) {
+        load6(K, v);
+      } else {
+#pragma unroll
+        for (int b = 0; b < ND; b++) v[b] = __ldg(K + b);
+      }
+    };
+    auto add = [&](const uint4& r, const double (&v)[ND]) {
+#pragma unroll
+      for (int b = 0; b < ND; b++) {
+        const int j = (int)space_off(r, b);
+        if (fits) buf[j][tid] += v[b];
+        else row[j] += v[b];
+      }
+    };
+    constexpr int U = 4;
+    for (int32_t s = s0; s < s1; s += U) {
+      uint4 r[U];
+      double v[U][ND];
+#pragma unroll
+      for (int u = 0; u < U; u++) r[u] = s + u < s1 ? inc[s + u] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (s + u < s1) load(r[u], v[u]);
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (s + u < s1) add(r[u], v[u]);
+    }
+  }
+  __syncthreads();
+  for (int32_t q = tid; q < total; q += BT) {
+    int r = nrow - 1;
+    if (q < CAP * BT) {
+      r = owner[q];
+    } else {  // (only where rows longer than the buffer make the tile longer than the table)
+      while (r > 0 && rowptr[i0 + r] - b0 > q) r--;
+    }
+    const int32_t p0 = rowptr[i0 + r];
+    if (rowptr[i0 + r + 1] - p0 > CAP) continue;  // that row was summed in place
+    vals[b0 + q] = buf[q - (p0 - b0)][r];
+  }
+}
+
 // ---------------------------------------------------------------- load vector
 template <int DEG>
 __global__ void __launch_bounds__(kGT) k_gen_source(int64_t ndof, const int32_t* __restrict__ inc_ptr,
@@ -523,9 +934,7 @@ __global__ void __launch_bounds__(kGT) k_gen_source(int64_t ndof, const int32_t*
     double acc = accumulate ? rhs[i] : 0.0;
     for (int32_t s = inc_ptr[i]; s < inc_ptr[i + 1]; s++) {
       const uint4 r = inc[s];
-      const double ar = area[r.x];
-#pragma unroll
-      for (int k = 0; k < NG; k++) acc += f[(int64_t)r.x * NG + k] * T.h[k][r.y] * weight_at(T, k, ar);
+      acc = fma(area[r.x], point_sum<NG>(f + (int64_t)r.x * NG, [&](int k) { return T.hw[k][r.y]; }), acc);
     }
     rhs[i] = acc;
   }
@@ -598,8 +1007,7 @@ __global__ void __launch_bounds__(kGT) k_gen_to_gauss_backward(int64_t nrow, con
         e = r.x;
         a = (int)r.y;
       }
-#pragma unroll
-      for (int k = 0; k < NG; k++) acc += gout[e * NG + k] * (VERT ? T.l[k][a] : T.h[k][a]);
+      acc += point_sum<NG>(gout + e * NG, [&](int k) { return VERT ? T.l[k][a] : T.h[k][a]; });
     }
     gu[i] = acc;
   }
@@ -646,16 +1054,20 @@ __global__ void __launch_bounds__(kRowBTs) k_gen_poisson_rows(
   for (int32_t s = inc_ptr[i]; s < inc_ptr[i + 1]; s++) {
     const uint4 rec = inc[s];
     const int a = (int)rec.y;
-    const double* K = ke + ((int64_t)rec.x * ND + a) * ND;
+    double K[ND];
+    if constexpr (ND == 6) {
+      load6(ke + ((int64_t)rec.x * ND + a) * ND, K);
+    } else {
+#pragma unroll
+      for (int b = 0; b < ND; b++) K[b] = __ldg(ke + ((int64_t)rec.x * ND + a) * ND + b);
+    }
 #pragma unroll
     for (int b = 0; b < ND; b++) {
       const unsigned o = space_off(rec, b);
       if (!ADFEM_DCHECK(o < (unsigned)w && o < (unsigned)MAXW)) continue;
       acc[o][t] += K[b];
     }
-    const double ar = area[rec.x];
-#pragma unroll
-    for (int k = 0; k < NG; k++) r += f[(int64_t)rec.x * NG + k] * T.h[k][a] * weight_at(T, k, ar);
+    r = fma(area[rec.x], point_sum<NG>(f + (int64_t)rec.x * NG, [&](int k) { return T.hw[k][a]; }), r);
   }
   if (tag == 2) {
     for (int k = 0; k < w; k++) {
@@ -750,7 +1162,8 @@ cudaError_t launch_gen_coo(const Mesh& m, const Space& sp, GenOp op, const doubl
   const double2* grad = m.d_grad.as<double2>();
   if (op == GenOp::LAPLACE)
     GEN_DISPATCH(sp, (k_gen_coo<1, 0><<<g, kGT, 0, st>>>(m.ne, dof, area, grad, coef, indices, vv)),
-                 (k_gen_coo<2, 0><<<g, kGT, 0, st>>>(m.ne, dof, area, grad, coef, indices, vv)));
+                 (k_p2_coo<<<grid_for(6 * m.ne, kCooPts), kCooT, 0, st>>>(m.ne, dof, m.d_geo.as<double4>(), coef,
+                                                                       reinterpret_cast<longlong2*>(indices), vv)));
   else
     GEN_DISPATCH(sp, (k_gen_coo<1, 1><<<g, kGT, 0, st>>>(m.ne, dof, area, grad, coef, indices, vv)),
                  (k_gen_coo<2, 1><<<g, kGT, 0, st>>>(m.ne, dof, area, grad, coef, indices, vv)));
@@ -766,7 +1179,8 @@ cudaError_t launch_gen_coo_backward(const Mesh& m, const Space& sp, GenOp op, co
   const double2* grad = m.d_grad.as<double2>();
   if (op == GenOp::LAPLACE)
     GEN_DISPATCH(sp, (k_gen_coo_backward<1, 0><<<g, 64 * 3, 0, st>>>(m.ne, area, grad, grad_vv, grad_coef)),
-                 (k_gen_coo_backward<2, 0><<<g, 64 * 6, 0, st>>>(m.ne, area, grad, grad_vv, grad_coef)));
+                 (k_p2_coo_backward<<<grid_for(ngp, kCooPts), kCooT, 0, st>>>(m.ne, m.d_geo.as<double4>(), grad_vv,
+                                                                           grad_coef)));
   else
     GEN_DISPATCH(sp, (k_gen_coo_backward<1, 1><<<g, 64 * 3, 0, st>>>(m.ne, area, grad, grad_vv, grad_coef)),
                  (k_gen_coo_backward<2, 1><<<g, 64 * 6, 0, st>>>(m.ne, area, grad, grad_vv, grad_coef)));
@@ -797,33 +1211,41 @@ cudaError_t launch_gen_stiffness_coo_backward(const Mesh& m, const Space& sp, co
 }
 
 constexpr int kRowBT = 128;     // rows per block of the row gathers
-constexpr int kRowCap1 = 32;    // buffered entries per scalar row
+constexpr int kRowCap0 = 20;    // buffered entries per scalar row (P2 vertices of valence up to 6: 19)
+constexpr int kRowCap1 = 32;    // the same for longer rows
 constexpr int kRowCap2 = 48;    // buffered entries per elasticity row (x and y columns)
+
+// element matrices of the space's operator
+static void launch_ke(const Mesh& m, const Space& sp, GenOp op, const double* coef, double* ke, cudaStream_t st) {
+  const int g = grid_for(m.ne);
+  const double* area = sp.d_area.as<double>();
+  const double2* grad = m.d_grad.as<double2>();
+  const double4* geo = m.d_geo.as<double4>();
+  if (op == GenOp::LAPLACE)
+    GEN_DISPATCH(sp, (k_gen_ke<1, 0><<<g, kGT, 0, st>>>(m.ne, area, grad, coef, ke)),
+                 (k_p2_ke<0><<<g, kGT, 0, st>>>(m.ne, geo, area, coef, ke)));
+  else
+    GEN_DISPATCH(sp, (k_gen_ke<1, 1><<<g, kGT, 0, st>>>(m.ne, area, grad, coef, ke)),
+                 (k_p2_ke<1><<<g, kGT, 0, st>>>(m.ne, geo, area, coef, ke)));
+}
 
 cudaError_t launch_gen_matrix(const Mesh& m, const Space& sp, GenOp op, const double* coef, double* ke, double* vals,
                               bool transpose, cudaStream_t st) {
   (void)transpose;  // Laplace and mass element matrices are symmetric: CSR and CSC values agree
-  const int g = grid_for(m.ne);
-  const double* area = sp.d_area.as<double>();
-  const double2* grad = m.d_grad.as<double2>();
-  if (op == GenOp::LAPLACE)
-    GEN_DISPATCH(sp, (k_gen_ke<1, 0><<<g, kGT, 0, st>>>(m.ne, area, grad, coef, ke)),
-                 (k_gen_ke<2, 0><<<g, kGT, 0, st>>>(m.ne, area, grad, coef, ke)));
-  else
-    GEN_DISPATCH(sp, (k_gen_ke<1, 1><<<g, kGT, 0, st>>>(m.ne, area, grad, coef, ke)),
-                 (k_gen_ke<2, 1><<<g, kGT, 0, st>>>(m.ne, area, grad, coef, ke)));
+  launch_ke(m, sp, op, coef, ke, st);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  const int gr = grid_for(sp.ndof, kRowBT);
-  const size_t smem = sizeof(double) * kRowCap1 * kRowBT;
   const int32_t* rp = sp.d_rowptr.as<int32_t>();
   const int32_t* ip = sp.d_inc_ptr.as<int32_t>();
   const uint4* inc = sp.d_inc.as<uint4>();
-  GEN_DISPATCH(sp,
-               (k_gen_rows<1, 1, kRowBT, kRowCap1><<<gr, kRowBT, smem, st>>>(sp.ndof, sp.nnz, rp, ip, inc, ke, vals,
-                                                                              false)),
-               (k_gen_rows<2, 1, kRowBT, kRowCap1><<<gr, kRowBT, smem, st>>>(sp.ndof, sp.nnz, rp, ip, inc, ke, vals,
-                                                                              false)));
+  const unsigned gr = (unsigned)((sp.ndof + kRowBT - 1) / kRowBT);
+  // (the smaller buffer where it holds every row: a third more blocks fit an SM)
+  if (sp.maxrow <= kRowCap0)
+    GEN_DISPATCH(sp, (k_gen_scalar_rows<1, kRowBT, kRowCap0><<<gr, kRowBT, 0, st>>>(sp.ndof, rp, ip, inc, ke, vals)),
+                 (k_gen_scalar_rows<2, kRowBT, kRowCap0><<<gr, kRowBT, 0, st>>>(sp.ndof, rp, ip, inc, ke, vals)));
+  else
+    GEN_DISPATCH(sp, (k_gen_scalar_rows<1, kRowBT, kRowCap1><<<gr, kRowBT, 0, st>>>(sp.ndof, rp, ip, inc, ke, vals)),
+                 (k_gen_scalar_rows<2, kRowBT, kRowCap1><<<gr, kRowBT, 0, st>>>(sp.ndof, rp, ip, inc, ke, vals)));
   return cudaGetLastError();
 }
 
@@ -831,11 +1253,8 @@ cudaError_t launch_gen_poisson_system(const Mesh& m, const Space& sp, const doub
                                       const uint8_t* isbd, const double* bdval, double* sell_vals, double* rhs,
                                       const int32_t* sptr, const int32_t* diagpos_space, const int32_t* nperm,
                                       const uint8_t* kperm, cudaStream_t st) {
-  const int g = grid_for(m.ne);
   const double* area = sp.d_area.as<double>();
-  const double2* grad = m.d_grad.as<double2>();
-  GEN_DISPATCH(sp, (k_gen_ke<1, 0><<<g, kGT, 0, st>>>(m.ne, area, grad, kappa, ke)),
-               (k_gen_ke<2, 0><<<g, kGT, 0, st>>>(m.ne, area, grad, kappa, ke)));
+  launch_ke(m, sp, GenOp::LAPLACE, kappa, ke, st);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   // (P2 rows of a triangle mesh: 19 entries for a vertex of valence 6, 25 for valence 8)
@@ -910,7 +1329,7 @@ cudaError_t launch_gen_source_backward(const Mesh& m, const Space& sp, const dou
   const int32_t* dof = sp.d_dof.as<int32_t>();
   const double* area = sp.d_area.as<double>();
   GEN_DISPATCH(sp, (k_gen_source_backward<1><<<g, kGT, 0, st>>>(m.ne, dof, area, grad_rhs, grad_f)),
-               (k_gen_source_backward<2><<<g, kGT, 0, st>>>(m.ne, dof, area, grad_rhs, grad_f)));
+               (k_p2_to_gauss<true><<<grid_for(m.ne), kGT, 0, st>>>(m.ne, dof, area, grad_rhs, grad_f)));
   return cudaGetLastError();
 }
 
@@ -924,7 +1343,7 @@ cudaError_t launch_gen_to_gauss(const Mesh& m, const Space& sp, bool vertex_only
                  (k_gen_to_gauss<2, true><<<g, kGT, 0, st>>>(m.ne, conn, dof, u, out)));
   else
     GEN_DISPATCH(sp, (k_gen_to_gauss<1, false><<<g, kGT, 0, st>>>(m.ne, conn, dof, u, out)),
-                 (k_gen_to_gauss<2, false><<<g, kGT, 0, st>>>(m.ne, conn, dof, u, out)));
+                 (k_p2_to_gauss<false><<<grid_for(m.ne), kGT, 0, st>>>(m.ne, dof, nullptr, u, out)));
   return cudaGetLastError();
 }
 
