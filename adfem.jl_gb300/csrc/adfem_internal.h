@@ -332,6 +332,7 @@ int system_solve_packed(adfem_system** sys, int count, double** out, const doubl
 // Device bytes held by a resident system (operator copies, Dirichlet data, solver
 // vectors) -- what the serving loop counts against its HBM budget.
 size_t system_device_bytes(const adfem_system* s);
+bool mg_wanted();
 // Mesh behind a handle (sizes for admission estimates).
 const Mesh* mesh_of(const adfem_mesh* h);
 

@@ -146,16 +146,6 @@ int system_set_bd(adfem_system* s, const long long* bd, long long nbd, const dou
   return ADFEM_OK;
 }
 
-// Solves of resident systems use the multigrid-preconditioned CG unless ADFEM_MG=0 or one of
-// the variables that pick a variant of the Jacobi iterations is set at creation.
-bool mg_wanted() {
-  const char* e = std::getenv("ADFEM_MG");
-  if (e && e[0] == '0') return false;
-  for (const char* v : {"ADFEM_ZCG", "ADFEM_ZCG64", "ADFEM_ZCG_SMAX", "ADFEM_ZCG_RING", "ADFEM_ZCG_RING_REFILL"})
-    if (std::getenv(v)) return false;
-  return true;
-}
-
 // vectors between the reference DOF order and the solver's
 bool mapped(const adfem_system* s) { return s->kind == ADFEM_SYS_ELASTICITY || s->renumbered; }
 int to_solver(adfem_system* s, const double* ref, double* sol, cudaStream_t st) {
@@ -168,6 +158,16 @@ int from_solver(adfem_system* s, const double* sol, double* ref, cudaStream_t st
 }  // namespace
 
 namespace adfem {
+
+// Solves of resident systems use the multigrid-preconditioned CG unless ADFEM_MG=0 or one of
+// the variables that pick a variant of the Jacobi iterations is set at creation.
+bool mg_wanted() {
+  const char* e = std::getenv("ADFEM_MG");
+  if (e && e[0] == '0') return false;
+  for (const char* v : {"ADFEM_ZCG", "ADFEM_ZCG64", "ADFEM_ZCG_SMAX", "ADFEM_ZCG_RING", "ADFEM_ZCG_RING_REFILL"})
+    if (std::getenv(v)) return false;
+  return true;
+}
 
 size_t system_device_bytes(const adfem_system* s) {
   size_t b = 0;

@@ -93,10 +93,21 @@ struct Worker {
 };
 
 constexpr int kPackers = 4;  // packer threads (concurrent packed launches)
-// Default packing threshold: up to ~4k DOFs a system solved by one thread block is about
-// as fast as the whole-GPU solver even alone, and packs of many run at a fraction of the
-// per-solve cost; larger systems are faster on the whole GPU unless many are packed.
-constexpr int kPackDefaultDof = 16384;
+// Default packing thresholds (DOFs).  A pack lasts as long as its slowest system's Jacobi CG,
+// whose iterations grow with the mesh; the resident solver's multigrid keeps some 20 (Poisson) to
+// 60 (elasticity), and its launches do not queue behind a pack that holds the SMs.  GB300, ms per
+// request, packs / resident solver, with 8 workers and with 64 (which fill larger packs):
+//   Poisson     2401 DOFs 0.42 / 0.22, 0.10 / 0.23     6561 0.66 / 0.33, 0.29 / 0.39
+//              16129      1.35 / 0.38, 0.58 / 0.40
+//   elasticity   338 DOFs 0.29 / 0.31, 0.09 / 0.37     1250 1.05 / 0.52, 0.23 / 0.64
+//               4802      3.79 / 1.00, 1.50 / 1.12
+// so the thresholds lie where the two meet, by the number of workers; Poisson stays packed up to
+// 2560 DOFs with few workers too (the launches saved are worth 0.2 ms to the others).  A system
+// that would be solved by Jacobi CG either way is packed up to the same size as before multigrid.
+constexpr int kPackManyWorkers = 32;
+constexpr int kPackPoisson = 2560, kPackPoissonMany = 8192;
+constexpr int kPackElastic = 640, kPackElasticMany = 2560;
+constexpr int kPackDefaultDof = 16384;  // without multigrid
 
 int ndof_of(const adfem::Mesh* m, int kind) { return (int)(kind == ADFEM_SYS_ELASTICITY ? 2 * m->nv : m->nv); }
 
@@ -143,6 +154,7 @@ struct adfem_server {
   std::vector<std::unique_ptr<Worker>> workers;
   // packer
   int pack_max_dof = 0, pack_max = 0;
+  bool default_packs = false;  // thresholds by kind and workers (systems are solved with multigrid)
   std::deque<PackTicket*> pack_queue;
   std::condition_variable cv_pack;       // pack queue non-empty or stopping
   std::condition_variable cv_pack_done;  // a ticket finished
@@ -182,8 +194,13 @@ struct adfem_server {
   // whether a request's solves run in packed launches
   bool goes_packed(const adfem_request& q) const {
     const int prec = q.precision >= 0 ? q.precision : cfg.opts.precision;
-    return pack_max_dof > 0 && prec == ADFEM_PREC_MIXED &&
-           (long long)ndof_of(adfem::mesh_of(q.mesh), q.kind) <= pack_max_dof;
+    int most = pack_max_dof;
+    if (default_packs && q.nbd > 0) {
+      const bool many = cfg.workers >= kPackManyWorkers;
+      most = std::min(most, q.kind == ADFEM_SYS_ELASTICITY ? (many ? kPackElasticMany : kPackElastic)
+                                                           : (many ? kPackPoissonMany : kPackPoisson));
+    }
+    return most > 0 && prec == ADFEM_PREC_MIXED && (long long)ndof_of(adfem::mesh_of(q.mesh), q.kind) <= most;
   }
   Resident* find_free(const adfem_mesh* mesh, int kind) {
     for (auto& r : residents)
@@ -520,6 +537,7 @@ int adfem_server_create(const adfem_server_config* cfg, adfem_server** out) {
   if (S->cfg.workers <= 0) S->cfg.workers = 8;
   if (S->cfg.workers > 256) return adfem::fail(ADFEM_ERR_INVALID, "server: at most 256 workers");
   if (S->cfg.max_queue <= 0) S->cfg.max_queue = 65536;
+  S->default_packs = S->cfg.pack_max_dof == 0 && adfem::mg_wanted();
   S->pack_max_dof = std::min(S->cfg.pack_max_dof == 0 ? kPackDefaultDof : std::max(S->cfg.pack_max_dof, 0),
                              adfem::pack_rows_limit());
   S->pack_max = S->cfg.pack_max <= 0 ? 64 : std::min(S->cfg.pack_max, adfem::kPackMaxSystems);

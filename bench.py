@@ -604,7 +604,7 @@ def run_serve(A, args, rank=0, world=1, dist=None):
                        "ratio 2^(1/4)), 50%% with a misfit gradient (1%% observations), each request's kappa or E "
                        "from its own seed" % len(SERVE_SIZES),
            "workers": args.serve_workers, "rtol": args.serve_rtol,
-           "pack_max_dof": args.serve_pack_max_dof if args.serve_pack_max_dof != 0 else 16384,
+           "pack_max_dof": args.serve_pack_max_dof if args.serve_pack_max_dof != 0 else "library default",
            "setup_s": setup_s, "arms": arms, "accuracy_vs_fp64": acc}
     head = arms.get("mixed") or next(iter(arms.values()))
     out.update({"p50_ms": head["p50_ms"], "p99_ms": head["p99_ms"], "latency_at_load": head["latency_at_load"],
