@@ -18,6 +18,12 @@ __device__ __forceinline__ int colof(const void* c, int64_t idx, int64_t r) {
   else return __ldg(reinterpret_cast<const int32_t*>(c) + idx);
 }
 
+// Programmatic dependent launch (launches with the programmatic-serialization attribute):
+// wait for the previous grid in the stream to complete with its memory visible (a no-op
+// when launched without the attribute), and let the next grid be scheduled.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 template <class T>
 __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll

@@ -46,7 +46,7 @@ struct Vec {
   float v[NB];
 };
 template <int NB>
-__device__ __forceinline__ Vec<NB> load_vec(const float* __restrict__ p, int64_t i) {
+__device__ __forceinline__ Vec<NB> load_vec(const float* p, int64_t i) {
   Vec<NB> r;
   if constexpr (NB == 2) {
     const float2 t = reinterpret_cast<const float2*>(p)[i];
@@ -125,74 +125,157 @@ struct Cols {
   }
 };
 
-// (A x)_r over the LPR lanes of row r (every lane gets the sum)
+// Row r of the level's operator for one of its LPR lanes.  The first group of entries is loaded
+// ahead: the operators do not change while a solve runs, so a kernel has its first rows in
+// registers when the launch before it ends.
 template <int NB, bool D16, int LPR>
-__device__ __forceinline__ Vec<NB> row_product(const MgLev& L, int r, int lane, const float* __restrict__ x) {
-  Vec<NB> acc;
-#pragma unroll
-  for (int c = 0; c < NB; c++) acc.v[c] = 0.0f;
-  const int s0 = __ldg(L.sptr + (r >> 5)), w = (__ldg(L.sptr + (r >> 5) + 1) - s0) >> 5, base = s0 + (r & 31);
-  const Cols<D16> cols(L, r);
+struct RowHead {
   // entries in groups whose loads are all in flight at once
-  constexpr int U = LPR == 1 ? (NB == 1 ? 8 : 4) : 2;
-  for (int k0 = lane; k0 < w; k0 += U * LPR) {
-    int j[U];
+  static constexpr int U = LPR == 1 ? (NB == 1 ? 8 : 4) : 2;
+  float v[U][NB * NB];
+  int j[U];
+  int base = 0, w = 0;
+  __device__ __forceinline__ void load(const MgLev& L, int r, int lane) {
+    const int s0 = __ldg(L.sptr + (r >> 5));
+    w = (__ldg(L.sptr + (r >> 5) + 1) - s0) >> 5;
+    base = s0 + (r & 31);
+    const Cols<D16> cols(L, r);
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      const int k = k0 + u * LPR;
+      const int k = lane + u * LPR;
       j[u] = k < w ? cols.at(k, base + 32 * k) : r;
       if (!ADFEM_DCHECK(j[u] >= 0 && j[u] < L.n)) j[u] = r;
-    }
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      const int k = k0 + u * LPR;
-      if (k < w) block_fma<NB, NB>(L.val, base + 32 * k, L.nv, load_vec<NB>(x, j[u]), acc);
+      if (k < w) load_block<NB, NB>(L.val, base + 32 * k, L.nv, v[u]);
     }
   }
-  if (LPR > 1) lane_sum<NB, LPR>(acc);
-  return acc;
+  // (A x)_r (every lane gets the sum)
+  __device__ __forceinline__ Vec<NB> product(const MgLev& L, int r, int lane, const float* x) const {
+    Vec<NB> acc;
+#pragma unroll
+    for (int c = 0; c < NB; c++) acc.v[c] = 0.0f;
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (lane + u * LPR < w) {
+        const Vec<NB> t = load_vec<NB>(x, j[u]);
+#pragma unroll
+        for (int a = 0; a < NB; a++)
+#pragma unroll
+          for (int c = 0; c < NB; c++) acc.v[a] = fmaf(v[u][a * NB + c], t.v[c], acc.v[a]);
+      }
+    const Cols<D16> cols(L, r);
+    for (int k0 = lane + U * LPR; k0 < w; k0 += U * LPR) {
+      int i[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int k = k0 + u * LPR;
+        i[u] = k < w ? cols.at(k, base + 32 * k) : r;
+        if (!ADFEM_DCHECK(i[u] >= 0 && i[u] < L.n)) i[u] = r;
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int k = k0 + u * LPR;
+        if (k < w) block_fma<NB, NB>(L.val, base + 32 * k, L.nv, load_vec<NB>(x, i[u]), acc);
+      }
+    }
+    if (LPR > 1) lane_sum<NB, LPR>(acc);
+    return acc;
+  }
+};
+
+// Sums over a grid: every block leaves its partial sum (block_partial), and the kernel that needs
+// the total forms it in each of its blocks, in one order, from the same words (grid_total).  The
+// kernel boundary in between is there anyway; a last block that adds up instead costs every block
+// a fence and a count (some 2 us in which its place on the SM is idle) and the registers of the
+// addition (last sweep of level 0 with its dot product: 45 against 34 us at 4M rows, 22 against 14 us
+// at 240k rows of P2).
+// A block's values go through shared memory to its first warp, eight to a lane (13 warp additions a
+// block instead of 40 of shuffle trees in every warp); FP32 values are added as FP32 pairs.
+template <class T>
+__device__ __forceinline__ void block_partial(T x, double* partials) {
+  __shared__ T sh[kT];
+  const int lane = threadIdx.x;
+  sh[threadIdx.x] = x;
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  double s;
+  if constexpr (sizeof(T) == 4) {
+    float2 w = make_float2(sh[lane], 0.0f);
+#pragma unroll
+    for (int k = 1; k < kT / 32; k++) w = pair_add(w, make_float2(sh[lane + 32 * k], 0.0f));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) w = pair_add(w, shfl_pair(w, o));
+    s = lane == 0 ? (double)w.x + (double)w.y : 0.0;
+  } else {
+    s = sh[lane];
+#pragma unroll
+    for (int k = 1; k < kT / 32; k++) s += sh[lane + 32 * k];
+    s = warp_sum(s);
+  }
+  if (lane == 0) partials[blockIdx.x] = s;
+}
+// The total as f makes two words of it.  (One warp adds and one thread runs f: an FP64 warp
+// instruction holds the SM's FP64 pipe for 16 cycles, and a division is some twenty of them, one
+// after the other: run by every thread, f cost 7 us a kernel.  So the state keeps reciprocals.
+// f also looks at st->done, which the first block may be setting: a block goes by one reading.)
+template <class F>
+__device__ __forceinline__ double2 grid_total(const double* partials, int count, F f) {
+  __shared__ double2 out;
+  if (threadIdx.x < 32) {
+    constexpr int K = 20;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int b0 = 0; b0 < count; b0 += 32 * K) {
+      double v[K];
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        const int b = b0 + 32 * k + (int)threadIdx.x;
+        v[k] = b < count ? partials[b] : 0.0;
+      }
+#pragma unroll
+      for (int k = 0; k < K; k++)
+        if (b0 + 32 * k < count) s[k & 3] += v[k];
+    }
+    double t = s[0];
+    if (count > 32) t = (t + s[1]) + (s[2] + s[3]);
+    t = warp_sum(t);
+    if (threadIdx.x == 0) out = f(t);
+  }
+  __syncthreads();
+  return out;
 }
 
 // ---------------------------------------------------------------------------
-// V-cycle kernels of the levels above the tail.
+// V-cycle kernels of the levels above the tail.  Every kernel of an iteration is a programmatic
+// dependent launch: its blocks start as the kernel before runs out, load what does not change
+// during a solve, and wait for that kernel before they read or write a vector (an iteration, with
+// the sums below: 277 -> 229 us at 1M unknowns, 235 -> 190 us elasticity at 320k, 57 -> 51 us at 4k).  (So vectors are
+// read by plain loads: the read-only path is for data that is constant while a kernel lives.)
 enum { kPre = 0, kStep = 1, kRes = 2, kLast = 3 };
-
-// r.z of the cycle (each thread's part), and beta from it
-__device__ __forceinline__ void rz_step(float dot, CgState* st, double* partials) {
-  float v[1] = {dot};
-  double tot[1];
-  if (reduce_grid_w<1, kT, true>(v, partials, &st->counter[0], tot) && threadIdx.x == 0 && !st->done) {
-    const double rz = tot[0] / st->ar;  // (b carries the factor st->ar, and so does z)
-    if (!(rz > 0.0) || !isfinite(rz)) {
-      st->done = 2;
-    } else {
-      st->beta = st->ap != 0.0 ? 0.0 : rz / st->rho;  // (ap: the direction starts anew)
-      st->ap = 0.0;
-      st->rho = rz;
-    }
-  }
-}
 
 // kPre:  two Chebyshev steps from x = 0: x1 = b / theta gathered from b, then step 2
 // kStep: one step: d <- c1 d + c2 (b - A x), out = x + d (c1 index < 0: first step, d unread)
 // kRes:  out = b - A x
-// kLast: kStep whose d is not needed again; on level 0 the products b.out give r.z
+// kLast: kStep whose d is not needed again; on level 0 (partials) also the products b.out, r.z
 template <int NB, bool D16, int LPR, int MODE>
-__global__ void __launch_bounds__(kT) k_mg_sweep(MgLev L, const float* __restrict__ x, float* __restrict__ out,
-                                                 int c1, int c2, int keep_d, CgState* st, double* partials) {
+__global__ void __launch_bounds__(kT) k_mg_sweep(MgLev L, const float* x, float* out, int c1, int c2, int keep_d,
+                                                 double* partials) {
+  pdl_trigger();
   float dot = 0.0f;
   const float th = MODE == kPre ? __ldg(L.coef) : 0.0f;
   const float a1 = c1 >= 0 ? __ldg(L.coef + c1) : 0.0f, a2 = c2 >= 0 ? __ldg(L.coef + c2) : 0.0f;
   const int64_t rows = (int64_t)L.n * LPR;
   const int64_t lim = LPR == 1 ? rows : (rows + 31) / 32 * 32;  // (whole warps stay together in lane_sum)
-  for (int64_t t = gtid(); t < lim; t += gstride()) {
+  int64_t t = gtid();
+  RowHead<NB, D16, LPR> row;
+  if (t < lim) row.load(L, min((int)(t / LPR), L.n - 1), (int)(t % LPR));
+  pdl_wait();
+  for (; t < lim;) {
     const int r0 = (int)(t / LPR), lane = (int)(t % LPR);
     const int r = r0 < L.n ? r0 : L.n - 1;
     const Vec<NB> bi = load_vec<NB>(L.b, r);
     const Vec<NB> xi = MODE == kPre ? bi : load_vec<NB>(x, r);
     Vec<NB> di;
     if ((MODE == kStep || MODE == kLast) && c1 >= 0) di = load_vec<NB>(L.d, r);
-    const Vec<NB> ax = row_product<NB, D16, LPR>(L, r, lane, MODE == kPre ? L.b : x);
+    const Vec<NB> ax = row.product(L, r, lane, MODE == kPre ? L.b : x);
     Vec<NB> o, d;
 #pragma unroll
     for (int c = 0; c < NB; c++) {
@@ -208,36 +291,40 @@ __global__ void __launch_bounds__(kT) k_mg_sweep(MgLev L, const float* __restric
         o.v[c] = xi.v[c] + d.v[c];
       }
     }
-    if (lane != 0 || r0 >= L.n) continue;
-    store_vec<NB>(out, r, o);
-    if ((MODE == kPre || MODE == kStep) && keep_d) store_vec<NB>(L.d, r, d);
-    if (MODE == kLast)
+    if (lane == 0 && r0 < L.n) {
+      store_vec<NB>(out, r, o);
+      if ((MODE == kPre || MODE == kStep) && keep_d) store_vec<NB>(L.d, r, d);
+      if (MODE == kLast)
 #pragma unroll
-      for (int c = 0; c < NB; c++) dot = fmaf(bi.v[c], o.v[c], dot);
+        for (int c = 0; c < NB; c++) dot = fmaf(bi.v[c], o.v[c], dot);
+    }
+    if (MODE != kLast) break;  // (the other modes have a lane group per row)
+    t += gstride();
+    if (t < lim) row.load(L, min((int)(t / LPR), L.n - 1), (int)(t % LPR));
   }
-  if (MODE == kLast && st) rz_step(dot, st, partials);
+  if (MODE == kLast && partials) block_partial(dot, partials);
 }
 
 // The sweeps of level 0 of a scalar system whose rows have at most 8 entries (P1: 7), on the
 // system's own pattern: straight-line code with 32-bit indices, all loads of a step issued
 // together (4M DOF: 23.2 -> 18.8 ms a solve against the generic form's loop; 2 or 3 rows per
 // thread with their loads side by side were no faster, the blocks' occupancy falls as the loads
-// in flight per thread rise).
+// in flight per thread rise).  32 registers, so that eight blocks are resident: 530 instead of
+// 568 us an iteration at 4M DOF with 36 to 38.
 template <int MODE>
-__global__ void __launch_bounds__(kT) k_mg_fine(MgLev L, const float* __restrict__ x, float* __restrict__ out, int c1,
-                                                int c2, CgState* st, double* partials) {
+__global__ void __launch_bounds__(kT, MODE == kLast ? 6 : 8) k_mg_fine(MgLev L, const float* x, float* out, int c1, int c2,
+                                                double* partials) {
+  pdl_trigger();
   constexpr int W = 8;
   const float th = MODE == kPre ? __ldg(L.coef) : 0.0f;
   const float a1 = c1 >= 0 ? __ldg(L.coef + c1) : 0.0f, a2 = c2 >= 0 ? __ldg(L.coef + c2) : 0.0f;
-  const float* __restrict__ g = MODE == kPre ? L.b : x;
+  const float* g = MODE == kPre ? L.b : x;
   float dot = 0.0f;
-  for (int r = blockIdx.x * kT + threadIdx.x; r < L.n; r += gridDim.x * kT) {
+  int j[W];
+  float v[W];
+  auto load = [&](int r) {
     const int sl = r >> 5, s0 = __ldg(L.sptr + sl), w = (__ldg(L.sptr + sl + 1) - s0) >> 5, so = __ldg(L.spat + sl);
     const int idx = s0 + (r & 31);
-    const float bi = __ldg(L.b + r), xi = MODE == kPre ? bi : __ldg(x + r);
-    const float di = (MODE == kStep || MODE == kLast) && c1 >= 0 ? L.d[r] : 0.0f;
-    int j[W];
-    float v[W];
 #pragma unroll
     for (int e = 0; e < W; e++) {
       j[e] = r;
@@ -246,9 +333,18 @@ __global__ void __launch_bounds__(kT) k_mg_fine(MgLev L, const float* __restrict
       v[e] = e < w ? __ldcs(L.val + idx + 32 * e) : 0.0f;
       if (!ADFEM_DCHECK(j[e] >= 0 && j[e] < L.n)) j[e] = r;
     }
-    float ax = 0.0f;
+  };
+  int r = blockIdx.x * kT + threadIdx.x;
+  if (r < L.n) load(r);
+  pdl_wait();
+  while (r < L.n) {
+    const float bi = L.b[r], xi = MODE == kPre ? bi : x[r];
+    const float di = (MODE == kStep || MODE == kLast) && c1 >= 0 ? L.d[r] : 0.0f;
+    float gx[W], ax = 0.0f;
 #pragma unroll
-    for (int e = 0; e < W; e++) ax = fmaf(v[e], __ldg(g + j[e]), ax);
+    for (int e = 0; e < W; e++) gx[e] = g[j[e]];
+#pragma unroll
+    for (int e = 0; e < W; e++) ax = fmaf(v[e], gx[e], ax);
     float o;
     if (MODE == kRes) {
       o = bi - ax;
@@ -262,13 +358,17 @@ __global__ void __launch_bounds__(kT) k_mg_fine(MgLev L, const float* __restrict
       if (MODE == kLast) dot = fmaf(bi, o, dot);
     }
     out[r] = o;
+    if (MODE != kLast) break;  // (the other modes have a thread per row)
+    r += gridDim.x * kT;
+    if (r < L.n) load(r);
   }
-  if (MODE == kLast) rz_step(dot, st, partials);
+  if (MODE == kLast) block_partial(dot, partials);
 }
 
 // out_J = sum_i P_iJ^T r_i
 template <int NB, int NC, int LPR>
-__global__ void __launch_bounds__(kT) k_mg_restrict(MgLev L, const float* __restrict__ r, float* __restrict__ out) {
+__global__ void __launch_bounds__(kT) k_mg_restrict(MgLev L, const float* r, float* out) {
+  pdl_trigger();
   const int64_t t = gtid();
   const int J0 = (int)(t / LPR), lane = (int)(t % LPR);
   const int J = J0 < L.nc ? J0 : L.nc - 1;
@@ -277,13 +377,32 @@ __global__ void __launch_bounds__(kT) k_mg_restrict(MgLev L, const float* __rest
   for (int c = 0; c < NC; c++) acc.v[c] = 0.0f;
   const int s0 = __ldg(L.pt_sptr + (J >> 5)), w = (__ldg(L.pt_sptr + (J >> 5) + 1) - s0) >> 5, base = s0 + (J & 31);
   constexpr int U = LPR == 1 ? 8 : 4;
-  for (int k0 = lane; k0 < w; k0 += U * LPR) {
-    int i[U];
+  int i[U];
+  auto cols = [&](int k0) {
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const int k = k0 + u * LPR;
       i[u] = k < w ? __ldg(L.pt_col + base + 32 * k) : 0;
     }
+  };
+  cols(lane);
+  // (the values of the first group, too)
+  float v[U][NB * NC];
+#pragma unroll
+  for (int u = 0; u < U; u++)
+    if (lane + u * LPR < w) load_block<NC, NB>(L.pt_val, base + 32 * (lane + u * LPR), L.npt, v[u]);
+  pdl_wait();
+#pragma unroll
+  for (int u = 0; u < U; u++)
+    if (lane + u * LPR < w) {
+      const Vec<NB> x = load_vec<NB>(r, i[u]);
+#pragma unroll
+      for (int a = 0; a < NC; a++)
+#pragma unroll
+        for (int c = 0; c < NB; c++) acc.v[a] = fmaf(v[u][a * NB + c], x.v[c], acc.v[a]);
+    }
+  for (int k0 = lane + U * LPR; k0 < w; k0 += U * LPR) {
+    cols(k0);
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const int k = k0 + u * LPR;
@@ -296,22 +415,38 @@ __global__ void __launch_bounds__(kT) k_mg_restrict(MgLev L, const float* __rest
 
 // x_i += sum_J P_iJ xc_J
 template <int NB, int NC>
-__global__ void __launch_bounds__(kT) k_mg_prolong(MgLev L, const float* __restrict__ xc, float* __restrict__ x) {
+__global__ void __launch_bounds__(kT) k_mg_prolong(MgLev L, const float* xc, float* x) {
+  pdl_trigger();
   const int64_t t = gtid();
-  if (t >= L.n) return;
-  const int i = (int)t;
+  const int i = (int)min(t, (int64_t)L.n - 1);
   const int s0 = __ldg(L.p_sptr + (i >> 5)), w = (__ldg(L.p_sptr + (i >> 5) + 1) - s0) >> 5, base = s0 + (i & 31);
-  Vec<NB> acc = load_vec<NB>(x, i);
   constexpr int U = 4;
-  for (int k0 = 0; k0 < w; k0 += U) {
-    int J[U];
+  int J[U];
+  float v[U][NB * NC];
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    J[u] = u < w ? __ldg(L.p_col + base + 32 * u) : 0;
+    if (u < w) load_block<NB, NC>(L.p_val, base + 32 * u, L.np, v[u]);
+  }
+  pdl_wait();
+  Vec<NB> acc = load_vec<NB>(x, i);
+#pragma unroll
+  for (int u = 0; u < U; u++)
+    if (u < w) {
+      const Vec<NC> y = load_vec<NC>(xc, J[u]);
+#pragma unroll
+      for (int a = 0; a < NB; a++)
+#pragma unroll
+        for (int c = 0; c < NC; c++) acc.v[a] = fmaf(v[u][a * NC + c], y.v[c], acc.v[a]);
+    }
+  for (int k0 = U; k0 < w; k0 += U) {
 #pragma unroll
     for (int u = 0; u < U; u++) J[u] = k0 + u < w ? __ldg(L.p_col + base + 32 * (k0 + u)) : 0;
 #pragma unroll
     for (int u = 0; u < U; u++)
       if (k0 + u < w) block_fma<NB, NC>(L.p_val, base + 32 * (k0 + u), L.np, load_vec<NC>(xc, J[u]), acc);
   }
-  store_vec<NB>(x, i, acc);
+  if (t < L.n) store_vec<NB>(x, i, acc);
 }
 
 // ---------------------------------------------------------------------------
@@ -347,7 +482,8 @@ struct TailArgs {
   const float* b;
   float* x;
   int reps;
-  int dot;       // level 0 in the tail: r.z from here
+  int dot;       // level 0 in the tail: r.z from here, to rz
+  double* rz;
   CgState* st;
 };
 struct TailVecs {
@@ -682,6 +818,7 @@ __global__ void __launch_bounds__(kTailT, 1) k_mg_tail(const __grid_constant__ T
     sm += tail_floats(n, nb, ex);
   }
   TailSync sync{bars, tokens, rank, a.st};
+  pdl_wait();
   const int n0 = a.L[0].n * NT, own0 = (v[0].r1 - v[0].r0) * NT, off0 = v[0].r0 * NT;
   for (int t = threadIdx.x; t < n0; t += T) v[0].y[t] = a.b[t];
   for (int t = threadIdx.x; t < own0; t += T) v[0].b[t] = a.b[off0 + t];
@@ -733,6 +870,7 @@ __global__ void __launch_bounds__(kTailT, 1) k_mg_tail(const __grid_constant__ T
       tail_smooth<EX, NT, T>(sync, L, v[0], deg, false, false);
     }
   }
+  pdl_trigger();  // (not before: blocks that wait would keep other solves' kernels off the SMs)
   float dot = 0.0f;
   for (int t = threadIdx.x; t < own0; t += T) {
     const float xi = v[0].x[off0 + t];
@@ -746,20 +884,13 @@ __global__ void __launch_bounds__(kTailT, 1) k_mg_tail(const __grid_constant__ T
       if (threadIdx.x == 0) store_rank(dots + rank, 0, w[0]);
       cluster_barrier();
     }
-    if (rank == 0 && threadIdx.x == 0 && !a.st->done) {
+    if (rank == 0 && threadIdx.x == 0) {
       float tot = w[0];
       if (EX) {
         tot = 0.0f;
         for (int k = 0; k < kTailC; k++) tot += dots[k];
       }
-      const double rz = (double)tot / a.st->ar;  // (b carries the factor st->ar, and so does z)
-      if (!(rz > 0.0) || !isfinite(rz)) {
-        a.st->done = 2;
-      } else {
-        a.st->beta = a.st->ap != 0.0 ? 0.0 : rz / a.st->rho;
-        a.st->ap = 0.0;
-        a.st->rho = rz;
-      }
+      a.rz[0] = (double)tot;
     }
   }
 }
@@ -1241,12 +1372,14 @@ __global__ void __launch_bounds__(kT) k_mg_init(int64_t n, const double* __restr
     // scale of the FP32 right-hand sides of the cycle
     const double g = tot[0] > 0.0 ? rsqrt(tot[0]) : 1.0;
     st->ar = isfinite(g) ? g : 1.0;
+    st->iar = 1.0 / st->ar;
   }
 }
 
 // The residual decides: converged, at its attainable floor, out of iterations, or go on (the
 // rules of replacement_step64, whose direction scalars do not apply here).
-__device__ __forceinline__ void mg_residual_step(CgState* st, double rr, bool first) {
+// rn: the recurrence's residual (its square, as rr)
+__device__ __forceinline__ void mg_residual_step(CgState* st, double rr, double rn, bool first) {
   const double prev = st->last_rr64;
   st->rr64 = rr;
   st->last_rr64 = rr;
@@ -1259,7 +1392,7 @@ __device__ __forceinline__ void mg_residual_step(CgState* st, double rr, bool fi
     return;
   }
   if (!first) {
-    const bool dropped = st->rho_new <= st->delta2 * prev;
+    const bool dropped = rn <= st->delta2 * prev;
     if (prev > 0.0 && rr > 0.0625 * prev && (dropped || st->final_seen)) {
       st->floor_hit = 1;
       st->done = 1;
@@ -1270,31 +1403,53 @@ __device__ __forceinline__ void mg_residual_step(CgState* st, double rr, bool fi
     st->done = 4;
     return;
   }
-  if (st->final_req) st->final_seen = 1;
-  st->final_req = 0;
+  if (!first && rn <= st->stop2) st->final_seen = 1;
   if (!first) st->updates += 1;
   // A residual that is not the recurrence's (near the attainable floor it can be many times
   // larger) has nothing to do with the directions so far: keeping them made the iteration
   // stagnate (elasticity, 320k DOF: over 200 iterations to the floor instead of 10).
-  if (first || rr > 1.21 * st->rho_new) st->ap = 1.0;
+  if (first || rr > 1.21 * rn) st->ap = 1.0;
+  st->fold = 1;
   st->ru2 = st->delta2 * rr;
   st->done = 0;
 }
 
 // r = b - K y in FP64, in difference form: row sums times the row's own unknowns plus entries
 // times differences, so that it rounds with the differences of the solution.
-// mode 0: start, 1: when due (st->done == 3), also the end of an iteration (sets the loop's
-// condition), 2: final value only
+// The iterate is y + z; the next direction kernel folds z into y (st->fold).
+// mode 0: start, 1: the end of an iteration (evaluated when the recurrence has met the tolerance,
+// has dropped far enough, or ends; sets the loop's condition), 2: final value only
 template <bool D16, int NB>
 __global__ void __launch_bounds__(kT) k_mg_residual(int64_t n, const int32_t* __restrict__ sptr,
                                                     const void* __restrict__ col, const double* __restrict__ val,
                                                     const double* __restrict__ rowsum, const float* __restrict__ sc,
-                                                    const double* __restrict__ b, const double* __restrict__ y,
-                                                    double* __restrict__ r64, float* __restrict__ b32, CgState* st,
+                                                    const double* b, const double* y, const double* z,
+                                                    double* r64, float* b32, CgState* st,
+                                                    const double* rn_part, int rn_count,
                                                     double* partials, int mode, cudaGraphConditionalHandle loop) {
-  if (mode == 1 && st->done != 3) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(loop, st->done == 0 ? 1 : 0);
-    return;
+  pdl_trigger();
+  pdl_wait();
+  const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+  double rn = 0.0;
+  if (mode == 1) {
+    const double2 v = grid_total(rn_part, rn_count, [&](double t) {
+      return make_double2(t * st->iar * st->iar, st->done ? 1.0 : 0.0);
+    });
+    if (v.y != 0.0) {
+      if (lead) cudaGraphSetConditional(loop, 0);
+      return;
+    }
+    rn = v.x;
+    const bool due = rn <= st->stop2 || rn <= st->ru2 || st->it >= st->max_iter;
+    if (!isfinite(rn) || !due) {
+      if (lead) {
+        st->iters = st->it;
+        st->rho_new = rn;
+        if (!isfinite(rn)) st->done = 2;
+        cudaGraphSetConditional(loop, isfinite(rn) ? 1 : 0);
+      }
+      return;
+    }
   }
   const double g = st->ar;
   double a0 = 0.0;
@@ -1305,7 +1460,7 @@ __global__ void __launch_bounds__(kT) k_mg_residual(int64_t n, const int32_t* __
     double yo[NB], s = 0.0;
 #pragma unroll
     for (int q = 0; q < NB; q++) {
-      yo[q] = y[r / NB * NB + q];
+      yo[q] = y[r / NB * NB + q] + z[r / NB * NB + q];
       s = fma(rowsum[NB * r + q], yo[q], s);
     }
     constexpr int U = 8;
@@ -1321,7 +1476,7 @@ __global__ void __launch_bounds__(kT) k_mg_residual(int64_t n, const int32_t* __
           j = colof<D16>(col, idx, r);
           if (!ADFEM_DCHECK(j >= 0 && j < n)) j = (int)r;
         }
-        x[u] = __ldg(y + j);
+        x[u] = y[j] + z[j];
       }
 #pragma unroll
       for (int u = 0; u < U; u++)
@@ -1336,23 +1491,41 @@ __global__ void __launch_bounds__(kT) k_mg_residual(int64_t n, const int32_t* __
   }
   double v[1] = {a0}, tot[1];
   if (reduce_grid<double, 1>(v, partials, &st->counter[1], tot) && threadIdx.x == 0) {
-    if (mode == 2) st->rr64 = tot[0];
-    else mg_residual_step(st, tot[0], mode == 0);
+    if (mode == 2) {
+      st->rr64 = tot[0];
+      return;
+    }
+    st->iters = st->it;
+    st->rho_new = rn;
+    mg_residual_step(st, tot[0], rn, mode == 0);
     if (mode == 1) cudaGraphSetConditional(loop, st->done == 0 ? 1 : 0);
   }
 }
 
-// p = S z + beta p, two unknowns per thread
-__global__ void __launch_bounds__(kT) k_mg_dir(int64_t n, const float* __restrict__ z, const float* __restrict__ s,
-                                               double* __restrict__ p, const CgState* st) {
-  if (st->done) return;
-  const double bt = st->beta;
-  const bool first = bt == 0.0;
+// p = S c + beta p (c: the cycle's correction, its r.z in rz_part), and after a residual
+// evaluation y += z, z = 0; two unknowns per thread
+__global__ void __launch_bounds__(kT) k_mg_dir(int64_t n, const float* c, const float* __restrict__ s, double* p,
+                                               double* y, double* z, CgState* st, const double* rz_part,
+                                               int rz_count) {
+  pdl_trigger();
+  pdl_wait();
+  const bool first = st->ap != 0.0;  // (the direction starts anew)
+  const double2 v = grid_total(rz_part, rz_count, [&](double t) {
+    const double rz = t * st->iar;  // (b carries the factor st->ar, and so does z)
+    const bool ok = rz > 0.0 && isfinite(rz) && !st->done;
+    if (blockIdx.x == 0 && !st->done) {
+      if (ok) st->rz = rz;
+      else st->done = 2;
+    }
+    return make_double2(ok ? 1.0 : 0.0, ok && !first ? rz * st->irz : 0.0);
+  });
+  if (v.x == 0.0) return;
+  const double bt = v.y;
   const int64_t n2 = n >> 1;
-#pragma unroll 2
+#pragma unroll 4
   for (int64_t i = gtid(); i < n2; i += gstride()) {
-    const float2 z2 = __ldg(reinterpret_cast<const float2*>(z) + i), s2 = __ldg(reinterpret_cast<const float2*>(s) + i);
-    double2 q = make_double2((double)(s2.x * z2.x), (double)(s2.y * z2.y));
+    const float2 c2 = reinterpret_cast<const float2*>(c)[i], s2 = __ldg(reinterpret_cast<const float2*>(s) + i);
+    double2 q = make_double2((double)(s2.x * c2.x), (double)(s2.y * c2.y));
     if (!first) {
       const double2 o = reinterpret_cast<const double2*>(p)[i];
       q.x = fma(bt, o.x, q.x);
@@ -1361,23 +1534,98 @@ __global__ void __launch_bounds__(kT) k_mg_dir(int64_t n, const float* __restric
     reinterpret_cast<double2*>(p)[i] = q;
   }
   if ((n & 1) && gtid() == 0) {
-    const double zi = (double)(s[n - 1] * z[n - 1]);
-    p[n - 1] = first ? zi : fma(bt, p[n - 1], zi);
+    const double ci = (double)(s[n - 1] * c[n - 1]);
+    p[n - 1] = first ? ci : fma(bt, p[n - 1], ci);
   }
+  if (st->fold)
+    for (int64_t i = gtid(); i < n; i += gstride()) {
+      y[i] += z[i];
+      z[i] = 0.0;
+    }
+}
+
+// q = K p and p.q, one row per thread, entries in groups of 8, the first loaded ahead (MORE: rows
+// may have more: P2, elasticity)
+template <bool D16, bool MORE>
+__global__ void __launch_bounds__(kT, MORE ? 3 : 4) k_mg_spmv(int64_t n, const int32_t* __restrict__ sptr,
+                                                   const void* __restrict__ col, const int32_t* __restrict__ spat,
+                                                   const int16_t* __restrict__ pat, int period,
+                                                   const double* __restrict__ val, const double* p, double* q,
+                                                   CgState* st, double* partials) {
+  constexpr int W = MORE ? 12 : 8;
+  pdl_trigger();
+  double v[W], acc = 0.0;
+  int j[W], w = 0;
+  int64_t base = 0;
+  const int16_t* pp = nullptr;
+  auto entries = [&](int r, int k0) {
+#pragma unroll
+    for (int u = 0; u < W; u++) {
+      const int k = k0 + u;
+      const int64_t idx = base + 32 * k;
+      v[u] = k < w ? __ldg(val + idx) : 0.0;
+      j[u] = r;
+      if (k < w) j[u] = pp ? r + (int)__ldg(pp + k) : colof<D16>(col, idx, r);
+      if (!ADFEM_DCHECK(j[u] >= 0 && j[u] < n)) j[u] = r;
+    }
+  };
+  auto load = [&](int r) {
+    sell_row(sptr, r, base, w);
+    const int32_t so = __ldg(spat + (r >> 5));
+    pp = so >= 0 ? pat + so + (period == 2 ? (r & 1) * w : 0) : nullptr;
+    entries(r, 0);
+  };
+  int r = blockIdx.x * kT + threadIdx.x;
+  const int rows = (int)n;
+  if (r < rows) load(r);
+  pdl_wait();
+  if (st->done) return;
+  // (state that the kernels before and after read and this one does not)
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    st->it += 1;
+    st->irz = 1.0 / st->rz;
+    st->ap = 0.0;
+    st->fold = 0;
+  }
+  while (r < rows) {
+    const double pr = p[r];
+    double s = 0.0;
+#pragma unroll
+    for (int u = 0; u < W; u++)
+      if (u < w) s = fma(v[u], p[j[u]], s);
+    if (MORE)
+      for (int k0 = W; k0 < w; k0 += W) {
+        entries(r, k0);
+#pragma unroll
+        for (int u = 0; u < W; u++)
+          if (k0 + u < w) s = fma(v[u], p[j[u]], s);
+      }
+    q[r] = s;
+    acc = fma(pr, s, acc);
+    r += gridDim.x * kT;
+    if (r < rows) load(r);
+  }
+  block_partial(acc, partials);
 }
 
 // z += alpha p, r -= alpha q (z: the correction since the last residual evaluation), and the
 // cycle's next right-hand side with its norm; two unknowns per thread
-__global__ void __launch_bounds__(kT) k_mg_update(int64_t n, double* __restrict__ z, double* __restrict__ r,
-                                                  const double* __restrict__ p, const double* __restrict__ q,
-                                                  const float* __restrict__ s, float* __restrict__ b32, CgState* st,
-                                                  double* partials) {
-  if (st->done) return;
-  const double a = st->alpha, g = st->ar;
+__global__ void __launch_bounds__(kT) k_mg_update(int64_t n, double* z, double* r, const double* p, const double* q,
+                                                  const float* __restrict__ s, float* b32, CgState* st,
+                                                  const double* pq_part, int pq_count, double* partials) {
+  pdl_trigger();
+  pdl_wait();
+  const double2 v = grid_total(pq_part, pq_count, [&](double pq) {
+    const bool ok = pq > 0.0 && isfinite(pq) && !st->done;
+    if (!ok && blockIdx.x == 0 && !st->done) st->done = 2;
+    return make_double2(ok ? 1.0 : 0.0, ok ? st->rz / pq : 0.0);
+  });
+  if (v.x == 0.0) return;
+  const double a = v.y, g = st->ar;
   float acc = 0.0f;
   const int64_t n2 = n >> 1;
   for (int64_t i = gtid(); i < n2; i += gstride()) {
-    const double2 pp = __ldg(reinterpret_cast<const double2*>(p) + i), qq = __ldg(reinterpret_cast<const double2*>(q) + i);
+    const double2 pp = reinterpret_cast<const double2*>(p)[i], qq = reinterpret_cast<const double2*>(q)[i];
     double2 zz = reinterpret_cast<const double2*>(z)[i], rr = reinterpret_cast<const double2*>(r)[i];
     const float2 ss = __ldg(reinterpret_cast<const float2*>(s) + i);
     zz.x = fma(a, pp.x, zz.x);
@@ -1400,21 +1648,7 @@ __global__ void __launch_bounds__(kT) k_mg_update(int64_t n, double* __restrict_
     b32[i] = t;
     acc = fmaf(t, t, acc);
   }
-  float v[1] = {acc};
-  double tot[1];
-  if (reduce_grid_w<1, kT, true>(v, partials + gridDim.x, &st->counter[2], tot) && threadIdx.x == 0) {
-    const double rn = tot[0] / (g * g);
-    st->iters += 1;
-    st->rho_new = rn;
-    if (!isfinite(rn)) {
-      st->done = 2;
-    } else if (rn <= st->stop2) {
-      st->final_req = 1;
-      st->done = 3;
-    } else if (rn <= st->ru2 || st->iters >= st->max_iter) {
-      st->done = 3;
-    }
-  }
+  block_partial(acc, partials);
 }
 
 __global__ void __launch_bounds__(kT) k_mg_out(int64_t n, const double* __restrict__ y,
@@ -1618,6 +1852,7 @@ int mg_plan(Solver& S) {
   }
   sl.room(&M.rowsum, (size_t)S.n * nb0);
   sl.room(&M.lam, kMgMaxLevels);
+  sl.room(&M.part, 3 * kMgGrid);
   for (int l = 0; l < M.nlev; l++) {
     MgLev& L = M.lev[l];
     const size_t nb = L.nb;
@@ -1629,6 +1864,9 @@ int mg_plan(Solver& S) {
     sl.room(&L.pt_val, (size_t)L.npt * nb * nbc);
   }
   M.ndense = M.lev[M.nlev - 1].n * M.lev[M.nlev - 1].nb;
+  int dev = 0;
+  ADFEM_CUDA(cudaGetDevice(&dev));
+  ADFEM_CUDA(cudaDeviceGetAttribute(&M.sms, cudaDevAttrMultiProcessorCount, dev));
   sl.room(&M.dense, (size_t)M.ndense * M.ndense);
   M.val_bytes = (int)(sl.total - val0);
   ADFEM_TRY(M.slab.alloc(sl.total));
@@ -1731,16 +1969,56 @@ int mg_values(Solver& S, cudaStream_t st) {
 
 namespace {
 
+// Launch of a kernel of an iteration (programmatic dependent launch unless ADFEM_ZCG_PDL=0).
+template <class... P, class... A>
+void mg_launch(const Solver& S, cudaStream_t st, void (*kern)(P...), unsigned grid, unsigned block, size_t smem,
+               unsigned cluster, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  int na = 0;
+  if (S.zpdl) {
+    at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[na++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    at[na].id = cudaLaunchAttributeClusterDimension;
+    at[na].val.clusterDim.x = cluster;
+    at[na].val.clusterDim.y = at[na].val.clusterDim.z = 1;
+    na++;
+  }
+  cfg.attrs = at;
+  cfg.numAttrs = na;
+  cudaLaunchKernelEx(&cfg, kern, P(args)...);  // (an error is reported by the caller's cudaGetLastError)
+}
+
+// Blocks of a kernel that sums over its grid or needs such a sum: at most one resident wave (every
+// block reads all partial sums of the kernel before).
+template <class K>
+unsigned sum_grid(const Solver& S, K kern, int64_t threads) {
+  int per = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kT, 0) != cudaSuccess || per < 1) per = 1;
+  return std::min(blocks(threads, kT), (unsigned)std::min(per * S.mg->sms, kMgGrid));
+}
+
 template <int MODE>
-void sweep(const Solver& S, const MgLev& L, const float* x, float* out, int c1, int c2, int keep, CgState* cs,
+void sweep(const Solver& S, const MgLev& L, const float* x, float* out, int c1, int c2, int keep, double* part,
            cudaStream_t st) {
-  double* part = S.partials.as<double>();
-  // (the kernel with the dot product keeps to the solver's grid: its partials have that size)
-  const unsigned g = MODE == kLast && cs ? (unsigned)S.grid : blocks((int64_t)L.n * L.lpr, kT);
-#define ADFEM_SWEEP(NB, D16, LPR) k_mg_sweep<NB, D16, LPR, MODE><<<g, kT, 0, st>>>(L, x, out, c1, c2, keep, cs, part)
+  const int64_t threads = (int64_t)L.n * L.lpr;
+  auto grid = [&](auto kern) {
+    if (MODE != kLast || !part) return blocks(threads, kT);
+    const unsigned g = sum_grid(S, kern, threads);
+    S.mg->nrz = (int)g;
+    return g;
+  };
+#define ADFEM_SWEEP(NB, D16, LPR)                                                                 \
+  mg_launch(S, st, k_mg_sweep<NB, D16, LPR, MODE>, grid(k_mg_sweep<NB, D16, LPR, MODE>), kT, 0, 1, L, x, out, c1, c2, \
+            keep, part)
   if (L.d16 && S.A->maxw <= 8) {
-    const unsigned gf = blocks(L.n, kT);
-    k_mg_fine<MODE><<<MODE == kLast ? std::min(gf, (unsigned)S.grid) : gf, kT, 0, st>>>(L, x, out, c1, c2, cs, part);
+    mg_launch(S, st, k_mg_fine<MODE>, grid(k_mg_fine<MODE>), kT, 0, 1, L, x, out, c1, c2, part);
     return;
   }
   if (L.nb == 1) {
@@ -1759,41 +2037,31 @@ void sweep(const Solver& S, const MgLev& L, const float* x, float* out, int c1, 
 #undef ADFEM_SWEEP
 }
 
-void restrict_to(const MgLev& L, const float* r, float* out, cudaStream_t st) {
+void restrict_to(const Solver& S, const MgLev& L, const float* r, float* out, cudaStream_t st) {
   const int lpr = L.nc >= 150000 ? 1 : 8;
   const unsigned g = blocks((int64_t)L.nc * lpr, kT);
 #define ADFEM_RES(NB, NC)                                                \
   do {                                                                   \
-    if (lpr == 1) k_mg_restrict<NB, NC, 1><<<g, kT, 0, st>>>(L, r, out); \
-    else k_mg_restrict<NB, NC, 8><<<g, kT, 0, st>>>(L, r, out);          \
+    if (lpr == 1) mg_launch(S, st, k_mg_restrict<NB, NC, 1>, g, kT, 0, 1, L, r, out); \
+    else mg_launch(S, st, k_mg_restrict<NB, NC, 8>, g, kT, 0, 1, L, r, out);          \
   } while (0)
   if (L.nb == 1) ADFEM_RES(1, 1);
   else if (L.nb == 2) ADFEM_RES(2, 3);
   else ADFEM_RES(3, 3);
 #undef ADFEM_RES
 }
-void prolong_from(const MgLev& L, const float* xc, float* x, cudaStream_t st) {
+void prolong_from(const Solver& S, const MgLev& L, const float* xc, float* x, cudaStream_t st) {
   const unsigned g = blocks(L.n, kT);
-  if (L.nb == 1) k_mg_prolong<1, 1><<<g, kT, 0, st>>>(L, xc, x);
-  else if (L.nb == 2) k_mg_prolong<2, 3><<<g, kT, 0, st>>>(L, xc, x);
-  else k_mg_prolong<3, 3><<<g, kT, 0, st>>>(L, xc, x);
+  if (L.nb == 1) mg_launch(S, st, k_mg_prolong<1, 1>, g, kT, 0, 1, L, xc, x);
+  else if (L.nb == 2) mg_launch(S, st, k_mg_prolong<2, 3>, g, kT, 0, 1, L, xc, x);
+  else mg_launch(S, st, k_mg_prolong<3, 3>, g, kT, 0, 1, L, xc, x);
 }
 
 template <int NT, int NC>
-void launch_tail(const Mg& M, const TailArgs& a, cudaStream_t st) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(M.cluster ? kTailC : 1);
-  cfg.blockDim = dim3(kTailT);
-  cfg.dynamicSmemBytes = M.tail_smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = kTailC;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = M.cluster ? 1 : 0;
-  if (M.cluster) cudaLaunchKernelEx(&cfg, k_mg_tail<NT, NC, true>, a);
-  else cudaLaunchKernelEx(&cfg, k_mg_tail<NT, NC, false>, a);
+void launch_tail(const Solver& S, const TailArgs& a, cudaStream_t st) {
+  const Mg& M = *S.mg;
+  if (M.cluster) mg_launch(S, st, k_mg_tail<NT, NC, true>, kTailC, kTailT, M.tail_smem, kTailC, a);
+  else mg_launch(S, st, k_mg_tail<NT, NC, false>, 1, kTailT, M.tail_smem, 1, a);
 }
 
 // One cycle: lev[0].b -> the vector returned; returns the launches through *count.
@@ -1815,7 +2083,7 @@ const float* enqueue_cycle(Solver& S, cudaStream_t st, int* count) {
     }
     // (d is free between the smoothers: the residual goes there)
     sweep<kRes>(S, L, x, L.d, -1, -1, 0, nullptr, st);
-    restrict_to(L, L.d, M.lev[l + 1].b, st);
+    restrict_to(S, L, L.d, M.lev[l + 1].b, st);
     nl += 2;
     xs[l] = x;
   }
@@ -1833,11 +2101,13 @@ const float* enqueue_cycle(Solver& S, cudaStream_t st, int* count) {
     a.x = M.lev[M.tail].x;
     a.reps = M.tail >= 3 ? 2 : 1;
     a.dot = M.tail == 0;
+    a.rz = M.part;
+    M.nrz = 1;  // (replaced by the last sweep of a level 0 above the tail)
     a.st = cs;
     const int nt = a.L[0].nb;
-    if (nt == 1) launch_tail<1, 1>(M, a, st);
-    else if (nt == 2) launch_tail<2, 3>(M, a, st);
-    else launch_tail<3, 3>(M, a, st);
+    if (nt == 1) launch_tail<1, 1>(S, a, st);
+    else if (nt == 2) launch_tail<2, 3>(S, a, st);
+    else launch_tail<3, 3>(S, a, st);
     xs[M.tail] = M.lev[M.tail].x;
     nl++;
   }
@@ -1845,12 +2115,12 @@ const float* enqueue_cycle(Solver& S, cudaStream_t st, int* count) {
     const MgLev& L = M.lev[l];
     const int deg = l == 0 ? kMgDeg0 : kMgDeg;
     float *x = xs[l], *y = x == L.x ? L.x2 : L.x;
-    prolong_from(L, xs[l + 1], x, st);
+    prolong_from(S, L, xs[l + 1], x, st);
     nl++;
     for (int k = 0; k < deg; k++) {
       const int c1 = k ? 2 * k : -1, c2 = k ? 2 * k + 1 : 0;
       if (k + 1 < deg) sweep<kStep>(S, L, x, y, c1, c2, 1, nullptr, st);
-      else sweep<kLast>(S, L, x, y, c1, c2, 0, l == 0 ? cs : nullptr, st);
+      else sweep<kLast>(S, L, x, y, c1, c2, 0, l == 0 ? M.part : nullptr, st);
       std::swap(x, y);
       nl++;
     }
@@ -1864,9 +2134,10 @@ void enqueue_residual(Solver& S, int mode, cudaGraphConditionalHandle loop, cuda
   Mg& M = *S.mg;
   const Sell& A = *S.A;
   auto go = [&](auto d16, auto nb) {
-    k_mg_residual<decltype(d16)::value, decltype(nb)::value><<<S.grid, kT, 0, st>>>(
-        S.n, A.sptr.as<int32_t>(), A.col.p, A.val64.as<double>(), M.rowsum, S.s32.as<float>(), S.b.as<double>(),
-        S.y64.as<double>(), S.r64.as<double>(), M.lev[0].b, S.state.as<CgState>(), S.partials.as<double>(), mode, loop);
+    auto k = k_mg_residual<decltype(d16)::value, decltype(nb)::value>;
+    mg_launch(S, st, k, (unsigned)S.grid, kT, 0, 1, S.n, A.sptr.as<int32_t>(), A.col.p, A.val64.as<double>(), M.rowsum,
+              S.s32.as<float>(), S.b.as<double>(), S.y64.as<double>(), S.z64.as<double>(), S.r64.as<double>(),
+              M.lev[0].b, S.state.as<CgState>(), M.part + 2 * kMgGrid, M.nrn, S.partials.as<double>(), mode, loop);
   };
   using std::integral_constant;
   if (M.lev[0].nb == 2) {
@@ -1884,13 +2155,31 @@ void enqueue_body(Solver& S, cudaGraphConditionalHandle loop, cudaStream_t st) {
   CgState* cs = S.state.as<CgState>();
   int nl = 0;
   const float* z = enqueue_cycle(S, st, &nl);
-  k_mg_dir<<<S.grid, kT, 0, st>>>(S.n, z, S.s32.as<float>(), S.p64.as<double>(), cs);
-  solver_enqueue_spmv64(S, S.A->val64.as<double>(), st);
-  k_mg_update<<<S.grid, kT, 0, st>>>(S.n, S.z64.as<double>(), S.r64.as<double>(), S.p64.as<double>(),
-                                     S.q64.as<double>(), S.s32.as<float>(), M.lev[0].b, cs, S.partials.as<double>());
-  solver_enqueue_fold64(S, 0, st);
+  const Sell& A = *S.A;
+  const int64_t n2 = (S.n + 1) / 2;
+  double *rz = M.part, *pq = rz + kMgGrid, *rn = pq + kMgGrid;
+  mg_launch(S, st, k_mg_dir, sum_grid(S, k_mg_dir, n2), kT, 0, 1, S.n, z, S.s32.as<float>(), S.p64.as<double>(),
+            S.y64.as<double>(), S.z64.as<double>(), cs, rz, M.nrz);
+  int npq = 0;
+  auto spmv = [&](auto d16, auto more) {
+    auto k = k_mg_spmv<decltype(d16)::value, decltype(more)::value>;
+    npq = (int)sum_grid(S, k, S.n);
+    mg_launch(S, st, k, (unsigned)npq, kT, 0, 1, S.n, A.sptr.as<int32_t>(), A.col.p, A.spat.as<int32_t>(),
+              A.pat.as<int16_t>(), A.pat_period, A.val64.as<double>(), S.p64.as<double>(), S.q64.as<double>(), cs, pq);
+  };
+  if (A.maxw <= 8) {
+    if (A.delta16) spmv(std::true_type{}, std::false_type{});
+    else spmv(std::false_type{}, std::false_type{});
+  } else {
+    if (A.delta16) spmv(std::true_type{}, std::true_type{});
+    else spmv(std::false_type{}, std::true_type{});
+  }
+  const unsigned gu = sum_grid(S, k_mg_update, n2);
+  mg_launch(S, st, k_mg_update, gu, kT, 0, 1, S.n, S.z64.as<double>(), S.r64.as<double>(), S.p64.as<double>(),
+            S.q64.as<double>(), S.s32.as<float>(), M.lev[0].b, cs, pq, npq, rn);
+  M.nrn = (int)gu;
   enqueue_residual(S, 1, loop, st);
-  M.body_launches = nl + 5;
+  M.body_launches = nl + 4;
 }
 
 int capture_solve(Solver& S) {

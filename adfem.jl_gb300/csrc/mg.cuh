@@ -25,6 +25,7 @@ constexpr int kMgDense = 160;     // unknowns of the directly solved coarsest le
 constexpr int kMgTailDofs = 5120; // unknowns of the largest level of the one-launch tail
 constexpr int kTailC = 8;         // blocks of the tail's cluster
 constexpr int kTailLocal = kMgTailDofs / kTailC;  // unknowns of a tail that one block runs alone
+constexpr int kMgGrid = 1280;     // blocks of the kernels that sum over the grid, at most
 constexpr int kMgDeg0 = 2, kMgDeg = 4;  // Chebyshev degree: level 0, coarser levels
 
 // Patterns of one level (host), rows in solver order at level 0.  Rows are in compressed
@@ -76,8 +77,11 @@ struct Mg {
   MgLev lev[kMgMaxLevels];
   float* dense = nullptr;      // inverse of the coarsest operator
   int ndense = 0;
+  int sms = 0;
+  int nrz = 0, nrn = 0;        // partial sums of r.z and of the residual's square
   double* rowsum = nullptr;    // FP64 row sums of K per component of the column (nb per row)
   int* lam = nullptr;          // MgLev::lam of every level
+  double* part = nullptr;      // partial sums of the iteration's three sums (kMgGrid each)
   DevBuf slab;                 // all of the above
   bool cluster = false;        // the tail's first level is shared by a cluster
   const char *pat = nullptr, *vals = nullptr;  // of the levels that a tail block runs alone

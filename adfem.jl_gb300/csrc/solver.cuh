@@ -27,6 +27,10 @@ struct CgState {
   int floor_hit;       // stopped at the attainable accuracy of the FP64 residual
   int final_seen;      // mixed: a replacement requested by rtol has already failed the true-residual test
   double last_rr64;    // FP64 residual norm^2 at the previous replacement (mixed: once final_seen)
+  int fold;            // multigrid CG: the correction z is to be folded into y
+  int it;              // multigrid CG: iterations including the current one
+  double rz, irz;      // multigrid CG: r.z of this iteration, reciprocal of the one before
+  double iar;          // multigrid CG: 1 / ar
   int fault;           // banded ring variant: a wait on a shared-memory stage timed out
   unsigned counter[4]; // last-block arrival counters (returned to 0 by the last block)
 };

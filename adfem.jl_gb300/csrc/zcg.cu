@@ -130,12 +130,6 @@ __device__ __forceinline__ float ld_stream(const float* a, uint64_t pol) {
   return v;
 }
 
-// Programmatic dependent launch (launches with the programmatic-serialization attribute):
-// wait for the previous grid in the stream to complete with its memory visible (a no-op
-// when launched without the attribute), and let the next grid be scheduled.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // ---- the matrix ring of the RING variants: each stage holds the fixed-width values of
 // BT consecutive rows (contiguous in global memory), copied by the bulk-copy engine
 // (cp.async.bulk, this GPU's memory into this CTA's shared memory) and tracked by a
