@@ -453,7 +453,9 @@ def solver_opts(precision: str = "fp64", rtol: float = 1e-12, max_iter: int = 20
 
 def solve(K, F, precision: str = "fp64", rtol: float = 1e-12, max_iter: int = 200000, return_stats: bool = False,
           u0=None):
-    """``K\\F`` for a symmetric positive definite sparse K (GPU Jacobi-CG); ``u0`` warm-starts."""
+    """``K\\F`` for a symmetric positive definite sparse K (conjugate gradients on the GPU,
+    preconditioned by multigrid where K is a scalar problem with eliminated rows and the precision
+    FP64, else by its diagonal); ``u0`` warm-starts."""
     K = sp.csc_matrix(K)
     K.sort_indices()
     n = K.shape[0]

@@ -937,6 +937,13 @@ static int check_symmetric(int64_t n, const std::vector<int32_t>& rp, const std:
       if (ci[k] == r) diag[r] += std::fabs(val[k]);
   std::vector<std::pair<int32_t, double>> row;
   for (int64_t r = 0; r < n; r++) {
+    // a row of distinct, sorted columns that are the transpose's, with equal values (the usual one)
+    const int32_t len = rp[r + 1] - rp[r];
+    bool same = len == tp[r + 1] - tp[r];
+    for (int32_t k = 0; k < len && same; k++)
+      same = ci[rp[r] + k] == tc[tp[r] + k] && val[rp[r] + k] == tv[tp[r] + k] &&
+             (k == 0 || ci[rp[r] + k] > ci[rp[r] + k - 1]);
+    if (same) continue;
     row.clear();
     for (int32_t k = rp[r]; k < rp[r + 1]; k++) row.emplace_back(ci[k], val[k]);
     std::stable_sort(row.begin(), row.end(),
@@ -970,6 +977,44 @@ static int check_symmetric(int64_t n, const std::vector<int32_t>& rp, const std:
     }
   }
   return ADFEM_OK;
+}
+
+// Whether K\F is worth a multigrid hierarchy, which is built for the one solve: a scalar problem
+// with eliminated rows (tagged in fixed: nothing but the diagonal), so that it is not singular, of
+// more unknowns than the directly solved level has.  The unknowns of a vector-valued problem (elasticity) come in sets with
+// one row pattern, whichever way they are numbered; the hierarchy here is a scalar one, so where
+// most rows have such a twin the Jacobi iteration is kept.  (Rows have to be sorted, without
+// repeated entries.)
+static bool csc_wants_mg(int64_t n, const std::vector<int32_t>& rp, const std::vector<int32_t>& ci,
+                         const double* val, std::vector<uint8_t>& fixed) {
+  // GB300, ms per call on P1 Poisson matrices, Jacobi / multigrid: 289 unknowns 2.4 / 1.1,
+  // 4225 6.6 / 2.8, 10201 10.7 / 4.2, 40401 20.0 / 11.4 (most of the rest is the hierarchy's set-up)
+  if (n <= kMgDense || !mg_wanted()) return false;
+  fixed.assign(n, 0);
+  int64_t nfixed = 0;
+  std::vector<uint64_t> key(n);
+  for (int64_t r = 0; r < n; r++) {
+    bool only = true;
+    uint64_t h = 0;
+    for (int32_t k = rp[r]; k < rp[r + 1]; k++) {
+      if (k > rp[r] && ci[k] <= ci[k - 1]) return false;
+      if (ci[k] != r && val[k] != 0.0) only = false;
+      h = (h ^ (uint64_t)ci[k]) * 0x9E3779B97F4A7C15ull;
+      h ^= h >> 29;
+    }
+    fixed[r] = only;
+    nfixed += only;
+    key[r] = h;
+  }
+  if (nfixed == 0) return false;
+  // (a twin has this row's pattern, diagonals included, so it is one of its columns)
+  int64_t twins = 0;
+  for (int64_t r = 0; r < n; r++) {
+    bool twin = false;
+    for (int32_t k = rp[r]; k < rp[r + 1] && !twin; k++) twin = ci[k] != r && key[ci[k]] == key[r];
+    twins += twin;
+  }
+  return 2 * twins <= n - nfixed;
 }
 
 int adfem_csc_solve(long long n, const long long* colptr1, const long long* rowval1, const double* nzval,
@@ -1016,6 +1061,17 @@ int adfem_csc_solve(long long n, const long long* colptr1, const long long* rowv
                  "csr to sell"));
   Solver sv;
   ADFEM_TRY(sv.init(&A, n));
+  std::vector<uint8_t> fixed;
+  DevBuf dfixed;
+  // (mixed precision names an iteration of its own here, which the callers of it keep)
+  if (o.precision == ADFEM_PREC_FP64 && csc_wants_mg(n, rp, ci, nzval, fixed)) {
+    ADFEM_TRY(to_dev(dfixed, fixed.data(), fixed.size()));
+    sv.mg_allowed = sv.mg_fixed = true;
+    sv.mg_nb = 1;
+    sv.mg_isbd = dfixed.as<uint8_t>();
+    sv.mg_rp = std::move(rp);
+    sv.mg_ci = std::move(ci);
+  }
   ADFEM_TRY(solver_prepare(sv, ddp.as<int32_t>(), nullptr));
   const int st = solver_solve(sv, db.as<double>(), du.as<double>(), nullptr, nullptr, nullptr, o, stats, nullptr);
   if (st != ADFEM_OK && st != ADFEM_ERR_NOT_CONVERGED) return st;

@@ -10,11 +10,16 @@ namespace {
 // taken becomes the root of an aggregate of itself and its neighbours.  Second pass: the
 // nodes left over join the neighbouring first-pass aggregate with which they share the most
 // edges (the lowest-numbered of equals); nodes without one become aggregates of their own.
+// Nodes without neighbours (eliminated rows of a user's matrix, whose interpolation is zero) are
+// dealt over the aggregates in node order: on their own they would be unknowns of every level.
 int64_t aggregate(int64_t n, const MgPattern& A, std::vector<int32_t>& agg) {
   agg.assign(n, -1);
   int32_t na = 0;
+  auto alone = [&](int64_t i) {
+    return A.rp[i + 1] == A.rp[i] || (A.rp[i + 1] == A.rp[i] + 1 && A.ci[A.rp[i]] == i);
+  };
   for (int64_t i = 0; i < n; i++) {
-    if (agg[i] >= 0) continue;
+    if (agg[i] >= 0 || alone(i)) continue;
     bool free = true;
     for (int32_t k = A.rp[i]; k < A.rp[i + 1] && free; k++) free = agg[A.ci[k]] < 0;
     if (!free) continue;
@@ -25,7 +30,7 @@ int64_t aggregate(int64_t n, const MgPattern& A, std::vector<int32_t>& agg) {
   std::vector<std::pair<int64_t, int32_t>> late;
   std::vector<int32_t> c;
   for (int64_t i = 0; i < n; i++) {
-    if (agg[i] >= 0) continue;
+    if (agg[i] >= 0 || alone(i)) continue;
     c.clear();
     for (int32_t k = A.rp[i]; k < A.rp[i + 1]; k++)
       if (agg[A.ci[k]] >= 0) c.push_back(agg[A.ci[k]]);
@@ -48,12 +53,17 @@ int64_t aggregate(int64_t n, const MgPattern& A, std::vector<int32_t>& agg) {
     late.emplace_back(i, best);
   }
   for (auto& p : late) agg[p.first] = p.second;
+  if (na == 0) return n;  // no edges at all
+  for (int64_t i = 0; i < n; i++)
+    if (agg[i] < 0) agg[i] = (int32_t)(i * na / n);
   return na;
 }
 
-// Pattern whose row i is the sorted set that emit(i, v) appends to v.
+// Pattern whose row i is the sorted set of the columns (below nc) that emit(i, add) adds.  (Repeated
+// ones are dropped as they come, by the row that last had the column: a coarse row meets each of its
+// some 7 columns 15 to 20 times.)
 template <class F>
-int64_t pattern(int64_t n, MgPattern& P, F emit) {
+int64_t pattern(int64_t n, int64_t nc, MgPattern& P, F emit) {
   constexpr int64_t kChunk = 16384;
   const int64_t nch = (n + kChunk - 1) / kChunk;
   std::vector<std::vector<int32_t>> part(nch);
@@ -61,13 +71,16 @@ int64_t pattern(int64_t n, MgPattern& P, F emit) {
   // (parallel_for splits by index; scale the chunk count up so that it threads)
   const int64_t m = n < 50000 ? nch : std::max<int64_t>(nch, 50000);
   parallel_for(m, [&](int64_t lo, int64_t hi) {
-    std::vector<int32_t> v;
+    std::vector<int32_t> v, seen(nc, -1);
     for (int64_t c = lo * nch / m; c < hi * nch / m; c++)
       for (int64_t i = c * kChunk; i < std::min(n, (c + 1) * kChunk); i++) {
         v.clear();
-        emit(i, v);
+        emit(i, [&](int32_t j) {
+          if (seen[j] == (int32_t)i) return;
+          seen[j] = (int32_t)i;
+          v.push_back(j);
+        });
         std::sort(v.begin(), v.end());
-        v.erase(std::unique(v.begin(), v.end()), v.end());
         part[c].insert(part[c].end(), v.begin(), v.end());
         P.rp[i + 1] = (int32_t)v.size();
       }
@@ -103,15 +116,15 @@ bool mg_build_host(int64_t n, std::vector<int32_t>&& rp, std::vector<int32_t>&& 
     if ((int)lv.size() == kMgMaxLevels) return false;
     const int64_t nc = aggregate(L.n, L.A, L.agg);
     if (2 * nc > L.n) return false;  // hardly any edges: no hierarchy
-    auto rows = [](const MgPattern& Q, int64_t i, std::vector<int32_t>& v) {
-      v.insert(v.end(), Q.ci.begin() + Q.rp[i], Q.ci.begin() + Q.rp[i + 1]);
+    auto rows = [](const MgPattern& Q, int64_t i, auto&& add) {
+      for (int32_t k = Q.rp[i]; k < Q.rp[i + 1]; k++) add(Q.ci[k]);
     };
-    if (pattern(L.n, L.P, [&](int64_t i, std::vector<int32_t>& v) {
-          for (int32_t k = L.A.rp[i]; k < L.A.rp[i + 1]; k++) v.push_back(L.agg[L.A.ci[k]]);
+    if (pattern(L.n, nc, L.P, [&](int64_t i, auto&& add) {
+          for (int32_t k = L.A.rp[i]; k < L.A.rp[i + 1]; k++) add(L.agg[L.A.ci[k]]);
         }) > kMgMaxP)
       return false;
-    if (pattern(L.n, L.AP, [&](int64_t i, std::vector<int32_t>& v) {
-          for (int32_t k = L.A.rp[i]; k < L.A.rp[i + 1]; k++) rows(L.P, L.A.ci[k], v);
+    if (pattern(L.n, nc, L.AP, [&](int64_t i, auto&& add) {
+          for (int32_t k = L.A.rp[i]; k < L.A.rp[i + 1]; k++) rows(L.P, L.A.ci[k], add);
         }) > kMgMaxAP)
       return false;
     // transpose of P, nodes ascending within each aggregate's row
@@ -131,8 +144,8 @@ bool mg_build_host(int64_t n, std::vector<int32_t>&& rp, std::vector<int32_t>&& 
     }
     MgHostLevel C;
     C.n = nc;
-    if (pattern(nc, C.A, [&](int64_t J, std::vector<int32_t>& v) {
-          for (int32_t q = L.PT.rp[J]; q < L.PT.rp[J + 1]; q++) rows(L.AP, L.PT.ci[q], v);
+    if (pattern(nc, nc, C.A, [&](int64_t J, auto&& add) {
+          for (int32_t q = L.PT.rp[J]; q < L.PT.rp[J + 1]; q++) rows(L.AP, L.PT.ci[q], add);
         }) > kMgMaxA)
       return false;
     if (!L.x.empty()) {
