@@ -32,6 +32,10 @@ def _dev(t, n=None, what="tensor"):
 
 
 def _cur_stream():
+    # (the stream object is made and thrown away on each call otherwise: 7 us)
+    C = _torch()._C
+    if hasattr(C, "_cuda_getCurrentRawStream"):
+        return ctypes.c_void_p(C._cuda_getCurrentRawStream(C._cuda_getDevice()))
     return stream_ptr(_torch().cuda.current_stream())
 
 
@@ -280,7 +284,8 @@ def source(mesh, f, rhs=None, accumulate=False):
     torch = _torch()
     _dev(f, _ng(mesh), "f")
     if rhs is None:
-        rhs = torch.zeros(mesh.ndof, dtype=torch.float64, device="cuda")
+        # (without accumulate every entry is written)
+        rhs = (torch.zeros if accumulate else torch.empty)(mesh.ndof, dtype=torch.float64, device="cuda")
     check(_lib.load().adfem_source_d(mesh.handle, ptr(f), ptr(rhs), int(accumulate), _cur_stream()), "source")
     return rhs
 

@@ -229,6 +229,10 @@ cudaError_t launch_element_prepass_unweighted(const Mesh& m, const double* kappa
 // Laplace values into the scalar pattern (CSR or sliced-ELL), no Dirichlet
 cudaError_t launch_laplace_rows(const Mesh& m, const double* sigma, double* vals, Layout lay, cudaStream_t st);
 // load vector: rhs[i] (+)= sum over incident elements of src_e[a]
+// rows straight from the Gauss-point inputs (small meshes)
+bool direct_rows(const Mesh& m);
+cudaError_t launch_laplace_rows_direct(const Mesh& m, const double* kappa, double* vals, cudaStream_t st);
+cudaError_t launch_source_rows_direct(const Mesh& m, const double* f, double* rhs, bool accumulate, cudaStream_t st);
 cudaError_t launch_source_rows(const Mesh& m, const double* src3, double* rhs, bool accumulate, cudaStream_t st);
 // unsummed COO of the reference op (FemLaplaceScalar_forward): 9 entries per Gauss point
 cudaError_t launch_laplace_coo(const Mesh& m, const double* kappa, long long* indices, double* vv, cudaStream_t st);

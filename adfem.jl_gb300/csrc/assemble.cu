@@ -219,6 +219,115 @@ cudaError_t launch_source_rows(const Mesh& m, const double* src3, double* rhs, b
 }
 
 // ---------------------------------------------------------------------------
+// Small meshes: the same rows straight from the Gauss-point inputs, without the element pass.  What
+// bounds them is latency, a launch and two dependent gathers per incidence; so one launch instead of
+// two, the loads of kIB incidences in flight together, and blocks of 64 rows, which spread the FP64
+// instructions over more SMs.  The element sums are formed once per incidence (three times each, as
+// in k_element_prepass, and in the same order: the results are the same bits).
+constexpr int kDirectB = 64, kIB = 4;
+
+template <int MAXW>
+__global__ void __launch_bounds__(kDirectB) k_laplace_rows_direct(
+    int64_t n, const int32_t* __restrict__ inc_ptr, const uint2* __restrict__ inc, const double4* __restrict__ geo,
+    const double* __restrict__ kappa, const int32_t* __restrict__ rowptr, const int32_t* __restrict__ diagpos,
+    double* __restrict__ vals) {
+  __shared__ double acc[MAXW][kDirectB];
+  const int t = threadIdx.x;
+  const int64_t i = gtid();
+  if (i >= n) return;
+  const int32_t r0 = rowptr[i], s0 = inc_ptr[i], s1 = inc_ptr[i + 1];
+  const int w = rowptr[i + 1] - r0, dp = diagpos[i];
+  for (int k = 0; k < w; k++) acc[k][t] = 0.0;
+  for (int32_t sb = s0; sb < s1; sb += kIB) {
+    uint2 rec[kIB];
+    double4 g[kIB];
+    double k0[kIB], k1[kIB], k2[kIB];
+#pragma unroll
+    for (int u = 0; u < kIB; u++) rec[u] = inc[min(sb + u, s1 - 1)];
+#pragma unroll
+    for (int u = 0; u < kIB; u++) {
+      const int64_t e = rec[u].x;
+      g[u] = geo[e];
+      k0[u] = kappa[3 * e];
+      k1[u] = kappa[3 * e + 1];
+      k2[u] = kappa[3 * e + 2];
+    }
+#pragma unroll
+    for (int u = 0; u < kIB; u++) {
+      if (sb + u >= s1) continue;
+      const double sg = k0[u] + k1[u] + k2[u];
+      const unsigned y = rec[u].y, a = inc_a(y), b = (a == 0) ? 1 : 0, c = (a == 2) ? 1 : 2;
+      const unsigned ob = inc_off(y, b), oc = inc_off(y, c);
+      if (!ADFEM_DCHECK(ob < (unsigned)w && oc < (unsigned)w && ob < MAXW && oc < MAXW)) continue;
+      acc[ob][t] = fma(gpair(g[u], a, b), sg, acc[ob][t]);
+      acc[oc][t] = fma(gpair(g[u], a, c), sg, acc[oc][t]);
+    }
+  }
+  double d = 0.0;
+  for (int k = 0; k < w; k++)
+    if (k != dp) d -= acc[k][t];
+  acc[dp][t] = d;
+  for (int k = 0; k < w; k++) vals[(int64_t)r0 + k] = acc[k][t];
+}
+
+__global__ void __launch_bounds__(kDirectB) k_source_rows_direct(int64_t n, const int32_t* __restrict__ inc_ptr,
+                                                                 const uint2* __restrict__ inc,
+                                                                 const double4* __restrict__ geo,
+                                                                 const double* __restrict__ f,
+                                                                 double* __restrict__ rhs, int accumulate) {
+  const int64_t i = gtid();
+  if (i >= n) return;
+  const int32_t s0 = inc_ptr[i], s1 = inc_ptr[i + 1];
+  double s = accumulate ? rhs[i] : 0.0;
+  for (int32_t sb = s0; sb < s1; sb += kIB) {
+    uint2 rec[kIB];
+    double w[kIB], f0[kIB], f1[kIB], f2[kIB];
+#pragma unroll
+    for (int u = 0; u < kIB; u++) rec[u] = inc[min(sb + u, s1 - 1)];
+#pragma unroll
+    for (int u = 0; u < kIB; u++) {
+      const int64_t e = rec[u].x;
+      w[u] = geo[e].w;
+      f0[u] = f[3 * e];
+      f1[u] = f[3 * e + 1];
+      f2[u] = f[3 * e + 2];
+    }
+#pragma unroll
+    for (int u = 0; u < kIB; u++) {
+      if (sb + u >= s1) continue;
+      const int a = (int)inc_a(rec[u].y);
+      const double wh = 0.5 * w[u], t = (f0[u] + f1[u] + f2[u]) * (w[u] * (1.0 / 6.0));
+      s += fma(a == 0 ? f0[u] : (a == 1 ? f2[u] : f1[u]), wh, t);
+    }
+  }
+  rhs[i] = s;
+}
+
+// GB300, us per call with the element pass / direct: 4225 nodes 27.1 / 23.4 (matrix), 25.6 / 21.3
+// (load); 66k 30.1 / 27.3, 28.4 / 25.0; 161k 36.6 / 33.5, 32.5 / 33.7; 491k 62.7 / 59.1, 48.4 / 60.9.
+bool direct_rows(const Mesh& m) {
+  constexpr int64_t kDirectNodes = 100000;
+  return m.maxrow <= 16 && m.nv <= kDirectNodes;
+}
+
+cudaError_t launch_laplace_rows_direct(const Mesh& m, const double* kappa, double* vals, cudaStream_t st) {
+  auto go = [&](auto kern) {
+    kern<<<nblocks(m.nv, kDirectB), kDirectB, 0, st>>>(m.nv, m.d_inc_ptr.as<int32_t>(), m.d_inc.as<uint2>(),
+                                                       m.d_geo.as<double4>(), kappa, m.d_rowptr.as<int32_t>(),
+                                                       m.d_diagpos.as<int32_t>(), vals);
+    return cudaGetLastError();
+  };
+  return m.maxrow <= 8 ? go(k_laplace_rows_direct<8>) : go(k_laplace_rows_direct<16>);
+}
+
+cudaError_t launch_source_rows_direct(const Mesh& m, const double* f, double* rhs, bool accumulate, cudaStream_t st) {
+  k_source_rows_direct<<<nblocks(m.nv, kDirectB), kDirectB, 0, st>>>(m.nv, m.d_inc_ptr.as<int32_t>(),
+                                                                     m.d_inc.as<uint2>(), m.d_geo.as<double4>(), f,
+                                                                     rhs, accumulate ? 1 : 0);
+  return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
 // Fused Poisson system: Laplace row + load + Dirichlet in one pass, into sliced-ELL.
 // isbd[i]: 0 interior, 1 Dirichlet node, 2 interior with a Dirichlet neighbour.
 // PERM: the system's DOFs are renumbered (nperm[node] = solver row); the row of mesh

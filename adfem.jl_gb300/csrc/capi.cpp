@@ -579,6 +579,11 @@ int adfem_laplace_csr_d(adfem_mesh* mesh, const double* kappa_d, double* vals_d,
   if (!mesh || !kappa_d || !vals_d) return fail(ADFEM_ERR_INVALID, "null argument");
   Mesh& m = *mesh->m;
   if (Space* sp = p2_space(m)) return gen_matrix_d(m, *sp, GenOp::LAPLACE, kappa_d, vals_d, false, S(stream));
+  if (direct_rows(m)) {
+    ADFEM_TRY(kerr(launch_laplace_rows_direct(m, kappa_d, vals_d, S(stream)), "laplace rows"));
+    ADFEM_CUDA(cudaStreamSynchronize(S(stream)));
+    return ADFEM_OK;
+  }
   std::lock_guard<std::mutex> lk(m.mu);
   ADFEM_TRY(m.s_el0.alloc(sizeof(double) * m.ne));
   ADFEM_TRY(kerr(launch_element_prepass(m, kappa_d, nullptr, m.s_el0.as<double>(), nullptr, S(stream)), "prepass"));
@@ -626,6 +631,11 @@ int adfem_source_d(adfem_mesh* mesh, const double* f_d, double* rhs_d, int accum
   Mesh& m = *mesh->m;
   if (Space* sp = p2_space(m)) {
     ADFEM_TRY(kerr(launch_gen_source(m, *sp, f_d, rhs_d, accumulate != 0, S(stream)), "source"));
+    ADFEM_CUDA(cudaStreamSynchronize(S(stream)));
+    return ADFEM_OK;
+  }
+  if (direct_rows(m)) {
+    ADFEM_TRY(kerr(launch_source_rows_direct(m, f_d, rhs_d, accumulate != 0, S(stream)), "source rows"));
     ADFEM_CUDA(cudaStreamSynchronize(S(stream)));
     return ADFEM_OK;
   }
