@@ -15,7 +15,8 @@
 //    the V-cycle gains most there), on [fr lam, lam] with lam = max q_i, an upper bound of the
 //    spectrum, so the cycle is symmetric positive definite for every input.
 //  * Every sum is formed by one thread or a fixed shuffle tree: results repeat bit for bit.
-//  * A solve is one CUDA graph: a while node around one iteration, left when a residual
+//  * A solve is one launch up to kMgTailDofs unknowns (k_mg_tail), above that one CUDA graph: a
+//    while node around one iteration, left when a residual
 //    evaluated in FP64 from the iterate meets the tolerance (or the iteration ends otherwise);
 //    the host waits once.
 #include <cmath>
@@ -451,6 +452,45 @@ __global__ void __launch_bounds__(kT) k_mg_prolong(MgLev L, const float* xc, flo
 }
 
 // ---------------------------------------------------------------------------
+// The residual decides: converged, at its attainable floor, out of iterations, or go on (the
+// rules of replacement_step64, whose direction scalars do not apply here).
+// rn: the recurrence's residual (its square, as rr)
+__device__ __forceinline__ void mg_residual_step(CgState* st, double rr, double rn, bool first) {
+  const double prev = st->last_rr64;
+  st->rr64 = rr;
+  st->last_rr64 = rr;
+  if (!isfinite(rr)) {
+    st->done = 2;
+    return;
+  }
+  if (rr <= st->stop2) {
+    st->done = 1;
+    return;
+  }
+  if (!first) {
+    const bool dropped = rn <= st->delta2 * prev;
+    if (prev > 0.0 && rr > 0.0625 * prev && (dropped || st->final_seen)) {
+      st->floor_hit = 1;
+      st->done = 1;
+      return;
+    }
+  }
+  if (st->iters >= st->max_iter) {
+    st->done = 4;
+    return;
+  }
+  if (!first && rn <= st->stop2) st->final_seen = 1;
+  if (!first) st->updates += 1;
+  // A residual that is not the recurrence's (near the attainable floor it can be many times
+  // larger) has nothing to do with the directions so far: keeping them made the iteration
+  // stagnate (elasticity, 320k DOF: over 200 iterations to the floor instead of 10).
+  if (first || rr > 1.21 * rn) st->ap = 1.0;
+  st->fold = 1;
+  st->ru2 = st->delta2 * rr;
+  st->done = 0;
+}
+
+// ---------------------------------------------------------------------------
 // The levels from Mg::tail on in one launch, `reps` cycles (two below three larger levels, where
 // the tail costs little beside them and its coarse problem is then solved nearly exactly: 35
 // instead of 44 iterations and 27.8 instead of 32.6 ms at 4M DOF; one below fewer levels: 41.1
@@ -483,8 +523,13 @@ struct TailArgs {
   const float* b;
   float* x;
   int reps;
-  int dot;       // level 0 in the tail: r.z from here, to rz
-  double* rz;
+  // a whole solve (k_mg_tail's SOLVE): the system's operator, right-hand side and iterate
+  const int32_t* sptr;
+  const void* col;
+  int d16;
+  const double *val, *rowsum, *rhs;
+  const float* s;
+  double* y;
   CgState* st;
 };
 struct TailVecs {
@@ -507,9 +552,6 @@ __device__ __forceinline__ unsigned rank_addr(const void* p, int rank) {
   unsigned m;
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(m) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
   return m;
-}
-__device__ __forceinline__ void store_rank(const float* p, int rank, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(rank_addr(p, rank)), "f"(v) : "memory");
 }
 
 // The exchanges of a block, numbered: exchange k counts on bar[k & 1] in its (k >> 1)-th phase.
@@ -597,6 +639,69 @@ struct RowCache {
     return acc;
   }
 };
+
+// Sum of a double per thread over the cluster, in a fixed order, in thread 0 of every block (sh: one
+// double per thread, slot: two sets of kTailC; the sets alternate, and the barrier of a sum has every
+// block past its reading of the one before).
+template <bool EX, int T>
+__device__ __forceinline__ double cluster_total(double x, double* sh, double* slot, int rank, int& phase) {
+  sh[threadIdx.x] = x;
+  __syncthreads();
+  double* set = slot + (phase & 1) * kTailC;
+  phase++;
+  double s = 0.0;
+  if (threadIdx.x < 32) {
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < T / 32; k++) v[k & 3] += sh[threadIdx.x + 32 * k];
+    s = warp_sum((v[0] + v[1]) + (v[2] + v[3]));
+    if (EX && threadIdx.x < kTailC)
+      asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(rank_addr(set + rank, threadIdx.x)), "d"(s) : "memory");
+  }
+  if (EX) {
+    cluster_barrier();
+    if (threadIdx.x == 0) {
+      static_assert(kTailC == 8, "pairs of pairs of pairs");
+      s = ((set[0] + set[1]) + (set[2] + set[3])) + ((set[4] + set[5]) + (set[6] + set[7]));
+    }
+  }
+  return s;
+}
+
+// The same of a float per thread, as FP32 pairs (48 bits): a dependent FP64 addition takes some 200
+// cycles here, a pair one 40 (a sum 3.9k instead of 5.2k cycles).
+template <bool EX, int T>
+__device__ __forceinline__ double cluster_total(float x, double* sh_, double* slot, int rank, int& phase) {
+  float* sh = reinterpret_cast<float*>(sh_);
+  sh[threadIdx.x] = x;
+  __syncthreads();
+  float2* set = reinterpret_cast<float2*>(slot + (phase & 1) * kTailC);
+  phase++;
+  float2 s = make_float2(0.0f, 0.0f);
+  if (threadIdx.x < 32) {
+    float2 v[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) v[k] = s;
+#pragma unroll
+    for (int k = 0; k < T / 32; k++) v[k & 3] = pair_add(v[k & 3], make_float2(sh[threadIdx.x + 32 * k], 0.0f));
+    s = pair_add(pair_add(v[0], v[1]), pair_add(v[2], v[3]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s = pair_add(s, shfl_pair(s, o));
+    if (EX && threadIdx.x < kTailC)
+      asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(rank_addr(set + rank, threadIdx.x)), "f"(s.x),
+                   "f"(s.y)
+                   : "memory");
+  }
+  if (EX) {
+    cluster_barrier();
+    if (threadIdx.x == 0) {
+      s = set[0];
+#pragma unroll
+      for (int k = 1; k < kTailC; k++) s = pair_add(s, set[k]);
+    }
+  }
+  return (double)s.x + (double)s.y;
+}
 
 constexpr int kTailT = kMgTailDofs / kTailC;  // threads of a tail block: one per own unknown
 
@@ -706,10 +811,10 @@ __device__ __forceinline__ int tail_lanes(int rows, int T) {
 
 // the levels from l on, each whole in this block: (b in y and b) -> x
 template <int NB, int T>
-__device__ __noinline__ void tail_local(TailSync& sync, const TailLev* L, TailVecs* v, int l0, int last, int dot,
+__device__ __noinline__ void tail_local(TailSync& sync, const TailLev* L, TailVecs* v, int l0, int last, int deg0,
                                         bool fresh0, const float* dense, int N) {
   for (int l = l0; l < last; l++) {
-    tail_smooth<false, NB, T>(sync, L[l], v[l], dot && l == 0 ? kMgDeg0 : kMgDeg, l > l0 || fresh0, true);
+    tail_smooth<false, NB, T>(sync, L[l], v[l], l == l0 ? deg0 : kMgDeg, l > l0 || fresh0, true);
     TailVecs& c = v[l + 1];
     tail_transfer<false, NB, NB, T>(sync, L[l].pt_sptr, L[l].pt_col, L[l].pt_val, L[l].npt, nullptr, 0, c.r1,
                                     tail_lanes(c.r1 * NB, T), v[l].y, nullptr, c.y, c.b);
@@ -731,7 +836,7 @@ __device__ __noinline__ void tail_local(TailSync& sync, const TailLev* L, TailVe
   for (int l = last - 1; l >= l0; l--) {
     tail_transfer<false, NB, NB, T>(sync, L[l].p_sptr, L[l].p_col, L[l].p_val, L[l].np, nullptr, 0, v[l].r1, 0,
                                     v[l + 1].x, v[l].x, v[l].x, nullptr);
-    tail_smooth<false, NB, T>(sync, L[l], v[l], dot && l == 0 ? kMgDeg0 : kMgDeg, false, false);
+    tail_smooth<false, NB, T>(sync, L[l], v[l], l == l0 ? deg0 : kMgDeg, false, false);
   }
 }
 
@@ -743,11 +848,16 @@ __host__ __device__ inline int tail_floats(int n, int nb, bool ex) {
 }
 
 // NT: unknowns per node of the tail's first level, NC: of the others
-template <int NT, int NC, bool EX>
+// SOLVE (level 0 is in the tail): the whole of the conjugate gradients around the cycle as well, one
+// unknown per thread.  A block keeps the direction of every row that its own rows refer to and
+// advances it from the cycle's result, which has reached it, so the direction needs no exchange; the
+// cycle's right-hand side needs one, and the three sums a barrier of the cluster each.  (As five
+// launches an iteration the same took 52.7 us at 4225 unknowns, here 40.0, of which the cycle 25.)
+template <int NT, int NC, bool EX, bool SOLVE>
 __global__ void __launch_bounds__(kTailT, 1) k_mg_tail(const __grid_constant__ TailArgs a) {
   constexpr int T = kTailT;
   extern __shared__ float4 tail_sm4[];
-  __shared__ float dots[kTailC], tokens[kTailC];
+  __shared__ float tokens[kTailC];
   __shared__ unsigned long long bars[3];
   __shared__ TailLev lev[kMgMaxTail];
   float* sm = reinterpret_cast<float*>(tail_sm4);
@@ -821,8 +931,10 @@ __global__ void __launch_bounds__(kTailT, 1) k_mg_tail(const __grid_constant__ T
   TailSync sync{bars, tokens, rank, a.st};
   pdl_wait();
   const int n0 = a.L[0].n * NT, own0 = (v[0].r1 - v[0].r0) * NT, off0 = v[0].r0 * NT;
-  for (int t = threadIdx.x; t < n0; t += T) v[0].y[t] = a.b[t];
-  for (int t = threadIdx.x; t < own0; t += T) v[0].b[t] = a.b[off0 + t];
+  if (!SOLVE) {
+    for (int t = threadIdx.x; t < n0; t += T) v[0].y[t] = a.b[t];
+    for (int t = threadIdx.x; t < own0; t += T) v[0].b[t] = a.b[off0 + t];
+  }
   // (EX also: no block stores to another's shared memory before that block runs and has its barriers)
   if (EX) cluster_barrier();
   else __syncthreads();
@@ -834,65 +946,216 @@ __global__ void __launch_bounds__(kTailT, 1) k_mg_tail(const __grid_constant__ T
                    : "=r"(ok)
                    : "r"(fill)
                    : "memory");
-    if (!ok) a.st->done = 5;
+    if (!ok) sync.st->done = 5;
   };
   const int last = a.nl - 1;
-  for (int rep = 0; rep < a.reps; rep++) {
-    if constexpr (!EX && NT == NC) {
-      if (rep == 0) filled();
-      tail_local<NC, T>(sync, lev, v, 0, last, a.dot, rep == 0, dense, a.N);
-    } else {
-      const TailLev& L = lev[0];
-      const int deg = a.dot ? kMgDeg0 : kMgDeg;
-      if (!EX && rep == 0) filled();
-      tail_smooth<EX, NT, T>(sync, L, v[0], deg, rep == 0, true);
-      TailVecs& c = v[1];
-      const int nc = lev[1].n;
-      if (EX) {
-        // coarse right-hand side: rows dealt in ranges, whole to every block
-        const int ch = tail_chunk(nc), c0 = min(nc, rank * ch), c1 = min(nc, c0 + ch);
-        sync.expect(nc * NC);
-        tail_transfer<true, NC, NT, T>(sync, L.pt_sptr, L.pt_col, L.pt_val, L.npt, nullptr, c0, c1,
-                                       tail_lanes(ch * NC, T), v[0].y, nullptr, c.y, nullptr);
-        for (int t = threadIdx.x; t < nc * NC; t += T) c.b[t] = c.y[t];
-        if (rep == 0) filled();
+  constexpr int deg0 = SOLVE ? kMgDeg0 : kMgDeg;
+  // SOLVE: the directions, scales and own vectors behind the levels' in shared memory
+  double* dir = reinterpret_cast<double*>(sm);
+  double* res = dir + n0;
+  double* cor = res + T;
+  double* sh = cor + T;
+  double* slot = sh + T;
+  float* sc = reinterpret_cast<float*>(slot + 2 * kTailC);
+  __shared__ CgState loc;
+  __shared__ double bc[2];
+  __shared__ int range[2], due;
+  const int t = threadIdx.x, u = off0 + t;
+  const bool live = t < own0;
+  constexpr int U = 8;  // entries of a row whose loads are in flight together
+  int64_t base = 0;
+  int w = 0, phase = 0;
+  unsigned ranks = 0;
+  auto column = [&](int k) {
+    const int64_t idx = base + 32 * (int64_t)k;
+    int j = a.d16 ? colof<true>(a.col, idx, u) : colof<false>(a.col, idx, u);
+    if (!ADFEM_DCHECK(j >= 0 && j < n0)) j = u;
+    return j;
+  };
+  if constexpr (SOLVE) {
+    if (t == 0) {
+      loc = *a.st;
+      range[0] = n0;
+      range[1] = 0;
+      due = 1;
+    }
+    cor[t] = 0.0;
+    __syncthreads();
+    if (live) {
+      sell_row(a.sptr, u, base, w);
+      int lo = u, hi = u;
+      for (int k = 0; k < w; k++) {
+        const int j = column(k);
+        lo = min(lo, j);
+        hi = max(hi, j);
+      }
+      atomicMin(&range[0], lo);
+      atomicMax(&range[1], hi + 1);
+      if (EX) ranks = lev[0].to[u / NT];
+    }
+    __syncthreads();
+    for (int i = range[0] + t; i < range[1]; i += T) sc[i] = __ldg(a.s + i);
+    __syncthreads();
+    sync.st = &loc;
+  }
+  bool start = true;
+  double rn = 0.0;
+  float bn = 0.0f;
+  for (;;) {
+    if constexpr (SOLVE) {
+      const double g = loc.ar;
+      if (due) {
+        // r = b - K y in difference form, as k_mg_residual does; before it y += z, z = 0
+        if (live && !start) {
+          a.y[u] += cor[t];
+          cor[t] = 0.0;
+        }
+        if (EX) cluster_barrier();
+        else __syncthreads();
+        double rr = 0.0;
+        if (live) {
+          double yo[NT], s = 0.0;
+#pragma unroll
+          for (int q = 0; q < NT; q++) {
+            yo[q] = __ldcg(a.y + u / NT * NT + q);
+            s = fma(__ldg(a.rowsum + NT * u + q), yo[q], s);
+          }
+          for (int k0 = 0; k0 < w; k0 += U) {
+            double vv[U], x[U];
+#pragma unroll
+            for (int e = 0; e < U; e++) {
+              vv[e] = k0 + e < w ? __ldg(a.val + base + 32 * (k0 + e)) : 0.0;
+              x[e] = __ldcg(a.y + (k0 + e < w ? column(k0 + e) : u));
+            }
+#pragma unroll
+            for (int e = 0; e < U; e++)
+              if (k0 + e < w) s = fma(vv[e], x[e] - (e & 1 ? yo[NT - 1] : yo[0]), s);
+          }
+          const double ri = a.rhs[u] - s, tr = (double)sc[u] * ri;
+          res[t] = ri;
+          bn = (float)(tr * g);
+          rr = tr * tr;
+        }
+        rr = cluster_total<EX, T>(rr, sh, slot, rank, phase);
+        if (t == 0) {
+          loc.iters = loc.it;
+          mg_residual_step(&loc, rr, rn, start);
+        }
+        start = false;
         __syncthreads();
-      } else {
-        tail_transfer<false, NC, NT, T>(sync, L.pt_sptr, L.pt_col, L.pt_val, L.npt, nullptr, 0, c.r1,
-                                        tail_lanes(c.r1 * NC, T), v[0].y, nullptr, c.y, c.b);
+        if (loc.done) break;
       }
-      tail_local<NC, T>(sync, lev, v, 1, last, 0, true, dense, a.N);
+      // the cycle's right-hand side
+      if (live) v[0].b[t] = bn;
       if (EX) sync.expect(v[0].floats);
-      tail_transfer<EX, NT, NC, T>(sync, L.p_sptr, L.p_col, L.p_val, L.np, L.to, v[0].r0, v[0].r1, 0, v[1].x, v[0].x,
-                                   v[0].y, nullptr);
-      float* s = v[0].x;
-      v[0].x = v[0].y;
-      v[0].y = s;
-      tail_smooth<EX, NT, T>(sync, L, v[0], deg, false, false);
+      if (live) tail_put<EX>(sync, ranks, v[0].y, u, bn);
+      tail_end<EX>(sync);
     }
-  }
-  pdl_trigger();  // (not before: blocks that wait would keep other solves' kernels off the SMs)
-  float dot = 0.0f;
-  for (int t = threadIdx.x; t < own0; t += T) {
-    const float xi = v[0].x[off0 + t];
-    a.x[off0 + t] = xi;
-    dot = fmaf(xi, v[0].b[t], dot);
-  }
-  if (a.dot) {
-    float w[1] = {dot};
-    block_sum<float, 1, T>(w);
-    if (EX) {
-      if (threadIdx.x == 0) store_rank(dots + rank, 0, w[0]);
-      cluster_barrier();
-    }
-    if (rank == 0 && threadIdx.x == 0) {
-      float tot = w[0];
-      if (EX) {
-        tot = 0.0f;
-        for (int k = 0; k < kTailC; k++) tot += dots[k];
+    for (int rep = 0; rep < (SOLVE ? 1 : a.reps); rep++) {
+      const bool first = rep == 0;
+      if constexpr (!EX && NT == NC) {
+        if (first) filled();
+        tail_local<NC, T>(sync, lev, v, 0, last, deg0, first, dense, a.N);
+      } else {
+        const TailLev& L = lev[0];
+        if (!EX && first) filled();
+        tail_smooth<EX, NT, T>(sync, L, v[0], deg0, first, true);
+        TailVecs& c = v[1];
+        const int nc = lev[1].n;
+        if (EX) {
+          // coarse right-hand side: rows dealt in ranges, whole to every block
+          const int ch = tail_chunk(nc), c0 = min(nc, rank * ch), c1 = min(nc, c0 + ch);
+          sync.expect(nc * NC);
+          tail_transfer<true, NC, NT, T>(sync, L.pt_sptr, L.pt_col, L.pt_val, L.npt, nullptr, c0, c1,
+                                         tail_lanes(ch * NC, T), v[0].y, nullptr, c.y, nullptr);
+          for (int q = threadIdx.x; q < nc * NC; q += T) c.b[q] = c.y[q];
+          if (first) filled();
+          __syncthreads();
+        } else {
+          tail_transfer<false, NC, NT, T>(sync, L.pt_sptr, L.pt_col, L.pt_val, L.npt, nullptr, 0, c.r1,
+                                          tail_lanes(c.r1 * NC, T), v[0].y, nullptr, c.y, c.b);
+        }
+        tail_local<NC, T>(sync, lev, v, 1, last, kMgDeg, true, dense, a.N);
+        if (EX) sync.expect(v[0].floats);
+        tail_transfer<EX, NT, NC, T>(sync, L.p_sptr, L.p_col, L.p_val, L.np, L.to, v[0].r0, v[0].r1, 0, v[1].x,
+                                     v[0].x, v[0].y, nullptr);
+        float* s = v[0].x;
+        v[0].x = v[0].y;
+        v[0].y = s;
+        tail_smooth<EX, NT, T>(sync, L, v[0], deg0, false, false);
       }
-      a.rz[0] = (double)tot;
     }
+    if constexpr (!SOLVE) break;
+    if constexpr (SOLVE) {
+      const float* x = v[0].x;
+      // (a wait that gave up in any block ends the solve in all of them)
+      float zb = live ? x[u] * v[0].b[t] : 0.0f;
+      if (loc.done) zb = nanf("");
+      double d = cluster_total<EX, T>(zb, sh, slot, rank, phase);
+      if (t == 0) {
+        const double rz = d * loc.iar;
+        if (!(rz > 0.0) || !isfinite(rz)) loc.done = 2;
+        bc[0] = loc.ap != 0.0 ? 0.0 : rz * loc.irz;
+        loc.rz = rz;
+        loc.ap = 0.0;
+      }
+      __syncthreads();
+      if (loc.done) break;
+      const double bt = bc[0];
+      for (int i = range[0] + t; i < range[1]; i += T) {
+        const double zi = (double)(sc[i] * x[i]);
+        dir[i] = bt == 0.0 ? zi : fma(bt, dir[i], zi);
+      }
+      __syncthreads();
+      if (t == T - 1) loc.irz = 1.0 / loc.rz;  // (beside the product: the division is read an iteration later)
+      double q = 0.0, pu = 0.0;
+      if (live) {
+        for (int k0 = 0; k0 < w; k0 += U) {
+          double vv[U];
+          int j[U];
+#pragma unroll
+          for (int e = 0; e < U; e++) {
+            vv[e] = k0 + e < w ? __ldg(a.val + base + 32 * (k0 + e)) : 0.0;
+            j[e] = k0 + e < w ? column(k0 + e) : u;
+          }
+#pragma unroll
+          for (int e = 0; e < U; e++)
+            if (k0 + e < w) q = fma(vv[e], dir[j[e]], q);
+        }
+        pu = dir[u];
+      }
+      d = cluster_total<EX, T>(pu * q, sh, slot, rank, phase);
+      if (t == 0) {
+        if (!(d > 0.0) || !isfinite(d)) loc.done = 2;
+        bc[1] = loc.rz / d;
+        loc.it += 1;
+      }
+      __syncthreads();
+      if (loc.done) break;
+      const double al = bc[1], g = loc.ar;
+      if (live) {
+        cor[t] = fma(al, pu, cor[t]);
+        const double ri = fma(-al, q, res[t]);
+        res[t] = ri;
+        bn = (float)(ri * g) * sc[u];
+      }
+      d = cluster_total<EX, T>(live ? bn * bn : 0.0f, sh, slot, rank, phase);
+      if (t == 0) {
+        rn = d * loc.iar * loc.iar;
+        loc.rho_new = rn;
+        loc.iters = loc.it;
+        if (!isfinite(rn)) loc.done = 2;
+        due = rn <= loc.stop2 || rn <= loc.ru2 || loc.it >= loc.max_iter;
+      }
+      __syncthreads();
+      if (loc.done) break;
+    }
+  }
+  if constexpr (SOLVE) {
+    if (rank == 0 && t == 0) *a.st = loc;
+  } else {
+    pdl_trigger();  // (not before: blocks that wait would keep other solves' kernels off the SMs)
+    for (int q = threadIdx.x; q < own0; q += T) a.x[off0 + q] = v[0].x[off0 + q];
   }
 }
 
@@ -1399,44 +1662,6 @@ __global__ void __launch_bounds__(kT) k_mg_init(int64_t n, const double* __restr
   }
 }
 
-// The residual decides: converged, at its attainable floor, out of iterations, or go on (the
-// rules of replacement_step64, whose direction scalars do not apply here).
-// rn: the recurrence's residual (its square, as rr)
-__device__ __forceinline__ void mg_residual_step(CgState* st, double rr, double rn, bool first) {
-  const double prev = st->last_rr64;
-  st->rr64 = rr;
-  st->last_rr64 = rr;
-  if (!isfinite(rr)) {
-    st->done = 2;
-    return;
-  }
-  if (rr <= st->stop2) {
-    st->done = 1;
-    return;
-  }
-  if (!first) {
-    const bool dropped = rn <= st->delta2 * prev;
-    if (prev > 0.0 && rr > 0.0625 * prev && (dropped || st->final_seen)) {
-      st->floor_hit = 1;
-      st->done = 1;
-      return;
-    }
-  }
-  if (st->iters >= st->max_iter) {
-    st->done = 4;
-    return;
-  }
-  if (!first && rn <= st->stop2) st->final_seen = 1;
-  if (!first) st->updates += 1;
-  // A residual that is not the recurrence's (near the attainable floor it can be many times
-  // larger) has nothing to do with the directions so far: keeping them made the iteration
-  // stagnate (elasticity, 320k DOF: over 200 iterations to the floor instead of 10).
-  if (first || rr > 1.21 * rn) st->ap = 1.0;
-  st->fold = 1;
-  st->ru2 = st->delta2 * rr;
-  st->done = 0;
-}
-
 // r = b - K y in FP64, in difference form: row sums times the row's own unknowns plus entries
 // times differences, so that it rounds with the differences of the solution.
 // The iterate is y + z; the next direction kernel folds z into y (st->fold).
@@ -1904,6 +2129,10 @@ int mg_plan(Solver& S) {
   size_t fl = 0;
   for (int l = M.tail; l < M.nlev; l++) fl += (size_t)tail_floats(M.lev[l].n, M.lev[l].nb, M.cluster && l == M.tail);
   M.tail_smem = sizeof(float) * fl;
+  if (M.tail == 0) {
+    const size_t n0 = (size_t)M.lev[0].n * M.lev[0].nb;
+    M.tail_smem += sizeof(double) * (n0 + 3 * kTailT + 2 * kTailC) + sizeof(float) * n0;
+  }
   M.pat = M.slab.as<char>() + pat0;
   M.vals = M.slab.as<char>() + val0;
   if (M.tail_smem + M.pat_bytes + M.val_bytes > kTailSmem) M.pat_bytes = M.val_bytes = 0;  // read through L1
@@ -1918,9 +2147,16 @@ int mg_plan(Solver& S) {
       const int dmax = (int)(sizeof(float) * (kMgDense * kMgDense + 4 * kMgDense));
       const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
       for (cudaError_t e :
-           {cudaFuncSetAttribute(k_mg_tail<1, 1, false>, a, tmax), cudaFuncSetAttribute(k_mg_tail<2, 3, false>, a, tmax),
-            cudaFuncSetAttribute(k_mg_tail<3, 3, false>, a, tmax), cudaFuncSetAttribute(k_mg_tail<1, 1, true>, a, tmax),
-            cudaFuncSetAttribute(k_mg_tail<2, 3, true>, a, tmax), cudaFuncSetAttribute(k_mg_tail<3, 3, true>, a, tmax),
+           {cudaFuncSetAttribute(k_mg_tail<1, 1, false, false>, a, tmax),
+            cudaFuncSetAttribute(k_mg_tail<2, 3, false, false>, a, tmax),
+            cudaFuncSetAttribute(k_mg_tail<3, 3, false, false>, a, tmax),
+            cudaFuncSetAttribute(k_mg_tail<1, 1, true, false>, a, tmax),
+            cudaFuncSetAttribute(k_mg_tail<2, 3, true, false>, a, tmax),
+            cudaFuncSetAttribute(k_mg_tail<3, 3, true, false>, a, tmax),
+            cudaFuncSetAttribute(k_mg_tail<1, 1, false, true>, a, tmax),
+            cudaFuncSetAttribute(k_mg_tail<2, 3, false, true>, a, tmax),
+            cudaFuncSetAttribute(k_mg_tail<1, 1, true, true>, a, tmax),
+            cudaFuncSetAttribute(k_mg_tail<2, 3, true, true>, a, tmax),
             cudaFuncSetAttribute(k_mg_dense<1>, a, dmax), cudaFuncSetAttribute(k_mg_dense<3>, a, dmax)})
         if (e != cudaSuccess) err = e;
     });
@@ -2082,11 +2318,38 @@ void prolong_from(const Solver& S, const MgLev& L, const float* xc, float* x, cu
   else mg_launch(S, st, k_mg_prolong<3, 3>, g, kT, 0, 1, L, xc, x);
 }
 
-template <int NT, int NC>
+template <int NT, int NC, bool SOLVE>
 void launch_tail(const Solver& S, const TailArgs& a, cudaStream_t st) {
   const Mg& M = *S.mg;
-  if (M.cluster) mg_launch(S, st, k_mg_tail<NT, NC, true>, kTailC, kTailT, M.tail_smem, kTailC, a);
-  else mg_launch(S, st, k_mg_tail<NT, NC, false>, 1, kTailT, M.tail_smem, 1, a);
+  if (M.cluster) mg_launch(S, st, k_mg_tail<NT, NC, true, SOLVE>, kTailC, kTailT, M.tail_smem, kTailC, a);
+  else mg_launch(S, st, k_mg_tail<NT, NC, false, SOLVE>, 1, kTailT, M.tail_smem, 1, a);
+}
+
+TailArgs tail_args(Solver& S) {
+  const Mg& M = *S.mg;
+  const Sell& A = *S.A;
+  TailArgs a;
+  a.nl = M.nlev - M.tail;
+  for (int l = 0; l < a.nl; l++) a.L[l] = M.lev[M.tail + l];
+  a.dense = M.dense;
+  a.N = M.ndense;
+  a.pat = M.pat;
+  a.vals = M.vals;
+  a.pat_bytes = M.pat_bytes;
+  a.val_bytes = M.val_bytes;
+  a.b = M.lev[M.tail].b;
+  a.x = M.lev[M.tail].x;
+  a.reps = M.tail >= 3 ? 2 : 1;
+  a.st = S.state.as<CgState>();
+  a.sptr = A.sptr.as<int32_t>();
+  a.col = A.col.p;
+  a.d16 = A.delta16 ? 1 : 0;
+  a.val = A.val64.as<double>();
+  a.rowsum = M.rowsum;
+  a.rhs = S.b.as<double>();
+  a.s = S.s32.as<float>();
+  a.y = S.y64.as<double>();
+  return a;
 }
 
 // One cycle: lev[0].b -> the vector returned; returns the launches through *count.
@@ -2113,26 +2376,11 @@ const float* enqueue_cycle(Solver& S, cudaStream_t st, int* count) {
     xs[l] = x;
   }
   {
-    TailArgs a;
-    a.nl = M.nlev - M.tail;
-    for (int l = 0; l < a.nl; l++) a.L[l] = M.lev[M.tail + l];
-    a.dense = M.dense;
-    a.N = M.ndense;
-    a.pat = M.pat;
-    a.vals = M.vals;
-    a.pat_bytes = M.pat_bytes;
-    a.val_bytes = M.val_bytes;
-    a.b = M.lev[M.tail].b;
-    a.x = M.lev[M.tail].x;
-    a.reps = M.tail >= 3 ? 2 : 1;
-    a.dot = M.tail == 0;
-    a.rz = M.part;
-    M.nrz = 1;  // (replaced by the last sweep of a level 0 above the tail)
-    a.st = cs;
+    const TailArgs a = tail_args(S);
     const int nt = a.L[0].nb;
-    if (nt == 1) launch_tail<1, 1>(S, a, st);
-    else if (nt == 2) launch_tail<2, 3>(S, a, st);
-    else launch_tail<3, 3>(S, a, st);
+    if (nt == 1) launch_tail<1, 1, false>(S, a, st);
+    else if (nt == 2) launch_tail<2, 3, false>(S, a, st);
+    else launch_tail<3, 3, false>(S, a, st);
     xs[M.tail] = M.lev[M.tail].x;
     nl++;
   }
@@ -2255,8 +2503,9 @@ int mg_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_rows, 
              bool* gave_up) {
   *gave_up = false;
   ADFEM_TRY(mg_values(S, user));
-  ADFEM_TRY(capture_solve(S));
   Mg& M = *S.mg;
+  const bool one = M.tail == 0;  // the whole solve in one launch
+  if (!one) ADFEM_TRY(capture_solve(S));
   cudaStream_t st = S.stream;
   ADFEM_CUDA(cudaEventRecord(S.ev[0], user));
   ADFEM_CUDA(cudaStreamWaitEvent(st, S.ev[0], 0));
@@ -2271,12 +2520,18 @@ int mg_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_rows, 
                                    o.warm_start ? u : nullptr, S.b.as<double>(), S.y64.as<double>(),
                                    S.z64.as<double>(), S.state.as<CgState>(), S.partials.as<double>(),
                                    o.rtol * o.rtol);
-  const cudaGraphConditionalHandle none{};
-  enqueue_residual(S, 0, none, st);
-  ADFEM_CUDA(cudaGetLastError());
-  ADFEM_CUDA(cudaGraphLaunch(M.solve, st));
-  solver_enqueue_fold64(S, 1, st);
-  enqueue_residual(S, 2, none, st);
+  if (one) {
+    const TailArgs a = tail_args(S);
+    if (M.lev[0].nb == 1) launch_tail<1, 1, true>(S, a, st);
+    else launch_tail<2, 3, true>(S, a, st);
+  } else {
+    const cudaGraphConditionalHandle none{};
+    enqueue_residual(S, 0, none, st);
+    ADFEM_CUDA(cudaGetLastError());
+    ADFEM_CUDA(cudaGraphLaunch(M.solve, st));
+    solver_enqueue_fold64(S, 1, st);
+    enqueue_residual(S, 2, none, st);
+  }
   // (the caller's vector is written after the outcome is known to be usable: a solve that gives
   // up leaves it as the other iteration's start)
   ADFEM_CUDA(cudaMemcpyAsync(&S.h_state[0], S.state.p, sizeof(CgState), cudaMemcpyDeviceToHost, st));
@@ -2304,7 +2559,7 @@ int mg_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_rows, 
     stats->relres = relres;
     stats->ms = ms;
     stats->status = status;
-    stats->launches = (long long)std::max(fin.iters, 1) * M.body_launches + 5;
+    stats->launches = one ? 3 : (long long)std::max(fin.iters, 1) * M.body_launches + 5;
   }
   if (status == ADFEM_ERR_NOT_CONVERGED)
     return fail(status, "CG did not reach rtol within max_iter (relres " + std::to_string(relres) + ")");
