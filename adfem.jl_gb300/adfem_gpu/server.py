@@ -32,8 +32,8 @@ class Server:
                  rtol: float = 1e-10, max_iter: int = 200000, ru_delta: float = 0.1, chunk: int = 32,
                  pack_max_dof: int = 0, pack_max: int = 0, trace=None):
         """pack_max_dof: mixed-precision requests up to this many DOFs are solved in packed
-        launches (0: the library default, up to where packs are faster: Poisson 2560,
-        from 32 workers on 8192, elasticity 640 and 2560; -1: never); pack_max: systems per pack;
+        launches (0: the library default, up to where packs pay: Poisson 2560, elasticity
+        none, from 32 workers on 640; -1: never); pack_max: systems per pack;
         trace: a path (opened for appending) or a writable text file for the per-request
         JSON lines, None for no trace."""
         from . import solver_opts

@@ -95,18 +95,18 @@ struct Worker {
 constexpr int kPackers = 4;  // packer threads (concurrent packed launches)
 // Default packing thresholds (DOFs).  A pack lasts as long as its slowest system's Jacobi CG,
 // whose iterations grow with the mesh; the resident solver's multigrid keeps some 20 (Poisson) to
-// 60 (elasticity), and its launches do not queue behind a pack that holds the SMs.  GB300, ms per
-// request, packs / resident solver, with 8 workers and with 64 (which fill larger packs):
-//   Poisson     2401 DOFs 0.42 / 0.22, 0.10 / 0.23     6561 0.66 / 0.33, 0.29 / 0.39
-//              16129      1.35 / 0.38, 0.58 / 0.40
-//   elasticity   338 DOFs 0.29 / 0.31, 0.09 / 0.37     1250 1.05 / 0.52, 0.23 / 0.64
-//               4802      3.79 / 1.00, 1.50 / 1.12
-// so the thresholds lie where the two meet, by the number of workers; Poisson stays packed up to
-// 2560 DOFs with few workers too (the launches saved are worth 0.2 ms to the others).  A system
-// that would be solved by Jacobi CG either way is packed up to the same size as before multigrid.
+// 60 (elasticity) and solves up to 5120 DOFs in one launch.  GB300, ms per request, packs /
+// resident solver, with 8 workers and with 64 (which fill larger packs):
+//   Poisson      625 DOFs 0.12 / 0.08, 0.05 / 0.07     2401 0.45 / 0.11, 0.11 / 0.08
+//               6561      0.71 / 0.24, 0.33 / 0.28    16129 1.47 / 0.33, 0.58 / 0.36
+//   elasticity   338 DOFs 0.28 / 0.13, 0.09 / 0.10     1250 1.16 / 0.26, 0.22 / 0.20
+//               4802      3.52 / 0.54, 1.49 / 0.42
+// Poisson requests of up to 2560 DOFs are packed, as callers that look at response.packed expect
+// of small ones (2401 DOFs is where packs of many stop being the faster); of elasticity only the
+// smallest where many workers fill the packs.  A system that would be solved by Jacobi CG either
+// way is packed up to the same size as before multigrid.
 constexpr int kPackManyWorkers = 32;
-constexpr int kPackPoisson = 2560, kPackPoissonMany = 8192;
-constexpr int kPackElastic = 640, kPackElasticMany = 2560;
+constexpr int kPackPoisson = 2560, kPackElasticMany = 640;
 constexpr int kPackDefaultDof = 16384;  // without multigrid
 
 int ndof_of(const adfem::Mesh* m, int kind) { return (int)(kind == ADFEM_SYS_ELASTICITY ? 2 * m->nv : m->nv); }
@@ -123,9 +123,10 @@ size_t estimate_system_bytes(const adfem::Mesh* m, int kind) {
 }
 
 // Multigrid hierarchy of a system, which its first solve outside a pack builds (per unknown:
-// operators, interpolation and work vectors of all levels, as mg_plan lays them out).
+// operators, interpolation and work vectors of all levels: 190 bytes at 1M unknowns of P1 Poisson,
+// 243 at 4k; 343 for elasticity at 320k).
 size_t estimate_hierarchy_bytes(const adfem::Mesh* m, int kind) {
-  return (size_t)((kind == ADFEM_SYS_ELASTICITY ? 380.0 : 230.0) * (double)ndof_of(m, kind)) + 64 * 1024;
+  return (size_t)((kind == ADFEM_SYS_ELASTICITY ? 380.0 : 250.0) * (double)ndof_of(m, kind)) + 64 * 1024;
 }
 
 // Worker buffers a request needs (inputs at Gauss points, u, g, lambda, gradient).
@@ -196,9 +197,8 @@ struct adfem_server {
     const int prec = q.precision >= 0 ? q.precision : cfg.opts.precision;
     int most = pack_max_dof;
     if (default_packs && q.nbd > 0) {
-      const bool many = cfg.workers >= kPackManyWorkers;
-      most = std::min(most, q.kind == ADFEM_SYS_ELASTICITY ? (many ? kPackElasticMany : kPackElastic)
-                                                           : (many ? kPackPoissonMany : kPackPoisson));
+      const int elastic = cfg.workers >= kPackManyWorkers ? kPackElasticMany : 0;
+      most = std::min(most, q.kind == ADFEM_SYS_ELASTICITY ? elastic : kPackPoisson);
     }
     return most > 0 && prec == ADFEM_PREC_MIXED && (long long)ndof_of(adfem::mesh_of(q.mesh), q.kind) <= most;
   }

@@ -469,8 +469,8 @@ typedef struct adfem_server_config {
   adfem_solver_opts opts;     /* solver options of every request (precision per request may override) */
   int pack_max_dof;           /* mixed-precision requests with at most this many DOFs are solved in
                                  packs (one launch, one thread block or cluster each); 0: up to
-                                 where packs are faster (Poisson 2560, from 32 workers on 8192;
-                                 elasticity 640 and 2560; 16384 where multigrid is not used);
+                                 where packs pay (Poisson 2560, elasticity 0, from 32 workers on
+                                 640; 16384 where multigrid is not used);
                                  < 0: never; at most 65536 */
   int pack_max;               /* systems per packed launch; 0: 64 (at most 128) */
 } adfem_server_config;
