@@ -146,11 +146,18 @@ __device__ __forceinline__ void elastic_row_add(const double* __restrict__ Db, c
     v1 = fma(ga.y, d[4], ga.x * d[7]);
     v2 = fma(ga.y, d[5], ga.x * d[8]);
   }
+  // (the six slots differ: read before any is written, their chains run side by side)
+  double ax[3], ay[3];
+#pragma unroll
+  for (int b = 0; b < 3; b++) {
+    ax[b] = acc[sl.x[b]][t];
+    ay[b] = acc[sl.y[b]][t];
+  }
 #pragma unroll
   for (int b = 0; b < 3; b++) {
     const double2 gb = gr[b];
-    acc[sl.x[b]][t] = fma(v0, gb.x, fma(v2, gb.y, acc[sl.x[b]][t]));
-    acc[sl.y[b]][t] = fma(v1, gb.y, fma(v2, gb.x, acc[sl.y[b]][t]));
+    acc[sl.x[b]][t] = fma(v0, gb.x, fma(v2, gb.y, ax[b]));
+    acc[sl.y[b]][t] = fma(v1, gb.y, fma(v2, gb.x, ay[b]));
   }
 }
 
