@@ -7,26 +7,31 @@ namespace adfem {
 namespace {
 
 // Aggregates of the graph.  First pass, in node order: a node none of whose neighbours is
-// taken becomes the root of an aggregate of itself and its neighbours.  Second pass: the
+// taken becomes the root of an aggregate of itself and its neighbours; with short_first, nodes with
+// fewer neighbours than the average before the others (P2: edges, 9 entries a row, before
+// vertices, 19, which makes aggregates of 9 instead of 16: 33 instead of 42 iterations at 5k DOF,
+// 35 instead of 43 at 44k, 40 instead of 42 at 243k).  Second pass: the
 // nodes left over join the neighbouring first-pass aggregate with which they share the most
 // edges (the lowest-numbered of equals); nodes without one become aggregates of their own.
 // Nodes without neighbours (eliminated rows of a user's matrix, whose interpolation is zero) are
 // dealt over the aggregates in node order: on their own they would be unknowns of every level.
-int64_t aggregate(int64_t n, const MgPattern& A, std::vector<int32_t>& agg) {
+int64_t aggregate(int64_t n, const MgPattern& A, std::vector<int32_t>& agg, bool short_first) {
   agg.assign(n, -1);
   int32_t na = 0;
   auto alone = [&](int64_t i) {
     return A.rp[i + 1] == A.rp[i] || (A.rp[i + 1] == A.rp[i] + 1 && A.ci[A.rp[i]] == i);
   };
-  for (int64_t i = 0; i < n; i++) {
-    if (agg[i] >= 0 || alone(i)) continue;
-    bool free = true;
-    for (int32_t k = A.rp[i]; k < A.rp[i + 1] && free; k++) free = agg[A.ci[k]] < 0;
-    if (!free) continue;
-    agg[i] = na;
-    for (int32_t k = A.rp[i]; k < A.rp[i + 1]; k++) agg[A.ci[k]] = na;
-    na++;
-  }
+  for (int pass = short_first ? 0 : 1; pass < 2; pass++)
+    for (int64_t i = 0; i < n; i++) {
+      if (agg[i] >= 0 || alone(i)) continue;
+      if (pass == 0 && n * (A.rp[i + 1] - A.rp[i]) >= (int64_t)A.rp[n]) continue;
+      bool free = true;
+      for (int32_t k = A.rp[i]; k < A.rp[i + 1] && free; k++) free = agg[A.ci[k]] < 0;
+      if (!free) continue;
+      agg[i] = na;
+      for (int32_t k = A.rp[i]; k < A.rp[i + 1]; k++) agg[A.ci[k]] = na;
+      na++;
+    }
   std::vector<std::pair<int64_t, int32_t>> late;
   std::vector<int32_t> c;
   for (int64_t i = 0; i < n; i++) {
@@ -114,7 +119,11 @@ bool mg_build_host(int64_t n, std::vector<int32_t>&& rp, std::vector<int32_t>&& 
     const int nb = lv.size() == 1 ? nb0 : nbc;
     if (L.n * nb <= kMgDense) break;
     if ((int)lv.size() == kMgMaxLevels) return false;
-    const int64_t nc = aggregate(L.n, L.A, L.agg);
+    // (rows of two kinds: on the system's own level, where the longest is 1.5 times the average)
+    int64_t longest = 0;
+    if (lv.size() == 1)
+      for (int64_t i = 0; i < L.n; i++) longest = std::max<int64_t>(longest, L.A.rp[i + 1] - L.A.rp[i]);
+    const int64_t nc = aggregate(L.n, L.A, L.agg, 2 * longest * L.n >= 3 * (int64_t)L.A.rp[L.n]);
     if (2 * nc > L.n) return false;  // hardly any edges: no hierarchy
     auto rows = [](const MgPattern& Q, int64_t i, auto&& add) {
       for (int32_t k = Q.rp[i]; k < Q.rp[i + 1]; k++) add(Q.ci[k]);
