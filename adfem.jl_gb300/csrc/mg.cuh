@@ -51,6 +51,7 @@ bool mg_build_host(int64_t n, std::vector<int32_t>&& rp, std::vector<int32_t>&& 
 struct MgLev {
   int n = 0, nc = 0, nb = 1, nbc = 1, lpr = 1;
   int nv = 0, np = 0, nap = 0, npt = 0;  // entries of val, p_val, ap_val, pt_val
+  int width = 0;               // longest row of the operator
   int d16 = 0;                 // level 0 only: the system's own pattern (int16 deltas, slice patterns)
   const int32_t *sptr = nullptr, *spat = nullptr;
   const void* col = nullptr;

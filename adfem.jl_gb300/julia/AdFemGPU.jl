@@ -159,7 +159,8 @@ struct SolverStats
     launches::Clonglong
 end
 
-"""`K\\F` on the GPU for a symmetric positive definite K (Jacobi-CG, FP64 or mixed)."""
+"""`K\\F` on the GPU for a symmetric positive definite K (conjugate gradients, FP64 or mixed; FP64
+with multigrid where K is a scalar problem with eliminated rows)."""
 function gpu_solve(K::SparseMatrixCSC{Float64,Int64}, F::Vector{Float64}; kw...)
     u = zeros(length(F))
     o = Ref(SolverOpts(; kw...))
