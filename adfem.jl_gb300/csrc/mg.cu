@@ -1873,15 +1873,18 @@ __global__ void __launch_bounds__(kT) k_mg_dir(int64_t n, const float* c, const 
     }
 }
 
-// q = K p and p.q, one row per thread, entries in groups of 8, the first loaded ahead (MORE: rows
-// may have more: P2, elasticity)
+// q = K p and p.q, one row per thread, entries in groups whose loads are in flight together, the
+// first loaded ahead.  Rows of up to 8 entries are one group; longer ones (MORE: P2, elasticity) go in
+// groups of 4, which leaves room for eight blocks on an SM: their scattered reads of p are what bounds
+// them, and those overlap by warps rather than within a row (P2 4M DOF, ms a solve: groups of 12 and
+// three blocks 79.3, 8 and five 73.2, 6 and six 71.1, 4 and eight 68.0).
 template <bool D16, bool MORE>
-__global__ void __launch_bounds__(kT, MORE ? 3 : 4) k_mg_spmv(int64_t n, const int32_t* __restrict__ sptr,
+__global__ void __launch_bounds__(kT, MORE ? 8 : 4) k_mg_spmv(int64_t n, const int32_t* __restrict__ sptr,
                                                    const void* __restrict__ col, const int32_t* __restrict__ spat,
                                                    const int16_t* __restrict__ pat, int period,
                                                    const double* __restrict__ val, const double* p, double* q,
                                                    CgState* st, double* partials) {
-  constexpr int W = MORE ? 12 : 8;
+  constexpr int W = MORE ? 4 : 8;
   pdl_trigger();
   double v[W], acc = 0.0;
   int j[W], w = 0;
