@@ -17,7 +17,7 @@
 // scatter (load vector, summed operators, interpolation transposes), walking the
 // DOF->element incidence in ascending element order, so results are deterministic
 // and no atomics are needed.  The per-point basis tables of the degree are built in
-// shared memory by every block from the rule (a few hundred flops).
+// shared memory by every block (formed from the rule by the compiler).
 #include <mutex>
 
 #include "adfem_internal.h"
@@ -33,7 +33,7 @@ constexpr int kRowBTs = 128;  // rows per block of the resident-system row kerne
 // rule points (xi, eta, weight) on the reference triangle: order 2 (3 points, P1) and
 // order 4 (6 points, P2: the published Strang-Fix/Dunavant rule); same constants as
 // the host tables of mesh.cpp
-__constant__ double c_rule[2][6][3] = {
+constexpr double c_rule[2][6][3] = {
     {{1.0 / 6.0, 1.0 / 6.0, 1.0 / 6.0},
      {1.0 / 6.0, 2.0 / 3.0, 1.0 / 6.0},
      {2.0 / 3.0, 1.0 / 6.0, 1.0 / 6.0},
@@ -62,14 +62,14 @@ struct Tab {
 // vertices and edge midpoints, vertex functions first, then edges (0,1), (1,2),
 // (2,0)): phi_a = l_a (2 l_a - 1), phi_ab = 4 l_a l_b.
 template <int DEG>
-__device__ void tab_init(Tab<DEG>& T) {
+constexpr Tab<DEG> make_tab() {
   constexpr int ND = Tab<DEG>::ND, NG = Tab<DEG>::NG;
-  for (int k = threadIdx.x; k < NG; k += blockDim.x) {
+  Tab<DEG> T{};
+  for (int k = 0; k < NG; k++) {
     const double xi = c_rule[DEG - 1][k][0], eta = c_rule[DEG - 1][k][1];
     const double l[3] = {1.0 - xi - eta, xi, eta};
     T.w[k] = c_rule[DEG - 1][k][2];
     for (int c = 0; c < 3; c++) T.l[k][c] = l[c];
-    for (int r = 0; r < ND; r++) T.t[k][r][0] = T.t[k][r][1] = T.t[k][r][2] = 0.0;
     if (DEG == 1) {
       for (int r = 0; r < 3; r++) {
         T.h[k][r] = l[r];
@@ -89,6 +89,20 @@ __device__ void tab_init(Tab<DEG>& T) {
     }
     for (int r = 0; r < ND; r++) T.hw[k][r] = T.h[k][r] * T.w[k] / 0.5;
   }
+  return T;
+}
+__device__ constexpr Tab<1> c_tab1 = make_tab<1>();
+__device__ constexpr Tab<2> c_tab2 = make_tab<2>();
+
+// The table in shared memory.  (Copied from memory: formed by a block's first threads, its chain of
+// FP64 operations held every block back: interpolation transpose 41 instead of 33 us at 641k rows.)
+template <int DEG>
+__device__ __forceinline__ void tab_init(Tab<DEG>& T) {
+  const double* src;
+  if constexpr (DEG == 1) src = reinterpret_cast<const double*>(&c_tab1);
+  else src = reinterpret_cast<const double*>(&c_tab2);
+  for (int i = threadIdx.x; i < (int)(sizeof(Tab<DEG>) / sizeof(double)); i += blockDim.x)
+    reinterpret_cast<double*>(&T)[i] = __ldg(src + i);
   __syncthreads();
 }
 
@@ -771,20 +785,18 @@ __global__ void __launch_bounds__(kGT) k_gen_ke_stiffness(int64_t ne, const doub
   }
 }
 
-// Summed rows, one thread per scalar DOF row (every FP64 add of a warp does 32 rows'
-// work): the row is accumulated in a per-thread shared-memory buffer of CAP entries in
-// ascending element order, then written out.  The block's rows occupy one contiguous
-// range of vals, written by the whole block in order.  NB = 1: scalar operator (row of
-// len entries).  NB = 2: [x; y] elasticity blocks; the thread owns the x row at
-// 2 rowptr[i] and the y row at 2 nnz + 2 rowptr[i], each with the x columns, then the y
-// columns, of the scalar row; transpose gives the CSC values.  Rows longer than the
-// buffer are summed in place in global memory.
-template <int DEG, int NB, int BT, int CAP>
+// Summed rows of [x; y] elasticity blocks, one thread per scalar DOF row (every FP64 add of a warp
+// does 32 rows' work): the thread owns the x row at 2 rowptr[i] and the y row at 2 nnz + 2 rowptr[i],
+// each with the x columns, then the y columns, of the scalar row, accumulated in a per-thread
+// shared-memory buffer of CAP entries in ascending element order; transpose gives the CSC values.
+// The block's rows occupy one contiguous range of each half of vals, written by the whole block in
+// order.  Rows longer than the buffer are summed in place in global memory.
+template <int DEG, int BT, int CAP>
 __global__ void __launch_bounds__(BT) k_gen_rows(int64_t ndof, int64_t nnz, const int32_t* __restrict__ rowptr,
                                                  const int32_t* __restrict__ inc_ptr, const uint4* __restrict__ inc,
                                                  const double* __restrict__ ke, double* __restrict__ vals,
                                                  bool transpose) {
-  constexpr int ND = Tab<DEG>::ND, KN = NB * ND;  // element matrix is KN x KN
+  constexpr int NB = 2, ND = Tab<DEG>::ND, KN = NB * ND;  // element matrix is KN x KN
   extern __shared__ double buf[];                 // [NB][CAP][BT]
   __shared__ int32_t srp[BT + 1];
   const int tid = threadIdx.x;
@@ -1310,8 +1322,8 @@ cudaError_t launch_gen_stiffness_matrix(const Mesh& m, const Space& sp, const do
   static std::once_flag once;
   std::call_once(once, [] {
     const int bytes = (int)(sizeof(double) * 2 * kRowCap2 * kRowBT);
-    cudaFuncSetAttribute(k_gen_rows<1, 2, kRowBT, kRowCap2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(k_gen_rows<2, 2, kRowBT, kRowCap2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaFuncSetAttribute(k_gen_rows<1, kRowBT, kRowCap2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaFuncSetAttribute(k_gen_rows<2, kRowBT, kRowCap2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   });
   const int gr = grid_for(sp.ndof, kRowBT);
   const size_t smem = sizeof(double) * 2 * kRowCap2 * kRowBT;
@@ -1319,9 +1331,9 @@ cudaError_t launch_gen_stiffness_matrix(const Mesh& m, const Space& sp, const do
   const int32_t* ip = sp.d_inc_ptr.as<int32_t>();
   const uint4* inc = sp.d_inc.as<uint4>();
   GEN_DISPATCH(sp,
-               (k_gen_rows<1, 2, kRowBT, kRowCap2><<<gr, kRowBT, smem, st>>>(sp.ndof, sp.nnz, rp, ip, inc, ke, vals,
+               (k_gen_rows<1, kRowBT, kRowCap2><<<gr, kRowBT, smem, st>>>(sp.ndof, sp.nnz, rp, ip, inc, ke, vals,
                                                                               transpose)),
-               (k_gen_rows<2, 2, kRowBT, kRowCap2><<<gr, kRowBT, smem, st>>>(sp.ndof, sp.nnz, rp, ip, inc, ke, vals,
+               (k_gen_rows<2, kRowBT, kRowCap2><<<gr, kRowBT, smem, st>>>(sp.ndof, sp.nnz, rp, ip, inc, ke, vals,
                                                                               transpose)));
   return cudaGetLastError();
 }

@@ -822,7 +822,7 @@ struct Timer {
   }
 };
 
-void solver_enqueue_spmv64(Solver& S, const double* vals, cudaStream_t st) {
+static void enqueue_spmv64(Solver& S, const double* vals, cudaStream_t st) {
   const Sell& A = *S.A;
   ADFEM_SELL_DISPATCH(S, k_cg64_spmv, S.grid_spmv, st, S.n, A.sptr.as<int32_t>(), A.col.p, sell_pat(A), vals,
                       S.p64.as<double>(), S.q64.as<double>(), S.state.as<CgState>(), S.partials.as<double>());
@@ -838,7 +838,7 @@ static void enqueue_cg64(Solver& S, cudaStream_t st, Timer* tm = nullptr) {
   if (!tm) tm = &none;
   auto* cs = S.state.as<CgState>();
   auto* part = S.partials.as<double>();
-  tm->run(0, st, [&] { solver_enqueue_spmv64(S, S.vals64.as<double>(), st); });
+  tm->run(0, st, [&] { enqueue_spmv64(S, S.vals64.as<double>(), st); });
   tm->run(1, st, [&] {
     k_cg64_update<<<S.grid, kT, 0, st>>>(S.n, S.z64.as<double>(), S.r64.as<double>(), S.p64.as<double>(),
                                          S.q64.as<double>(), cs, part);

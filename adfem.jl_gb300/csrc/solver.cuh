@@ -141,7 +141,6 @@ int mg_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_rows, 
 size_t mg_device_bytes(const Solver& S);
 // kernels of the FP64 CG that mg.cu shares: q64 = K p64 with alpha = rho / p.q for the given
 // values, and y64 += z64, z64 = 0 (when a residual is due, or forced)
-void solver_enqueue_spmv64(Solver& S, const double* vals, cudaStream_t st);
 void solver_enqueue_fold64(Solver& S, int force, cudaStream_t st);
 
 // Banded mixed path (zcg.cu).  zcg_plan decides whether the operator's band fits
