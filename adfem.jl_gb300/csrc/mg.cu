@@ -2277,7 +2277,9 @@ void level_values(const MgLev& L, const MgLev& C, bool top, cudaStream_t st) {
 
 }  // namespace
 
-// values of the hierarchy for the current assembly (s32 is current)
+// Enqueues the values of the hierarchy for the current assembly (s32 is current).  They count as
+// made (Mg::current) once the host has seen the stream past them, in mg_solve: on a stream that is
+// being captured nothing runs, and a call that fails before then leaves them to the next.
 int mg_values(Solver& S, cudaStream_t st) {
   Mg& M = *S.mg;
   if (M.current) return ADFEM_OK;
@@ -2313,7 +2315,6 @@ int mg_values(Solver& S, cudaStream_t st) {
   if (C.nb == 1) k_mg_dense<1><<<1, 1024, dsm, st>>>(C, M.dense);
   else k_mg_dense<3><<<1, 1024, dsm, st>>>(C, M.dense);
   ADFEM_CUDA(cudaGetLastError());
-  M.current = true;
   return ADFEM_OK;
 }
 
@@ -2591,10 +2592,10 @@ int mg_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_rows, 
              const double* fix_vals, const adfem_solver_opts& o, adfem_solver_stats* stats, cudaStream_t user,
              bool* gave_up) {
   *gave_up = false;
-  ADFEM_TRY(mg_values(S, user));
   Mg& M = *S.mg;
   const bool one = M.tail == 0;  // the whole solve in one launch
   if (!one) ADFEM_TRY(capture_solve(S));
+  ADFEM_TRY(mg_values(S, user));
   cudaStream_t st = S.stream;
   ADFEM_CUDA(cudaEventRecord(S.ev[0], user));
   ADFEM_CUDA(cudaStreamWaitEvent(st, S.ev[0], 0));
@@ -2627,6 +2628,7 @@ int mg_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_rows, 
   ADFEM_CUDA(cudaEventRecord(S.ev[2], st));
   ADFEM_CUDA(cudaGetLastError());
   ADFEM_CUDA(cudaEventSynchronize(S.ev[2]));
+  M.current = true;
   const CgState fin = S.h_state[0];
   if (fin.done != 1 && !(fin.done == 4 && fin.iters >= o.max_iter)) {
     *gave_up = true;

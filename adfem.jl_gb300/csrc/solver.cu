@@ -1013,6 +1013,11 @@ int solver_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_ro
   const bool mixed = o.precision == ADFEM_PREC_MIXED;
   if (o.precision != ADFEM_PREC_FP64 && !mixed) return fail(ADFEM_ERR_INVALID, "solver: unknown precision");
   if (!(o.rtol > 0.0) || o.max_iter < 1) return fail(ADFEM_ERR_INVALID, "solver: rtol must be > 0, max_iter >= 1");
+  // (a solve waits for its stream; refused before anything is enqueued, the capture stays valid)
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(user, &cap) != cudaSuccess) cudaGetLastError();
+  if (cap != cudaStreamCaptureStatusNone)
+    return fail(ADFEM_ERR_UNSUPPORTED, "solver: a solve cannot be captured (the stream is being captured)");
   if (S.mg_allowed && S.mg_fixed && !prof) {
     ADFEM_TRY(mg_plan(S));
     if (S.mg) {

@@ -1,0 +1,58 @@
+"""When a solve's results are there, and what a refused one leaves behind.
+
+* A solve on a stream that is being captured is refused and leaves the capture and the system as
+  they were: the hierarchy values of a later solve belong to the last assembly.
+
+Bars: 1e-9 relative (max norm) against the direct solve, as for every solve of this suite.
+"""
+import ctypes
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from adfem_gpu import _lib, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float(np.max(np.abs(a.cpu().numpy() - b)) / np.max(np.abs(b)))
+
+
+def t(a):
+    return torch.tensor(np.asarray(a, dtype=np.float64), device="cuda")
+
+
+# nodes: 169 (one block), 4225 (a cluster), 10201 (a graph)
+@pytest.mark.parametrize("m", [12, 64, 100])
+def test_refused_capture_leaves_the_system_as_it_was(oracle, gpulib, m):
+    coords, elems = synth.jittered_square(m, seed=2)
+    O = oracle.OracleMesh(coords, elems)
+    rng = np.random.default_rng(m)
+    bd = O.bcnode()
+    bv = rng.random(bd.size)
+    S = gpulib.PoissonSystem(gpulib.Mesh(coords, elems))
+    S.set_dirichlet(bd, bv)
+    f = rng.random(O.ngauss)
+    S.assemble(t(1.0 + rng.random(O.ngauss)), t(f))
+    S.solve(rtol=1e-12)  # (the hierarchy holds the values of this assembly)
+    kappa = 1e3 * (1.0 + 9.0 * rng.random(O.ngauss))
+    S.assemble(t(kappa), t(f))
+    u = torch.zeros(O.ndof, dtype=torch.float64, device="cuda")
+    o, st = gpulib.solver_opts(rtol=1e-12), _lib.SolverStats()
+    s, g, x = torch.cuda.Stream(), torch.cuda.CUDAGraph(), torch.zeros(8, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g, stream=s):
+        x.add_(1.0)
+        r = _lib.load().adfem_system_solve_d(S.handle, _lib.ptr(u), ctypes.byref(o), ctypes.byref(st),
+                                             _lib.stream_ptr(s))
+        x.add_(1.0)
+    assert r == _lib.ERR_UNSUPPORTED and "captured" in _lib.load().adfem_last_error().decode()
+    g.replay()
+    torch.cuda.synchronize()
+    assert float(x[0]) == 2.0
+    B, b = oracle.dirichlet_csc(O.laplace_csc(kappa), O.source(f), bd, bv)
+    assert rel(S.solve(rtol=1e-12), oracle.spsolve(B, b)) < 1e-9
+    assert S.last_stats.iterations < 60  # (not the Jacobi iteration)
