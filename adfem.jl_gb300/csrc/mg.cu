@@ -2638,12 +2638,12 @@ int mg_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_rows, 
   k_mg_out<<<blocks(S.n, kT), kT, 0, st>>>(S.n, S.y64.as<double>(), fix_rows, fix_vals, u);
   ADFEM_CUDA(cudaGetLastError());
   ADFEM_CUDA(cudaEventRecord(S.ev[3], st));
+  ADFEM_CUDA(cudaEventSynchronize(S.ev[3]));  // (u is written when the call returns, on any stream)
   ADFEM_CUDA(cudaStreamWaitEvent(user, S.ev[3], 0));
   const int status = fin.done == 1 ? ADFEM_OK : ADFEM_ERR_NOT_CONVERGED;
   const double relres = fin.bnorm2 > 0.0 ? std::sqrt(fin.rr64 / fin.bnorm2) : 0.0;
   if (stats) {
     float ms = 0.0f;
-    ADFEM_CUDA(cudaEventSynchronize(S.ev[3]));
     cudaEventElapsedTime(&ms, S.ev[1], S.ev[3]);
     stats->iterations = fin.iters;
     stats->updates = fin.updates;

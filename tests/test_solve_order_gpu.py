@@ -2,6 +2,7 @@
 
 * A solve on a stream that is being captured is refused and leaves the capture and the system as
   they were: the hierarchy values of a later solve belong to the last assembly.
+* The solution is written when the call returns, with or without statistics asked for.
 
 Bars: 1e-9 relative (max norm) against the direct solve, as for every solve of this suite.
 """
@@ -56,3 +57,26 @@ def test_refused_capture_leaves_the_system_as_it_was(oracle, gpulib, m):
     B, b = oracle.dirichlet_csc(O.laplace_csc(kappa), O.source(f), bd, bv)
     assert rel(S.solve(rtol=1e-12), oracle.spsolve(B, b)) < 1e-9
     assert S.last_stats.iterations < 60  # (not the Jacobi iteration)
+
+
+def test_solution_is_there_when_the_call_returns(gpulib):
+    # the caller's vector is pinned host memory, which the device writes slower than its own and the
+    # host can look at at once; natural numbering, so that the solver writes it itself
+    M = gpulib.Mesh(*synth.jittered_square(1000, seed=1))
+    S = gpulib.PoissonSystem(M)
+    S.set_dirichlet(gpulib.bcnode(M))
+    ng = gpulib.get_ngauss(M)
+    S.assemble(t(np.ones(ng)), t(np.ones(ng)))
+    assert S.solver_info()["renumbered"] == 0
+    ref = S.solve(rtol=1e-3).cpu().numpy()
+    u = torch.empty(ref.size, dtype=torch.float64).pin_memory()
+    h, o = u.numpy(), gpulib.solver_opts(rtol=1e-3)
+    solve = _lib.load().adfem_system_solve_d
+    for stats in (None, _lib.SolverStats()):
+        args = (S.handle, _lib.ptr(u), ctypes.byref(o), ctypes.byref(stats) if stats else None, _lib.stream_ptr(0))
+        for _ in range(5):
+            h[:] = np.nan
+            r = solve(*args)
+            last = h[-2000:].copy()
+            torch.cuda.synchronize()
+            assert r == 0 and np.array_equal(last, ref[-2000:]) and np.array_equal(h, ref)
