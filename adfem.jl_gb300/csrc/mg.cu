@@ -939,6 +939,8 @@ __global__ void __launch_bounds__(kTailT, 1) k_mg_tail(const __grid_constant__ T
   // (EX also: no block stores to another's shared memory before that block runs and has its barriers)
   if (EX) cluster_barrier();
   else __syncthreads();
+  // (also before the block leaves: a solve whose start has converged never ran a cycle, and the copies
+  // may still be on their way into its shared memory)
   auto filled = [&] {
     if (!copy) return;
     unsigned ok = 0;
@@ -1152,6 +1154,7 @@ __global__ void __launch_bounds__(kTailT, 1) k_mg_tail(const __grid_constant__ T
       if (loc.done) break;
     }
   }
+  filled();
   if constexpr (SOLVE) {
     if (rank == 0 && t == 0) *a.st = loc;
   } else {

@@ -3,6 +3,7 @@
 * A solve on a stream that is being captured is refused and leaves the capture and the system as
   they were: the hierarchy values of a later solve belong to the last assembly.
 * The solution is written when the call returns, with or without statistics asked for.
+* Solves that end before their first iteration disturb none that follows.
 
 Bars: 1e-9 relative (max norm) against the direct solve, as for every solve of this suite.
 """
@@ -80,3 +81,19 @@ def test_solution_is_there_when_the_call_returns(gpulib):
             last = h[-2000:].copy()
             torch.cuda.synchronize()
             assert r == 0 and np.array_equal(last, ref[-2000:]) and np.array_equal(h, ref)
+
+
+@pytest.mark.parametrize("m", [24, 60])  # one block, a cluster
+def test_solves_whose_start_has_converged(gpulib, m):
+    # they end before the first cycle, which is what first waits for the block's bulk copies; other
+    # solves take the same places on the device right behind them
+    M = gpulib.Mesh(*synth.jittered_square(m, seed=1))
+    ng, bd = gpulib.get_ngauss(M), gpulib.bcnode(M)
+    A, B = gpulib.PoissonSystem(M), gpulib.PoissonSystem(M)
+    for S in (A, B):
+        S.set_dirichlet(bd)
+        S.assemble(t(np.ones(ng)), t(np.ones(ng)))
+    ref, zero = B.solve(rtol=1e-12), torch.zeros(M.nnode, dtype=torch.float64, device="cuda")
+    for _ in range(100):
+        assert not bool(A.adjoint(zero).any()) and A.last_stats.iterations == 0
+        assert torch.equal(B.solve(rtol=1e-12), ref)
