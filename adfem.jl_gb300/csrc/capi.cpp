@@ -169,6 +169,11 @@ bool mg_wanted() {
   return true;
 }
 
+// ADFEM_MG_SPIN=0 (a test hook): every wait in the one-launch levels gives up at once.
+static void mg_env(Solver& s) {
+  if (const char* e = std::getenv("ADFEM_MG_SPIN")) s.mg_spin = std::atoi(e);
+}
+
 size_t system_device_bytes(const adfem_system* s) {
   size_t b = 0;
   const Sell& A = s->A;
@@ -1077,6 +1082,7 @@ int adfem_csc_solve(long long n, const long long* colptr1, const long long* rowv
   if (o.precision == ADFEM_PREC_FP64 && csc_wants_mg(n, rp, ci, nzval, fixed)) {
     ADFEM_TRY(to_dev(dfixed, fixed.data(), fixed.size()));
     sv.mg_allowed = sv.mg_fixed = true;
+    mg_env(sv);
     sv.mg_nb = 1;
     sv.mg_isbd = dfixed.as<uint8_t>();
     sv.mg_rp = std::move(rp);
@@ -1236,6 +1242,7 @@ int adfem_system_create(adfem_mesh* mesh, int kind, adfem_system** out) {
   if (mg_wanted()) {
     Solver& sv = s->solver;
     sv.mg_allowed = true;
+    mg_env(sv);
     sv.mg_nb = kind == ADFEM_SYS_ELASTICITY ? 2 : 1;
     sv.mg_rp = std::move(rpS);
     sv.mg_ci = std::move(ciS);

@@ -524,6 +524,7 @@ struct TailArgs {
   const float* b;
   float* x;
   int reps;
+  int spin;      // tries of a wait
   // a whole solve (k_mg_tail's SOLVE): the system's operator, right-hand side and iterate
   const int32_t* sptr;
   const void* col;
@@ -555,13 +556,37 @@ __device__ __forceinline__ unsigned rank_addr(const void* p, int rank) {
   return m;
 }
 
+// Whether the given phase of an mbarrier has completed, after at most `spin` tries.
+__device__ __forceinline__ bool mbar_wait(const void* bar, unsigned parity, int spin) {
+  unsigned ok = 0;
+  for (int i = 0; i < spin && !ok; i++)
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok)
+                 : "r"((unsigned)__cvta_generic_to_shared(bar)), "r"(parity)
+                 : "memory");
+  return ok;
+}
+
 // The exchanges of a block, numbered: exchange k counts on bar[k & 1] in its (k >> 1)-th phase.
+//
+// Waits are bounded (`spin` tries).  A block whose wait gives up is dead: it takes part in no further
+// exchange (an arrival in a phase that has not completed would corrupt the barrier) and uses no
+// indices that it waited for, so the blocks that wait for it give up as well, one exchange later at
+// most.  The launch then ends with st->done set, and the solve is left to the Jacobi iteration.  Every block of a
+// cluster stays until all have ended their sends (k_mg_tail's last barrier), and a dead one until what
+// was on its way to it has had time to arrive.
 struct TailSync {
   unsigned long long* bar;
   float* tok;    // kTailC words
   int rank;
   CgState* st;
+  int spin;
+  bool dead = false;  // the same in all threads
   int k = 0;
+  __device__ __forceinline__ void give_up() {
+    if (threadIdx.x == 0) st->done = 5;
+    dead = true;
+  }
   // this exchange brings `floats` values here
   __device__ __forceinline__ void expect(int floats) {
     if (threadIdx.x == 0)
@@ -578,20 +603,17 @@ struct TailSync {
   // the block has sent its rows: tell every block, and wait for what it needs itself
   __device__ __forceinline__ void exchange() {
     __syncthreads();
+    bool ok = true;
     if (threadIdx.x < 32) {
       if (threadIdx.x < kTailC) send(tok + rank, threadIdx.x, 0.0f);
-      const unsigned a = (unsigned)__cvta_generic_to_shared(bar + (k & 1)), parity = (k >> 1) & 1;
-      unsigned ok = 0;
-      // (bounded: a wait that gives up ends the solve, which falls back to the Jacobi iteration)
-      for (int i = 0; i < (1 << 16) && !ok; i++)
-        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-                     : "=r"(ok)
-                     : "r"(a), "r"(parity)
-                     : "memory");
-      if (!ok) st->done = 5;
+      ok = mbar_wait(bar + (k & 1), (k >> 1) & 1, spin);
     }
-    __syncthreads();
-    k++;
+    if (__syncthreads_and(ok)) k++;
+    else give_up();
+  }
+  // dead, and no block sends any more: some 0.2 ms for what is on its way to this one
+  __device__ __forceinline__ void drain() const {
+    for (int i = 0; i < 200; i++) __nanosleep(1000);
   }
 };
 
@@ -739,6 +761,7 @@ __device__ __forceinline__ void tail_smooth(TailSync& sync, const TailLev& L, Ta
   const float th = L.coef[0];
   const int k1 = res ? deg + 1 : deg;
   for (int k = fresh ? 1 : 0; k < k1; k++) {
+    if (EX && sync.dead) break;
     const bool pre = fresh && k == 1, last = k == deg;
     const float a1 = k > 0 && !last ? L.coef[2 * k] : 0.0f;
     const float a2 = k > 0 && !last ? L.coef[2 * k + 1] : th;
@@ -781,6 +804,7 @@ template <bool EX, int R, int X, int T>
 __device__ __forceinline__ void tail_transfer(TailSync& sync, const int32_t* sp, const int32_t* col, const float* val,
                                               int nent, const uint8_t* to, int r0, int r1, int lg, const float* x,
                                               const float* add, float* out, float* own) {
+  if (EX && sync.dead) return;
   const int lane = threadIdx.x & ((1 << lg) - 1), rows = (r1 - r0) * R;
   for (int q0 = 0; q0 < rows; q0 += T >> lg) {
     if (q0 + ((int)(threadIdx.x & ~31u) >> lg) >= rows) break;  // (whole warps without a row)
@@ -929,7 +953,7 @@ __global__ void __launch_bounds__(kTailT, 1) k_mg_tail(const __grid_constant__ T
     v[l].floats = ex ? nb * __ldg(a.L[l].cnt + rank) : 0;
     sm += tail_floats(n, nb, ex);
   }
-  TailSync sync{bars, tokens, rank, a.st};
+  TailSync sync{bars, tokens, rank, a.st, a.spin};
   pdl_wait();
   const int n0 = a.L[0].n * NT, own0 = (v[0].r1 - v[0].r0) * NT, off0 = v[0].r0 * NT;
   if (!SOLVE) {
@@ -941,15 +965,11 @@ __global__ void __launch_bounds__(kTailT, 1) k_mg_tail(const __grid_constant__ T
   else __syncthreads();
   // (also before the block leaves: a solve whose start has converged never ran a cycle, and the copies
   // may still be on their way into its shared memory)
-  auto filled = [&] {
-    if (!copy) return;
-    unsigned ok = 0;
-    for (int i = 0; i < (1 << 16) && !ok; i++)
-      asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\nselp.u32 %0, 1, 0, p;\n}"
-                   : "=r"(ok)
-                   : "r"(fill)
-                   : "memory");
-    if (!ok) sync.st->done = 5;
+  bool full = !copy;
+  auto filled = [&](int spin) {
+    if (full) return;
+    full = __syncthreads_and(mbar_wait(bars + 2, 0, spin));
+    if (!full) sync.give_up();
   };
   const int last = a.nl - 1;
   constexpr int deg0 = SOLVE ? kMgDeg0 : kMgDeg;
@@ -1057,23 +1077,26 @@ __global__ void __launch_bounds__(kTailT, 1) k_mg_tail(const __grid_constant__ T
     for (int rep = 0; rep < (SOLVE ? 1 : a.reps); rep++) {
       const bool first = rep == 0;
       if constexpr (!EX && NT == NC) {
-        if (first) filled();
+        if (first) filled(a.spin);
+        if (sync.dead) break;
         tail_local<NC, T>(sync, lev, v, 0, last, deg0, first, dense, a.N);
       } else {
         const TailLev& L = lev[0];
-        if (!EX && first) filled();
+        if (!EX && first) filled(a.spin);
+        if (sync.dead) break;
         tail_smooth<EX, NT, T>(sync, L, v[0], deg0, first, true);
         TailVecs& c = v[1];
         const int nc = lev[1].n;
         if (EX) {
           // coarse right-hand side: rows dealt in ranges, whole to every block
           const int ch = tail_chunk(nc), c0 = min(nc, rank * ch), c1 = min(nc, c0 + ch);
-          sync.expect(nc * NC);
+          if (!sync.dead) sync.expect(nc * NC);
           tail_transfer<true, NC, NT, T>(sync, L.pt_sptr, L.pt_col, L.pt_val, L.npt, nullptr, c0, c1,
                                          tail_lanes(ch * NC, T), v[0].y, nullptr, c.y, nullptr);
           for (int q = threadIdx.x; q < nc * NC; q += T) c.b[q] = c.y[q];
-          if (first) filled();
+          if (first) filled(a.spin);
           __syncthreads();
+          if (sync.dead) break;
         } else {
           tail_transfer<false, NC, NT, T>(sync, L.pt_sptr, L.pt_col, L.pt_val, L.npt, nullptr, 0, c.r1,
                                           tail_lanes(c.r1 * NC, T), v[0].y, nullptr, c.y, c.b);
@@ -1093,7 +1116,7 @@ __global__ void __launch_bounds__(kTailT, 1) k_mg_tail(const __grid_constant__ T
       const float* x = v[0].x;
       // (a wait that gave up in any block ends the solve in all of them)
       float zb = live ? x[u] * v[0].b[t] : 0.0f;
-      if (loc.done) zb = nanf("");
+      if (sync.dead) zb = nanf("");
       double d = cluster_total<EX, T>(zb, sh, slot, rank, phase);
       if (t == 0) {
         const double rz = d * loc.iar;
@@ -1154,7 +1177,11 @@ __global__ void __launch_bounds__(kTailT, 1) k_mg_tail(const __grid_constant__ T
       if (loc.done) break;
     }
   }
-  filled();
+  if (EX) {
+    cluster_barrier();
+    if (sync.dead) sync.drain();
+  }
+  filled(kTailSpin);
   if constexpr (SOLVE) {
     if (rank == 0 && t == 0) *a.st = loc;
   } else {
@@ -2434,6 +2461,7 @@ TailArgs tail_args(Solver& S) {
   a.x = M.lev[M.tail].x;
   a.reps = M.tail >= 3 ? 2 : 1;
   a.st = S.state.as<CgState>();
+  a.spin = S.mg_spin;
   a.sptr = A.sptr.as<int32_t>();
   a.col = A.col.p;
   a.d16 = A.delta16 ? 1 : 0;

@@ -24,6 +24,7 @@ constexpr int kMgMaxA = 64;       // entries per coarse row
 constexpr int kMgDense = 160;     // unknowns of the directly solved coarsest level
 constexpr int kMgTailDofs = 5120; // unknowns of the largest level of the one-launch tail
 constexpr int kTailC = 8;         // blocks of the tail's cluster
+constexpr int kTailSpin = 1 << 16;  // tries of a wait in the tail before it gives up
 constexpr int kTailLocal = kMgTailDofs / kTailC;  // unknowns of a tail that one block runs alone
 constexpr int kMgGrid = 1280;     // blocks of the kernels that sum over the grid, at most
 constexpr int kMgDeg0 = 2, kMgDeg = 4;  // Chebyshev degree: level 0, coarser levels

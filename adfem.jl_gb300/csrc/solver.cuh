@@ -100,6 +100,7 @@ struct Solver {
   std::vector<double> mg_x, mg_y;
   const uint8_t* mg_isbd = nullptr;  // device: Dirichlet tags in solver order
   bool mg_fixed = false;             // there are Dirichlet rows (the operator is not singular)
+  int mg_spin = kTailSpin;           // tries of a wait in the one-launch tail
   std::unique_ptr<Mg> mg;
   DevBuf vals64;           // Jacobi-scaled FP64 copy (A->val64 keeps the assembled values)
   DevBuf bad;              // int: a diagonal entry is not positive and finite
