@@ -44,9 +44,11 @@ struct MgHostLevel {
 };
 // Hierarchy of a graph of n nodes with nb0 unknowns each on level 0 and nbc on the others;
 // x, y (may be empty): node positions for the rotation mode.  false: the graph does not
-// coarsen to a size the tail can hold (the system keeps the Jacobi iteration).
+// coarsen to a size the tail can hold, or a pattern has more than `limit` entries (they are
+// numbered with 32 bits); the system keeps the Jacobi iteration.
 bool mg_build_host(int64_t n, std::vector<int32_t>&& rp, std::vector<int32_t>&& ci, int nb0, int nbc,
-                   std::vector<double>&& x, std::vector<double>&& y, std::vector<MgHostLevel>& lv);
+                   std::vector<double>&& x, std::vector<double>&& y, std::vector<MgHostLevel>& lv,
+                   int64_t limit = INT32_MAX);
 
 // Device view of one level
 struct MgLev {

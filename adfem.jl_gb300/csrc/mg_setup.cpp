@@ -66,9 +66,11 @@ int64_t aggregate(int64_t n, const MgPattern& A, std::vector<int32_t>& agg, bool
 
 // Pattern whose row i is the sorted set of the columns (below nc) that emit(i, add) adds.  (Repeated
 // ones are dropped as they come, by the row that last had the column: a coarse row meets each of its
-// some 7 columns 15 to 20 times.)
+// some 7 columns 15 to 20 times.)  Returns the longest row's entries, or kTooMany for more than limit
+// entries in all (which are counted with 64 bits, but kept as 32).
+constexpr int64_t kTooMany = INT64_MAX;
 template <class F>
-int64_t pattern(int64_t n, int64_t nc, MgPattern& P, F emit) {
+int64_t pattern(int64_t n, int64_t nc, int64_t limit, MgPattern& P, F emit) {
   constexpr int64_t kChunk = 16384;
   const int64_t nch = (n + kChunk - 1) / kChunk;
   std::vector<std::vector<int32_t>> part(nch);
@@ -90,10 +92,12 @@ int64_t pattern(int64_t n, int64_t nc, MgPattern& P, F emit) {
         P.rp[i + 1] = (int32_t)v.size();
       }
   });
-  int64_t w = 0;
+  int64_t w = 0, total = 0;
   for (int64_t i = 0; i < n; i++) {
     w = std::max<int64_t>(w, P.rp[i + 1]);
-    P.rp[i + 1] += P.rp[i];
+    total += P.rp[i + 1];
+    if (total > limit) return kTooMany;
+    P.rp[i + 1] = (int32_t)total;
   }
   P.ci.resize(P.rp[n]);
   parallel_for(m, [&](int64_t lo, int64_t hi) {
@@ -103,10 +107,23 @@ int64_t pattern(int64_t n, int64_t nc, MgPattern& P, F emit) {
   return w;
 }
 
+// whether a pattern in slices of 32 rows has at most limit / nb entries (a slice has at most 32 times
+// its rows' entries: no need to look at most patterns)
+bool fits(int64_t n, const MgPattern& P, int nb, int64_t limit) {
+  if (32 * (int64_t)P.rp[n] * nb <= limit) return true;
+  int64_t s = 0;
+  for (int64_t r0 = 0; r0 < n; r0 += 32) {
+    int64_t w = 0;
+    for (int64_t r = r0; r < std::min(n, r0 + 32); r++) w = std::max<int64_t>(w, P.rp[r + 1] - P.rp[r]);
+    s += 32 * w;
+  }
+  return s * nb <= limit;
+}
+
 }  // namespace
 
 bool mg_build_host(int64_t n, std::vector<int32_t>&& rp, std::vector<int32_t>&& ci, int nb0, int nbc,
-                   std::vector<double>&& x, std::vector<double>&& y, std::vector<MgHostLevel>& lv) {
+                   std::vector<double>&& x, std::vector<double>&& y, std::vector<MgHostLevel>& lv, int64_t limit) {
   lv.clear();
   lv.emplace_back();
   lv[0].n = n;
@@ -117,6 +134,7 @@ bool mg_build_host(int64_t n, std::vector<int32_t>&& rp, std::vector<int32_t>&& 
   for (;;) {
     MgHostLevel& L = lv.back();
     const int nb = lv.size() == 1 ? nb0 : nbc;
+    if (!fits(L.n, L.A, nb, limit)) return false;
     if (L.n * nb <= kMgDense) break;
     if ((int)lv.size() == kMgMaxLevels) return false;
     // (rows of two kinds: on the system's own level, where the longest is 1.5 times the average)
@@ -128,11 +146,11 @@ bool mg_build_host(int64_t n, std::vector<int32_t>&& rp, std::vector<int32_t>&& 
     auto rows = [](const MgPattern& Q, int64_t i, auto&& add) {
       for (int32_t k = Q.rp[i]; k < Q.rp[i + 1]; k++) add(Q.ci[k]);
     };
-    if (pattern(L.n, nc, L.P, [&](int64_t i, auto&& add) {
+    if (pattern(L.n, nc, limit, L.P, [&](int64_t i, auto&& add) {
           for (int32_t k = L.A.rp[i]; k < L.A.rp[i + 1]; k++) add(L.agg[L.A.ci[k]]);
         }) > kMgMaxP)
       return false;
-    if (pattern(L.n, nc, L.AP, [&](int64_t i, auto&& add) {
+    if (pattern(L.n, nc, limit, L.AP, [&](int64_t i, auto&& add) {
           for (int32_t k = L.A.rp[i]; k < L.A.rp[i + 1]; k++) rows(L.P, L.A.ci[k], add);
         }) > kMgMaxAP)
       return false;
@@ -151,9 +169,10 @@ bool mg_build_host(int64_t n, std::vector<int32_t>&& rp, std::vector<int32_t>&& 
           L.PTslot[q] = k - L.P.rp[i];
         }
     }
+    if (!fits(L.n, L.P, 1, limit) || !fits(L.n, L.AP, 1, limit) || !fits(nc, L.PT, 1, limit)) return false;
     MgHostLevel C;
     C.n = nc;
-    if (pattern(nc, nc, C.A, [&](int64_t J, auto&& add) {
+    if (pattern(nc, nc, limit, C.A, [&](int64_t J, auto&& add) {
           for (int32_t q = L.PT.rp[J]; q < L.PT.rp[J + 1]; q++) rows(L.AP, L.PT.ci[q], add);
         }) > kMgMaxA)
       return false;
