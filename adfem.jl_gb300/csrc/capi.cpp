@@ -1078,8 +1078,13 @@ int adfem_csc_solve(long long n, const long long* colptr1, const long long* rowv
   ADFEM_TRY(sv.init(&A, n));
   std::vector<uint8_t> fixed;
   DevBuf dfixed;
+  bool wants_mg = false;
+  try {
+    wants_mg = csc_wants_mg(n, rp, ci, nzval, fixed);
+  } catch (const std::bad_alloc&) {
+  }
   // (mixed precision names an iteration of its own here, which the callers of it keep)
-  if (o.precision == ADFEM_PREC_FP64 && csc_wants_mg(n, rp, ci, nzval, fixed)) {
+  if (o.precision == ADFEM_PREC_FP64 && wants_mg) {
     ADFEM_TRY(to_dev(dfixed, fixed.data(), fixed.size()));
     sv.mg_allowed = sv.mg_fixed = true;
     mg_env(sv);

@@ -2091,27 +2091,26 @@ int lanes_per_row(int64_t n) {
 
 }  // namespace
 
-int mg_plan(Solver& S) {
-  if (S.mg || !S.mg_allowed) return ADFEM_OK;
+static int plan(Solver& S) {
   const int nb0 = S.mg_nb, nbc = nb0 == 2 ? 3 : 1;
   std::vector<MgHostLevel> lv;
-  if (!mg_build_host((int64_t)S.mg_rp.size() - 1, std::move(S.mg_rp), std::move(S.mg_ci), nb0, nbc,
-                     std::move(S.mg_x), std::move(S.mg_y), lv)) {
-    S.mg_allowed = false;
-    return ADFEM_OK;
-  }
-  // (a plan that ends in an error gives the graph back: the next solve tries again)
+  // (a plan that ends in an error or an exception gives the graph back: the next solve tries again)
   struct GiveBack {
     Solver& S;
     std::vector<MgHostLevel>& lv;
     ~GiveBack() {
-      if (S.mg || !S.mg_allowed) return;
+      if (S.mg || !S.mg_allowed || lv.empty()) return;
       S.mg_rp = std::move(lv[0].A.rp);
       S.mg_ci = std::move(lv[0].A.ci);
       S.mg_x = std::move(lv[0].x);
       S.mg_y = std::move(lv[0].y);
     }
   } give_back{S, lv};
+  if (!mg_build_host((int64_t)S.mg_rp.size() - 1, std::move(S.mg_rp), std::move(S.mg_ci), nb0, nbc,
+                     std::move(S.mg_x), std::move(S.mg_y), lv)) {
+    S.mg_allowed = false;
+    return ADFEM_OK;
+  }
   std::unique_ptr<Mg> mg(new Mg());
   Mg& M = *mg;
   M.nlev = (int)lv.size();
@@ -2283,6 +2282,15 @@ int mg_plan(Solver& S) {
   }
   S.mg = std::move(mg);
   return ADFEM_OK;
+}
+
+int mg_plan(Solver& S) {
+  if (S.mg || !S.mg_allowed) return ADFEM_OK;
+  try {
+    return plan(S);
+  } catch (const std::bad_alloc&) {
+    return ADFEM_OK;  // (no host memory for the patterns: this solve takes the Jacobi iteration)
+  }
 }
 
 // ---------------------------------------------------------------------------

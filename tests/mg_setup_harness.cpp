@@ -1,9 +1,13 @@
 // CPU harness for the multigrid set-up code (adfem.jl_gb300/csrc/mg_setup.cpp, host_par.h), built and
 // run by tests/test_mg_setup_cpu.py.  Test infrastructure only: nothing in the library uses it.
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <new>
+#include <stdexcept>
 
+#include "host_par.h"
 #include "mg.cuh"
 
 namespace adfem {
@@ -11,6 +15,16 @@ Mg::~Mg() {}
 void DevBuf::release() {}
 }  // namespace adfem
 using namespace adfem;
+
+// the k-th following allocation fails, whichever thread makes it (k < 0: none)
+static std::atomic<long long> g_fail{-1};
+void* operator new(std::size_t n) {
+  if (g_fail.load() >= 0 && g_fail.fetch_sub(1) == 0) throw std::bad_alloc();
+  if (void* p = std::malloc(n ? n : 1)) return p;
+  throw std::bad_alloc();
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, std::size_t) noexcept { std::free(p); }
 
 #define REQUIRE(c)                                          \
   do {                                                      \
@@ -81,6 +95,43 @@ int main(int argc, char** argv) {
     check(lv, &most);
     REQUIRE(build(90, 70, lv, most));
     for (int64_t limit = most - 1; limit > 0; limit /= 2) REQUIRE(!build(90, 70, lv, limit));
+  }
+  if (!std::strcmp(argv[1], "exceptions")) {
+    // an exception of one thread's part reaches the caller, after all parts have ended
+    std::atomic<int64_t> done{0};
+    bool caught = false;
+    try {
+      parallel_for(100000, [&](int64_t lo, int64_t hi) {
+        done += hi - lo;
+        if (lo <= 70000 && 70000 < hi) throw std::runtime_error("part");
+      });
+    } catch (const std::runtime_error&) {
+      caught = true;
+    }
+    REQUIRE(caught && done.load() == 100000);
+    // every allocation of a set-up (90k nodes: threaded, the threads' own included) fails in turn: the
+    // caller gets std::bad_alloc (or the whole hierarchy, where only a thread was not to be had) and
+    // still has the graph
+    std::vector<int32_t> rp0, ci0;
+    graph(299, 299, rp0, ci0);
+    int64_t most = 0;
+    int thrown = 0;
+    bool whole = false;
+    for (long long k = 0; !whole; k += 1 + k / 16) {
+      std::vector<MgHostLevel> lv;
+      std::vector<int32_t> rp = rp0, ci = ci0;
+      g_fail = k;
+      try {
+        REQUIRE(mg_build_host(90000, std::move(rp), std::move(ci), 1, 1, {}, {}, lv));
+        whole = g_fail.exchange(-1) >= 0;
+        check(lv, &most);
+      } catch (const std::bad_alloc&) {
+        g_fail = -1;
+        thrown++;
+        REQUIRE(lv.empty() ? rp == rp0 && ci == ci0 : lv[0].A.rp == rp0 && lv[0].A.ci == ci0);
+      }
+    }
+    REQUIRE(thrown > 20);
   }
   std::printf("mg setup ok\n");
   return 0;

@@ -22,7 +22,7 @@ def harness(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["limit"])
+@pytest.mark.parametrize("what", ["limit", "exceptions"])
 def test_mg_setup(harness, what):
     r = subprocess.run([harness, what], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "mg setup ok" in r.stdout, (r.stdout[-2000:], r.stderr[-2000:])
