@@ -110,7 +110,7 @@ struct Sell {
   int pat_period = 1;
   int64_t uniform_slices = 0;
   int64_t uniform_entries = 0;  // stored entries of the uniform slices
-  DevBuf val64;         // double [nent]  (as assembled)
+  DevBuf val64;         // double [nent]  (as assembled; see Solver::val64_scaled)
   DevBuf valD64;        // double [nent]  (Jacobi-scaled, difference form, for FP64 residuals)
   DevBuf val32;         // float  [nent]
 };

@@ -65,7 +65,7 @@ __global__ void k_scale_diag(int64_t n, const int32_t* __restrict__ sptr, const 
   s[r] = rsqrtf(df);
 }
 
-// vals <- s_i K_ij s_j (FP64, standard form).  The difference-form copies
+// vals <- s_i K_ij s_j (FP64, standard form; may be val itself).  The difference-form copies
 // (FP64 valD for residuals, FP32 val32 for the inner iteration) hold w_ij = s_i K_ij
 // in off-diagonal slots and d_i = s_i^2 sum_j K_ij (the row sum, zero for rows of a
 // pure Laplacian) in the diagonal slot, so that
@@ -75,8 +75,7 @@ __global__ void k_scale_diag(int64_t n, const int32_t* __restrict__ sptr, const 
 // their accuracy; a plain FP32 copy of K~ loses them once cond(K~) * 2^-24 ~ 1.
 template <bool D16>
 __global__ void k_scale_values(int64_t n, const int32_t* __restrict__ sptr, const void* __restrict__ col,
-                               const double* __restrict__ val, double* __restrict__ vals,
-                               double* __restrict__ valD, float* __restrict__ val32,
+                               const double* val, double* vals, double* __restrict__ valD, float* __restrict__ val32,
                                const float* __restrict__ s, const int32_t* __restrict__ diagpos) {
   const int64_t r = gtid();
   if (r >= n) return;
@@ -539,10 +538,11 @@ __global__ void k_unscale(int64_t n, const double* __restrict__ y, const float* 
   else u[i] = (double)s[i] * y[i];
 }
 
-// y = K x
-template <bool D16>
+// y = K x; SCALED: val holds K~, y = S^-1 K~ S^-1 x
+template <bool D16, bool SCALED>
 __global__ void k_apply(int64_t n, const int32_t* __restrict__ sptr, const void* __restrict__ col,
-                        const double* __restrict__ val, const double* __restrict__ x, double* __restrict__ y) {
+                        const double* __restrict__ val, const float* __restrict__ s, const double* __restrict__ x,
+                        double* __restrict__ y) {
   const int64_t r = gtid();
   if (r >= n) return;
   int64_t base;
@@ -553,9 +553,9 @@ __global__ void k_apply(int64_t n, const int32_t* __restrict__ sptr, const void*
     const int64_t idx = base + 32 * (int64_t)k;
     int j = colof<D16>(col, idx, r);
     if (!ADFEM_DCHECK(j >= 0 && j < n)) j = (int)r;
-    acc = fma(val[idx], x[j], acc);
+    acc = fma(val[idx], SCALED ? x[j] / (double)s[j] : x[j], acc);
   }
-  y[r] = acc;
+  y[r] = SCALED ? acc / (double)s[r] : acc;
 }
 
 // ---------------------------------------------------------------------------
@@ -714,6 +714,7 @@ int solver_prepare(Solver& S, const int32_t* diagpos_dev, cudaStream_t user) {
   S.prepared = false;
   S.prep_scaled = false;
   S.prep_vals64 = false;
+  S.val64_scaled = false;
   S.prep_z = false;
   if (S.mg) S.mg->current = false;
   if (!diagpos_dev) return fail(ADFEM_ERR_INVALID, "solver_prepare: diagonal positions required");
@@ -732,15 +733,22 @@ int solver_prepare(Solver& S, const int32_t* diagpos_dev, cudaStream_t user) {
   return ADFEM_OK;
 }
 
-// Jacobi-scaled copies: s_i = rsqrt(K_ii), vals64 = s_i K_ij s_j (standard form), valD64 / val32
-// the FP64 / FP32 difference forms (k_scale_values).  Once per assembly.  standard64: vals64 is
-// needed (the FP64 iterations).
+// whether the solves of this assembly read the assembled values (multigrid)
+static bool solves_with_mg(const Solver& S) { return S.mg_allowed && S.mg_fixed; }
+
+// Jacobi-scaled copies: s_i = rsqrt(K_ii), scaled64() = s_i K_ij s_j (standard form), valD64 / val32
+// the FP64 / FP32 difference forms (k_scale_values).  Once per assembly.  standard64: scaled64() is
+// needed (the FP64 iterations): it takes the place of the assembled values, so that a solve needs no
+// memory beyond the system's own, except for a profiled solve of a system that multigrid solves.
 int solver_ensure_scaled(Solver& S, bool standard64, cudaStream_t user) {
   if (S.prep_scaled && (S.prep_vals64 || !standard64)) return ADFEM_OK;
   if (!S.diagpos) return fail(ADFEM_ERR_INVALID, "solver: operator not prepared");
   const Sell& A = *S.A;
-  if (standard64) ADFEM_TRY(S.vals64.alloc(sizeof(double) * (size_t)std::max<int64_t>(A.nent, 1)));
-  double* vals = standard64 ? S.vals64.as<double>() : nullptr;
+  const bool in_place = standard64 && !solves_with_mg(S);
+  if (in_place && S.zcg) ADFEM_TRY(ensure_banded(S, user));  // (made from the assembled values)
+  if (standard64 && !in_place) ADFEM_TRY(S.vals64.alloc(sizeof(double) * (size_t)std::max<int64_t>(A.nent, 1)));
+  if (in_place) S.val64_scaled = true;
+  double* vals = standard64 ? S.scaled64() : nullptr;
   ADFEM_CUDA(cudaMemsetAsync(S.bad.p, 0, sizeof(int), user));
   const unsigned nb = (unsigned)((S.n + kT - 1) / kT);
   enqueue_scale_diag(S, user);
@@ -838,7 +846,7 @@ static void enqueue_cg64(Solver& S, cudaStream_t st, Timer* tm = nullptr) {
   if (!tm) tm = &none;
   auto* cs = S.state.as<CgState>();
   auto* part = S.partials.as<double>();
-  tm->run(0, st, [&] { enqueue_spmv64(S, S.vals64.as<double>(), st); });
+  tm->run(0, st, [&] { enqueue_spmv64(S, S.scaled64(), st); });
   tm->run(1, st, [&] {
     k_cg64_update<<<S.grid, kT, 0, st>>>(S.n, S.z64.as<double>(), S.r64.as<double>(), S.p64.as<double>(),
                                          S.q64.as<double>(), cs, part);
@@ -1018,7 +1026,7 @@ int solver_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_ro
   if (cudaStreamIsCapturing(user, &cap) != cudaSuccess) cudaGetLastError();
   if (cap != cudaStreamCaptureStatusNone)
     return fail(ADFEM_ERR_UNSUPPORTED, "solver: a solve cannot be captured (the stream is being captured)");
-  if (S.mg_allowed && S.mg_fixed && !prof) {
+  if (solves_with_mg(S) && !prof) {
     ADFEM_TRY(mg_plan(S));
     if (S.mg) {
       bool gave_up = false;
@@ -1035,14 +1043,16 @@ int solver_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_ro
                         : (path == Path::MIXED ? &S.g32 : (path == Path::BANDED ? &S.gz : &S.gd));
   int* gc = path == Path::FP64 ? &S.g64_chunk
             : (path == Path::MIXED ? &S.g32_chunk : (path == Path::BANDED ? &S.gz_chunk : &S.gd_chunk));
+  const bool fp64 = path == Path::FP64 || path == Path::DBANDED;
   if (!prof) {
-    if (*gx && *gc != chunk) {
+    if (*gx && (*gc != chunk || (fp64 && S.g64_vals != S.scaled64()))) {
       cudaGraphExecDestroy(*gx);
       *gx = nullptr;
     }
     if (!*gx) {
       ADFEM_TRY(capture_chunk(S, path, chunk, gx));
       *gc = chunk;
+      if (fp64) S.g64_vals = S.scaled64();
     }
   }
   long long launches = 0;
@@ -1203,10 +1213,11 @@ int solver_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_ro
 int solver_apply(Solver& S, const double* x, double* y, cudaStream_t user) {
   const Sell& A = *S.A;
   const unsigned nb = (unsigned)((S.n + kT - 1) / kT);
-  if (A.delta16)
-    k_apply<true><<<nb, kT, 0, user>>>(S.n, A.sptr.as<int32_t>(), A.col.p, A.val64.as<double>(), x, y);
-  else
-    k_apply<false><<<nb, kT, 0, user>>>(S.n, A.sptr.as<int32_t>(), A.col.p, A.val64.as<double>(), x, y);
+  auto go = [&](auto k) {
+    k<<<nb, kT, 0, user>>>(S.n, A.sptr.as<int32_t>(), A.col.p, A.val64.as<double>(), S.s32.as<float>(), x, y);
+  };
+  if (A.delta16) S.val64_scaled ? go(k_apply<true, true>) : go(k_apply<true, false>);
+  else S.val64_scaled ? go(k_apply<false, true>) : go(k_apply<false, false>);
   ADFEM_CUDA(cudaGetLastError());
   return ADFEM_OK;
 }

@@ -40,7 +40,7 @@ struct Solver {
   int grid = 0;            // blocks of the grid-stride kernels (resident blocks per SM x SMs)
   int grid_spmv = 0;       // same for the unrolled SpMV kernels (higher register use)
   bool prefetch = false;   // SpMV software pipelining (ADFEM_SPMV_PREFETCH=1)
-  const Sell* A = nullptr; // sliced-ELL operator (val64 as assembled, val32 scaled copy)
+  const Sell* A = nullptr; // sliced-ELL operator (val64 as assembled unless val64_scaled, val32 scaled copy)
   DevBuf s32;              // Jacobi scaling s_i = 1/sqrt(K_ii) (float, exact in double)
   DevBuf state;            // CgState
   DevBuf partials;         // 4 * grid doubles
@@ -57,7 +57,8 @@ struct Solver {
   int g64_chunk = 0, g32_chunk = 0;
   bool prepared = false;
   bool prep_scaled = false;        // the Jacobi-scaled copies are current (see solver_ensure_scaled)
-  bool prep_vals64 = false;        // vals64 too
+  bool prep_vals64 = false;        // scaled64() too
+  bool val64_scaled = false;       // A->val64 holds the scaled values (see solver_ensure_scaled)
   const int32_t* diagpos = nullptr; // device: entry index of the diagonal in each row
   // banded mixed path (zcg.cu): used by mixed solves when the band fits the ring
   bool zcg = false;
@@ -102,7 +103,9 @@ struct Solver {
   bool mg_fixed = false;             // there are Dirichlet rows (the operator is not singular)
   int mg_spin = kTailSpin;           // tries of a wait in the one-launch tail
   std::unique_ptr<Mg> mg;
-  DevBuf vals64;           // Jacobi-scaled FP64 copy (A->val64 keeps the assembled values)
+  DevBuf vals64;           // Jacobi-scaled FP64 copy where A->val64 has to keep the assembled values
+  double* scaled64() const { return val64_scaled ? A->val64.as<double>() : vals64.as<double>(); }
+  const double* g64_vals = nullptr;  // the values that g64 (or gd) was captured with
   DevBuf bad;              // int: a diagonal entry is not positive and finite
   bool prep_z = false;     // the banded mixed copies are current
   ~Solver();
@@ -112,8 +115,8 @@ struct Solver {
 // After an assembly (diagpos: entry index k of the diagonal in row i): makes the copies
 // the default solve needs now and marks the others for first use.
 int solver_prepare(Solver& S, const int32_t* diagpos_dev, cudaStream_t user);
-// The Jacobi-scaled copies: s_i = rsqrt(K_ii) (FP32), vals64 = s_i K_ij s_j, valD64 / val32
-// the FP64 / FP32 difference-form copies (see k_scale_values); standard64: vals64 too; no-op when
+// The Jacobi-scaled copies: s_i = rsqrt(K_ii) (FP32), scaled64() = s_i K_ij s_j, valD64 / val32
+// the FP64 / FP32 difference-form copies (see k_scale_values); standard64: scaled64() too; no-op when
 // current.
 int solver_ensure_scaled(Solver& S, bool standard64, cudaStream_t user);
 // Per-kernel timing of a profiled solve: 0 SpMV+dot, 1 update+dot, 2 p update / fold,

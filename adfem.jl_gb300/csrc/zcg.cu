@@ -1474,7 +1474,7 @@ static DcgArgs dcg_args(Solver& S) {
   d.npool = S.znpool;
   d.colz = S.colz16.as<int16_t>();
   d.sptr = A.sptr.as<int32_t>();
-  d.val = S.vals64.as<double>();
+  d.val = S.scaled64();
   d.r[0] = S.r64.as<double>();
   d.r[1] = S.dr1.as<double>();
   d.p[0] = S.p64.as<double>();
