@@ -169,8 +169,10 @@ bool mg_wanted() {
   return true;
 }
 
+// ADFEM_MG_MAX_ITER: multigrid iterations before a solve is left to the Jacobi iteration;
 // ADFEM_MG_SPIN=0 (a test hook): every wait in the one-launch levels gives up at once.
 static void mg_env(Solver& s) {
+  if (const char* e = std::getenv("ADFEM_MG_MAX_ITER")) s.mg_cap = std::max(1, std::atoi(e));
   if (const char* e = std::getenv("ADFEM_MG_SPIN")) s.mg_spin = std::atoi(e);
 }
 

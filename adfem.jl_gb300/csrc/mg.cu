@@ -42,7 +42,6 @@ namespace {
 constexpr float kFrac0 = 0.125f, kFrac = 0.06f;  // lower end of the Chebyshev interval over lam
 constexpr int kCoef = 2 * kMgDeg;
 constexpr size_t kTailSmem = 224 * 1024;  // shared memory of a tail block, at most
-constexpr int kMgIterations = 300;  // a solve that needs more is left to the Jacobi iteration
 
 template <int NB>
 struct Vec {
@@ -2641,7 +2640,7 @@ int mg_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_rows, 
   ADFEM_CUDA(cudaEventRecord(S.ev[1], st));
   CgState init;
   std::memset(&init, 0, sizeof(init));
-  init.max_iter = std::min(o.max_iter, kMgIterations);
+  init.max_iter = std::min(o.max_iter, S.mg_cap);
   init.delta2 = 1e-6;  // residual evaluated in FP64 after each drop of the recurrence by 1e-3
   S.h_state[1] = init;
   ADFEM_CUDA(cudaMemcpyAsync(S.state.p, &S.h_state[1], sizeof(CgState), cudaMemcpyHostToDevice, st));

@@ -27,6 +27,7 @@ constexpr int kTailC = 8;         // blocks of the tail's cluster
 constexpr int kTailSpin = 1 << 16;  // tries of a wait in the tail before it gives up
 constexpr int kTailLocal = kMgTailDofs / kTailC;  // unknowns of a tail that one block runs alone
 constexpr int kMgGrid = 1280;     // blocks of the kernels that sum over the grid, at most
+constexpr int kMgIterations = 300;  // a solve that needs more is left to the Jacobi iteration
 constexpr int kMgDeg0 = 2, kMgDeg = 4;  // Chebyshev degree: level 0, coarser levels
 
 // Patterns of one level (host), rows in solver order at level 0.  Rows are in compressed

@@ -716,6 +716,7 @@ int solver_prepare(Solver& S, const int32_t* diagpos_dev, cudaStream_t user) {
   S.prep_vals64 = false;
   S.val64_scaled = false;
   S.prep_z = false;
+  S.mg_skip = false;
   if (S.mg) S.mg->current = false;
   if (!diagpos_dev) return fail(ADFEM_ERR_INVALID, "solver_prepare: diagonal positions required");
   S.diagpos = diagpos_dev;
@@ -734,7 +735,7 @@ int solver_prepare(Solver& S, const int32_t* diagpos_dev, cudaStream_t user) {
 }
 
 // whether the solves of this assembly read the assembled values (multigrid)
-static bool solves_with_mg(const Solver& S) { return S.mg_allowed && S.mg_fixed; }
+static bool solves_with_mg(const Solver& S) { return S.mg_allowed && S.mg_fixed && !S.mg_skip; }
 
 // Jacobi-scaled copies: s_i = rsqrt(K_ii), scaled64() = s_i K_ij s_j (standard form), valD64 / val32
 // the FP64 / FP32 difference forms (k_scale_values).  Once per assembly.  standard64: scaled64() is
@@ -1033,6 +1034,8 @@ int solver_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_ro
       const int r = mg_solve(S, rhs, u, zero_rows, fix_rows, fix_vals, o, stats, user, &gave_up);
       if (!gave_up) return r;
     }
+    // (the assembly's later solves do not try again: what it gave up on is the operator)
+    S.mg_skip = true;
   }
   const int chunk = std::max(1, std::min(o.chunk > 0 ? o.chunk : 32, 512));
   const Path path = !mixed ? (S.dcg ? Path::DBANDED : Path::FP64) : (S.zcg ? Path::BANDED : Path::MIXED);

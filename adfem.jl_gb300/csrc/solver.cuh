@@ -101,7 +101,9 @@ struct Solver {
   std::vector<double> mg_x, mg_y;
   const uint8_t* mg_isbd = nullptr;  // device: Dirichlet tags in solver order
   bool mg_fixed = false;             // there are Dirichlet rows (the operator is not singular)
+  bool mg_skip = false;              // this assembly's solves take the Jacobi iteration: multigrid gave one up
   int mg_spin = kTailSpin;           // tries of a wait in the one-launch tail
+  int mg_cap = kMgIterations;        // iterations of a solve before it is left to the Jacobi iteration
   std::unique_ptr<Mg> mg;
   DevBuf vals64;           // Jacobi-scaled FP64 copy where A->val64 has to keep the assembled values
   double* scaled64() const { return val64_scaled ? A->val64.as<double>() : vals64.as<double>(); }

@@ -338,9 +338,10 @@ enum { ADFEM_SYS_POISSON = 0, ADFEM_SYS_ELASTICITY = 1 };
  * once per assembly): tens of iterations at every size where Jacobi-CG needs thousands.  The
  * Jacobi iterations serve systems without Dirichlet DOFs (singular), graphs that do not
  * coarsen, solves in which the preconditioned iteration breaks down (indefinite operators) or
- * needs more than 300 iterations, profiled solves, and systems created while ADFEM_MG=0 or one
- * of ADFEM_ZCG, ADFEM_ZCG64, ADFEM_ZCG_SMAX, ADFEM_ZCG_RING, ADFEM_ZCG_RING_REFILL (which pick
- * a variant of them) is set in the environment.
+ * needs more than 300 iterations (ADFEM_MG_MAX_ITER in the environment at creation; from then on
+ * every solve of that assembly), profiled solves, and systems created while ADFEM_MG=0 or one of
+ * ADFEM_ZCG, ADFEM_ZCG64, ADFEM_ZCG_SMAX, ADFEM_ZCG_RING, ADFEM_ZCG_RING_REFILL (which pick a
+ * variant of them) is set in the environment.
  * Poisson systems on P1 or P2 meshes (P2: the vertex-then-edge DOFs of the mesh's space,
  * kappa and f at the 6 points per element of the order-4 rule; DOFs renumbered for the
  * solver by reverse Cuthill-McKee, inputs and outputs in the reference order); elasticity

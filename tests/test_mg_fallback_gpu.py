@@ -61,3 +61,52 @@ def test_waits_that_give_up(oracle, gpulib, monkeypatch, m, elastic, precision):
     # the device is as it was for the systems that do wait
     S, ref, _ = system(oracle, gpulib, m, elastic)
     assert rel(S.solve(precision=precision, rtol=1e-12), ref) < 1e-9 and S.last_stats.iterations < JACOBI
+
+
+@pytest.mark.parametrize("m,elastic", [(23, 0), (60, 0), (100, 0), (25, 1), (70, 1)])
+def test_iteration_cap(oracle, gpulib, monkeypatch, m, elastic):
+    cap = 25 if elastic else 8  # enough for a residual of 1e-2, too few for 1e-12
+    monkeypatch.setenv("ADFEM_MG_MAX_ITER", str(cap))
+    S, ref, args = system(oracle, gpulib, m, elastic)
+    for precision in ("fp64", "mixed"):
+        S.solve(precision=precision, rtol=1e-2)
+        few = S.last_stats.iterations
+        assert few < cap
+        u = S.solve(precision=precision, rtol=1e-12)
+        assert S.last_stats.iterations > JACOBI and rel(u, ref) < 1e-9
+        # the start of a warm solve is the caller's vector, as before the multigrid iterations
+        w = S.solve(t(ref), precision=precision, rtol=1e-8, warm=True)
+        assert S.last_stats.iterations == 0 and rel(w, ref) < 1e-9
+        # the assembly's later solves do not try again, the next assembly's do
+        S.solve(precision=precision, rtol=1e-2)
+        assert S.last_stats.iterations > few
+        S.assemble(*args)
+        S.solve(precision=precision, rtol=1e-2)
+        assert S.last_stats.iterations == few
+        S.assemble(*args)
+        w = S.solve(t(ref * (1 + 1e-3 * np.sin(np.arange(ref.size)))), precision=precision, rtol=1e-12, warm=True)
+        assert S.last_stats.iterations > JACOBI / 2 and rel(w, ref) < 1e-9
+        S.assemble(*args)
+
+
+def test_indefinite_operator_with_a_positive_diagonal(oracle, gpulib):
+    coords, elems = synth.jittered_square(20, seed=1)
+    O = oracle.OracleMesh(coords, elems)
+    k = np.arange(len(elems))
+    x, y = k // 2 % 20, k // 2 // 20
+    kappa = np.repeat(np.where((x % 4 == 2) & (y % 4 == 2) & (k % 2 == 0), -0.6, 1.0 / 3), 3)
+    f, bd = np.ones(O.ngauss), O.bcnode()
+    B, _ = oracle.dirichlet_csc(O.laplace_csc(kappa), O.source(f), bd, np.zeros(bd.size))
+    assert B.diagonal().min() > 0.01 and np.linalg.eigvalsh(B.toarray()).min() < -0.1
+    S = gpulib.PoissonSystem(gpulib.Mesh(coords, elems))
+    S.set_dirichlet(bd)
+    for _ in range(2):
+        S.assemble(t(kappa), t(f))
+        for precision in ("fp64", "mixed", "fp64"):
+            with pytest.raises(gpulib.AdFemError) as e:
+                S.solve(precision=precision, rtol=1e-12)
+            assert e.value.status == gpulib._lib.ERR_BREAKDOWN
+    # the system is as before for an operator that is definite
+    S.assemble(t(np.ones(O.ngauss)), t(f))
+    B, r = oracle.dirichlet_csc(O.laplace_csc(np.ones(O.ngauss)), O.source(f), bd, np.zeros(bd.size))
+    assert rel(S.solve(rtol=1e-12), oracle.spsolve(B, r)) < 1e-9 and S.last_stats.iterations < JACOBI
