@@ -170,9 +170,11 @@ bool mg_wanted() {
 }
 
 // ADFEM_MG_MAX_ITER: multigrid iterations before a solve is left to the Jacobi iteration;
+// ADFEM_MG_MAX_BYTES: a hierarchy that would take more is not made;
 // ADFEM_MG_SPIN=0 (a test hook): every wait in the one-launch levels gives up at once.
 static void mg_env(Solver& s) {
   if (const char* e = std::getenv("ADFEM_MG_MAX_ITER")) s.mg_cap = std::max(1, std::atoi(e));
+  if (const char* e = std::getenv("ADFEM_MG_MAX_BYTES")) s.mg_limit = (size_t)std::max(0ll, std::atoll(e));
   if (const char* e = std::getenv("ADFEM_MG_SPIN")) s.mg_spin = std::atoi(e);
 }
 

@@ -2090,6 +2090,13 @@ int lanes_per_row(int64_t n) {
 
 }  // namespace
 
+// the device has less than this left (a failed allocation is then no error of its own)
+static bool short_of(size_t bytes) {
+  size_t freeb = 0, total = 0;
+  cudaGetLastError();
+  return cudaMemGetInfo(&freeb, &total) == cudaSuccess && freeb < bytes + ((size_t)64 << 20);
+}
+
 static int plan(Solver& S) {
   const int nb0 = S.mg_nb, nbc = nb0 == 2 ? 3 : 1;
   std::vector<MgHostLevel> lv;
@@ -2232,7 +2239,11 @@ static int plan(Solver& S) {
   ADFEM_CUDA(cudaDeviceGetAttribute(&M.sms, cudaDevAttrMultiProcessorCount, dev));
   sl.room(&M.dense, (size_t)M.ndense * M.ndense);
   M.val_bytes = (int)(sl.total - val0);
-  ADFEM_TRY(M.slab.alloc(sl.total));
+  S.mg_need = sl.total;
+  if (S.mg_need > S.mg_limit) return ADFEM_OK;
+  const int got = M.slab.alloc(sl.total);
+  if (got == ADFEM_ERR_NOMEM && short_of(sl.total)) return ADFEM_OK;
+  ADFEM_TRY(got);
   sl.resolve(M.slab.as<char>());
   for (int l = 0; l < M.nlev; l++) M.lev[l].lam = M.lam + l;
   ADFEM_CUDA(cudaMemcpy(M.slab.p, sl.host.data(), sl.host.size(), cudaMemcpyHostToDevice));
@@ -2285,6 +2296,8 @@ static int plan(Solver& S) {
 
 int mg_plan(Solver& S) {
   if (S.mg || !S.mg_allowed) return ADFEM_OK;
+  // (a hierarchy that did not fit before: the patterns are not made again to find that out)
+  if (S.mg_limit == 0 || S.mg_need > S.mg_limit || (S.mg_need > 0 && short_of(S.mg_need))) return ADFEM_OK;
   try {
     return plan(S);
   } catch (const std::bad_alloc&) {

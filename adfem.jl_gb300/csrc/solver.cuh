@@ -101,7 +101,10 @@ struct Solver {
   std::vector<double> mg_x, mg_y;
   const uint8_t* mg_isbd = nullptr;  // device: Dirichlet tags in solver order
   bool mg_fixed = false;             // there are Dirichlet rows (the operator is not singular)
-  bool mg_skip = false;              // this assembly's solves take the Jacobi iteration: multigrid gave one up
+  bool mg_skip = false;              // this assembly's solves take the Jacobi iteration: multigrid gave one
+                                     // up, or there was no room for the hierarchy
+  size_t mg_limit = SIZE_MAX;        // bytes the hierarchy may take
+  size_t mg_need = 0;                // bytes it takes (0: not known yet)
   int mg_spin = kTailSpin;           // tries of a wait in the one-launch tail
   int mg_cap = kMgIterations;        // iterations of a solve before it is left to the Jacobi iteration
   std::unique_ptr<Mg> mg;
@@ -138,7 +141,7 @@ int solver_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_ro
 int solver_apply(Solver& S, const double* x, double* y, cudaStream_t user);
 
 // Multigrid-preconditioned FP64 CG (mg.cu): hierarchy on first use (clears mg_allowed when the
-// graph does not coarsen), its values once per assembly, the solve.  gave_up: no outcome (a
+// graph does not coarsen, makes none where the device or mg_limit has no room for it), its values once per assembly, the solve.  gave_up: no outcome (a
 // breakdown, or more iterations than the multigrid cap); u untouched, the caller falls back.
 int mg_plan(Solver& S);
 int mg_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_rows, const uint8_t* fix_rows,

@@ -337,7 +337,8 @@ enum { ADFEM_SYS_POISSON = 0, ADFEM_SYS_ELASTICITY = 1 };
  * aggregation multigrid (hierarchy of the matrix graph built by the first solve, its values
  * once per assembly): tens of iterations at every size where Jacobi-CG needs thousands.  The
  * Jacobi iterations serve systems without Dirichlet DOFs (singular), graphs that do not
- * coarsen, solves in which the preconditioned iteration breaks down (indefinite operators) or
+ * coarsen, hierarchies that the device has no memory for (200 to 350 bytes per DOF;
+ * ADFEM_MG_MAX_BYTES in the environment at creation caps them), solves in which the preconditioned iteration breaks down (indefinite operators) or
  * needs more than 300 iterations (ADFEM_MG_MAX_ITER in the environment at creation; from then on
  * every solve of that assembly), profiled solves, and systems created while ADFEM_MG=0 or one of
  * ADFEM_ZCG, ADFEM_ZCG64, ADFEM_ZCG_SMAX, ADFEM_ZCG_RING, ADFEM_ZCG_RING_REFILL (which pick a

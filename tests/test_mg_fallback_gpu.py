@@ -110,3 +110,30 @@ def test_indefinite_operator_with_a_positive_diagonal(oracle, gpulib):
     S.assemble(t(np.ones(O.ngauss)), t(f))
     B, r = oracle.dirichlet_csc(O.laplace_csc(np.ones(O.ngauss)), O.source(f), bd, np.zeros(bd.size))
     assert rel(S.solve(rtol=1e-12), oracle.spsolve(B, r)) < 1e-9 and S.last_stats.iterations < JACOBI
+
+
+@pytest.mark.parametrize("m,elastic", [(23, 0), (100, 0), (25, 1)])
+def test_hierarchy_without_room(oracle, gpulib, monkeypatch, m, elastic):
+    monkeypatch.setenv("ADFEM_MG_MAX_BYTES", "10000")  # (these take 100 KB and more)
+    S, ref, args = system(oracle, gpulib, m, elastic)
+    monkeypatch.delenv("ADFEM_MG_MAX_BYTES")
+    L = gpulib._lib.load()
+    for _ in range(2):
+        for precision in ("fp64", "mixed"):
+            try:
+                L.adfem_debug_fail_alloc(0)  # (nothing is allocated for the Jacobi iteration either)
+                u = S.solve(precision=precision, rtol=1e-12)
+            finally:
+                L.adfem_debug_fail_alloc(-1)
+            assert S.last_stats.iterations > JACOBI and rel(u, ref) < 1e-9
+        S.assemble(*args)
+    # with room, an allocation that fails although the device is not short is reported, and tried again
+    S, ref, _ = system(oracle, gpulib, m, elastic)
+    try:
+        L.adfem_debug_fail_alloc(0)
+        with pytest.raises(gpulib.AdFemError) as e:
+            S.solve(rtol=1e-12)
+    finally:
+        L.adfem_debug_fail_alloc(-1)
+    assert e.value.status == gpulib._lib.ERR_NOMEM
+    assert rel(S.solve(rtol=1e-12), ref) < 1e-9 and S.last_stats.iterations < JACOBI
