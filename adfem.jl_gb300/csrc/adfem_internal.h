@@ -336,7 +336,11 @@ int system_solve_packed(adfem_system** sys, int count, double** out, const doubl
 // Device bytes held by a resident system (operator copies, Dirichlet data, solver
 // vectors) -- what the serving loop counts against its HBM budget.
 size_t system_device_bytes(const adfem_system* s);
+// Multigrid of resident systems: whether it is in use at all, whether the system's next solve (with
+// Dirichlet DOFs, outside a pack) builds the hierarchy, and whether it may.
 bool mg_wanted();
+bool system_builds_hierarchy(const adfem_system* s);
+void system_allow_hierarchy(adfem_system* s, bool allow);
 // Mesh behind a handle (sizes for admission estimates).
 const Mesh* mesh_of(const adfem_mesh* h);
 

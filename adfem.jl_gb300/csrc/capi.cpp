@@ -178,6 +178,9 @@ static void mg_env(Solver& s) {
   if (const char* e = std::getenv("ADFEM_MG_SPIN")) s.mg_spin = std::atoi(e);
 }
 
+bool system_builds_hierarchy(const adfem_system* s) { return s->solver.mg_allowed && !s->solver.mg; }
+void system_allow_hierarchy(adfem_system* s, bool allow) { s->solver.mg_room = allow; }
+
 size_t system_device_bytes(const adfem_system* s) {
   size_t b = 0;
   const Sell& A = s->A;

@@ -2297,7 +2297,7 @@ static int plan(Solver& S) {
 int mg_plan(Solver& S) {
   if (S.mg || !S.mg_allowed) return ADFEM_OK;
   // (a hierarchy that did not fit before: the patterns are not made again to find that out)
-  if (S.mg_limit == 0 || S.mg_need > S.mg_limit || (S.mg_need > 0 && short_of(S.mg_need))) return ADFEM_OK;
+  if (!S.mg_room || S.mg_limit == 0 || S.mg_need > S.mg_limit || (S.mg_need > 0 && short_of(S.mg_need))) return ADFEM_OK;
   try {
     return plan(S);
   } catch (const std::bad_alloc&) {

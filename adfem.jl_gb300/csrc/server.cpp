@@ -10,9 +10,10 @@
 //    reused by later requests on the same mesh; several instances of one (mesh, kind)
 //    serve concurrent requests; the last solution of an instance is kept for warm starts;
 //  * HBM admission: resident systems and worker buffers are counted against a budget;
-//    idle systems are evicted least-recently-used when a new one does not fit; a request
-//    that does not fit even into an empty server is rejected with ADFEM_ERR_BUSY (never
-//    an abort), one that fits later waits in the queue;
+//    idle systems are evicted least-recently-used when a new one, or the multigrid hierarchy
+//    that a solve adds to one, does not fit; a request that does not fit even into an empty
+//    server is rejected with ADFEM_ERR_BUSY (never an abort), one that fits later waits in the
+//    queue, one that only its hierarchy keeps from fitting is solved without it;
 //  * packing: the solves of small mixed-precision requests (at most pack_max_dof DOFs)
 //    are handed to a packer thread that solves all waiting ones in one graph-captured
 //    launch, one thread block per system (pack.cu); packs grow with the load;
@@ -112,7 +113,7 @@ constexpr int kPackDefaultDof = 16384;  // without multigrid
 int ndof_of(const adfem::Mesh* m, int kind) { return (int)(kind == ADFEM_SYS_ELASTICITY ? 2 * m->nv : m->nv); }
 
 // Device bytes of a resident system before it exists (admission): per stored operator
-// entry 8+8+4 (scaled FP64 standard and difference forms, FP32) + 8+4 (banded path
+// entry 8+8+4 (FP64 values, FP64 and FP32 difference forms) + 8+4 (banded path
 // copies) + 2+2 (column deltas) = 36 B with 15% padding; per DOF ~210 B of solver and
 // Dirichlet vectors; per element ~96 B of element scratch and Gauss-point staging.
 size_t estimate_system_bytes(const adfem::Mesh* m, int kind) {
@@ -124,7 +125,8 @@ size_t estimate_system_bytes(const adfem::Mesh* m, int kind) {
 
 // Multigrid hierarchy of a system, which its first solve outside a pack builds (per unknown:
 // operators, interpolation and work vectors of all levels: 190 bytes at 1M unknowns of P1 Poisson,
-// 243 at 4k; 343 for elasticity at 320k).
+// 243 at 4k; 343 for elasticity at 320k).  It is an extra: a request is admitted by the system and
+// its buffers alone, and solved without a hierarchy where the budget has no room for one.
 size_t estimate_hierarchy_bytes(const adfem::Mesh* m, int kind) {
   return (size_t)((kind == ADFEM_SYS_ELASTICITY ? 380.0 : 250.0) * (double)ndof_of(m, kind)) + 64 * 1024;
 }
@@ -155,7 +157,8 @@ struct adfem_server {
   std::vector<std::unique_ptr<Worker>> workers;
   // packer
   int pack_max_dof = 0, pack_max = 0;
-  bool default_packs = false;  // thresholds by kind and workers (systems are solved with multigrid)
+  bool multigrid = false;      // systems are solved with multigrid
+  bool default_packs = false;  // thresholds by kind and workers (as they are)
   std::deque<PackTicket*> pack_queue;
   std::condition_variable cv_pack;       // pack queue non-empty or stopping
   std::condition_variable cv_pack_done;  // a ticket finished
@@ -202,6 +205,11 @@ struct adfem_server {
     }
     return most > 0 && prec == ADFEM_PREC_MIXED && (long long)ndof_of(adfem::mesh_of(q.mesh), q.kind) <= most;
   }
+  // bytes by which a request's solve may make its system (null: a new one) larger
+  size_t growth(const adfem_request& q, const Resident* r) const {
+    if (!multigrid || q.nbd == 0 || goes_packed(q) || (r && !adfem::system_builds_hierarchy(r->sys))) return 0;
+    return estimate_hierarchy_bytes(adfem::mesh_of(q.mesh), q.kind);
+  }
   Resident* find_free(const adfem_mesh* mesh, int kind) {
     for (auto& r : residents)
       if (!r->busy && r->sys && r->mesh == mesh && r->kind == kind) return r.get();
@@ -224,6 +232,28 @@ struct adfem_server {
     for (auto& r : residents)
       if (r->busy) return true;
     return false;
+  }
+  // Make room for `base` more bytes and, where the budget holds them, the hierarchy's beside the system
+  // `keep` (or a new one): 1 done (*hier: the hierarchy's bytes that fit, all or none), 0 wait for
+  // running requests, -1 does not fit.  patient: the request may wait for the hierarchy's room.
+  int make_room(size_t base, size_t* hier, bool patient, Resident* keep) {
+    size_t others = 0, idle = 0;
+    for (auto& r : residents) {
+      if (r.get() == keep) continue;
+      others += r->bytes;
+      if (!r->busy && r->sys) idle += r->bytes;
+    }
+    if (used - others + base + *hier > budget ||  // (not even without any other system)
+        (!patient && used - idle + base + *hier > budget))
+      *hier = 0;
+    const size_t need = base + *hier;
+    if (need == 0) return 1;
+    if (used - idle + need > budget) return running == 0 && !any_busy() ? -1 : 0;
+    if (keep) keep->busy = true;
+    while (used + need > budget && evict_one_idle()) {
+    }
+    if (keep) keep->busy = false;
+    return 1;
   }
   void run_worker(int wid);
   void run_packer(int pid);
@@ -432,6 +462,8 @@ void adfem_server::run_worker(int wid) {
     std::shared_ptr<Job> job;
     Resident* R = nullptr;
     bool create = false;
+    size_t hier = 0;  // bytes booked for a hierarchy that this request may build
+    bool allow = true;
     {
       std::unique_lock<std::mutex> lk(mu);
       cv_work.wait(lk, [&] { return stopping || !queue.empty(); });
@@ -445,32 +477,34 @@ void adfem_server::run_worker(int wid) {
         continue;
       }
       R = find_free(job->req.mesh, job->req.kind);
+      const size_t base = R ? 0 : estimate_system_bytes(adfem::mesh_of(job->req.mesh), job->req.kind);
+      const size_t more = growth(job->req, R);
+      hier = more;
+      const int room = make_room(base, &hier, job->req.deadline_ms <= 0.0, R);
+      if (room < 0) {
+        std::snprintf(job->resp.message, sizeof(job->resp.message), "does not fit the HBM budget");
+        finish(job, ADFEM_ERR_BUSY);
+        continue;
+      }
+      if (room == 0) {
+        // wait for running requests to release memory, then try again
+        queue.push_front(job);
+        cv_done.wait(lk);
+        continue;
+      }
+      allow = hier == more;
       if (R) {
         hits++;
+        R->bytes += hier;
+        used += hier;
       } else {
-        const adfem::Mesh* m = adfem::mesh_of(job->req.mesh);
-        const size_t est = estimate_system_bytes(m, job->req.kind) +
-                           (goes_packed(job->req) ? 0 : estimate_hierarchy_bytes(m, job->req.kind));
-        while (used + est > budget && evict_one_idle()) {
-        }
-        if (used + est > budget) {
-          if (running == 0 && !any_busy()) {
-            std::snprintf(job->resp.message, sizeof(job->resp.message), "does not fit the HBM budget");
-            finish(job, ADFEM_ERR_BUSY);
-            continue;
-          }
-          // wait for running requests to release memory, then try again
-          queue.push_front(job);
-          cv_done.wait(lk);
-          continue;
-        }
         misses++;
         residents.push_back(std::make_unique<Resident>());
         R = residents.back().get();
         R->mesh = job->req.mesh;
         R->kind = job->req.kind;
-        R->bytes = est;
-        used += est;
+        R->bytes = base + hier;
+        used += R->bytes;
         create = true;
       }
       R->busy = true;
@@ -484,13 +518,15 @@ void adfem_server::run_worker(int wid) {
       std::lock_guard<std::mutex> lk(mu);
       if (status == ADFEM_OK) {
         // (the hierarchy is built by the first solve: its estimate stays booked until then)
-        const size_t actual = adfem::system_device_bytes(R->sys) +
-                              (goes_packed(job->req) ? 0 : estimate_hierarchy_bytes(adfem::mesh_of(R->mesh), R->kind));
+        const size_t actual = adfem::system_device_bytes(R->sys) + hier;
         used = used - R->bytes + actual;
         R->bytes = actual;
       }
     }
-    if (status == ADFEM_OK) status = run_job(W, *R, *job);
+    if (status == ADFEM_OK) {
+      adfem::system_allow_hierarchy(R->sys, allow);
+      status = run_job(W, *R, *job);
+    }
     if (status != ADFEM_OK) std::snprintf(job->resp.message, sizeof(job->resp.message), "%s", adfem_last_error());
     {
       std::lock_guard<std::mutex> lk(mu);
@@ -537,7 +573,8 @@ int adfem_server_create(const adfem_server_config* cfg, adfem_server** out) {
   if (S->cfg.workers <= 0) S->cfg.workers = 8;
   if (S->cfg.workers > 256) return adfem::fail(ADFEM_ERR_INVALID, "server: at most 256 workers");
   if (S->cfg.max_queue <= 0) S->cfg.max_queue = 65536;
-  S->default_packs = S->cfg.pack_max_dof == 0 && adfem::mg_wanted();
+  S->multigrid = adfem::mg_wanted();
+  S->default_packs = S->cfg.pack_max_dof == 0 && S->multigrid;
   S->pack_max_dof = std::min(S->cfg.pack_max_dof == 0 ? kPackDefaultDof : std::max(S->cfg.pack_max_dof, 0),
                              adfem::pack_rows_limit());
   S->pack_max = S->cfg.pack_max <= 0 ? 64 : std::min(S->cfg.pack_max, adfem::kPackMaxSystems);
@@ -615,8 +652,7 @@ int adfem_server_submit(adfem_server* srv, const adfem_request* req, long long* 
     return adfem::fail(ADFEM_ERR_INVALID, "server: unknown precision");
   std::lock_guard<std::mutex> lk(srv->mu);
   if (srv->stopping) return adfem::fail(ADFEM_ERR_INVALID, "server: shutting down");
-  const size_t need = estimate_system_bytes(m, req->kind) + estimate_worker_bytes(m, req->kind) +
-                      (srv->goes_packed(*req) ? 0 : estimate_hierarchy_bytes(m, req->kind));
+  const size_t need = estimate_system_bytes(m, req->kind) + estimate_worker_bytes(m, req->kind);
   if (need > srv->budget) {
     srv->rejected++;
     return adfem::fail(ADFEM_ERR_BUSY, "server: request needs ~" + std::to_string(need >> 20) +

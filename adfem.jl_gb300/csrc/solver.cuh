@@ -104,6 +104,7 @@ struct Solver {
   bool mg_skip = false;              // this assembly's solves take the Jacobi iteration: multigrid gave one
                                      // up, or there was no room for the hierarchy
   size_t mg_limit = SIZE_MAX;        // bytes the hierarchy may take
+  bool mg_room = true;               // it may be built (the server's budget has room for it)
   size_t mg_need = 0;                // bytes it takes (0: not known yet)
   int mg_spin = kTailSpin;           // tries of a wait in the one-launch tail
   int mg_cap = kMgIterations;        // iterations of a solve before it is left to the Jacobi iteration
