@@ -2,8 +2,9 @@
 //
 // Jacobi-CG needs 5,000 to 16,000 iterations at 1M to 4M unknowns, each near the memory
 // bound already, so the time of a solve is their number.  Here the preconditioner is one
-// V-cycle of smoothed aggregation in FP32 and the CG around it is FP64 throughout (iterate,
-// residual, direction, products), which needs 20 to 90 iterations at every size.
+// V-cycle of smoothed aggregation in FP32, and the CG around it is FP64: iterate, residual,
+// direction, products with K and every sum (r.z is the FP64 sum over the cycle's FP32 input and
+// output).  Iterations at 625 to 4M unknowns: P1 Poisson 14 to 36, P2 33 to 43, elasticity 36 to 58.
 //  * Patterns (aggregates, interpolation, A P, coarse operators) are made once per system on
 //    the host (mg_setup.cpp); after an assembly the kernels below fill in the values.
 //  * Level 0 is S K S, S = diag(K_ii^-1/2) as in the Jacobi iterations, so the stopping
@@ -191,28 +192,19 @@ struct RowHead {
 // addition (last sweep of level 0 with its dot product: 45 against 34 us at 4M rows, 22 against 14 us
 // at 240k rows of P2).
 // A block's values go through shared memory to its first warp, eight to a lane (13 warp additions a
-// block instead of 40 of shuffle trees in every warp); FP32 values are added as FP32 pairs.
-template <class T>
-__device__ __forceinline__ void block_partial(T x, double* partials) {
-  __shared__ T sh[kT];
+// block instead of 40 of shuffle trees in every warp).  The products are FP64 too, as in the Jacobi
+// iterations: in FP32 and FP32 pairs an iteration takes 235 instead of 243 us at 1M unknowns, 42.4
+// instead of 44.5 at 4225, 194 instead of 198 for elasticity at 320k, and the iterations are the same.
+__device__ __forceinline__ void block_partial(double x, double* partials) {
+  __shared__ double sh[kT];
   const int lane = threadIdx.x;
   sh[threadIdx.x] = x;
   __syncthreads();
   if (threadIdx.x >= 32) return;
-  double s;
-  if constexpr (sizeof(T) == 4) {
-    float2 w = make_float2(sh[lane], 0.0f);
+  double s = sh[lane];
 #pragma unroll
-    for (int k = 1; k < kT / 32; k++) w = pair_add(w, make_float2(sh[lane + 32 * k], 0.0f));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) w = pair_add(w, shfl_pair(w, o));
-    s = lane == 0 ? (double)w.x + (double)w.y : 0.0;
-  } else {
-    s = sh[lane];
-#pragma unroll
-    for (int k = 1; k < kT / 32; k++) s += sh[lane + 32 * k];
-    s = warp_sum(s);
-  }
+  for (int k = 1; k < kT / 32; k++) s += sh[lane + 32 * k];
+  s = warp_sum(s);
   if (lane == 0) partials[blockIdx.x] = s;
 }
 // The total as f makes two words of it.  (One warp adds and one thread runs f: an FP64 warp
@@ -261,7 +253,7 @@ template <int NB, bool D16, int LPR, int MODE>
 __global__ void __launch_bounds__(kT) k_mg_sweep(MgLev L, const float* x, float* out, int c1, int c2, int keep_d,
                                                  double* partials) {
   pdl_trigger();
-  float dot = 0.0f;
+  double dot = 0.0;
   const float th = MODE == kPre ? __ldg(L.coef) : 0.0f;
   const float a1 = c1 >= 0 ? __ldg(L.coef + c1) : 0.0f, a2 = c2 >= 0 ? __ldg(L.coef + c2) : 0.0f;
   const int64_t rows = (int64_t)L.n * LPR;
@@ -298,7 +290,7 @@ __global__ void __launch_bounds__(kT) k_mg_sweep(MgLev L, const float* x, float*
       if ((MODE == kPre || MODE == kStep) && keep_d) store_vec<NB>(L.d, r, d);
       if (MODE == kLast)
 #pragma unroll
-        for (int c = 0; c < NB; c++) dot = fmaf(bi.v[c], o.v[c], dot);
+        for (int c = 0; c < NB; c++) dot = fma((double)bi.v[c], (double)o.v[c], dot);
     }
     if (MODE != kLast) break;  // (the other modes have a lane group per row)
     t += gstride();
@@ -321,7 +313,7 @@ __global__ void __launch_bounds__(kT, MODE == kLast ? 6 : 8) k_mg_fine(MgLev L, 
   const float th = MODE == kPre ? __ldg(L.coef) : 0.0f;
   const float a1 = c1 >= 0 ? __ldg(L.coef + c1) : 0.0f, a2 = c2 >= 0 ? __ldg(L.coef + c2) : 0.0f;
   const float* g = MODE == kPre ? L.b : x;
-  float dot = 0.0f;
+  double dot = 0.0;
   int j[W];
   float v[W];
   auto load = [&](int r) {
@@ -357,7 +349,7 @@ __global__ void __launch_bounds__(kT, MODE == kLast ? 6 : 8) k_mg_fine(MgLev L, 
       const float d = fmaf(a1, di, a2 * (bi - ax));
       o = xi + d;
       if (MODE == kStep) L.d[r] = d;
-      if (MODE == kLast) dot = fmaf(bi, o, dot);
+      if (MODE == kLast) dot = fma((double)bi, (double)o, dot);
     }
     out[r] = o;
     if (MODE != kLast) break;  // (the other modes have a thread per row)
@@ -694,41 +686,6 @@ __device__ __forceinline__ double cluster_total(double x, double* sh, double* sl
     }
   }
   return s;
-}
-
-// The same of a float per thread, as FP32 pairs (48 bits): a dependent FP64 addition takes some 200
-// cycles here, a pair one 40 (a sum 3.9k instead of 5.2k cycles).
-template <bool EX, int T>
-__device__ __forceinline__ double cluster_total(float x, double* sh_, double* slot, int rank, int& phase) {
-  float* sh = reinterpret_cast<float*>(sh_);
-  sh[threadIdx.x] = x;
-  __syncthreads();
-  float2* set = reinterpret_cast<float2*>(slot + (phase & 1) * kTailC);
-  phase++;
-  float2 s = make_float2(0.0f, 0.0f);
-  if (threadIdx.x < 32) {
-    float2 v[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) v[k] = s;
-#pragma unroll
-    for (int k = 0; k < T / 32; k++) v[k & 3] = pair_add(v[k & 3], make_float2(sh[threadIdx.x + 32 * k], 0.0f));
-    s = pair_add(pair_add(v[0], v[1]), pair_add(v[2], v[3]));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s = pair_add(s, shfl_pair(s, o));
-    if (EX && threadIdx.x < kTailC)
-      asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(rank_addr(set + rank, threadIdx.x)), "f"(s.x),
-                   "f"(s.y)
-                   : "memory");
-  }
-  if (EX) {
-    cluster_barrier();
-    if (threadIdx.x == 0) {
-      s = set[0];
-#pragma unroll
-      for (int k = 1; k < kTailC; k++) s = pair_add(s, set[k]);
-    }
-  }
-  return (double)s.x + (double)s.y;
 }
 
 constexpr int kTailT = kMgTailDofs / kTailC;  // threads of a tail block: one per own unknown
@@ -1125,8 +1082,8 @@ __global__ void __launch_bounds__(kTailT, 1) k_mg_tail(const __grid_constant__ T
     if constexpr (SOLVE) {
       const float* x = v[0].x;
       // (a wait that gave up in any block ends the solve in all of them)
-      float zb = live ? x[u] * v[0].b[t] : 0.0f;
-      if (EX && sync.dead) zb = nanf("");
+      double zb = live ? (double)x[u] * (double)v[0].b[t] : 0.0;
+      if (EX && sync.dead) zb = nan("");
       double d = cluster_total<EX, T>(zb, sh, slot, rank, phase);
       if (t == 0) {
         const double rz = d * loc.iar;
@@ -1169,13 +1126,15 @@ __global__ void __launch_bounds__(kTailT, 1) k_mg_tail(const __grid_constant__ T
       __syncthreads();
       if (loc.done) break;
       const double al = bc[1], g = loc.ar;
+      double tn = 0.0;
       if (live) {
         cor[t] = fma(al, pu, cor[t]);
         const double ri = fma(-al, q, res[t]);
         res[t] = ri;
-        bn = (float)(ri * g) * sc[u];
+        tn = ri * g * (double)sc[u];
+        bn = (float)tn;
       }
-      d = cluster_total<EX, T>(live ? bn * bn : 0.0f, sh, slot, rank, phase);
+      d = cluster_total<EX, T>(tn * tn, sh, slot, rank, phase);
       if (t == 0) {
         rn = d * loc.iar * loc.iar;
         loc.rho_new = rn;
@@ -1994,7 +1953,7 @@ __global__ void __launch_bounds__(kT) k_mg_update(int64_t n, double* z, double* 
   });
   if (v.x == 0.0) return;
   const double a = v.y, g = st->ar;
-  float acc = 0.0f;
+  double acc = 0.0;
   const int64_t n2 = n >> 1;
   for (int64_t i = gtid(); i < n2; i += gstride()) {
     const double2 pp = reinterpret_cast<const double2*>(p)[i], qq = reinterpret_cast<const double2*>(q)[i];
@@ -2006,19 +1965,19 @@ __global__ void __launch_bounds__(kT) k_mg_update(int64_t n, double* z, double* 
     rr.y = fma(-a, qq.y, rr.y);
     reinterpret_cast<double2*>(z)[i] = zz;
     reinterpret_cast<double2*>(r)[i] = rr;
-    const float2 t = make_float2((float)(rr.x * g) * ss.x, (float)(rr.y * g) * ss.y);
-    reinterpret_cast<float2*>(b32)[i] = t;
-    acc = fmaf(t.x, t.x, acc);
-    acc = fmaf(t.y, t.y, acc);
+    const double tx = rr.x * g * (double)ss.x, ty = rr.y * g * (double)ss.y;
+    reinterpret_cast<float2*>(b32)[i] = make_float2((float)tx, (float)ty);
+    acc = fma(tx, tx, acc);
+    acc = fma(ty, ty, acc);
   }
   if ((n & 1) && gtid() == 0) {
     const int64_t i = n - 1;
     z[i] = fma(a, p[i], z[i]);
     const double ri = fma(-a, q[i], r[i]);
     r[i] = ri;
-    const float t = (float)(ri * g) * s[i];
-    b32[i] = t;
-    acc = fmaf(t, t, acc);
+    const double t = ri * g * (double)s[i];
+    b32[i] = (float)t;
+    acc = fma(t, t, acc);
   }
   block_partial(acc, partials);
 }

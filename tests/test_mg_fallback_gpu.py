@@ -137,3 +137,13 @@ def test_hierarchy_without_room(oracle, gpulib, monkeypatch, m, elastic):
         L.adfem_debug_fail_alloc(-1)
     assert e.value.status == gpulib._lib.ERR_NOMEM
     assert rel(S.solve(rtol=1e-12), ref) < 1e-9 and S.last_stats.iterations < JACOBI
+
+
+@pytest.mark.parametrize("m", [23, 60, 100])
+def test_warm_start_far_from_the_solution(oracle, gpulib, m):
+    # residuals of 1e20 |b| and more, whose squares are no FP32 numbers: the multigrid iteration takes
+    # them (36 digits at some 0.7 of a digit an iteration), without the Jacobi iteration's help
+    S, ref, _ = system(oracle, gpulib, m)
+    u = 1e24 * np.random.default_rng(m).standard_normal(ref.size)
+    w = S.solve(t(u), rtol=1e-12, warm=True)
+    assert rel(w, ref) < 1e-9 and S.last_stats.iterations < JACOBI
