@@ -1007,11 +1007,33 @@ static int check_symmetric(int64_t n, const std::vector<int32_t>& rp, const std:
 // one row pattern, whichever way they are numbered; the hierarchy here is a scalar one, so where
 // most rows have such a twin the Jacobi iteration is kept.  (Rows have to be sorted, without
 // repeated entries.)
+//
+// The hierarchy costs some 0.15 us an unknown, a Jacobi iteration 15 us and 36 ps an unknown, and
+// Jacobi needs about 20 / sqrt(lam) of them for 1e-12, lam the smallest eigenvalue of D^-1 K: what a
+// smooth vector sees of it, the row sums over the diagonal (away from the eliminated rows, so their
+// median), and some 6 / n for the gradients of the smoothest one.  GB300, ms per call, Jacobi / multigrid
+// of P1 matrices (mass M, Laplace K, cells of size h):
+//   unknowns   M            M + h2 K     M + 10 h2 K   M + 100 h2 K   K
+//   441        2.1 / 1.3    2.5 / 1.3    2.8 / 1.3     2.9 / 1.3      2.9 / 1.3
+//   4225       2.5 / 2.7    3.0 / 2.8    4.2 / 2.9     6.1 / 2.9      6.5 / 3.0
+//   40401      5.2 / 11.2   5.7 / 11.1   7.3 / 11.4    12.4 / 11.4    19.0 / 11.8
+//   251001     19 / 47      19 / 46      22 / 47       32 / 47        74 / 48
 static bool csc_wants_mg(int64_t n, const std::vector<int32_t>& rp, const std::vector<int32_t>& ci,
                          const double* val, std::vector<uint8_t>& fixed) {
-  // GB300, ms per call on P1 Poisson matrices, Jacobi / multigrid: 289 unknowns 2.4 / 1.1,
-  // 4225 6.6 / 2.8, 10201 10.7 / 4.2, 40401 20.0 / 11.4 (most of the rest is the hierarchy's set-up)
   if (n <= kMgDense || !mg_wanted()) return false;
+  std::vector<double> low;  // row sum over diagonal of the rows that are not eliminated (of some 4000)
+  for (int64_t r = 0; r < n; r += std::max<int64_t>(1, n / 4096)) {
+    double sum = 0.0, off = 0.0, diag = 0.0;
+    for (int32_t k = rp[r]; k < rp[r + 1]; k++) {
+      sum += val[k];
+      if (ci[k] == r) diag = val[k];
+      else off += std::fabs(val[k]);
+    }
+    if (off > 0.0) low.push_back(diag > 0.0 && sum > 0.0 ? sum / diag : 0.0);
+  }
+  std::nth_element(low.begin(), low.begin() + low.size() / 2, low.end());
+  const double lam = (low.empty() ? 0.0 : low[low.size() / 2]) + 6.0 / (double)n;
+  if (20.0 / std::sqrt(lam) * (15e-6 + 36e-12 * (double)n) < 0.15e-6 * (double)n) return false;
   fixed.assign(n, 0);
   int64_t nfixed = 0;
   std::vector<uint64_t> key(n);

@@ -323,7 +323,8 @@ ADFEM_API void adfem_solver_opts_default(adfem_solver_opts *opts);
  * Dirichlet entry), host pointers.  Replaces Julia SparseArrays' `\` on this path
  * (README.md:54) with CG on the GPU; u receives the solution.  In FP64, a scalar problem with
  * eliminated rows (nothing but the diagonal; more than 160 unknowns, sorted columns, no repeated
- * entries) is preconditioned by multigrid; every other matrix by its diagonal. */
+ * entries) that its diagonal alone would take many iterations for is preconditioned by multigrid;
+ * every other matrix by its diagonal. */
 ADFEM_API int adfem_csc_solve(long long n, const long long *colptr1, const long long *rowval1, const double *nzval,
                               const double *rhs, double *u, const adfem_solver_opts *opts,
                               adfem_solver_stats *stats);
