@@ -97,3 +97,34 @@ def test_solves_whose_start_has_converged(gpulib, m):
     for _ in range(100):
         assert not bool(A.adjoint(zero).any()) and A.last_stats.iterations == 0
         assert torch.equal(B.solve(rtol=1e-12), ref)
+
+
+@pytest.mark.parametrize("m", [64, 100, 300])  # a cluster, graphs
+def test_warm_start_that_is_there_right_after_an_assembly(oracle, gpulib, m):
+    # (it is found by its residual, before the hierarchy has the assembly's values, which the solves
+    # after it need)
+    coords, elems = synth.jittered_square(m, seed=2)
+    O = oracle.OracleMesh(coords, elems)
+    rng = np.random.default_rng(m)
+    bd = O.bcnode()
+    bv = rng.random(bd.size)
+    S = gpulib.PoissonSystem(gpulib.Mesh(coords, elems))
+    S.set_dirichlet(bd, bv)
+    f = rng.random(O.ngauss)
+    for scale in (1.0, 1e3):
+        kappa = scale * (1.0 + 9.0 * rng.random(O.ngauss))
+        B, b = oracle.dirichlet_csc(O.laplace_csc(kappa), O.source(f), bd, bv)
+        ref = oracle.spsolve(B, b)
+        S.assemble(t(kappa), t(f))
+        for precision in ("mixed", "fp64"):
+            w = S.solve(t(ref), precision=precision, rtol=1e-8, warm=True)
+            assert S.last_stats.iterations == 0 and rel(w, ref) < 1e-9
+        w = S.solve(t(0.0 * ref), rtol=1e-12, warm=True)  # (far from there)
+        assert 0 < S.last_stats.iterations < 60 and rel(w, ref) < 1e-9
+        u = S.solve(rtol=1e-12)
+        assert rel(u, ref) < 1e-9 and rel(S.solve(t(ref), rtol=1e-8, warm=True), ref) < 1e-9
+        # a NaN start is no start: the solve ends with a status, and the next is as before
+        with pytest.raises(gpulib.AdFemError):
+            S.solve(torch.full_like(u, float("nan")), rtol=1e-12, warm=True)
+        S.assemble(t(kappa), t(f))
+        assert torch.equal(S.solve(rtol=1e-12), u)
