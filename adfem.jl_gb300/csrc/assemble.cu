@@ -305,6 +305,7 @@ __global__ void __launch_bounds__(kDirectB) k_source_rows_direct(int64_t n, cons
 
 // GB300, us per call with the element pass / direct: 4225 nodes 27.1 / 23.4 (matrix), 25.6 / 21.3
 // (load); 66k 30.1 / 27.3, 28.4 / 25.0; 161k 36.6 / 33.5, 32.5 / 33.7; 491k 62.7 / 59.1, 48.4 / 60.9.
+// The line is the load's, whose crossing lies between 66k and 161k; the matrix's is beyond 491k.
 bool direct_rows(const Mesh& m) {
   constexpr int64_t kDirectNodes = 100000;
   return m.maxrow <= 16 && m.nv <= kDirectNodes;

@@ -518,8 +518,7 @@ struct TailArgs {
   int spin;      // tries of a wait
   // a whole solve (k_mg_tail's SOLVE): the system's operator, right-hand side and iterate
   const int32_t* sptr;
-  const void* col;
-  int d16;
+  const void* col;  // (int16 differences: a system of that size has no others)
   const double *val, *rowsum, *rhs;
   const float* s;
   double* y;
@@ -956,7 +955,7 @@ __global__ void __launch_bounds__(kTailT, 1) k_mg_tail(const __grid_constant__ T
   unsigned ranks = 0;
   auto column = [&](int k) {
     const int64_t idx = base + 32 * (int64_t)k;
-    int j = a.d16 ? colof<true>(a.col, idx, u) : colof<false>(a.col, idx, u);
+    int j = colof<true>(a.col, idx, u);
     if (!ADFEM_DCHECK(j >= 0 && j < n0)) j = u;
     return j;
   };
@@ -2460,7 +2459,6 @@ TailArgs tail_args(Solver& S) {
   a.spin = S.mg_spin;
   a.sptr = A.sptr.as<int32_t>();
   a.col = A.col.p;
-  a.d16 = A.delta16 ? 1 : 0;
   a.val = A.val64.as<double>();
   a.rowsum = M.rowsum;
   a.rhs = S.b.as<double>();
@@ -2472,7 +2470,6 @@ TailArgs tail_args(Solver& S) {
 // One cycle: lev[0].b -> the vector returned; returns the launches through *count.
 const float* enqueue_cycle(Solver& S, cudaStream_t st, int* count) {
   Mg& M = *S.mg;
-  CgState* cs = S.state.as<CgState>();
   int nl = 0;
   float* xs[kMgMaxLevels];
   for (int l = 0; l < M.tail; l++) {

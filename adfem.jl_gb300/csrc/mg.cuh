@@ -4,7 +4,7 @@
 // aggregated level by level once per system on the host (mg_setup.cpp: patterns only), and
 // after every assembly the device forms the interpolation values P = P0 - c D^-1 A P0 and the
 // coarse operators P^T A P on those fixed patterns (mg.cu).  Every level is scaled to unit
-// diagonal, so its smoother (Chebyshev) needs no diagonal; levels of at most kTailDofs
+// diagonal, so its smoother (Chebyshev) needs no diagonal; levels of at most kMgTailDofs
 // unknowns run in one launch (k_mg_tail).
 #pragma once
 #include <stdint.h>
@@ -39,7 +39,7 @@ struct MgHostLevel {
   int64_t n = 0;
   MgPattern A;                 // graph of the level
   std::vector<int32_t> agg;    // aggregate of each node (empty on the coarsest level)
-  MgPattern P, AP, PT;         // interpolation, A P, transpose (PT entry -> P entry in PTsrc)
+  MgPattern P, AP, PT;         // interpolation, A P, transpose of P
   std::vector<int32_t> PTslot; // position of each PT entry within its P row
   std::vector<double> x, y;    // node positions (2-D elasticity only)
 };

@@ -102,9 +102,10 @@ constexpr int kPackers = 4;  // packer threads (concurrent packed launches)
 //               6561      0.71 / 0.24, 0.33 / 0.28    16129 1.47 / 0.33, 0.58 / 0.36
 //   elasticity   338 DOFs 0.28 / 0.13, 0.09 / 0.10     1250 1.16 / 0.26, 0.22 / 0.20
 //               4802      3.52 / 0.54, 1.49 / 0.42
-// Poisson requests of up to 2560 DOFs are packed, as callers that look at response.packed expect
-// of small ones (2401 DOFs is where packs of many stop being the faster); of elasticity only the
-// smallest where many workers fill the packs.  A system that would be solved by Jacobi CG either
+// Poisson requests of up to 2560 DOFs are packed whatever the workers, as callers that look at
+// response.packed expect of small ones: with 64 workers packs are the faster at 625 and no longer at 2401, with 8 the
+// resident solver is at every size (by 0.04 ms a request at 625 DOFs, 0.34 at 2401).  Of elasticity
+// only the smallest are, where many workers fill the packs.  A system that would be solved by Jacobi CG either
 // way is packed up to the same size as before multigrid.
 constexpr int kPackManyWorkers = 32;
 constexpr int kPackPoisson = 2560, kPackElasticMany = 640;

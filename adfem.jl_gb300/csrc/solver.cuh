@@ -142,20 +142,20 @@ int solver_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_ro
 int solver_apply(Solver& S, const double* x, double* y, cudaStream_t user);
 
 // Multigrid-preconditioned FP64 CG (mg.cu): hierarchy on first use (clears mg_allowed when the
-// graph does not coarsen, makes none where the device or mg_limit has no room for it), its values once per assembly, the solve.  gave_up: no outcome (a
-// breakdown, or more iterations than the multigrid cap); u untouched, the caller falls back.
+// graph does not coarsen, makes none where the device or mg_limit has no room for it), its values
+// once per assembly, the solve.  gave_up: no outcome (a breakdown, a wait that gave up, or more
+// iterations than the multigrid cap); u untouched, the caller falls back.
 int mg_plan(Solver& S);
 int mg_solve(Solver& S, const double* rhs, double* u, const uint8_t* zero_rows, const uint8_t* fix_rows,
              const double* fix_vals, const adfem_solver_opts& o, adfem_solver_stats* stats, cudaStream_t user,
              bool* gave_up);
 size_t mg_device_bytes(const Solver& S);
-// kernels of the FP64 CG that mg.cu shares: q64 = K p64 with alpha = rho / p.q for the given
-// values, and y64 += z64, z64 = 0 (when a residual is due, or forced)
+// the kernel of the FP64 CG that mg.cu shares: y64 += z64, z64 = 0 (when a residual is due, or forced)
 void solver_enqueue_fold64(Solver& S, int force, cudaStream_t st);
 
 // Banded mixed path (zcg.cu).  zcg_plan decides whether the operator's band fits
 // the shared-memory ring and allocates the path's buffers; zcg_prepare derives its
-// operator copies from the unscaled FP64 values (before they are scaled in place).
+// operator copies from the unscaled FP64 values (before solver_ensure_scaled scales them in place).
 int zcg_plan(Solver& S, int sms);
 int zcg_prepare(Solver& S, const int32_t* diagpos_dev, int* bad_dev, cudaStream_t st);
 int zcg_clear(Solver& S, cudaStream_t st);
