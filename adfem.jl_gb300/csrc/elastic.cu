@@ -329,10 +329,11 @@ cudaError_t launch_elastic_system(const Mesh& m, const double* Dbar, const doubl
 
 // ---------------------------------------------------------------------------
 // Unsummed COO of ComputeFemStiffnessMatrixMfem_forward: entry 108 e + 36 k + 6 l + s of
-// NN_k = w B^T D_k B.  The gradients of the three vertices sum to zero, so the rows and columns
-// of vertex 2 are the negated sums of the other two: one thread per Gauss point forms the 4 x 4
-// block of vertices 0 and 1 and extends it, 80 FP64 operations instead of 144 (FP64 issue bounds
-// the kernel); the block then writes values and indices in order through shared memory.
+// NN_k = w B^T D_k B.  FP64 issue bounds the kernel: one thread per Gauss point, the weight in the
+// rows' gradients (114 operations); the block then writes values and indices in order through
+// shared memory.  Every entry comes from the gradients of its own two vertices.  (Rows and columns of
+// vertex 2 as negated sums of the others' take 80 operations, but lose digits to cancellation where
+// that vertex' gradient is the small one: 6 of 16 in elements of aspect 1000.)
 constexpr int kStiffPts = 126, kStiffT = 128;  // whole elements; every warp of the block has points
 __global__ void __launch_bounds__(kStiffT) k_stiffness_coo(int64_t ne, int64_t ndof, const int4* __restrict__ conn,
                                                        const double2* __restrict__ grad,
@@ -344,35 +345,24 @@ __global__ void __launch_bounds__(kStiffT) k_stiffness_coo(int64_t ne, int64_t n
   const int np = (int)min((int64_t)kStiffPts, 3 * (ne - e0));
   if ((int)threadIdx.x < np) {
     const int64_t e = e0 + threadIdx.x / 3;
-    const double2 h0 = grad[3 * e], h1 = grad[3 * e + 1];
+    const double2 h[3] = {grad[3 * e], grad[3 * e + 1], grad[3 * e + 2]};
     const double w = geo[e].w;
     double d[9];
 #pragma unroll
     for (int q = 0; q < 9; q++) d[q] = __ldg(D + 27 * e0 + 9 * threadIdx.x + q);
     double* N = sv[threadIdx.x];
-    // row l of the 4 x 4 block: x of vertex i (B column (hx, 0, hy)), y of vertex i ((0, hy, hx))
-    auto row = [&](int l, const double2& h, bool y) {
-      const double a = w * h.x, b = w * h.y;
+    // row l: x of vertex l (B column (hx, 0, hy)), y of vertex l - 3 ((0, hy, hx))
+#pragma unroll
+    for (int l = 0; l < 6; l++) {
+      const double a = w * h[l % 3].x, b = w * h[l % 3].y;
       double v[3];
 #pragma unroll
-      for (int q = 0; q < 3; q++) v[q] = y ? fma(b, d[3 + q], a * d[6 + q]) : fma(a, d[q], b * d[6 + q]);
-      const double x0 = fma(v[0], h0.x, v[2] * h0.y), x1 = fma(v[0], h1.x, v[2] * h1.y);
-      const double y0 = fma(v[1], h0.y, v[2] * h0.x), y1 = fma(v[1], h1.y, v[2] * h1.x);
-      N[6 * l] = x0;
-      N[6 * l + 1] = x1;
-      N[6 * l + 2] = -(x0 + x1);
-      N[6 * l + 3] = y0;
-      N[6 * l + 4] = y1;
-      N[6 * l + 5] = -(y0 + y1);
-    };
-    row(0, h0, false);
-    row(1, h1, false);
-    row(3, h0, true);
-    row(4, h1, true);
+      for (int q = 0; q < 3; q++) v[q] = l < 3 ? fma(a, d[q], b * d[6 + q]) : fma(b, d[3 + q], a * d[6 + q]);
 #pragma unroll
-    for (int q = 0; q < 6; q++) {
-      N[12 + q] = -(N[q] + N[6 + q]);
-      N[30 + q] = -(N[18 + q] + N[24 + q]);
+      for (int c = 0; c < 3; c++) {
+        N[6 * l + c] = fma(v[0], h[c].x, v[2] * h[c].y);
+        N[6 * l + 3 + c] = fma(v[1], h[c].y, v[2] * h[c].x);
+      }
     }
     if (threadIdx.x % 3 == 0) {
       const int4 cn = conn[e];
@@ -397,10 +387,9 @@ cudaError_t launch_stiffness_coo(const Mesh& m, const double* D, long long* indi
   return cudaGetLastError();
 }
 
-// ComputeFemStiffnessMatrixMfem_backward: grad_D_k = w B G B^T, G = grad_vv block (6x6).  By the
-// same zero sum G enters through the differences of its rows and columns to those of vertex 2: a
-// 4 x 4 block (40 additions), then 60 operations, against 126 on the full block.  The block reads
-// and writes its points' entries in order through shared memory.
+// ComputeFemStiffnessMatrixMfem_backward: grad_D_k = w B G B^T, G = grad_vv block (6x6): 117
+// operations (100 with G's differences to the rows and columns of vertex 2, at up to six times the
+// error).  The block reads and writes its points' entries in order through shared memory.
 __global__ void __launch_bounds__(kStiffT) k_stiffness_coo_backward(int64_t ne, const double2* __restrict__ grad,
                                                                 const double4* __restrict__ geo,
                                                                 const double* __restrict__ gvv,
@@ -422,37 +411,38 @@ __global__ void __launch_bounds__(kStiffT) k_stiffness_coo_backward(int64_t ne, 
   __syncthreads();
   if ((int)threadIdx.x < np) {
     const int64_t e = e0 + threadIdx.x / 3;
-    const double2 h0 = grad[3 * e], h1 = grad[3 * e + 1];
+    const double2 h[3] = {grad[3 * e], grad[3 * e + 1], grad[3 * e + 2]};
     const double w = geo[e].w;
     double* G = sv[threadIdx.x];
-    // H: rows and columns x0, x1, y0, y1
-    double H[4][4];
+    double T[3][6];  // B G
 #pragma unroll
-    for (int r = 0; r < 4; r++) {
-      const int gr = r < 2 ? r : r + 1, g2 = r < 2 ? 2 : 5;
-      double R[6];
+    for (int c = 0; c < 6; c++) {
+      T[0][c] = h[0].x * G[c];
+      T[1][c] = h[0].y * G[18 + c];
+      T[2][c] = h[0].y * G[c];
 #pragma unroll
-      for (int c = 0; c < 6; c++) R[c] = G[6 * gr + c] - G[6 * g2 + c];
-      H[r][0] = R[0] - R[2];
-      H[r][1] = R[1] - R[2];
-      H[r][2] = R[3] - R[5];
-      H[r][3] = R[4] - R[5];
-    }
-    double T[3][4];
-    {
-      const double a0 = w * h0.x, a1 = w * h1.x, b0 = w * h0.y, b1 = w * h1.y;
-#pragma unroll
-      for (int c = 0; c < 4; c++) {
-        T[0][c] = fma(a0, H[0][c], a1 * H[1][c]);
-        T[1][c] = fma(b0, H[2][c], b1 * H[3][c]);
-        T[2][c] = fma(b0, H[0][c], fma(b1, H[1][c], fma(a0, H[2][c], a1 * H[3][c])));
+      for (int l = 1; l < 3; l++) {
+        T[0][c] = fma(h[l].x, G[6 * l + c], T[0][c]);
+        T[1][c] = fma(h[l].y, G[18 + 6 * l + c], T[1][c]);
+        T[2][c] = fma(h[l].y, G[6 * l + c], T[2][c]);
       }
+#pragma unroll
+      for (int l = 0; l < 3; l++) T[2][c] = fma(h[l].x, G[18 + 6 * l + c], T[2][c]);
     }
 #pragma unroll
     for (int p = 0; p < 3; p++) {
-      G[3 * p] = fma(T[p][0], h0.x, T[p][1] * h1.x);
-      G[3 * p + 1] = fma(T[p][2], h0.y, T[p][3] * h1.y);
-      G[3 * p + 2] = fma(T[p][0], h0.y, fma(T[p][1], h1.y, fma(T[p][2], h0.x, T[p][3] * h1.x)));
+      double x = T[p][0] * h[0].x, y = T[p][3] * h[0].y, z = T[p][0] * h[0].y;
+#pragma unroll
+      for (int l = 1; l < 3; l++) {
+        x = fma(T[p][l], h[l].x, x);
+        y = fma(T[p][3 + l], h[l].y, y);
+        z = fma(T[p][l], h[l].y, z);
+      }
+#pragma unroll
+      for (int l = 0; l < 3; l++) z = fma(T[p][3 + l], h[l].x, z);
+      G[3 * p] = x * w;
+      G[3 * p + 1] = y * w;
+      G[3 * p + 2] = z * w;
     }
   }
   __syncthreads();
