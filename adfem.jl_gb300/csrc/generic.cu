@@ -331,15 +331,32 @@ __device__ __forceinline__ void p2_factors(int k, double (&t)[3], double (&l4)[3
   }
 }
 
+// Gradients of the six basis functions at point k
+__device__ __forceinline__ void p2_gradients(int k, const double2 (&g)[3], double (&hx)[6], double (&hy)[6]) {
+  double t[3], l4[3];
+  p2_factors(k, t, l4);
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    const int b = (a + 1) % 3;
+    hx[a] = t[a] * g[a].x;
+    hy[a] = t[a] * g[a].y;
+    hx[3 + a] = fma(l4[b], g[a].x, l4[a] * g[b].x);
+    hy[3 + a] = fma(l4[b], g[a].y, l4[a] * g[b].y);
+  }
+}
+
 // Unsummed P2 Laplace COO: a block takes kCooPts Gauss points; one thread per point forms the 21
-// distinct entries from the element's g_ab (51 FP64 operations; recomputing the gradients per row
-// took ~400), all threads write values and indices in order through shared memory.
+// distinct entries from the gradients there (75 FP64 operations; recomputing the gradients per row
+// took ~400), all threads write values and indices in order through shared memory.  (From the three
+// g_ab of the P1 geometry record they take 51, but the products with a vertex of small gradient lose
+// digits to cancellation: 3 of 16 in elements of aspect 10^4.)
 // (The points fill every warp of the block: two warps of eight left half of the SM's FP64 pipes
 // idle, 54 instead of 40 us at 39k elements.)
 constexpr int kCooPts = 126, kCooT = 128;  // whole elements
 __global__ void __launch_bounds__(kCooT) k_p2_coo(int64_t ne, const int32_t* __restrict__ dof,
-                                                const double4* __restrict__ geo, const double* __restrict__ coef,
-                                                longlong2* __restrict__ idx, double* __restrict__ vv) {
+                                                const double* __restrict__ area, const double2* __restrict__ grad,
+                                                const double* __restrict__ coef, longlong2* __restrict__ idx,
+                                                double* __restrict__ vv) {
   __shared__ double sv[kCooPts][37];
   __shared__ int32_t sd[kCooPts / 6][6];
   const int64_t ngp = 6 * ne;
@@ -352,31 +369,17 @@ __global__ void __launch_bounds__(kCooT) k_p2_coo(int64_t ne, const int32_t* __r
     if ((int)threadIdx.x < np) {
       const int64_t gp = g0 + threadIdx.x, e = gp / 6;
       const int k = (int)(gp - 6 * e);
-      const double4 gr = geo[e];
-      const double cw = coef[gp] * (6 * p2::W[k >= 3 ? 1 : 0]);
-      const double x = gr.x * cw, y = gr.y * cw, z = gr.z * cw;
-      const double g[3][3] = {{-(x + y), x, y}, {x, -(x + z), z}, {y, z, -(y + z)}};
-      double t[3], l4[3], h[3][3];  // h[i][c] = (edge i's gradient) . grad_c
-      p2_factors(k, t, l4);
+      double2 g[3];
+      load_grad(grad, e, g);
+      const double cw = coef[gp] * (2 * p2::W[k >= 3 ? 1 : 0] * area[e]);
+      double hx[6], hy[6];
+      p2_gradients(k, g, hx, hy);
       double* K = sv[threadIdx.x];
 #pragma unroll
-      for (int i = 0; i < 3; i++) {
-        const int q = (i + 1) % 3;
+      for (int i = 0; i < 6; i++) {
+        const double x = cw * hx[i], y = cw * hy[i];
 #pragma unroll
-        for (int c = 0; c < 3; c++) h[i][c] = fma(l4[q], g[i][c], l4[i] * g[q][c]);
-      }
-#pragma unroll
-      for (int i = 0; i < 3; i++) {
-        K[6 * i + i] = t[i] * t[i] * g[i][i];
-#pragma unroll
-        for (int j = 0; j < i; j++) K[6 * i + j] = K[6 * j + i] = t[i] * t[j] * g[i][j];
-#pragma unroll
-        for (int j = 0; j < 3; j++) K[6 * (3 + j) + i] = K[6 * i + 3 + j] = t[i] * h[j][i];
-#pragma unroll
-        for (int j = 0; j <= i; j++) {
-          const int s = (j + 1) % 3;
-          K[6 * (3 + i) + 3 + j] = K[6 * (3 + j) + 3 + i] = fma(l4[s], h[i][j], l4[j] * h[i][s]);
-        }
+        for (int j = 0; j <= i; j++) K[6 * i + j] = K[6 * j + i] = fma(x, hx[j], y * hy[j]);
       }
     }
     __syncthreads();
@@ -390,9 +393,10 @@ __global__ void __launch_bounds__(kCooT) k_p2_coo(int64_t ne, const int32_t* __r
 }
 
 // Its transpose: grad_coef[gp] = sum_pq grad_vv[gp, p, q] (d N_pq / d coef).  The block reads its
-// points' entries in order into shared memory, one thread per point contracts them with the
-// basis' gradient factors to the 3 x 3 matrix of the barycentric gradients, then with the g_ab.
-__global__ void __launch_bounds__(kCooT) k_p2_coo_backward(int64_t ne, const double4* __restrict__ geo,
+// points' entries in order into shared memory, one thread per point multiplies them with the
+// gradients from both sides (104 operations).
+__global__ void __launch_bounds__(kCooT) k_p2_coo_backward(int64_t ne, const double* __restrict__ area,
+                                                         const double2* __restrict__ grad,
                                                          const double* __restrict__ gv, double* __restrict__ out) {
   __shared__ double sv[kCooPts][37];
   const int64_t ngp = 6 * ne;
@@ -413,29 +417,22 @@ __global__ void __launch_bounds__(kCooT) k_p2_coo_backward(int64_t ne, const dou
     if ((int)threadIdx.x < np) {
       const int64_t gp = g0 + threadIdx.x, e = gp / 6;
       const int k = (int)(gp - 6 * e);
-      double t[3], l4[3], S[3][3];
-      p2_factors(k, t, l4);
+      double2 g[3];
+      load_grad(grad, e, g);
+      double hx[6], hy[6], v = 0.0;
+      p2_gradients(k, g, hx, hy);
       const double* G = sv[threadIdx.x];
-      double y[6][3];
 #pragma unroll
-      for (int p = 0; p < 6; p++)
+      for (int p = 0; p < 6; p++) {
+        double x = G[6 * p] * hx[0], y = G[6 * p] * hy[0];
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-          const int q = (c + 1) % 3, r = (c + 2) % 3;  // edges c = (c, q) and r = (r, c) touch vertex c
-          y[p][c] = fma(t[c], G[6 * p + c], fma(l4[q], G[6 * p + 3 + c], l4[r] * G[6 * p + 3 + r]));
+        for (int q = 1; q < 6; q++) {
+          x = fma(G[6 * p + q], hx[q], x);
+          y = fma(G[6 * p + q], hy[q], y);
         }
-#pragma unroll
-      for (int b = 0; b < 3; b++)
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-          const int q = (b + 1) % 3, r = (b + 2) % 3;
-          S[b][c] = fma(t[b], y[b][c], fma(l4[q], y[3 + b][c], l4[r] * y[3 + r][c]));
-        }
-      const double4 gr = geo[e];
-      double v = gr.x * ((S[0][1] + S[1][0]) - (S[0][0] + S[1][1]));
-      v = fma(gr.y, (S[0][2] + S[2][0]) - (S[0][0] + S[2][2]), v);
-      v = fma(gr.z, (S[1][2] + S[2][1]) - (S[1][1] + S[2][2]), v);
-      out[gp] = v * (6 * p2::W[k >= 3 ? 1 : 0]);
+        v = fma(hx[p], x, fma(hy[p], y, v));
+      }
+      out[gp] = v * (2 * p2::W[k >= 3 ? 1 : 0] * area[e]);
     }
   }
 }
@@ -1188,7 +1185,7 @@ cudaError_t launch_gen_coo(const Mesh& m, const Space& sp, GenOp op, const doubl
   const double2* grad = m.d_grad.as<double2>();
   if (op == GenOp::LAPLACE)
     GEN_DISPATCH(sp, (k_gen_coo<1, 0><<<g, kGT, 0, st>>>(m.ne, dof, area, grad, coef, indices, vv)),
-                 (k_p2_coo<<<grid_for(6 * m.ne, kCooPts), kCooT, 0, st>>>(m.ne, dof, m.d_geo.as<double4>(), coef,
+                 (k_p2_coo<<<grid_for(6 * m.ne, kCooPts), kCooT, 0, st>>>(m.ne, dof, area, grad, coef,
                                                                        reinterpret_cast<longlong2*>(indices), vv)));
   else
     GEN_DISPATCH(sp, (k_gen_coo<1, 1><<<g, kGT, 0, st>>>(m.ne, dof, area, grad, coef, indices, vv)),
@@ -1205,8 +1202,7 @@ cudaError_t launch_gen_coo_backward(const Mesh& m, const Space& sp, GenOp op, co
   const double2* grad = m.d_grad.as<double2>();
   if (op == GenOp::LAPLACE)
     GEN_DISPATCH(sp, (k_gen_coo_backward<1, 0><<<g, 64 * 3, 0, st>>>(m.ne, area, grad, grad_vv, grad_coef)),
-                 (k_p2_coo_backward<<<grid_for(ngp, kCooPts), kCooT, 0, st>>>(m.ne, m.d_geo.as<double4>(), grad_vv,
-                                                                           grad_coef)));
+                 (k_p2_coo_backward<<<grid_for(ngp, kCooPts), kCooT, 0, st>>>(m.ne, area, grad, grad_vv, grad_coef)));
   else
     GEN_DISPATCH(sp, (k_gen_coo_backward<1, 1><<<g, 64 * 3, 0, st>>>(m.ne, area, grad, grad_vv, grad_coef)),
                  (k_gen_coo_backward<2, 1><<<g, 64 * 6, 0, st>>>(m.ne, area, grad, grad_vv, grad_coef)));

@@ -43,6 +43,28 @@ def gradients(coords, elems):
     return g, abs(det) / 2
 
 
+def p2_points(g):
+    """gradients at the six points of the order-4 rule (ne, 6 points, 6 functions, 2), their lengths
+    before cancellation, and the weights (of an area of 1)"""
+    r = LD(8) - np.sqrt(LD(10))
+    s = np.sqrt(LD(38) - 44 * np.sqrt(LD(2) / 5))
+    a = [(r - s) / 18, (r + s) / 18]
+    w = [(620 - np.sqrt(LD(213125) - 53320 * np.sqrt(LD(10)))) / 3720,
+         (620 + np.sqrt(LD(213125) - 53320 * np.sqrt(LD(10)))) / 3720]
+    out, mag, ws = [], [], []
+    for o in range(2):
+        for xi, eta in ((a[o], a[o]), (a[o], 1 - 2 * a[o]), (1 - 2 * a[o], a[o])):
+            l = [1 - xi - eta, xi, eta]
+            T = np.zeros((6, 3), LD)
+            for i in range(3):
+                T[i, i] = 4 * l[i] - 1
+                T[3 + i, i], T[3 + i, (i + 1) % 3] = 4 * l[(i + 1) % 3], 4 * l[i]
+            out.append(np.einsum("fc,ecd->efd", T, g))
+            mag.append(np.einsum("fc,ec->ef", abs(T), np.sqrt((g * g).sum(-1))))
+            ws.append(w[o])
+    return np.stack(out, 1), np.stack(mag, 1), np.array(ws)
+
+
 def worst(got, want, scale, area=None):
     """largest error in roundings, and the factors by which the elements' areas differ"""
     got = got.cpu().numpy() if hasattr(got, "cpu") else got
@@ -77,3 +99,26 @@ def test_elasticity(gpulib):
     want = np.einsum("epl,eklc,eqc->ekpq", B, G.astype(LD), B) * w
     scale = np.einsum("epl,eklc,eqc->ekpq", abs(B), abs(G).astype(LD), abs(B)) * w
     assert worst(gD, want, scale, area)[0] < 64
+
+
+def test_p2_laplace_coo(gpulib):
+    from adfem_gpu import system as S
+
+    coords, elems = thin_mesh()
+    g, area = gradients(coords, elems)
+    N, mag, ws = p2_points(g)
+    w = ws[None, :] * area[:, None]
+    M = gpulib.Mesh(coords, elems, degree=2)
+    ne = len(N)
+    rng = np.random.default_rng(6)
+    kappa = 1 + rng.random((ne, 6))
+    G = rng.standard_normal((ne, 6, 6, 6))
+    _, vv = S.laplace_coo(M, torch.tensor(kappa.reshape(-1), device="cuda"))
+    want = np.einsum("ekpd,ekqd->ekpq", N, N) * (w * kappa)[..., None, None]
+    scale = mag[..., :, None] * mag[..., None, :] * (w * kappa)[..., None, None]
+    err, area = worst(vv, want, scale)
+    assert err < 32
+    gk = S.laplace_coo_backward(M, torch.tensor(G.reshape(-1), device="cuda"))
+    want = np.einsum("ekpd,ekpq,ekqd->ek", N, G.astype(LD), N) * w
+    scale = np.einsum("ekp,ekpq,ekq->ek", mag, abs(G).astype(LD), mag) * w
+    assert worst(gk, want, scale, area)[0] < 64
