@@ -1021,15 +1021,16 @@ static int check_symmetric(int64_t n, const std::vector<int32_t>& rp, const std:
 static bool csc_wants_mg(int64_t n, const std::vector<int32_t>& rp, const std::vector<int32_t>& ci,
                          const double* val, std::vector<uint8_t>& fixed) {
   if (n <= kMgDense || !mg_wanted()) return false;
-  std::vector<double> low;  // row sum over diagonal of the rows that are not eliminated (of some 4000)
-  for (int64_t r = 0; r < n; r += std::max<int64_t>(1, n / 4096)) {
+  std::vector<double> low;  // row sum over diagonal of the rows that are not eliminated (of some 1000)
+  for (int64_t r = 0; r < n; r += std::max<int64_t>(1, n / 1024)) {
     double sum = 0.0, off = 0.0, diag = 0.0;
     for (int32_t k = rp[r]; k < rp[r + 1]; k++) {
       sum += val[k];
       if (ci[k] == r) diag = val[k];
       else off += std::fabs(val[k]);
     }
-    if (off > 0.0) low.push_back(diag > 0.0 && sum > 0.0 ? sum / diag : 0.0);
+    const double q = diag > 0.0 ? sum / diag : 0.0;
+    if (off > 0.0) low.push_back(q > 0.0 && std::isfinite(q) ? q : 0.0);  // (no NaN: they are ordered below)
   }
   std::nth_element(low.begin(), low.begin() + low.size() / 2, low.end());
   const double lam = (low.empty() ? 0.0 : low[low.size() / 2]) + 6.0 / (double)n;
@@ -1109,11 +1110,11 @@ int adfem_csc_solve(long long n, const long long* colptr1, const long long* rowv
   DevBuf dfixed;
   bool wants_mg = false;
   try {
-    wants_mg = csc_wants_mg(n, rp, ci, nzval, fixed);
+    // (mixed precision names an iteration of its own here, which the callers of it keep)
+    wants_mg = o.precision == ADFEM_PREC_FP64 && csc_wants_mg(n, rp, ci, nzval, fixed);
   } catch (const std::bad_alloc&) {
   }
-  // (mixed precision names an iteration of its own here, which the callers of it keep)
-  if (o.precision == ADFEM_PREC_FP64 && wants_mg) {
+  if (wants_mg) {
     ADFEM_TRY(to_dev(dfixed, fixed.data(), fixed.size()));
     sv.mg_allowed = sv.mg_fixed = true;
     mg_env(sv);

@@ -33,3 +33,18 @@ def test_choice_of_preconditioner(oracle, gpulib, m, c, multigrid):
     ref = oracle.spsolve(B, r)
     assert st.status == 0 and np.linalg.norm(u - ref) < 1e-7 * np.linalg.norm(ref)
     assert (st.iterations < 22) == multigrid
+
+
+@pytest.mark.parametrize("bad", [np.inf, np.nan, 0.0, -1.0])
+@pytest.mark.parametrize("every", [1, 7])
+def test_diagonal_that_is_not_positive_and_finite_is_refused(oracle, gpulib, bad, every):
+    coords, elems = synth.jittered_square(20, seed=1)
+    O = oracle.OracleMesh(coords, elems)
+    K = sp.csc_matrix(O.laplace_csc(np.ones(O.ngauss)))
+    bd = O.bcnode()
+    B, r = oracle.dirichlet_csc(K, np.ones(O.ndof), bd, np.zeros(bd.size))
+    B = sp.csc_matrix(B)
+    d = np.flatnonzero(np.repeat(np.arange(O.ndof), np.diff(B.indptr)) == B.indices)
+    B.data[d[::every]] = bad
+    with pytest.raises(gpulib.AdFemError):
+        gpulib.solve(B, r, rtol=1e-12)
