@@ -174,8 +174,8 @@ int grid_for(int64_t n, int bt = kGT) {
 // what bounds these kernels (FP64 issues at 1/64 of FP32 here).  Laplace: the basis gradients
 // are combinations of the barycentric ones, so the matrix is a contraction of the moments
 //   VV_ab = sum c w t_a t_b, Q_ab = sum c w t_a 4 l_b, R_ab = sum c w 16 l_a l_b  (t = 4 l - 1)
-// with the three products g_ab of the P1 geometry record.  ~125 FP64 operations per element
-// against ~500 with gradients formed at every point.
+// with the three products g_ab of the P1 geometry record, the diagonal from the zero row sums.  ~125
+// FP64 operations per element against ~500 with gradients formed at every point.
 namespace p2 {
 __device__ constexpr double A[2] = {0.091576213509770743460, 0.44594849091596488632};
 __device__ constexpr double B[2] = {0.81684757298045851308, 0.10810301816807022736};

@@ -4,7 +4,7 @@
 // bound already, so the time of a solve is their number.  Here the preconditioner is one
 // V-cycle of smoothed aggregation in FP32, and the CG around it is FP64: iterate, residual,
 // direction, products with K and every sum (r.z is the FP64 sum over the cycle's FP32 input and
-// output).  Iterations at 625 to 4M unknowns: P1 Poisson 14 to 36, P2 33 to 43, elasticity 36 to 58.
+// output).  Iterations at 625 to 4M unknowns: P1 Poisson 14 to 36, P2 33 to 53, elasticity 36 to 70.
 //  * Patterns (aggregates, interpolation, A P, coarse operators) are made once per system on
 //    the host (mg_setup.cpp); after an assembly the kernels below fill in the values.
 //  * Level 0 is S K S, S = diag(K_ii^-1/2) as in the Jacobi iterations, so the stopping

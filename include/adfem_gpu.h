@@ -339,11 +339,12 @@ enum { ADFEM_SYS_POISSON = 0, ADFEM_SYS_ELASTICITY = 1 };
  * once per assembly): tens of iterations at every size where Jacobi-CG needs thousands.  The
  * Jacobi iterations serve systems without Dirichlet DOFs (singular), graphs that do not
  * coarsen, hierarchies that the device has no memory for (200 to 350 bytes per DOF;
- * ADFEM_MG_MAX_BYTES in the environment at creation caps them), solves in which the preconditioned iteration breaks down (indefinite operators) or
- * needs more than 300 iterations (ADFEM_MG_MAX_ITER in the environment at creation; from then on
- * every solve of that assembly), profiled solves, and systems created while ADFEM_MG=0 or one of
- * ADFEM_ZCG, ADFEM_ZCG64, ADFEM_ZCG_SMAX, ADFEM_ZCG_RING, ADFEM_ZCG_RING_REFILL (which pick a
- * variant of them) is set in the environment.
+ * ADFEM_MG_MAX_BYTES in the environment at creation caps them), solves in which the preconditioned
+ * iteration breaks down (indefinite operators) or needs more than 300 iterations
+ * (ADFEM_MG_MAX_ITER in the environment at creation; from then on every solve of that
+ * assembly), profiled solves, and systems created while ADFEM_MG=0 or one of ADFEM_ZCG,
+ * ADFEM_ZCG64, ADFEM_ZCG_SMAX, ADFEM_ZCG_RING, ADFEM_ZCG_RING_REFILL (which pick a variant of
+ * them) is set in the environment.
  * Poisson systems on P1 or P2 meshes (P2: the vertex-then-edge DOFs of the mesh's space,
  * kappa and f at the 6 points per element of the order-4 rule; DOFs renumbered for the
  * solver by reverse Cuthill-McKee, inputs and outputs in the reference order); elasticity
@@ -367,10 +368,11 @@ ADFEM_API int adfem_system_assemble_poisson_profiled_d(adfem_system *sys, const 
                                                        double *ms, void *stream);
 ADFEM_API int adfem_system_assemble_elasticity_d(adfem_system *sys, const double *E_d, const double *nu_d,
                                                  const double *fx_d, const double *fy_d, void *stream);
-/* Solve the assembled system; u_d: ndof (nv or 2nv, reference DOF ordering). */
+/* Solve the assembled system; u_d: ndof (nv or 2nv, reference DOF ordering), written when the call
+ * returns, with or without stats.  A stream that is being captured is refused (ADFEM_ERR_UNSUPPORTED). */
 ADFEM_API int adfem_system_solve_d(adfem_system *sys, double *u_d, const adfem_solver_opts *opts,
                                    adfem_solver_stats *stats, void *stream);
-/* Adjoint solve K lambda = g (K symmetric); lambda is zero on Dirichlet DOFs. */
+/* Adjoint solve K lambda = g (K symmetric); lambda is zero on Dirichlet DOFs.  As the solve otherwise. */
 ADFEM_API int adfem_system_adjoint_d(adfem_system *sys, const double *g_d, double *lam_d,
                                      const adfem_solver_opts *opts, adfem_solver_stats *stats, void *stream);
 /* dL/dkappa at every Gauss point: -w (grad lam).(grad u) at the point (P1: equal for the 3
